@@ -43,7 +43,47 @@ __device__ __forceinline__ float clamp_h(float x) { return fminf(fmaxf(x, -65504
 // 8 bits instead of 15: h = round(x * 127 / amax), l = 0 and sx = amax / (127 * 128), so every consumer reads the same
 // format and the W4A8 arm of the streaming kernel may skip the low plane.
 constexpr int ACT_A8 = 0x2000;
+// With ACT_FRAG the chunk is for the 16-bit tensor path (gemv_mma.cu): eight bf16 = x * 2^64, an exponent shift; elements 2, 3,
+// 6 and 7, which meet the nibbles that carry a factor 16, are x * 2^60 (with ACT_A8, x is the 8-bit integer and sx its scale).
+// xsum is stored in the unit of the products, n * 2^-133 * x * 2^64. With ACT_NV as well (NVFP4 weights) the elements come in
+// the order 0 4 1 5 2 6 3 7, all times 2^64 (and with ACT_A8 the rounded activations themselves: there is no scale to apply).
+constexpr int ACT_FRAG = 0x4000, ACT_NV = 0x8000;
+constexpr float ACT_FRAG_UNIT = 590295810358705651712.f;      // 2^69 = 2^133 / 2^64
+__device__ __forceinline__ uint4 actpack_frag(const float* v, int cpg, float& sx, float& xsum) {
+  const bool a8 = (cpg & (ACT_A8 >> 3)) != 0, nv = (cpg & (ACT_NV >> 3)) != 0;
+  cpg &= (ACT_A8 >> 3) - 1;
+  float x[8], sum = 0.f;
+  sx = 1.f;
+  if (a8) {
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    for (int o = cpg >> 1; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    sx = fmaxf(amax, 1e-30f) * (1.f / 127.f);
+    const float inv = 1.f / sx;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = (float)__float2int_rn(v[i] * inv);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = v[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) sum += x[i];
+  for (int o = cpg >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  xsum = sum * sx * (1.f / ACT_FRAG_UNIT);
+  if (nv && a8) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] *= sx;
+  }
+  const float e = 18446744073709551616.f, e16 = nv ? e : e / 16.f;
+  float y[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) y[i] = x[i] * ((i & 2) ? e16 : e);
+  if (nv) return make_uint4(pack_bf16(y[0], y[4]), pack_bf16(y[1], y[5]), pack_bf16(y[2], y[6]), pack_bf16(y[3], y[7]));
+  return make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
+}
 __device__ __forceinline__ uint4 actpack_emit(const float* v, int cpg, float& sx, float& xsum) {
+  if (cpg & (ACT_FRAG >> 3)) return actpack_frag(v, cpg, sx, xsum);
   const bool a8 = (cpg & (ACT_A8 >> 3)) != 0;
   cpg &= (ACT_A8 >> 3) - 1;
   float pb[4], pl[4];   // pl: activations of the low nibbles, pb: of the high nibbles
@@ -101,20 +141,33 @@ __device__ __forceinline__ uint4 actpack_emit(const float* v, int cpg, float& sx
 //   [128/G groups][8 tokens] float2 (sx, xsum)
 // so the consumer fetches everything a weight block needs with one bulk copy. `xs` is unused.
 // Tokens 8..15, 16..23, ... go to further buffers of the same size that follow the first one.
+// Fragment layout (ACT_FRAG): see actpack_store; the buffers hold the tokens rounded up to a multiple of 8.
 constexpr int ACT_TILES = 0x1000;
 __host__ __device__ constexpr int actpack_tile_bytes(int G) { return 2048 + 64 * (128 / G); }
 
 // Group argument check of the producers' launchers: 32 / 128, optionally | ACT_TILES.
 inline bool actpack_group_ok(int G, int tokens) {
-  const int g = G & ~(ACT_TILES | 0x2000);       // 0x2000: ACT_A8
+  const int g = G & ~(ACT_TILES | ACT_A8 | ACT_FRAG | ACT_NV);
   (void)tokens;
+  if ((G & ACT_FRAG) && (G & ACT_TILES)) return false;
+  if ((G & ACT_NV) && !(G & ACT_FRAG)) return false;
   return g == 32 || g == 128;
 }
 
 __device__ __forceinline__ void actpack_store(uint4* xpack, float2* xs, int tiles, int G, int token, int c8, int nchunks,
                                               const uint4& pk, float sx, float xsum) {
-  G &= ~ACT_A8;
+  const int frag = G & ACT_FRAG, nv = G & ACT_NV;
+  G &= ~(ACT_A8 | ACT_FRAG | ACT_NV);
   const int cpg = G >> 3;
+  if (frag) {
+    // fragment layout: blocks of 8 tokens; per block and 128-k record [4 words][8 tokens][4 quarters] chunks and per group
+    // [8 tokens] pairs. A lane of the consumer reads word w of quarter t; NVFP4 codes run the other way round.
+    const int kt = c8 >> 4, hi = (c8 >> 2) & 3, lo = c8 & 3, w = nv ? lo : hi, t = nv ? hi : lo;
+    const size_t blk = (size_t)(token >> 3);
+    xpack[(blk * (nchunks >> 4) + kt) * 128 + w * 32 + (token & 7) * 4 + t] = pk;
+    if (!nv && (c8 % cpg) == 0) xs[(blk * (nchunks / cpg) + c8 / cpg) * 8 + (token & 7)] = make_float2(sx, xsum);
+    return;
+  }
   if (!tiles) {
     xpack[(size_t)token * nchunks + c8] = pk;
     if ((c8 % cpg) == 0) xs[(size_t)token * (nchunks / cpg) + c8 / cpg] = make_float2(sx, xsum);

@@ -415,7 +415,8 @@ class HybridRunner:
         self.sp_prefill = True          # tensor-parallel prefill through the GEMM-fused reduce-scatter / all-gather path
         self.gdn_save = None            # (qkvz [n_gdn, M, nq], ab [n_gdn, M, ldab]): GDN inputs of the last step, kept for fold()
         # one-token steps: "fma" = the half-precision FMA projection with the norm / residual / activation glue folded in
-        # (5 launches per GDN layer, 7 per attention layer); "dp4a" = the integer arm with separate norm and pack launches
+        # (5 launches per GDN layer, 7 per attention layer); "dp4a" = the integer arms with separate norm and pack launches,
+        # for every row count
         self.decode_gemv = "fma"
         self.mix = bf(M, max(spec.value_dim, spec.hq * spec.hd))   # mixer output (GDN / attention) of the fused one-token path
         self.h_alt = bf(M, H)           # second residual-stream buffer of the one-token path with split projections
@@ -432,10 +433,31 @@ class HybridRunner:
                     gslot=i[lay.gslot:lay.gslot + lay.b], bt_row=i[lay.bt_row:lay.bt_row + lay.b])
 
     # -- building blocks ---------------------------------------------------------------------
-    def _grp(self) -> int:
-        """``group`` argument for the ActPack producers: the tile layout when the tcgen05 streaming kernel consumes it."""
+    def _grp(self, m: int) -> int:
+        """``group`` argument for the ActPack producers of an ``m``-row step: the tile layout when the tcgen05 streaming kernel
+        consumes it, fragments for the 16-bit tensor streaming kernel."""
         g = (self.G | K.ACT_TILES) if self.tiles else self.G
+        if self._mma(m):
+            g |= K.ACT_FRAG | (K.ACT_NV if self.w.layout == "nvfp4" else 0)
         return g | K.ACT_A8 if self.act_bits == 8 else g
+
+    def _dense16(self, m: int) -> bool:
+        """An ``m``-row step multiplies the resident dense copy of the int4 weights. (Not under uniform_rows: a speculating
+        engine needs the same arithmetic for every row count.)"""
+        sp = self.spec
+        return m >= self.BATCH_GEMM_FROM and self.prefill_gemm in ("tcr", "tc8r") and self.w.layout == "slice" \
+            and not self.uniform_rows and not any(k % 128 for k in (sp.hidden, sp.inter, sp.value_dim, sp.hq * sp.hd))
+
+    def _mma(self, m: int) -> bool:
+        """The projections of an ``m``-row step run on the 16-bit tensor streaming kernel (``csrc/gemv_mma.cu``): one GPU,
+        slice-major int4 or NVFP4 weights. The tensor-parallel arms (push, symmetric all-reduce) and the fused-norm variant
+        stay on the integer kernels, whose epilogues they are."""
+        sp = self.spec
+        if self._dense16(m):
+            return False
+        if self.decode_gemv == "dp4a" or self.fuse_norm or self.w.layout not in ("slice", "nvfp4") or not self.w.layers:
+            return False
+        return (self.comm is None or sp.tp_world == 1) and not any(k % 128 for k in (sp.hidden, sp.inter, sp.value_dim, sp.hq * sp.hd))
 
     def _pf_hook(self, w, after: bool) -> None:
         """Weight-stream bookkeeping around a projection: the warm-up pass of a capture records the weight tensors in launch
@@ -459,20 +481,21 @@ class HybridRunner:
         with torch.cuda.stream(side):
             K.l2_prefetch(nxt, int(self.l2_prefetch_mb * (1 << 20)))
 
-    def _gemv(self, w, xp, xs, out, m: int, *, residual=None, epi: int = K.EPI_STORE, ldo=None, pdl: bool = False) -> None:
-        """out[m] = W x on the weight-streaming kernel that matches the weight's record layout."""
+    def _gemv(self, w, xp, xs, out, m: int, *, residual=None, epi: int = K.EPI_STORE, ldo=None, pdl: bool = False, **ab) -> None:
+        """out[m] = W x on the weight-streaming kernel that matches the weight's record layout. ``ab``: the dense rows that
+        the 16-bit tensor kernel computes beside the matrix."""
         self._pf_hook(w, False)
-        self._gemv_inner(w, xp, xs, out, m, residual=residual, epi=epi, ldo=ldo, pdl=pdl)
+        if self._mma(m):
+            K.w4_mma(w, xp, xs, out, m, residual=residual, epi=epi, ldo=ldo, a8=self.act_bits == 8, pdl=pdl, **ab)
+        else:
+            self._gemv_inner(w, xp, xs, out, m, residual=residual, epi=epi, ldo=ldo, pdl=pdl)
         self._pf_hook(w, True)
 
     def _gemv_inner(self, w, xp, xs, out, m: int, *, residual=None, epi: int = K.EPI_STORE, ldo=None, pdl: bool = False) -> None:
         if w.layout == "nvfp4":
             self._gemv_nvfp4(w, xp, xs, out, m, residual, epi, ldo)
             return
-        # (not under uniform_rows: a speculating engine needs the same arithmetic for every row count, and the dense product
-        # rounds differently from the integer arm that plain steps of a few rows use)
-        if m >= self.BATCH_GEMM_FROM and self.prefill_gemm in ("tcr", "tc8r") and w.layout == "slice" and w.k % 128 == 0 \
-                and epi in (K.EPI_STORE, K.EPI_RESIDUAL, K.EPI_SILU_MUL) and not self.uniform_rows:
+        if self._dense16(m) and w.layout == "slice" and epi in (K.EPI_STORE, K.EPI_RESIDUAL, K.EPI_SILU_MUL):
             self._gemv_dense16(w, xp, xs, out, m, residual, epi, ldo)
             return
         if w.layout != "block":
@@ -546,7 +569,7 @@ class HybridRunner:
     def _norm(self, m: int, w, *, want_xn: bool, want_pack: bool = True) -> None:
         sp = self.spec
         K.rmsnorm_pack(self.h, w, normed=self.xn if want_xn else None, xpack=self.xp_h if want_pack else None,
-                       xs=self.xs_h if want_pack else None, m=m, k=sp.hidden, group=self._grp(), eps=sp.eps, pdl=self.pdl)
+                       xs=self.xs_h if want_pack else None, m=m, k=sp.hidden, group=self._grp(m), eps=sp.eps, pdl=self.pdl)
 
     def _row_parallel(self, which: int, w, xp, xs, m: int, next_norm, *, want_xn: bool, want_pack: bool = True) -> None:
         """h += W x for a row-parallel projection, then x_next = rmsnorm(h) * (1 + next_norm).
@@ -563,7 +586,7 @@ class HybridRunner:
                     self._norm_count = torch.zeros(1, dtype=torch.int32, device=self.device)
                 K.w4a16_skinny_norm(w, xp, xs, self.h, next_norm, self._norm_count, m, normed=self.xn if want_xn else None,
                                     norm_pack=self.xp_h if want_pack else None, norm_xs=self.xs_h if want_pack else None,
-                                    group=self._grp(), eps=sp.eps, pdl=self.pdl, force_mma=self.uniform_rows and m == 1)
+                                    group=self._grp(m), eps=sp.eps, pdl=self.pdl, force_mma=self.uniform_rows and m == 1)
                 return
             self._gemv(w, xp, xs, self.h, m, residual=self.h, epi=K.EPI_RESIDUAL, pdl=self.pdl)
             self._norm(m, next_norm, want_xn=want_xn, want_pack=want_pack)
@@ -574,12 +597,12 @@ class HybridRunner:
             symm.gemv_push(which, w, xp, xs, m, pdl=self.pdl, force_mma=self.uniform_rows and m == 1)
             symm.push_residual_norm(which, self.h, m, next_norm, normed=self.xn if want_xn else None,
                                     xpack=self.xp_h if want_pack else None, xs=self.xs_h if want_pack else None,
-                                    group=self._grp(), eps=sp.eps, pdl=self.pdl)
+                                    group=self._grp(m), eps=sp.eps, pdl=self.pdl)
         elif symm is not None:
             self._gemv(w, xp, xs, symm.partial(which), m, pdl=self.pdl)
             symm.ar_residual_norm(which, self.h, m, next_norm, normed=self.xn if want_xn else None,
                                   xpack=self.xp_h if want_pack else None, xs=self.xs_h if want_pack else None,
-                                  group=self._grp(), eps=sp.eps, pdl=self.pdl)
+                                  group=self._grp(m), eps=sp.eps, pdl=self.pdl)
         else:
             self._gemv(w, xp, xs, self.partial, m, pdl=self.pdl)
             self.comm.allreduce_add_residual(self.partial, self.h, m)
@@ -590,23 +613,28 @@ class HybridRunner:
         # silu(gate)*up is written as bf16 and packed by a small kernel: the fused pack epilogue
         # (EPI_SILU_PACK) needs 16 row tiles per CTA, which leaves too few CTAs at this size
         self._gemv(lw.gate_up, self.xp_h, self.xs_h, self.act, m, epi=K.EPI_SILU_MUL, ldo=sp.inter, pdl=self.pdl)
-        K.act_pack(self.act, self.xp_i, self.xs_i, m, sp.inter, self._grp(), pdl=self.pdl)
+        K.act_pack(self.act, self.xp_i, self.xs_i, m, sp.inter, self._grp(m), pdl=self.pdl)
         self._row_parallel(1, lw.down, self.xp_i, self.xs_i, m, next_norm, want_xn=want_xn, want_pack=want_pack)
 
     def _gdn(self, lw: LayerWeights, li: int, lay: StepLayout, v: dict) -> None:
         sp, m = self.spec, lay.m
-        # fork: the tiny dense a/b projection runs beside the big qkvz stream
-        main = torch.cuda.current_stream()
         # a speculative verify step keeps every layer's GDN inputs so that fold() can replay a prefix
         qo, ao = (self.qkvz_out, self.ab_out) if self.gdn_save is None else (self.gdn_save[0][li], self.gdn_save[1][li])
-        self.side.wait_stream(main)
-        with torch.cuda.stream(self.side):
-            K.dense_skinny(lw.ab, self.xn, ao, m, pdl=False)
-        self._gemv(lw.qkvz, self.xp_h, self.xs_h, qo, m, pdl=False)
-        main.wait_stream(self.side)
+        pdl = self._mma(m) and self.pdl
+        if self._mma(m):
+            # the small dense a/b projection runs on CTAs of the qkvz launch (a forked branch of the graph cost 10 us a layer)
+            self._gemv(lw.qkvz, self.xp_h, self.xs_h, qo, m, pdl=pdl, ab_w=lw.ab_dense, ab_x=self.xn, ab_out=ao)
+        else:
+            # fork: the tiny dense a/b projection runs beside the big qkvz stream
+            main = torch.cuda.current_stream()
+            self.side.wait_stream(main)
+            with torch.cuda.stream(self.side):
+                K.dense_skinny(lw.ab, self.xn, ao, m, pdl=False)
+            self._gemv(lw.qkvz, self.xp_h, self.xs_h, qo, m, pdl=False)
+            main.wait_stream(self.side)
         K.gdn_decode(qo, qo.shape[1], ao, self.ldab, lw.conv_w, lw.a_log, lw.dt_bias,
                      lw.gamma, self.pool.conv_state[li], self.pool.rec_state[li], v["gslot"], xpack=self.xp_v,
-                     xs=self.xs_v, batch=lay.b, t=lay.t, nk=sp.nk, nv=sp.nv, group=self._grp(), eps=sp.eps, pdl=False)
+                     xs=self.xs_v, batch=lay.b, t=lay.t, nk=sp.nk, nv=sp.nv, group=self._grp(m), eps=sp.eps, pdl=pdl)
         self._row_parallel(0, lw.out_proj, self.xp_v, self.xs_v, m, lw.ln2, want_xn=False)
 
     def _pick_splits(self, b: int, ctx_hint: int) -> int:
@@ -634,7 +662,7 @@ class HybridRunner:
                      pdl=self.pdl, scales=self.pool.scales(li),
                      per_pages=((ctx_hint + PAGE - 1) // PAGE + splits - 1) // splits if self.uniform_rows and ctx_hint else 0)
         K.attn_reduce(self.part_o, self.part_ml, splits, self.qkv_out, self.qkv_n, m, sp.hq, xpack=self.xp_a,
-                      xs=self.xs_a, group=self._grp(), pdl=self.pdl)
+                      xs=self.xs_a, group=self._grp(m), pdl=self.pdl)
         self._row_parallel(0, lw.o_proj, self.xp_a, self.xs_a, m, lw.ln2, want_xn=False)
 
     def _head(self, m: int, sample: bool = True) -> None:

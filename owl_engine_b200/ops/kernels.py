@@ -181,6 +181,8 @@ class StreamTcWorkspace:
 
 ACT_TILES = 0x1000     # OR into a producer's ``group`` argument: write ActPack in the tile layout
 ACT_A8 = 0x2000        # OR into a producer's ``group`` argument: round the activations to 8 bits (low plane zero)
+ACT_FRAG = 0x4000      # OR into a producer's ``group`` argument: bf16 fragments for w4_mma (buffers hold rows rounded up to 8)
+ACT_NV = 0x8000        # with ACT_FRAG: the element order of nvfp4_mma
 
 
 def act_tile_bytes(k: int, group: int) -> int:
@@ -233,6 +235,26 @@ def w4_fma(w, x, out, *, norm_w=None, residual=None, epi: int = EPI_STORE, ab_w=
     assert w.layout == "slice" and w.group == 128, "w4_fma reads slice-major group-128 records"
     call("owl_w4_fma", ptr(w.records), ptr(x), ptr(norm_w), ptr(out), ptr(residual), ptr(ab_w), ptr(ab_out), ab_rows,
          ptr(x_out), w.n, w.k, int(norm_w is not None), epi, eps, int(one_plus_w), groups_per_cta, int(pdl), stream())
+
+
+register("owl_w4_mma", [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P])
+register("owl_nvfp4_mma", [_P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P])
+
+
+def w4_mma(w, xpack, xs, out, m: int, *, residual=None, epi: int = EPI_STORE, ldo: int | None = None, a8: bool = False,
+           ab_w=None, ab_x=None, ab_out=None, pdl: bool = False) -> None:
+    """out[m, :] = dequant(w) @ x for m <= 32 rows on the 16-bit tensor path (``csrc/gemv_mma.cu``): int4 slice-major records
+    with activations packed ``ACT_FRAG`` (and ``ACT_A8`` with ``a8``), or an ``NvFp4Linear`` with ``ACT_FRAG | ACT_NV``.
+    ``ab_w`` bf16 ``[r, K]``: dense rows multiplied with the plain bf16 rows ``ab_x`` into ``ab_out`` by the same launch."""
+    ldo = out.shape[-1] if ldo is None else ldo
+    ab = (ptr(ab_w), ptr(ab_x), ptr(ab_out), ab_w.shape[0] if ab_w is not None else 0, ab_out.shape[-1] if ab_w is not None else 0)
+    if w.layout == "nvfp4":
+        call("owl_nvfp4_mma", ptr(w.codes), ptr(w.scales), float(w.alpha), ptr(w.row_scale), ptr(xpack), ptr(out), ptr(residual), *ab,
+             m, w.n, w.k, ldo, epi, int(pdl), stream())
+        return
+    assert w.layout == "slice", "w4_mma reads slice-major records"
+    call("owl_w4_mma", ptr(w.records), ptr(xpack), ptr(xs), ptr(out), ptr(residual), *ab, m, w.n, w.k, ldo, w.group, epi, int(a8),
+         int(pdl), stream())
 
 
 def fma_status() -> int:

@@ -90,10 +90,11 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.Ten
             # a handful of rows (the tail chunk after the last block boundary): the weight-streaming kernel
             t, k = x.shape
             xb = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
-            xp = torch.empty(t, 2 * k, dtype=torch.uint8, device=x.device)
-            xs = torch.empty(t, k // w.group, 2, dtype=torch.float32, device=x.device)
-            K.act_pack(xb, xp, xs, t, k, w.group)
-            K.w4a16_skinny(w, xp, xs, out, t, ldo=out.stride(0))
+            rows = (t + 7) // 8 * 8
+            xp = torch.empty(rows, 2 * k, dtype=torch.uint8, device=x.device)
+            xs = torch.empty(rows, k // w.group, 2, dtype=torch.float32, device=x.device)
+            K.act_pack(xb, xp, xs, t, k, w.group | K.ACT_FRAG)
+            K.w4_mma(w, xp, xs, out, t, ldo=out.stride(0))
             return out
         if x.shape[0] >= DEQUANT_FROM:
             return gemm_tc.f16_gemm(x, w4_dense(w, x.dtype, x.device, resident=resident), out)

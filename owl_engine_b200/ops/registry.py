@@ -39,6 +39,8 @@ _T = [
     KernelSpec("owl_bf16_skinny", "gemv.cu", "gemv", gen="mma.sync+bulk-copy"),
     KernelSpec("owl_w8a16_skinny", "gemv.cu", "gemv", gen="mma.sync+bulk-copy"),
     KernelSpec("owl_skinny_status", "gemv.cu", "status", capture=False),
+    KernelSpec("owl_w4_mma", "gemv_mma.cu", "gemv", gen="mma.sync+cp.async+dsmem"),
+    KernelSpec("owl_nvfp4_mma", "gemv_mma.cu", "gemv", gen="mma.sync+cp.async+dsmem"),
     KernelSpec("owl_w4_fma", "gemv_fma.cu", "gemv", gen="hfma2+bulk-copy"),
     KernelSpec("owl_w4_fma_tp", "gemv_fma.cu", "gemv", gen="hfma2+bulk-copy+p2p"),
     KernelSpec("owl_fma_status", "gemv_fma.cu", "status", capture=False),
