@@ -455,6 +455,8 @@ class HybridRunner:
         sp = self.spec
         if self._dense16(m):
             return False
+        if m == 1 and self.act_bits == 8 and not self.uniform_rows and self.w.layout == "slice":
+            return False          # one row of 8-bit activations: dp4a needs half the products and streams faster (10 against 13 us)
         if self.decode_gemv == "dp4a" or self.fuse_norm or self.w.layout not in ("slice", "nvfp4") or not self.w.layers:
             return False
         return (self.comm is None or sp.tp_world == 1) and not any(k % 128 for k in (sp.hidden, sp.inter, sp.value_dim, sp.hq * sp.hd))
@@ -1040,8 +1042,9 @@ class HybridRunner:
             h.copy_(embeds)
         fi = gi = 0
         use_state = pos0 > 0
+        y = None                    # the last MLP's output, not yet added to h: the next norm adds it on its way
         for i, lw in enumerate(self.w.layers):
-            K.rmsnorm_pack(h, lw.ln1, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps)
+            K.rmsnorm_pack(h, lw.ln1, delta=y, out_h=h if y is not None else None, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps)
             if lw.kind == "gdn":
                 nq = sp.conv_dim + sp.value_dim
                 wide = ws["wide"].view(-1)[:t * nq].view(t, nq)
@@ -1067,14 +1070,19 @@ class HybridRunner:
             if self.comm is not None and sp.tp_world > 1:
                 self.comm.allreduce_prefill(ws["y"][:t])
             K.rmsnorm_pack(h, lw.ln2, delta=ws["y"][:t], out_h=h, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps)
-            gu = ws["wide"].view(-1)[:t * 2 * sp.inter].view(t, 2 * sp.inter)
-            self._gemm(lw.gate_up, x, gu)
-            K.silu_mul(gu, t, sp.inter, out=ws["act"][:t], group=self.G)
+            if not linear.w4_gemm_silu(lw.gate_up, x, ws["act"][:t], arm=self.prefill_gemm):
+                gu = ws["wide"].view(-1)[:t * 2 * sp.inter].view(t, 2 * sp.inter)
+                self._gemm(lw.gate_up, x, gu)
+                K.silu_mul(gu, t, sp.inter, out=ws["act"][:t], group=self.G)
             self._gemm(lw.down, ws["act"][:t], ws["y"][:t])
             if self.comm is not None and sp.tp_world > 1:
                 self.comm.allreduce_prefill(ws["y"][:t])
-            h.add_(ws["y"][:t])
-            if self.taps is not None and i in self.taps and "prefill" in self.taps:
+            y = ws["y"][:t]
+            tap = self.taps is not None and i in self.taps and "prefill" in self.taps
+            if tap or i + 1 == len(self.w.layers):
+                h.add_(y)
+                y = None
+            if tap:
                 self.taps["prefill"][i] = h.clone()
         if self.taps is not None and self.tap_sink is not None and "prefill" in self.taps:
             self.tap_sink(pos0, t, self.taps["prefill"])

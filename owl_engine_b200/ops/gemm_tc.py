@@ -78,6 +78,20 @@ def f16_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, force_small: b
     return out
 
 
+K.register("owl_gemm_silu", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p])
+
+
+def gemm_silu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, sx: torch.Tensor | None = None, sw: torch.Tensor | None = None) -> torch.Tensor:
+    """out[T, N/2] (fp16) = silu(gate) * up of x @ w^T, gate / up rows of ``w`` interleaved in eights, in the GEMM's epilogue;
+    with ``sx`` / ``sw`` both operands are e4m3 bytes with per-row scales."""
+    assert x.dtype == w.dtype and out.dtype == torch.float16 and out.stride(-1) == 1
+    ensure_scratch(x.device)
+    fmt = 2 if sx is not None else 1 if x.dtype == torch.bfloat16 else 0
+    K.call("owl_gemm_silu", K.ptr(x), x.stride(0), K.ptr(sx), K.ptr(w), w.stride(0), K.ptr(sw), K.ptr(out), x.shape[0], w.shape[0],
+           x.shape[1], out.stride(0), fmt, K.stream())
+    return out
+
+
 def gemm_status() -> int:
     f = K.fn("owl_gemm_status")
     f.argtypes = []

@@ -73,14 +73,7 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.Ten
     if arm in ("tc8", "tc8r") and x.shape[0] >= DEQUANT_FROM and w.k % 128 == 0:
         from . import gemm_tc
 
-        cached = getattr(w, "_owl_e4m3", None) if resident else None
-        if cached is None:
-            dense = K.w4_dequant(w, _dense_scratch(w.n, w.k, x.device, torch.float16))
-            cached = gemm_tc.quant_e4m3_rows(dense) if resident else gemm_tc.quant_e4m3_rows(dense, *_fp8_scratch("w", w.n, w.k, x.device))
-            if resident:
-                _ledger(x.device).track("resident e4m3 weight copy", "resident copies", cached[0])
-                w._owl_e4m3 = cached
-        wq, sw = cached
+        wq, sw = _e4m3_weight(w, x.device, resident)
         xq, sx = gemm_tc.quant_e4m3_rows(x, *_fp8_scratch("x", x.shape[0], w.k, x.device))
         return gemm_tc.e4m3_gemm(xq, sx, wq, sw, out)
     if arm in ("tc", "tc8", "tcr", "tc8r"):
@@ -100,6 +93,42 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.Ten
             return gemm_tc.f16_gemm(x, w4_dense(w, x.dtype, x.device, resident=resident), out)
         return gemm_tc.w4a16_gemm(w, x, out)
     raise ValueError(f"unknown prefill GEMM arm {arm!r}")
+
+
+def _e4m3_weight(w, device, resident: bool):
+    """The weight as e4m3 rows with their scales: its resident copy (made on first use), or the shared scratch."""
+    from . import gemm_tc
+
+    cached = getattr(w, "_owl_e4m3", None) if resident else None
+    if cached is None:
+        dense = K.w4_dequant(w, _dense_scratch(w.n, w.k, device, torch.float16))
+        cached = gemm_tc.quant_e4m3_rows(dense) if resident else gemm_tc.quant_e4m3_rows(dense, *_fp8_scratch("w", w.n, w.k, device))
+        if resident:
+            _ledger(device).track("resident e4m3 weight copy", "resident copies", cached[0])
+            w._owl_e4m3 = cached
+    return cached
+
+
+SILU_FROM = 256         # tokens from which the persistent GEMM, which has the silu(gate) * up epilogue, multiplies fp16 weights
+
+
+def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> bool:
+    """out[T, N/2] (fp16) = silu(gate) * up of the merged gate / up projection in one launch. False (and nothing done) where the
+    arm or the shape has no such epilogue: the caller multiplies and activates in two steps."""
+    from . import gemm_tc
+
+    t = x.shape[0]
+    if w.layout == "nvfp4" or x.dtype != torch.float16 or out.dtype != torch.float16 or out.stride(0) % 8:
+        return False
+    if arm in ("tc8", "tc8r") and t >= DEQUANT_FROM and w.k % 128 == 0:
+        wq, sw = _e4m3_weight(w, x.device, arm == "tc8r")
+        xq, sx = gemm_tc.quant_e4m3_rows(x, *_fp8_scratch("x", t, w.k, x.device))
+        gemm_tc.gemm_silu(xq, wq, out, sx, sw)
+        return True
+    if arm in ("tc", "tc4", "tcr", "tc8", "tc8r") and t >= SILU_FROM and w.n >= 512:
+        gemm_tc.gemm_silu(x, w4_dense(w, x.dtype, x.device, resident=arm in ("tcr", "tc8r")), out)
+        return True
+    return False
 
 
 def nvfp4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.Tensor:
@@ -174,4 +203,6 @@ def dense_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, arm: str = "
             cache = w.to(x.dtype)
             w._owl_cast = cache
         w = cache
-    return gemm_tc.f16_gemm(x, w, out)
+    # few weight rows (the 96 of the a / b projection): the persistent kernel cuts k so that every SM has a part (2048 tokens:
+    # 37 us on the 16 tiles of the other kernel)
+    return gemm_tc.f16_gemm(x, w, out, force_persist=x.shape[0] >= 256)

@@ -39,6 +39,7 @@ _T = [
     KernelSpec("owl_bf16_skinny", "gemv.cu", "gemv", gen="mma.sync+bulk-copy"),
     KernelSpec("owl_w8a16_skinny", "gemv.cu", "gemv", gen="mma.sync+bulk-copy"),
     KernelSpec("owl_skinny_status", "gemv.cu", "status", capture=False),
+    KernelSpec("owl_gemm_silu", "gemm_dense.cu", "gemm_act", gen="tcgen05+tma"),
     KernelSpec("owl_w4_mma", "gemv_mma.cu", "gemv", gen="mma.sync+cp.async+dsmem"),
     KernelSpec("owl_nvfp4_mma", "gemv_mma.cu", "gemv", gen="mma.sync+cp.async+dsmem"),
     KernelSpec("owl_w4_fma", "gemv_fma.cu", "gemv", gen="hfma2+bulk-copy"),
