@@ -241,47 +241,55 @@ __global__ void __launch_bounds__(256) gdn_decode_kernel(GdnDecodeParams p) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Prefill conv: one warp per (t, 128-channel segment). Segments 0..2nk-1 are q/k heads (get
-// l2norm), the rest are v heads. Reads the 3-sample history from conv_state for t < 3 and
-// (blockIdx.z == last time tile) writes the new history. Output bf16 [T][conv_dim].
+// Prefill conv: one warp per (TR consecutive t, 128-channel segment). Segments 0..2nk-1 are q/k heads (get
+// l2norm), the rest are v heads. Reads the 3-sample history from conv_state for t < 3. Output bf16 [T][conv_dim].
+// Memory bound (every input read once, every output written once: 13 us at 2048 tokens of 10240 channels). With one t per
+// warp (TR = 1) the four taps were four loads and the weights four more per output row: 56 us; TR = 8 loads 11 rows for 8
+// outputs, all of them before the first is used. Short prompts keep TR = 1 for its eight times as many warps.
 // ---------------------------------------------------------------------------------------
+template <int TR>
 __global__ void __launch_bounds__(256) gdn_conv_fwd_kernel(const __nv_bfloat16* __restrict__ x, int ld,
                                                            const float* __restrict__ conv_w, float* conv_state,
                                                            int slot, __nv_bfloat16* out, int T, int nk, int nv,
                                                            int use_state) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int seg = blockIdx.x;
-  const int t = blockIdx.y * 8 + warp;
+  const int t0 = (blockIdx.y * 8 + warp) * TR;
   const int K = nk * GD, conv_dim = 2 * K + nv * GD;
-  if (t >= T) return;
+  if (t0 >= T) return;
   const int ch0 = seg * GD + lane * 4;
-  float acc[4];
-  float xin[4][4];  // [tap][channel]
+  float xin[TR + 3][4];  // rows t0 - 3 .. t0 + TR - 1
 #pragma unroll
-  for (int tap = 0; tap < 4; ++tap) {
-    const int tt = t - 3 + tap;
-    if (tt >= 0) {
-      const uint2 u = *reinterpret_cast<const uint2*>(x + (size_t)tt * ld + ch0);
-      xin[tap][0] = bf16_lo(u.x); xin[tap][1] = bf16_hi(u.x); xin[tap][2] = bf16_lo(u.y); xin[tap][3] = bf16_hi(u.y);
-    } else {
+  for (int i = 0; i < TR + 3; ++i) {
+    const int tt = t0 - 3 + i;
+    uint2 u = make_uint2(0, 0);
+    if (tt >= 0 && tt < T) u = *reinterpret_cast<const uint2*>(x + (size_t)tt * ld + ch0);
+    xin[i][0] = bf16_lo(u.x); xin[i][1] = bf16_hi(u.x); xin[i][2] = bf16_lo(u.y); xin[i][3] = bf16_hi(u.y);
+    if (tt < 0) {
 #pragma unroll
       for (int c = 0; c < 4; ++c)
-        xin[tap][c] = use_state ? conv_state[((size_t)slot * conv_dim + ch0 + c) * 3 + (3 + tt)] : 0.f;
+        xin[i][c] = use_state ? conv_state[((size_t)slot * conv_dim + ch0 + c) * 3 + (3 + tt)] : 0.f;
     }
   }
+  float4 w4[4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const float4 w4 = *reinterpret_cast<const float4*>(conv_w + (size_t)(ch0 + c) * 4);
-    acc[c] = silu_f(w4.x * xin[0][c] + w4.y * xin[1][c] + w4.z * xin[2][c] + w4.w * xin[3][c]);
-  }
-  if (seg < 2 * nk) {
-    float ss = warp_sum(acc[0] * acc[0] + acc[1] * acc[1] + acc[2] * acc[2] + acc[3] * acc[3]);
-    const float rinv = rsqrtf(ss + 1e-6f);
+  for (int c = 0; c < 4; ++c) w4[c] = *reinterpret_cast<const float4*>(conv_w + (size_t)(ch0 + c) * 4);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[c] *= rinv;
+  for (int i = 0; i < TR; ++i) {
+    if (t0 + i >= T) break;
+    float acc[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      acc[c] = silu_f(w4[c].x * xin[i][c] + w4[c].y * xin[i + 1][c] + w4[c].z * xin[i + 2][c] + w4[c].w * xin[i + 3][c]);
+    if (seg < 2 * nk) {
+      const float ss = warp_sum(acc[0] * acc[0] + acc[1] * acc[1] + acc[2] * acc[2] + acc[3] * acc[3]);
+      const float rinv = rsqrtf(ss + 1e-6f);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[c] *= rinv;
+    }
+    *reinterpret_cast<uint2*>(out + (size_t)(t0 + i) * conv_dim + ch0) =
+        make_uint2(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]));
   }
-  *reinterpret_cast<uint2*>(out + (size_t)t * conv_dim + ch0) =
-      make_uint2(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]));
 }
 // New conv history after a prefill chunk: the last 3 inputs (falling back to the old history
 // when the chunk is shorter than 3). One thread per channel. Runs after gdn_conv_fwd_kernel.
@@ -572,9 +580,14 @@ OWL_API int owl_gdn_conv_fwd(const void* x, int ld, const void* conv_w, void* co
                              int nk, int nv, int use_state, cudaStream_t st) {
   if (T < 1 || nk < 1 || nv < 1 || (ld & 3)) return OWL_ERR_BAD_ARG;
   const int conv_dim = (2 * nk + nv) * GD;
-  gdn_conv_fwd_kernel<<<dim3(2 * nk + nv, (T + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)x, ld, (const float*)conv_w,
-                                                                      (float*)conv_state, slot,
-                                                                      (__nv_bfloat16*)out, T, nk, nv, use_state);
+  const int tr = T >= 512 ? 8 : 1;
+  const dim3 grid(2 * nk + nv, (T + 8 * tr - 1) / (8 * tr));
+  if (tr == 8)
+    gdn_conv_fwd_kernel<8><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (const float*)conv_w, (float*)conv_state, slot,
+                                                 (__nv_bfloat16*)out, T, nk, nv, use_state);
+  else
+    gdn_conv_fwd_kernel<1><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (const float*)conv_w, (float*)conv_state, slot,
+                                                 (__nv_bfloat16*)out, T, nk, nv, use_state);
   OWL_LAUNCH_CHECK();
   gdn_conv_state_kernel<<<(conv_dim + 255) / 256, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (float*)conv_state, slot, T,
                                                                 conv_dim, use_state);

@@ -1,0 +1,105 @@
+"""Prompt-sized forms of the prefill kernels against the forms that short inputs take."""
+import pytest
+import torch
+
+from owl_engine_b200.ops import gemm_tc, linear
+from owl_engine_b200.ops import kernels as K
+from owl_engine_b200.ops import quant as Q
+from owl_engine_b200.ops import reference as R
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("t", [512, 513, 519, 700])
+@pytest.mark.parametrize("use_state", [False, True])
+def test_conv_of_long_chunks_equals_short_chunks(t, use_state):
+    """Eight rows per warp (from 512 rows) against one row per warp, fed the same rows in pieces with the history between them:
+    the same products in the same order, so the same bits."""
+    nk, nv, slot = 2, 4, 1
+    gen = torch.Generator(device=DEV).manual_seed(t)
+    cd = (2 * nk + nv) * 128
+    x = torch.randn(t, cd + 64, device=DEV, generator=gen).bfloat16()
+    w = torch.randn(cd, 4, device=DEV, generator=gen)
+    hist = torch.randn(3, cd, 3, device=DEV, generator=gen)
+    h1, h2 = hist.clone(), hist.clone()
+    a, b = (torch.zeros(t, cd, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    K.gdn_conv_fwd(x, cd + 64, w, h1, slot, a, t, nk, nv, use_state)
+    for r in range(0, t, 256):
+        n = min(256, t - r)
+        K.gdn_conv_fwd(x[r:], cd + 64, w, h2, slot, b[r:], n, nk, nv, use_state or r > 0)
+    assert torch.equal(a, b) and torch.equal(h1, h2)
+
+
+@pytest.mark.parametrize("pool", ["fp8", "int8", "f16"])
+@pytest.mark.parametrize("rows,hq,hkv,rot", [(128, 24, 4, 64), (131, 6, 2, 256), (200, 2, 1, 16)])
+def test_qknorm_rope_of_many_rows_equals_few_rows(pool, rows, hq, hkv, rot):
+    """A CTA per row (from 128 rows) against a CTA per (row, head): sums in another order, so one bf16 (or e4m3 / int8) step."""
+    hd = 256
+    gen = torch.Generator(device=DEV).manual_seed(rows)
+    ld = 2 * hq * hd + 2 * hkv * hd
+    wide = torch.randn(rows, ld, device=DEV, generator=gen).bfloat16()
+    qw, kw = ((torch.randn(hd, device=DEV, generator=gen) * 0.1).bfloat16() for _ in range(2))
+    pos3 = torch.randint(0, 200000, (3, rows), device=DEV, generator=gen, dtype=torch.int32)
+    inv = R.rope_inv_freq(rot, 1e7).to(DEV)
+    section = torch.tensor([j % 3 for j in range(rot // 2)], dtype=torch.uint8, device=DEV)
+    slots = torch.randperm(16 * 16, device=DEV, generator=gen)[:rows].int()
+    slots[3] = -1
+
+    def run(step):
+        dt = torch.float16 if pool == "f16" else torch.uint8
+        kp, vp = (torch.zeros(16, 16, hkv, hd, dtype=dt, device=DEV) for _ in range(2))
+        sc = (torch.zeros(16, 16, hkv, device=DEV), torch.zeros(16, 16, hkv, device=DEV)) if pool == "int8" else None
+        q = torch.zeros(rows, hq, hd, dtype=torch.bfloat16, device=DEV)
+        for r in range(0, rows, step):
+            n = min(step, rows - r)
+            x = wide[r:r + n]
+            K.qknorm_rope_insert(x, ld, x[:, 2 * hq * hd:], ld, x[:, 2 * hq * hd + hkv * hd:], ld, qw, kw,
+                                 pos3[:, r:r + n].contiguous(), inv, section, slots[r:r + n], q[r:], kp, vp, n, hq, hkv, hd, rot, scales=sc)
+        f = (lambda p: p.float()) if pool == "f16" else (lambda p: p.view(torch.int8 if pool == "int8" else torch.float8_e4m3fn).float())
+        return [q.float(), f(kp), f(vp)] + list(sc or ())
+    for a, b in zip(run(rows), run(64)):
+        assert (a - b).abs().max() <= 2.0 ** -3 * b.abs().max() and (a != b).float().mean() < 0.02
+        assert (a - b).norm() <= 2e-3 * b.norm()
+
+
+@pytest.mark.parametrize("t", [256, 300])
+@pytest.mark.parametrize("n,k", [(512, 128), (1072, 1024), (40960, 128)])
+@pytest.mark.parametrize("fmt", ["f16", "bf16", "e4m3"])
+def test_silu_epilogue(t, n, k, fmt):
+    """Edges of the 256-column tile (1072 = 4 tiles + 48), the k-split form (few tiles, 16 k steps) and the unsplit one."""
+    gen = torch.Generator(device=DEV).manual_seed(n + t)
+    x, w = torch.randn(t, k, device=DEV, generator=gen), torch.randn(n, k, device=DEV, generator=gen) * 0.05
+    out = torch.zeros(t, n // 2 + 8, dtype=torch.float16, device=DEV)
+    if fmt == "e4m3":
+        xq, sx = gemm_tc.quant_e4m3_rows(x.half())
+        wq, sw = gemm_tc.quant_e4m3_rows(w.half())
+        gemm_tc.gemm_silu(xq, wq, out, sx, sw)
+        xd, wd = xq.view(torch.float8_e4m3fn).double() * sx[:, None], wq.view(torch.float8_e4m3fn).double() * sw[:, None]
+    else:
+        dt = torch.float16 if fmt == "f16" else torch.bfloat16
+        x, w = x.to(dt), w.to(dt)
+        gemm_tc.gemm_silu(x, w, out)
+        xd, wd = x.double(), w.double()
+    y = (xd @ wd.t()).view(t, n // 16, 2, 8)
+    want = (y[:, :, 0] * torch.sigmoid(y[:, :, 0]) * y[:, :, 1]).reshape(t, n // 2)
+    got = out[:, :n // 2].double()
+    assert (out[:, n // 2:] == 0).all()
+    # fp16 result (2^-11), fp32 sums, the fast exponential (2 ulp)
+    assert ((got - want).abs() <= want.abs() * 2.0 ** -10 + 2.0 ** -16 * y.abs().amax() ** 2 + 2.0 ** -24).all()
+    assert gemm_tc.gemm_status() == 0
+
+
+def test_gate_up_with_activation_matches_two_steps():
+    gen = torch.Generator().manual_seed(1)
+    c = Q.pack_skinny(Q.quantize_w4(torch.randn(1024, 512, generator=gen) * 0.05, 128)).to(DEV)
+    for t in (100, 255, 256):
+        x = torch.randn(t, 512, generator=gen).half().to(DEV)
+        out = torch.zeros(t, 512, dtype=torch.float16, device=DEV)
+        done = linear.w4_gemm_silu(c, x, out, arm="tc")
+        assert done == (t >= linear.SILU_FROM)
+        if done:
+            gu = linear.w4_gemm(c, x, torch.empty(t, 1024, dtype=torch.bfloat16, device=DEV), arm="tc")
+            two = torch.empty_like(out)
+            K.silu_mul(gu, t, 512, out=two)
+            assert (out.float() - two.float()).norm() < 6e-3 * two.float().norm()      # the two-step form rounds gate and up to bf16
