@@ -8,11 +8,15 @@
 //   S  <- e^{gc_last} S + (e^{gc_last - gc} k)^T v'
 // (every exponential has a non-positive argument). Two kernels:
 //   gdn_chunk_prep_kernel  one CTA per (chunk, v-head), all chunks in parallel: the 64x64 products and the two 64x128
-//                          products on mma.sync (bf16 in, fp32 accumulate), the triangular inverse by forward substitution
-//                          with one column per thread; writes w, u, scaled q, scaled k^T and attn
+//                          products on mma.sync (bf16 in, fp32 accumulate), the triangular inverse in fp32 by blocks (16 x 16
+//                          by substitution, then two doublings); writes w, u, scaled q, scaled k and attn
 //   gdn_chunk_scan_kernel  one CTA per (v-head, half of the value columns), the chunks in order: three small tensor-core
 //                          products per chunk against the fp32 state kept in MMA accumulator registers (a bf16 copy in
 //                          shared memory is the B operand), operands prefetched one chunk ahead with cp.async
+// Every tile stays in the row order it has in global memory; the products that need it the other way round read it with
+// ldmatrix.trans. Before that the tiles were transposed through shared memory (8-way bank conflicts) and the fragments
+// fetched word by word, and the inverse ran one column per thread through 2016 dependent steps: 168 us (preparation) and
+// 117 us (recurrence) a layer at 2048 tokens x 48 heads; memory traffic would take 31 and 20 us.
 // followed by the gated RMSNorm kernel of gdn.cu. q and k arrive l2-normalised from the convolution kernel.
 //
 // Reference counterpart: the chunk-64 delta-rule kernels (cumsum, kkt, solve_tril, wu, h, o) that the reference compiles
@@ -34,16 +38,27 @@ __device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uin
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// A fragment (16 x 16) of a row-major bf16 tile; B fragment (16 x 8) of a tile stored [n][k]
-__device__ __forceinline__ void frag_a(const __nv_bfloat16* s, int ld, int m0, int k0, int g, int t, uint32_t* a) {
-  a[0] = *reinterpret_cast<const uint32_t*>(s + (m0 + g) * ld + k0 + 2 * t);
-  a[1] = *reinterpret_cast<const uint32_t*>(s + (m0 + g + 8) * ld + k0 + 2 * t);
-  a[2] = *reinterpret_cast<const uint32_t*>(s + (m0 + g) * ld + k0 + 2 * t + 8);
-  a[3] = *reinterpret_cast<const uint32_t*>(s + (m0 + g + 8) * ld + k0 + 2 * t + 8);
+// Fragments through ldmatrix; ld in elements (rows of 16-byte multiples, 16 bytes past a multiple of 128: conflict-free).
+__device__ __forceinline__ void ldm4(uint32_t* r, const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
 }
-__device__ __forceinline__ void frag_b(const __nv_bfloat16* s, int ld, int n0, int k0, int g, int t, uint32_t* b) {
-  b[0] = *reinterpret_cast<const uint32_t*>(s + (n0 + g) * ld + k0 + 2 * t);
-  b[1] = *reinterpret_cast<const uint32_t*>(s + (n0 + g) * ld + k0 + 2 * t + 8);
+__device__ __forceinline__ void ldm4t(uint32_t* r, const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+// A (16 x 16) of a tile stored [m][k] / [k][m]; B (16 x 16: two n-tiles, registers 0-1 and 2-3) stored [n][k] / [k][n]
+__device__ __forceinline__ void frag_a(uint32_t* r, const __nv_bfloat16* s, int ld, int m0, int k0, int l) {
+  ldm4(r, s + (m0 + (l & 15)) * ld + k0 + (l >> 4) * 8);
+}
+__device__ __forceinline__ void frag_at(uint32_t* r, const __nv_bfloat16* s, int ld, int m0, int k0, int l) {
+  ldm4t(r, s + (k0 + (l & 7) + (l >> 4) * 8) * ld + m0 + ((l >> 3) & 1) * 8);
+}
+__device__ __forceinline__ void frag_b(uint32_t* r, const __nv_bfloat16* s, int ld, int n0, int k0, int l) {
+  ldm4(r, s + (n0 + (l & 7) + (l >> 4) * 8) * ld + k0 + ((l >> 3) & 1) * 8);
+}
+__device__ __forceinline__ void frag_bt(uint32_t* r, const __nv_bfloat16* s, int ld, int n0, int k0, int l) {
+  ldm4t(r, s + (k0 + (l & 15)) * ld + n0 + (l >> 4) * 8);
 }
 __device__ __forceinline__ void ck_cp16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
@@ -58,84 +73,92 @@ struct GdnChunkParams {
   __nv_bfloat16* w;             // [Tpad][nv][128]
   float* u;                     // [Tpad][nv][128] (fp32: v' = u - w S cancels)
   __nv_bfloat16* qg;            // [Tpad][nv][128]   scale e^{gc} q
-  __nv_bfloat16* kdT;           // [nv][chunks][128][64]   (e^{gc_last - gc} k)^T
+  __nv_bfloat16* kd;            // [nv][chunks][64][128]   e^{gc_last - gc} k
   __nv_bfloat16* attn;          // [nv][chunks][64][64]
   float* eglast;                // [nv][chunks]
   int ldab, nk, nv, T, slot, use_state, chunks;
 };
 
-// ---- preparation: one CTA per (chunk, v-head), 256 threads -----------------------------------------------------------
+// ---- preparation: one CTA per (chunk, v-head), 256 threads, three CTAs per SM -------------------------------------------
 struct PrepSmem {
-  __nv_bfloat16 k[CK_C][CK_LD];       // k rows
-  __nv_bfloat16 q[CK_C][CK_LD];       // q rows; later T as bf16 ([64][CK_LT] inside the same bytes)
-  __nv_bfloat16 vbT[CK_D][CK_LT];     // (beta v)^T
-  __nv_bfloat16 kgT[CK_D][CK_LT];     // (beta e^{gc} k)^T; first the staging area of the raw v rows ([64][CK_LD])
-  float a[CK_C][CK_C + 1];            // A' (strictly lower)
-  float g[CK_C], gc[CK_C], beta[CK_C];
+  __nv_bfloat16 k[CK_C][CK_LD];
+  __nv_bfloat16 v[CK_C][CK_LD];
+  union {
+    __nv_bfloat16 q[CK_C][CK_LD];
+    float t[CK_C][CK_C + 4];          // T = (I + A')^-1 (q is consumed by then)
+  };
+  union {
+    float a[CK_C][CK_C + 4];          // A' (strictly lower)
+    __nv_bfloat16 tb[2][CK_C][CK_LT]; // T diag(beta), T diag(beta e^{gc})
+  };
+  float x[32][36];
+  float gc[CK_C], beta[CK_C], eg[CK_C], el[CK_C];       // el: e^{gc_last - gc}
 };
-__global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(GdnChunkParams p) {
+__global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkParams p) {
   extern __shared__ __align__(16) uint8_t ck_smem[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(ck_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
   const int c = blockIdx.x, h = blockIdx.y, R = p.nv / p.nk, hk = h / R;
   const int K = p.nk * CK_D, V = p.nv * CK_D, conv_dim = 2 * K + V, r0 = c * CK_C;
   const float scale = rsqrtf((float)CK_D);
-  __nv_bfloat16(*vraw)[CK_LD] = reinterpret_cast<__nv_bfloat16(*)[CK_LD]>(&sm.kgT[0][0]);
   // 1. tiles (zero rows past T) and per-token scalars
   for (int i = tid; i < CK_C * 16; i += 256) {
     const int t = i >> 4, piece = (i & 15) * 8, r = r0 + t;
-    uint4 qv = make_uint4(0, 0, 0, 0), kv = qv, vv = qv;
     if (r < p.T) {
       const __nv_bfloat16* xr = p.qkv + (size_t)r * conv_dim;
-      qv = *reinterpret_cast<const uint4*>(xr + hk * CK_D + piece);
-      kv = *reinterpret_cast<const uint4*>(xr + K + hk * CK_D + piece);
-      vv = *reinterpret_cast<const uint4*>(xr + 2 * K + h * CK_D + piece);
+      ck_cp16(&sm.q[t][piece], xr + hk * CK_D + piece);
+      ck_cp16(&sm.k[t][piece], xr + K + hk * CK_D + piece);
+      ck_cp16(&sm.v[t][piece], xr + 2 * K + h * CK_D + piece);
+    } else {
+      const uint4 z = make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(&sm.q[t][piece]) = z;
+      *reinterpret_cast<uint4*>(&sm.k[t][piece]) = z;
+      *reinterpret_cast<uint4*>(&sm.v[t][piece]) = z;
     }
-    *reinterpret_cast<uint4*>(&sm.q[t][piece]) = qv;
-    *reinterpret_cast<uint4*>(&sm.k[t][piece]) = kv;
-    *reinterpret_cast<uint4*>(&vraw[t][piece]) = vv;
   }
-  if (tid < CK_C) {
-    const int r = r0 + tid;
-    float gg = 0.f, bb = 0.f;
-    if (r < p.T) {
-      const float a = __bfloat162float(p.ab[(size_t)r * p.ldab + h]);
-      const float b = __bfloat162float(p.ab[(size_t)r * p.ldab + p.nv + h]);
-      gg = -__expf(p.a_log[h]) * softplus_f(a + p.dt_bias[h]);
-      bb = sigmoid_f(b);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  if (warp == 0) {                    // two tokens per lane, inclusive sums by shuffles
+    float gg[2], acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int r = r0 + 2 * lane + e;
+      gg[e] = 0.f;
+      float bb = 0.f;
+      if (r < p.T) {
+        const float a = __bfloat162float(p.ab[(size_t)r * p.ldab + h]);
+        const float b = __bfloat162float(p.ab[(size_t)r * p.ldab + p.nv + h]);
+        gg[e] = -__expf(p.a_log[h]) * softplus_f(a + p.dt_bias[h]);
+        bb = sigmoid_f(b);
+      }
+      sm.beta[2 * lane + e] = bb;
+      acc += gg[e];
     }
-    sm.g[tid] = gg;
-    sm.beta[tid] = bb;
+    float sum = acc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float n = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += n;
+    }
+    const float last = __shfl_sync(0xffffffffu, sum, 31);
+    const float g0 = sum - gg[1], g1 = sum;
+    sm.gc[2 * lane] = g0; sm.gc[2 * lane + 1] = g1;
+    sm.eg[2 * lane] = __expf(g0); sm.eg[2 * lane + 1] = __expf(g1);
+    sm.el[2 * lane] = __expf(last - g0); sm.el[2 * lane + 1] = __expf(last - g1);
+    if (lane == 0) p.eglast[(size_t)h * p.chunks + c] = __expf(last);
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  if (tid == 0) {
-    float acc = 0.f;
-    for (int i = 0; i < CK_C; ++i) { acc += sm.g[i]; sm.gc[i] = acc; }
-    p.eglast[(size_t)h * p.chunks + c] = __expf(acc);
-  }
-  __syncthreads();
-  const float gc_last = sm.gc[CK_C - 1];
-  // 2. (beta v)^T, scaled q rows and scaled k^T to global; all read the row tiles
-  for (int i = tid; i < CK_D * (CK_C / 2); i += 256) {
-    const int d = i / (CK_C / 2), j = (i % (CK_C / 2)) * 2;
-    const float v0 = __bfloat162float(vraw[j][d]) * sm.beta[j], v1 = __bfloat162float(vraw[j + 1][d]) * sm.beta[j + 1];
-    *reinterpret_cast<uint32_t*>(&sm.vbT[d][j]) = pack_bf16(v0, v1);
-    const float k0 = __bfloat162float(sm.k[j][d]), k1 = __bfloat162float(sm.k[j + 1][d]);
-    *reinterpret_cast<uint32_t*>(p.kdT + (((size_t)h * p.chunks + c) * CK_D + d) * CK_C + j) =
-        pack_bf16(k0 * __expf(gc_last - sm.gc[j]), k1 * __expf(gc_last - sm.gc[j + 1]));
-  }
-  for (int i = tid; i < CK_C * (CK_D / 2); i += 256) {
-    const int t = i / (CK_D / 2), d = (i % (CK_D / 2)) * 2;
-    const float e = scale * __expf(sm.gc[t]);
-    *reinterpret_cast<uint32_t*>(p.qg + ((size_t)(r0 + t) * p.nv + h) * CK_D + d) =
-        pack_bf16(__bfloat162float(sm.q[t][d]) * e, __bfloat162float(sm.q[t][d + 1]) * e);
-  }
-  __syncthreads();                                     // the raw v rows are consumed: their bytes become kgT
-  for (int i = tid; i < CK_D * (CK_C / 2); i += 256) {
-    const int d = i / (CK_C / 2), j = (i % (CK_C / 2)) * 2;
-    const float k0 = __bfloat162float(sm.k[j][d]) * sm.beta[j] * __expf(sm.gc[j]);
-    const float k1 = __bfloat162float(sm.k[j + 1][d]) * sm.beta[j + 1] * __expf(sm.gc[j + 1]);
-    *reinterpret_cast<uint32_t*>(&sm.kgT[d][j]) = pack_bf16(k0, k1);
+  // 2. scaled q rows and scaled k rows to global
+  for (int i = tid; i < CK_C * 16; i += 256) {
+    const int t = i >> 4, d = (i & 15) * 8;
+    const uint4 qu = *reinterpret_cast<const uint4*>(&sm.q[t][d]), ku = *reinterpret_cast<const uint4*>(&sm.k[t][d]);
+    const float e = scale * sm.eg[t], l = sm.el[t];
+    *reinterpret_cast<uint4*>(p.qg + ((size_t)(r0 + t) * p.nv + h) * CK_D + d) =
+        make_uint4(pack_bf16(bf16_lo(qu.x) * e, bf16_hi(qu.x) * e), pack_bf16(bf16_lo(qu.y) * e, bf16_hi(qu.y) * e),
+                   pack_bf16(bf16_lo(qu.z) * e, bf16_hi(qu.z) * e), pack_bf16(bf16_lo(qu.w) * e, bf16_hi(qu.w) * e));
+    *reinterpret_cast<uint4*>(p.kd + (((size_t)h * p.chunks + c) * CK_C + t) * CK_D + d) =
+        make_uint4(pack_bf16(bf16_lo(ku.x) * l, bf16_hi(ku.x) * l), pack_bf16(bf16_lo(ku.y) * l, bf16_hi(ku.y) * l),
+                   pack_bf16(bf16_lo(ku.z) * l, bf16_hi(ku.z) * l), pack_bf16(bf16_lo(ku.w) * l, bf16_hi(ku.w) * l));
   }
   // 3. k k^T and q k^T (64 x 64 x 128): warp -> rows 16 (warp & 3), columns 32 (warp >> 2)
   {
@@ -148,14 +171,16 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(GdnChunkParams p) {
 #pragma unroll
     for (int ks = 0; ks < CK_D / 16; ++ks) {
       uint32_t ak[4], aq[4];
-      frag_a(&sm.k[0][0], CK_LD, m0, ks * 16, g, t4, ak);
-      frag_a(&sm.q[0][0], CK_LD, m0, ks * 16, g, t4, aq);
+      frag_a(ak, &sm.k[0][0], CK_LD, m0, ks * 16, lane);
+      frag_a(aq, &sm.q[0][0], CK_LD, m0, ks * 16, lane);
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        uint32_t b[2];
-        frag_b(&sm.k[0][0], CK_LD, nh + n * 8, ks * 16, g, t4, b);
+      for (int n = 0; n < 4; n += 2) {
+        uint32_t b[4];
+        frag_b(b, &sm.k[0][0], CK_LD, nh + n * 8, ks * 16, lane);
         mma_bf16(kk[n], ak[0], ak[1], ak[2], ak[3], b[0], b[1]);
         mma_bf16(qk[n], aq[0], aq[1], aq[2], aq[3], b[0], b[1]);
+        mma_bf16(kk[n + 1], ak[0], ak[1], ak[2], ak[3], b[2], b[3]);
+        mma_bf16(qk[n + 1], aq[0], aq[1], aq[2], aq[3], b[2], b[3]);
       }
     }
     __nv_bfloat16* at = p.attn + ((size_t)h * p.chunks + c) * CK_C * CK_C;
@@ -175,23 +200,76 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(GdnChunkParams p) {
         *reinterpret_cast<uint32_t*>(at + i * CK_C + j) = pack_bf16(av[0], av[1]);
       }
   }
+  __syncthreads();                    // q is consumed: its bytes become T
+  // 4. T = (I + A')^-1, fp32. The four 16 x 16 diagonal blocks by forward substitution (a column per thread) ...
+  for (int i = tid; i < CK_C * (CK_C + 4) / 4; i += 256) reinterpret_cast<float4*>(&sm.t[0][0])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
-  // 4. T = (I + A')^-1 by forward substitution: thread c owns column c (rows above the diagonal are zero)
-  __nv_bfloat16(*tb)[CK_LT] = reinterpret_cast<__nv_bfloat16(*)[CK_LT]>(&sm.q[0][0]);
   if (tid < CK_C) {
-    float col[CK_C];
+    const int b = tid & ~15, cc = tid & 15;
+    float col[16];
 #pragma unroll
-    for (int i = 0; i < CK_C; ++i) {
-      float acc = (i == tid) ? 1.f : 0.f;
+    for (int i = 0; i < 16; ++i) {
+      float acc = (i == cc) ? 1.f : 0.f;
 #pragma unroll
-      for (int j = 0; j < i; ++j) acc -= sm.a[i][j] * col[j];
+      for (int j = 0; j < i; ++j) acc -= sm.a[b + i][b + j] * col[j];
       col[i] = acc;
     }
 #pragma unroll
-    for (int i = 0; i < CK_C; ++i) tb[i][tid] = __float2bfloat16(col[i]);
+    for (int i = 0; i < 16; ++i) sm.t[b + i][b + cc] = col[i];
   }
   __syncthreads();
-  // 5. u = T (beta v), w = T (beta e^{gc} k)  (64 x 128 x 64): warp -> rows 16 (warp & 3), columns 64 (warp >> 2)
+  // ... then T21 = -T22 (A21 T11), for the two pairs of 16 and the pair of 32
+  {
+    const int i = tid >> 4, j = tid & 15;
+    float x0 = 0.f, x1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      x0 += sm.a[16 + i][k] * sm.t[k][j];
+      x1 += sm.a[48 + i][32 + k] * sm.t[32 + k][32 + j];
+    }
+    sm.x[i][j] = x0;
+    sm.x[16 + i][j] = x1;
+    __syncthreads();
+    x0 = x1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      x0 -= sm.t[16 + i][16 + k] * sm.x[k][j];
+      x1 -= sm.t[48 + i][48 + k] * sm.x[16 + k][j];
+    }
+    sm.t[16 + i][j] = x0;
+    sm.t[48 + i][32 + j] = x1;
+  }
+  __syncthreads();
+  {
+    const int i = tid >> 3, j = (tid & 7) * 4;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+      const float a = sm.a[32 + i][k];
+      const float4 t = *reinterpret_cast<const float4*>(&sm.t[k][j]);
+      x.x += a * t.x; x.y += a * t.y; x.z += a * t.z; x.w += a * t.w;
+    }
+    *reinterpret_cast<float4*>(&sm.x[i][j]) = x;
+    __syncthreads();
+    x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+      const float a = sm.t[32 + i][32 + k];
+      const float4 t = *reinterpret_cast<const float4*>(&sm.x[k][j]);
+      x.x -= a * t.x; x.y -= a * t.y; x.z -= a * t.z; x.w -= a * t.w;
+    }
+    *reinterpret_cast<float4*>(&sm.t[32 + i][j]) = x;
+  }
+  __syncthreads();                    // A' is consumed: its bytes become the two bf16 operands
+  for (int i = tid; i < CK_C * CK_C / 2; i += 256) {
+    const int r = i >> 5, j = (i & 31) * 2;
+    const float2 t = *reinterpret_cast<const float2*>(&sm.t[r][j]);
+    const float b0 = t.x * sm.beta[j], b1 = t.y * sm.beta[j + 1];
+    *reinterpret_cast<uint32_t*>(&sm.tb[0][r][j]) = pack_bf16(b0, b1);
+    *reinterpret_cast<uint32_t*>(&sm.tb[1][r][j]) = pack_bf16(b0 * sm.eg[j], b1 * sm.eg[j + 1]);
+  }
+  __syncthreads();
+  // 5. u = (T beta) v, w = (T beta e^{gc}) k  (64 x 128 x 64): warp -> rows 16 (warp & 3), columns 64 (warp >> 2)
   {
     const int m0 = (warp & 3) * 16, nh = (warp >> 2) * 64;
     float uu[8][4], ww[8][4];
@@ -201,15 +279,18 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(GdnChunkParams p) {
       for (int i = 0; i < 4; ++i) uu[n][i] = ww[n][i] = 0.f;
 #pragma unroll
     for (int ks = 0; ks < CK_C / 16; ++ks) {
-      uint32_t a[4];
-      frag_a(&tb[0][0], CK_LT, m0, ks * 16, g, t4, a);
+      uint32_t a[4], aw[4];
+      frag_a(a, &sm.tb[0][0][0], CK_LT, m0, ks * 16, lane);
+      frag_a(aw, &sm.tb[1][0][0], CK_LT, m0, ks * 16, lane);
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        uint32_t bv[2], bk[2];
-        frag_b(&sm.vbT[0][0], CK_LT, nh + n * 8, ks * 16, g, t4, bv);
-        frag_b(&sm.kgT[0][0], CK_LT, nh + n * 8, ks * 16, g, t4, bk);
+      for (int n = 0; n < 8; n += 2) {
+        uint32_t bv[4], bk[4];
+        frag_bt(bv, &sm.v[0][0], CK_LD, nh + n * 8, ks * 16, lane);
+        frag_bt(bk, &sm.k[0][0], CK_LD, nh + n * 8, ks * 16, lane);
         mma_bf16(uu[n], a[0], a[1], a[2], a[3], bv[0], bv[1]);
-        mma_bf16(ww[n], a[0], a[1], a[2], a[3], bk[0], bk[1]);
+        mma_bf16(ww[n], aw[0], aw[1], aw[2], aw[3], bk[0], bk[1]);
+        mma_bf16(uu[n + 1], a[0], a[1], a[2], a[3], bv[2], bv[3]);
+        mma_bf16(ww[n + 1], aw[0], aw[1], aw[2], aw[3], bk[2], bk[3]);
       }
     }
 #pragma unroll
@@ -227,14 +308,14 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(GdnChunkParams p) {
 struct ScanBuf {
   __nv_bfloat16 w[CK_C][CK_LD];
   __nv_bfloat16 qg[CK_C][CK_LD];
-  __nv_bfloat16 kdT[CK_D][CK_LT];
+  __nv_bfloat16 kd[CK_C][CK_LD];
   __nv_bfloat16 attn[CK_C][CK_LT];
   float u[CK_C][CK_NC + 4];         // this CTA's 64 columns (fp32)
 };
 struct ScanSmem {
   ScanBuf buf[2];
-  __nv_bfloat16 sT[CK_NC][CK_LD];   // state^T as bf16: [value column][k]
-  __nv_bfloat16 vnT[CK_NC][CK_LT];  // v'^T: [value column][token]
+  __nv_bfloat16 s[CK_D][CK_LT];     // the state as bf16: [k][value column]
+  __nv_bfloat16 vn[CK_C][CK_LT];    // v': [token][value column]
 };
 __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
   extern __shared__ __align__(16) uint8_t ck_smem[];
@@ -249,8 +330,9 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int k = warp * 16 + g + half * 8, col = cb + n * 8 + 2 * t4;
-      S[n][half * 2] = p.use_state ? sp[(size_t)k * CK_D + col] : 0.f;
-      S[n][half * 2 + 1] = p.use_state ? sp[(size_t)k * CK_D + col + 1] : 0.f;
+      const float2 v = p.use_state ? *reinterpret_cast<const float2*>(sp + (size_t)k * CK_D + col) : make_float2(0.f, 0.f);
+      S[n][half * 2] = v.x;
+      S[n][half * 2 + 1] = v.y;
     }
   auto issue = [&](int c) {
     if (c < p.chunks) {
@@ -261,18 +343,12 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
         const size_t o = ((size_t)(r0 + t) * p.nv + h) * CK_D + piece;
         ck_cp16(&b.w[t][piece], p.w + o);
         ck_cp16(&b.qg[t][piece], p.qg + o);
+        ck_cp16(&b.kd[t][piece], p.kd + (((size_t)h * p.chunks + c) * CK_C + t) * CK_D + piece);
+        ck_cp16(&b.u[t][piece / 2], p.u + ((size_t)(r0 + t) * p.nv + h) * CK_D + cb + piece / 2);
       }
       for (int i = tid; i < CK_C * 8; i += 256) {
         const int t = i >> 3, piece = (i & 7) * 8;
         ck_cp16(&b.attn[t][piece], p.attn + (((size_t)h * p.chunks + c) * CK_C + t) * CK_C + piece);
-      }
-      for (int i = tid; i < CK_C * 16; i += 256) {
-        const int t = i >> 4, piece = (i & 15) * 4;
-        ck_cp16(&b.u[t][piece], p.u + ((size_t)(r0 + t) * p.nv + h) * CK_D + cb + piece);
-      }
-      for (int i = tid; i < CK_D * 8; i += 256) {
-        const int d = i >> 3, piece = (i & 7) * 8;
-        ck_cp16(&b.kdT[d][piece], p.kdT + (((size_t)h * p.chunks + c) * CK_D + d) * CK_C + piece);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -281,15 +357,13 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
   for (int c = 0; c < p.chunks; ++c) {
     ScanBuf& b = sm.buf[c & 1];
     const int r0 = c * CK_C;
-    // the state as the B operand of this chunk
+    const float eg = p.eglast[(size_t)h * p.chunks + c];
+    // the state as the B operand of this chunk (the last reads of s are two barriers back)
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int k = warp * 16 + g + half * 8, col = n * 8 + 2 * t4;
-        sm.sT[col][k] = __float2bfloat16(S[n][half * 2]);
-        sm.sT[col + 1][k] = __float2bfloat16(S[n][half * 2 + 1]);
-      }
+      for (int half = 0; half < 2; ++half)
+        *reinterpret_cast<uint32_t*>(&sm.s[warp * 16 + g + half * 8][n * 8 + 2 * t4]) = pack_bf16(S[n][half * 2], S[n][half * 2 + 1]);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                 // chunk c and the state copy are visible; everyone is done with chunk c - 1
     issue(c + 1);
@@ -303,14 +377,16 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
 #pragma unroll
     for (int ks = 0; ks < CK_D / 16; ++ks) {
       uint32_t aw[4], aq[4];
-      frag_a(&b.w[0][0], CK_LD, m0, ks * 16, g, t4, aw);
-      frag_a(&b.qg[0][0], CK_LD, m0, ks * 16, g, t4, aq);
+      frag_a(aw, &b.w[0][0], CK_LD, m0, ks * 16, lane);
+      frag_a(aq, &b.qg[0][0], CK_LD, m0, ks * 16, lane);
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        uint32_t bs[2];
-        frag_b(&sm.sT[0][0], CK_LD, nh + n * 8, ks * 16, g, t4, bs);
+      for (int n = 0; n < 4; n += 2) {
+        uint32_t bs[4];
+        frag_bt(bs, &sm.s[0][0], CK_LT, nh + n * 8, ks * 16, lane);
         mma_bf16(pv[n], aw[0], aw[1], aw[2], aw[3], bs[0], bs[1]);
         mma_bf16(ov[n], aq[0], aq[1], aq[2], aq[3], bs[0], bs[1]);
+        mma_bf16(pv[n + 1], aw[0], aw[1], aw[2], aw[3], bs[2], bs[3]);
+        mma_bf16(ov[n + 1], aq[0], aq[1], aq[2], aq[3], bs[2], bs[3]);
       }
     }
 #pragma unroll
@@ -319,20 +395,33 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
       for (int half = 0; half < 2; ++half) {
         const int i = m0 + g + half * 8, col = nh + n * 8 + 2 * t4;
         const float2 uw = *reinterpret_cast<const float2*>(&b.u[i][col]);
-        sm.vnT[col][i] = __float2bfloat16(uw.x - pv[n][half * 2]);
-        sm.vnT[col + 1][i] = __float2bfloat16(uw.y - pv[n][half * 2 + 1]);
+        *reinterpret_cast<uint32_t*>(&sm.vn[i][col]) = pack_bf16(uw.x - pv[n][half * 2], uw.y - pv[n][half * 2 + 1]);
       }
     __syncthreads();
-    // o += attn v'  (K = 64 tokens)
+    // S <- e^{gc_last} S + (e^{gc_last - gc} k)^T v': warp -> state rows 16 warp .. +15, all 64 columns
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) S[n][i] *= eg;
+    // and o += attn v'  (K = 64 tokens)
 #pragma unroll
     for (int ks = 0; ks < CK_C / 16; ++ks) {
-      uint32_t a[4];
-      frag_a(&b.attn[0][0], CK_LT, m0, ks * 16, g, t4, a);
+      uint32_t a[4], ak[4];
+      frag_at(ak, &b.kd[0][0], CK_LD, warp * 16, ks * 16, lane);
+      frag_a(a, &b.attn[0][0], CK_LT, m0, ks * 16, lane);
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        uint32_t bv[2];
-        frag_b(&sm.vnT[0][0], CK_LT, nh + n * 8, ks * 16, g, t4, bv);
+      for (int n = 0; n < 8; n += 2) {
+        uint32_t bv[4];
+        frag_bt(bv, &sm.vn[0][0], CK_LT, n * 8, ks * 16, lane);
+        mma_bf16(S[n], ak[0], ak[1], ak[2], ak[3], bv[0], bv[1]);
+        mma_bf16(S[n + 1], ak[0], ak[1], ak[2], ak[3], bv[2], bv[3]);
+      }
+#pragma unroll
+      for (int n = 0; n < 4; n += 2) {
+        uint32_t bv[4];
+        frag_bt(bv, &sm.vn[0][0], CK_LT, nh + n * 8, ks * 16, lane);
         mma_bf16(ov[n], a[0], a[1], a[2], a[3], bv[0], bv[1]);
+        mma_bf16(ov[n + 1], a[0], a[1], a[2], a[3], bv[2], bv[3]);
       }
     }
 #pragma unroll
@@ -344,24 +433,6 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
           *reinterpret_cast<float2*>(p.raw + (size_t)r * V + h * CK_D + cb + nh + n * 8 + 2 * t4) =
               make_float2(ov[n][half * 2], ov[n][half * 2 + 1]);
       }
-    // S <- e^{gc_last} S + (e^{gc_last - gc} k)^T v': warp -> state rows 16 warp .. +15, all 64 columns
-    const float eg = p.eglast[(size_t)h * p.chunks + c];
-#pragma unroll
-    for (int n = 0; n < 8; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) S[n][i] *= eg;
-#pragma unroll
-    for (int ks = 0; ks < CK_C / 16; ++ks) {
-      uint32_t a[4];
-      frag_a(&b.kdT[0][0], CK_LT, warp * 16, ks * 16, g, t4, a);
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        uint32_t bv[2];
-        frag_b(&sm.vnT[0][0], CK_LT, n * 8, ks * 16, g, t4, bv);
-        mma_bf16(S[n], a[0], a[1], a[2], a[3], bv[0], bv[1]);
-      }
-    }
-    __syncthreads();                 // all reads of sT and vnT are done before the next chunk rewrites them
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
@@ -410,8 +481,8 @@ OWL_API int owl_gdn_chunk_scan(const void* qkv, const void* ab, int ldab, const 
   auto* base = reinterpret_cast<__nv_bfloat16*>(work);
   p.u = reinterpret_cast<float*>(base);                 // 2 * rows bf16-sized elements
   p.w = base + 2 * rows; p.qg = base + 3 * rows;
-  p.kdT = base + 4 * rows;
-  p.attn = p.kdT + (size_t)nv * p.chunks * CK_D * CK_C;
+  p.kd = base + 4 * rows;
+  p.attn = p.kd + (size_t)nv * p.chunks * CK_D * CK_C;
   p.eglast = reinterpret_cast<float*>(p.attn + (size_t)nv * p.chunks * CK_C * CK_C);
   gdn_chunk_prep_kernel<<<dim3(p.chunks, nv), 256, sizeof(PrepSmem), st>>>(p);
   OWL_LAUNCH_CHECK();

@@ -110,11 +110,15 @@ __device__ __forceinline__ uint32_t gd_ld_acquire_sys(const uint32_t* p) {
   return v;
 }
 
-// silu(gate) * up of 16 columns (8 gate, 8 up) -> 8 fp16 values
+// silu(gate) * up of 16 columns (8 gate, 8 up) -> 8 fp16 values. Gate and up are rounded to bf16 first: the bits are those of the
+// product stored and activated by a second kernel, whichever of the two forms a shape takes.
 __device__ __forceinline__ uint4 gd_silu8(const float* v) {
   float y[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) y[i] = fminf(fmaxf(silu_f(v[i]) * v[8 + i], -65504.f), 65504.f);
+  for (int i = 0; i < 8; ++i) {
+    const float g = __bfloat162float(__float2bfloat16(v[i])), u = __bfloat162float(__float2bfloat16(v[8 + i]));
+    y[i] = fminf(fmaxf(silu_f(g) * u, -65504.f), 65504.f);
+  }
   return make_uint4(pack_f16(y[0], y[1]), pack_f16(y[2], y[3]), pack_f16(y[4], y[5]), pack_f16(y[6], y[7]));
 }
 
