@@ -8,15 +8,16 @@
 //   S  <- e^{gc_last} S + (e^{gc_last - gc} k)^T v'
 // (every exponential has a non-positive argument). Two kernels:
 //   gdn_chunk_prep_kernel  one CTA per (chunk, v-head), all chunks in parallel: the 64x64 products and the two 64x128
-//                          products on mma.sync (bf16 in, fp32 accumulate), the triangular inverse in fp32 by blocks (16 x 16
-//                          by substitution, then two doublings); writes w, u, scaled q, scaled k and attn
+//                          products on mma.sync (bf16 in, fp32 accumulate), the triangular inverse by forward substitution
+//                          with four threads per column; writes w, u, scaled q, scaled k and attn
 //   gdn_chunk_scan_kernel  one CTA per (v-head, half of the value columns), the chunks in order: three small tensor-core
 //                          products per chunk against the fp32 state kept in MMA accumulator registers (a bf16 copy in
 //                          shared memory is the B operand), operands prefetched one chunk ahead with cp.async
 // Every tile stays in the row order it has in global memory; the products that need it the other way round read it with
 // ldmatrix.trans. Before that the tiles were transposed through shared memory (8-way bank conflicts) and the fragments
 // fetched word by word, and the inverse ran one column per thread through 2016 dependent steps: 168 us (preparation) and
-// 117 us (recurrence) a layer at 2048 tokens x 48 heads; memory traffic would take 31 and 20 us.
+// 117 us (recurrence) a layer at 2048 tokens x 48 heads; memory traffic would take 31 and 20 us. The operands, their rounding
+// and the order of every sum are those of that form: the outputs are the same bits.
 // followed by the gated RMSNorm kernel of gdn.cu. q and k arrive l2-normalised from the convolution kernel.
 //
 // Reference counterpart: the chunk-64 delta-rule kernels (cumsum, kkt, solve_tril, wu, h, o) that the reference compiles
@@ -81,19 +82,23 @@ struct GdnChunkParams {
 
 // ---- preparation: one CTA per (chunk, v-head), 256 threads, three CTAs per SM -------------------------------------------
 struct PrepSmem {
-  __nv_bfloat16 k[CK_C][CK_LD];
-  __nv_bfloat16 v[CK_C][CK_LD];
+  __nv_bfloat16 k[CK_C][CK_LD];       // k rows, later beta e^{gc} k
+  __nv_bfloat16 v[CK_C][CK_LD];       // v rows, then beta v
   union {
     __nv_bfloat16 q[CK_C][CK_LD];
-    float t[CK_C][CK_C + 4];          // T = (I + A')^-1 (q is consumed by then)
+    __nv_bfloat16 tb[CK_C][CK_LT];    // T as bf16 (q is consumed by then)
   };
-  union {
-    float a[CK_C][CK_C + 4];          // A' (strictly lower)
-    __nv_bfloat16 tb[2][CK_C][CK_LT]; // T diag(beta), T diag(beta e^{gc})
-  };
-  float x[32][36];
-  float gc[CK_C], beta[CK_C], eg[CK_C], el[CK_C];       // el: e^{gc_last - gc}
+  float at[CK_C][CK_C + 4];           // A'^T (column j of A' is row j)
+  float g[CK_C], gc[CK_C], beta[CK_C], eg[CK_C], el[CK_C];       // eg: e^{gc}, el: e^{gc_last - gc}
 };
+__device__ __forceinline__ uint4 scale_bf16x8(const uint4& u, float s) {
+  return make_uint4(pack_bf16(bf16_lo(u.x) * s, bf16_hi(u.x) * s), pack_bf16(bf16_lo(u.y) * s, bf16_hi(u.y) * s),
+                    pack_bf16(bf16_lo(u.z) * s, bf16_hi(u.z) * s), pack_bf16(bf16_lo(u.w) * s, bf16_hi(u.w) * s));
+}
+__device__ __forceinline__ uint4 scale2_bf16x8(const uint4& u, float s, float e) {      // (x s) e
+  return make_uint4(pack_bf16(bf16_lo(u.x) * s * e, bf16_hi(u.x) * s * e), pack_bf16(bf16_lo(u.y) * s * e, bf16_hi(u.y) * s * e),
+                    pack_bf16(bf16_lo(u.z) * s * e, bf16_hi(u.z) * s * e), pack_bf16(bf16_lo(u.w) * s * e, bf16_hi(u.w) * s * e));
+}
 __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkParams p) {
   extern __shared__ __align__(16) uint8_t ck_smem[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(ck_smem);
@@ -117,48 +122,48 @@ __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkParams p
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
-  if (warp == 0) {                    // two tokens per lane, inclusive sums by shuffles
-    float gg[2], acc = 0.f;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int r = r0 + 2 * lane + e;
-      gg[e] = 0.f;
-      float bb = 0.f;
-      if (r < p.T) {
-        const float a = __bfloat162float(p.ab[(size_t)r * p.ldab + h]);
-        const float b = __bfloat162float(p.ab[(size_t)r * p.ldab + p.nv + h]);
-        gg[e] = -__expf(p.a_log[h]) * softplus_f(a + p.dt_bias[h]);
-        bb = sigmoid_f(b);
-      }
-      sm.beta[2 * lane + e] = bb;
-      acc += gg[e];
+  if (tid < CK_C) {
+    const int r = r0 + tid;
+    float gg = 0.f, bb = 0.f;
+    if (r < p.T) {
+      const float a = __bfloat162float(p.ab[(size_t)r * p.ldab + h]);
+      const float b = __bfloat162float(p.ab[(size_t)r * p.ldab + p.nv + h]);
+      gg = -__expf(p.a_log[h]) * softplus_f(a + p.dt_bias[h]);
+      bb = sigmoid_f(b);
     }
-    float sum = acc;
+    sm.g[tid] = gg;
+    sm.beta[tid] = bb;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    float4 gv[CK_C / 4];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float n = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= o) sum += n;
+    for (int i = 0; i < CK_C / 4; ++i) gv[i] = *reinterpret_cast<const float4*>(&sm.g[i * 4]);
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < CK_C / 4; ++i) {
+      float4 o;
+      acc += gv[i].x; o.x = acc; acc += gv[i].y; o.y = acc; acc += gv[i].z; o.z = acc; acc += gv[i].w; o.w = acc;
+      *reinterpret_cast<float4*>(&sm.gc[i * 4]) = o;
     }
-    const float last = __shfl_sync(0xffffffffu, sum, 31);
-    const float g0 = sum - gg[1], g1 = sum;
-    sm.gc[2 * lane] = g0; sm.gc[2 * lane + 1] = g1;
-    sm.eg[2 * lane] = __expf(g0); sm.eg[2 * lane + 1] = __expf(g1);
-    sm.el[2 * lane] = __expf(last - g0); sm.el[2 * lane + 1] = __expf(last - g1);
-    if (lane == 0) p.eglast[(size_t)h * p.chunks + c] = __expf(last);
+    p.eglast[(size_t)h * p.chunks + c] = __expf(acc);
+  }
+  __syncthreads();
+  if (tid < CK_C) {
+    sm.eg[tid] = __expf(sm.gc[tid]);
+    sm.el[tid] = __expf(sm.gc[CK_C - 1] - sm.gc[tid]);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  // 2. scaled q rows and scaled k rows to global
+  // 2. scaled q rows and scaled k rows to global, beta v in place
   for (int i = tid; i < CK_C * 16; i += 256) {
     const int t = i >> 4, d = (i & 15) * 8;
-    const uint4 qu = *reinterpret_cast<const uint4*>(&sm.q[t][d]), ku = *reinterpret_cast<const uint4*>(&sm.k[t][d]);
-    const float e = scale * sm.eg[t], l = sm.el[t];
     *reinterpret_cast<uint4*>(p.qg + ((size_t)(r0 + t) * p.nv + h) * CK_D + d) =
-        make_uint4(pack_bf16(bf16_lo(qu.x) * e, bf16_hi(qu.x) * e), pack_bf16(bf16_lo(qu.y) * e, bf16_hi(qu.y) * e),
-                   pack_bf16(bf16_lo(qu.z) * e, bf16_hi(qu.z) * e), pack_bf16(bf16_lo(qu.w) * e, bf16_hi(qu.w) * e));
+        scale_bf16x8(*reinterpret_cast<const uint4*>(&sm.q[t][d]), scale * sm.eg[t]);
     *reinterpret_cast<uint4*>(p.kd + (((size_t)h * p.chunks + c) * CK_C + t) * CK_D + d) =
-        make_uint4(pack_bf16(bf16_lo(ku.x) * l, bf16_hi(ku.x) * l), pack_bf16(bf16_lo(ku.y) * l, bf16_hi(ku.y) * l),
-                   pack_bf16(bf16_lo(ku.z) * l, bf16_hi(ku.z) * l), pack_bf16(bf16_lo(ku.w) * l, bf16_hi(ku.w) * l));
+        scale_bf16x8(*reinterpret_cast<const uint4*>(&sm.k[t][d]), sm.el[t]);
+    uint4* v = reinterpret_cast<uint4*>(&sm.v[t][d]);
+    *v = scale_bf16x8(*v, sm.beta[t]);
   }
   // 3. k k^T and q k^T (64 x 64 x 128): warp -> rows 16 (warp & 3), columns 32 (warp >> 2)
   {
@@ -194,82 +199,47 @@ __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkParams p
         for (int e = 0; e < 2; ++e) {
           const int jj = j + e;
           const float dec = jj <= i ? __expf(sm.gc[i] - sm.gc[jj]) : 0.f;
-          sm.a[i][jj] = jj < i ? sm.beta[i] * kk[n][half * 2 + e] * dec : 0.f;
+          sm.at[jj][i] = jj < i ? sm.beta[i] * kk[n][half * 2 + e] * dec : 0.f;
           av[e] = scale * qk[n][half * 2 + e] * dec;
         }
         *reinterpret_cast<uint32_t*>(at + i * CK_C + j) = pack_bf16(av[0], av[1]);
       }
   }
-  __syncthreads();                    // q is consumed: its bytes become T
-  // 4. T = (I + A')^-1, fp32. The four 16 x 16 diagonal blocks by forward substitution (a column per thread) ...
-  for (int i = tid; i < CK_C * (CK_C + 4) / 4; i += 256) reinterpret_cast<float4*>(&sm.t[0][0])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  __syncthreads();
-  if (tid < CK_C) {
-    const int b = tid & ~15, cc = tid & 15;
-    float col[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float acc = (i == cc) ? 1.f : 0.f;
-#pragma unroll
-      for (int j = 0; j < i; ++j) acc -= sm.a[b + i][b + j] * col[j];
-      col[i] = acc;
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) sm.t[b + i][b + cc] = col[i];
+  __syncthreads();                    // q and k rows are consumed
+  for (int i = tid; i < CK_C * 16; i += 256) {
+    const int t = i >> 4, d = (i & 15) * 8;
+    uint4* k = reinterpret_cast<uint4*>(&sm.k[t][d]);
+    *k = scale2_bf16x8(*k, sm.beta[t], sm.eg[t]);
   }
-  __syncthreads();
-  // ... then T21 = -T22 (A21 T11), for the two pairs of 16 and the pair of 32
+  // 4. T = (I + A')^-1 by forward substitution. Four threads share column c; thread r holds rows 16 q + 4 r + e. When row j is
+  // final, its holder tells the other three, and every later row takes its term: per element the terms come in order of j.
   {
-    const int i = tid >> 4, j = tid & 15;
-    float x0 = 0.f, x1 = 0.f;
+    const int cc = tid >> 2, r = tid & 3;
+    float acc[4][4];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      x0 += sm.a[16 + i][k] * sm.t[k][j];
-      x1 += sm.a[48 + i][32 + k] * sm.t[32 + k][32 + j];
-    }
-    sm.x[i][j] = x0;
-    sm.x[16 + i][j] = x1;
-    __syncthreads();
-    x0 = x1 = 0.f;
+    for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      x0 -= sm.t[16 + i][16 + k] * sm.x[k][j];
-      x1 -= sm.t[48 + i][48 + k] * sm.x[16 + k][j];
+      for (int e = 0; e < 4; ++e) acc[q][e] = (16 * q + 4 * r + e == cc) ? 1.f : 0.f;
+#pragma unroll
+    for (int j = 0; j < CK_C - 1; ++j) {
+      const float x = __shfl_sync(0xffffffffu, acc[j >> 4][j & 3], (lane & ~3) | ((j >> 2) & 3));
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (16 * q + 15 <= j) continue;
+        const float4 a = *reinterpret_cast<const float4*>(&sm.at[j][16 * q + 4 * r]);
+        const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (16 * q > j || 16 * q + 4 * r + e > j) acc[q][e] -= av[e] * x;
+      }
     }
-    sm.t[16 + i][j] = x0;
-    sm.t[48 + i][32 + j] = x1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sm.tb[16 * q + 4 * r + e][cc] = __float2bfloat16(acc[q][e]);
   }
   __syncthreads();
-  {
-    const int i = tid >> 3, j = (tid & 7) * 4;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-      const float a = sm.a[32 + i][k];
-      const float4 t = *reinterpret_cast<const float4*>(&sm.t[k][j]);
-      x.x += a * t.x; x.y += a * t.y; x.z += a * t.z; x.w += a * t.w;
-    }
-    *reinterpret_cast<float4*>(&sm.x[i][j]) = x;
-    __syncthreads();
-    x = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-      const float a = sm.t[32 + i][32 + k];
-      const float4 t = *reinterpret_cast<const float4*>(&sm.x[k][j]);
-      x.x -= a * t.x; x.y -= a * t.y; x.z -= a * t.z; x.w -= a * t.w;
-    }
-    *reinterpret_cast<float4*>(&sm.t[32 + i][j]) = x;
-  }
-  __syncthreads();                    // A' is consumed: its bytes become the two bf16 operands
-  for (int i = tid; i < CK_C * CK_C / 2; i += 256) {
-    const int r = i >> 5, j = (i & 31) * 2;
-    const float2 t = *reinterpret_cast<const float2*>(&sm.t[r][j]);
-    const float b0 = t.x * sm.beta[j], b1 = t.y * sm.beta[j + 1];
-    *reinterpret_cast<uint32_t*>(&sm.tb[0][r][j]) = pack_bf16(b0, b1);
-    *reinterpret_cast<uint32_t*>(&sm.tb[1][r][j]) = pack_bf16(b0 * sm.eg[j], b1 * sm.eg[j + 1]);
-  }
-  __syncthreads();
-  // 5. u = (T beta) v, w = (T beta e^{gc}) k  (64 x 128 x 64): warp -> rows 16 (warp & 3), columns 64 (warp >> 2)
+  // 5. u = T (beta v), w = T (beta e^{gc} k)  (64 x 128 x 64): warp -> rows 16 (warp & 3), columns 64 (warp >> 2)
   {
     const int m0 = (warp & 3) * 16, nh = (warp >> 2) * 64;
     float uu[8][4], ww[8][4];
@@ -279,18 +249,17 @@ __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkParams p
       for (int i = 0; i < 4; ++i) uu[n][i] = ww[n][i] = 0.f;
 #pragma unroll
     for (int ks = 0; ks < CK_C / 16; ++ks) {
-      uint32_t a[4], aw[4];
-      frag_a(a, &sm.tb[0][0][0], CK_LT, m0, ks * 16, lane);
-      frag_a(aw, &sm.tb[1][0][0], CK_LT, m0, ks * 16, lane);
+      uint32_t a[4];
+      frag_a(a, &sm.tb[0][0], CK_LT, m0, ks * 16, lane);
 #pragma unroll
       for (int n = 0; n < 8; n += 2) {
         uint32_t bv[4], bk[4];
         frag_bt(bv, &sm.v[0][0], CK_LD, nh + n * 8, ks * 16, lane);
         frag_bt(bk, &sm.k[0][0], CK_LD, nh + n * 8, ks * 16, lane);
         mma_bf16(uu[n], a[0], a[1], a[2], a[3], bv[0], bv[1]);
-        mma_bf16(ww[n], aw[0], aw[1], aw[2], aw[3], bk[0], bk[1]);
+        mma_bf16(ww[n], a[0], a[1], a[2], a[3], bk[0], bk[1]);
         mma_bf16(uu[n + 1], a[0], a[1], a[2], a[3], bv[2], bv[3]);
-        mma_bf16(ww[n + 1], aw[0], aw[1], aw[2], aw[3], bk[2], bk[3]);
+        mma_bf16(ww[n + 1], a[0], a[1], a[2], a[3], bk[2], bk[3]);
       }
     }
 #pragma unroll

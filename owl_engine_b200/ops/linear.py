@@ -203,6 +203,4 @@ def dense_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, arm: str = "
             cache = w.to(x.dtype)
             w._owl_cast = cache
         w = cache
-    # few weight rows (the 96 of the a / b projection): the persistent kernel cuts k so that every SM has a part (2048 tokens:
-    # 37 us on the 16 tiles of the other kernel)
-    return gemm_tc.f16_gemm(x, w, out, force_persist=x.shape[0] >= 256)
+    return gemm_tc.f16_gemm(x, w, out)
