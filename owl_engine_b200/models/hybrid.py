@@ -646,10 +646,10 @@ class HybridRunner:
         if self.uniform_rows:
             b = 8        # a speculating engine: the split of the keys (and with it the order of the partial sums) must not
                          # depend on how many sequences share the step, or batched verify rows round differently from plain ones
-        # four CTAs per SM: a CTA walks its keys one page after the other and is bound by their latency, and with sequences of
-        # unequal lengths the longest part is what the launch takes
-        want = max(1, (4 * 148) // max(1, b * self.spec.hkv))
-        return max(1, min(self.max_splits * self.MAX_ROWS // max(b, 8), want, (pages + 3) // 4))
+        # two CTAs per SM, four for many sequences: with unequal lengths the longest part is what the launch takes (32 sequences of
+        # 1k to 8k tokens: 125 against 149 us a layer; 8 sequences: 24 against 20, the parts get too short)
+        want = max(1, ((4 if b >= 16 else 2) * 148) // max(1, b * self.spec.hkv))
+        return max(1, min(self.max_splits, want, (pages + 3) // 4))
 
     def _full(self, lw: LayerWeights, li: int, lay: StepLayout, v: dict, splits: int, ctx_hint: int = 0) -> None:
         sp, m = self.spec, lay.m
