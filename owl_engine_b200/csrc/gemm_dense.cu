@@ -392,6 +392,24 @@ constexpr int GD_MAX_DEV = 64;
 static float* g_ks_scratch[GD_MAX_DEV] = {nullptr};
 static size_t g_ks_scratch_bytes[GD_MAX_DEV] = {0};
 
+namespace owl {
+// The split-k scratch registered for the current device (null: none), and the sum of fp32 k parts [ks][T][ldp] (gemm_w4.cu).
+float* gd_split_scratch(size_t* bytes) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= GD_MAX_DEV) return nullptr;
+  *bytes = g_ks_scratch_bytes[dev];
+  return g_ks_scratch[dev];
+}
+int gd_split_reduce(const float* partial, void* out, int T, int N, int ldp, int ldo, int ks, int silu, cudaStream_t st) {
+  if (silu)
+    gemm_ksplit_silu_kernel<<<dim3((N + 4095) / 4096, T), 256, 0, st>>>(partial, (__nv_bfloat16*)out, T, N, ldp, ldo, ks);
+  else
+    gemm_ksplit_reduce_kernel<<<dim3((N + 1023) / 1024, T), 256, 0, st>>>(partial, (__nv_bfloat16*)out, T, N, ldp, ldo, ks);
+  OWL_LAUNCH_CHECK();
+  return OWL_OK;
+}
+}  // namespace owl
+
 static int gd_launch(const void* x, int ldx, const void* w, int ldw, GdParams& p, int mode, cudaStream_t st) {
   const int kmask = p.fmt == 2 ? 127 : 63, ldmask = p.fmt == 2 ? 15 : 7;
   if (p.T < 1 || p.N < 1 || p.K <= kmask || (p.K & kmask) || (ldx & ldmask) || (ldw & ldmask) || (p.ldo & 7) || p.fmt < 0 ||

@@ -63,6 +63,14 @@ def _fp8_scratch(tag: str, r: int, k: int, device):
     return buf[0][:r * k].view(r, k), buf[1][:r]
 
 
+def _rows_ok(w, x: torch.Tensor, out: torch.Tensor) -> bool:
+    """Up to 256 rows of fp16: one launch reads the int4 records and dequantises each weight once."""
+    from . import gemm_tc
+
+    return w.layout == "slice" and x.dtype == torch.float16 and x.shape[0] <= gemm_tc.ROWS_UPTO and x.stride(0) % 8 == 0 \
+        and out.stride(0) % 8 == 0 and (x.data_ptr() | out.data_ptr()) % 16 == 0
+
+
 def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.Tensor:
     arm = "tc" if arm == "tc4" else arm                    # the 4-bit float product exists for NVFP4 weights only
     if arm == "baseline":
@@ -89,6 +97,8 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.Ten
             K.act_pack(xb, xp, xs, t, k, w.group | K.ACT_FRAG)
             K.w4_mma(w, xp, xs, out, t, ldo=out.stride(0))
             return out
+        if _rows_ok(w, x, out):
+            return gemm_tc.w4_gemm_rows(w, x, out)
         if x.shape[0] >= DEQUANT_FROM:
             return gemm_tc.f16_gemm(x, w4_dense(w, x.dtype, x.device, resident=resident), out)
         return gemm_tc.w4a16_gemm(w, x, out)
@@ -124,6 +134,9 @@ def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> bool
         wq, sw = _e4m3_weight(w, x.device, arm == "tc8r")
         xq, sx = gemm_tc.quant_e4m3_rows(x, *_fp8_scratch("x", t, w.k, x.device))
         gemm_tc.gemm_silu(xq, wq, out, sx, sw)
+        return True
+    if arm in ("tc", "tc4", "tcr", "tc8", "tc8r") and t > SKINNY_UPTO and _rows_ok(w, x, out):
+        gemm_tc.w4_gemm_rows(w, x, out, silu=True)
         return True
     if arm in ("tc", "tc4", "tcr", "tc8", "tc8r") and t >= SILU_FROM and w.n >= 512:
         gemm_tc.gemm_silu(x, w4_dense(w, x.dtype, x.device, resident=arm in ("tcr", "tc8r")), out)

@@ -109,3 +109,30 @@ def test_gate_up_with_activation_matches_two_steps():
             two = torch.empty_like(out)
             K.silu_mul(gu, t, 512, out=two)
             assert torch.equal(out, two)
+
+
+# every token width of the MMA (64, 128, 192, 256) at its edges; one row tile, a last row block of 1 to 7 tiles, slices of unequal
+# length, and row counts that are cut along k (K from 1024 on)
+@pytest.mark.parametrize("t", [1, 64, 65, 137, 192, 256])
+@pytest.mark.parametrize("n,k", [(16, 128), (144, 384), (1040, 2176), (5120, 1024), (20480, 128)])
+@pytest.mark.parametrize("group", [128, 32])
+def test_rows_gemm_dequantises_once(t, n, k, group):
+    gen = torch.Generator().manual_seed(n + k + t)
+    c = Q.quantize_w4(torch.randn(n, k, generator=gen) * 0.05, group)
+    if t == 65:
+        c.zeros.add_(0.3)          # fractional zero points, as converted Q4_K blocks have
+    w = Q.pack_skinny(c).to(DEV)
+    x = torch.randn(t, k, generator=gen).half().to(DEV)
+    dense = K.w4_dequant(w, torch.empty(n, k, dtype=torch.float16, device=DEV)).double()
+    want = x.double() @ dense.t()
+    out = torch.zeros(t, n + 8, dtype=torch.bfloat16, device=DEV)
+    gemm_tc.w4_gemm_rows(w, x, out)
+    # bf16 result + fp32 sums of products of the same fp16 weights
+    size = x.double().abs() @ dense.abs().t()
+    assert (out[:, n:] == 0).all()
+    assert ((out[:, :n].double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -18).all()
+    act = torch.zeros(t, n // 2 + 8, dtype=torch.float16, device=DEV)
+    gemm_tc.w4_gemm_rows(w, x, act, silu=True)
+    assert (act[:, n // 2:] == 0).all()
+    torch.testing.assert_close(act[:, :n // 2].float(), _silu_ref(out[:, :n].contiguous()).float(), rtol=2.0 ** -9, atol=2.0 ** -20)
+    assert K.all_status()["gemm_w4"] == 0
