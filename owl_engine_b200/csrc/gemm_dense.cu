@@ -82,7 +82,7 @@ __device__ __forceinline__ bool gd_wait(uint64_t* bar, uint32_t parity, GdCtl* c
 // The producer's and the MMA issuer's waits: one thread each, polling with test_wait (a suspended thread's wake-up adds to
 // every stage's round trip).
 __device__ __forceinline__ bool gd_spin(uint64_t* bar, uint32_t parity, GdCtl* c, int code) {
-  uint64_t t0 = 0;                          // the clock is read only when there is something to wait for
+  uint64_t t0 = 0;                          // reading the clock takes about as long as a stage: not before a thousand polls
   for (uint32_t i = 0;; ++i) {
     uint32_t ok;
     asm volatile(
@@ -91,10 +91,10 @@ __device__ __forceinline__ bool gd_spin(uint64_t* bar, uint32_t parity, GdCtl* c
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     if (ok) return true;
-    if (i == 0) t0 = global_ns();
-    if ((i & 63u) == 63u) {
+    if ((i & 1023u) == 1023u) {
       if (c->abort_flag) return false;
-      if (wait_expired(t0)) break;
+      if (t0 == 0) t0 = global_ns();
+      else if (wait_expired(t0)) break;
     }
   }
   c->abort_flag = 1;
