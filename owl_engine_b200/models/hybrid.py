@@ -341,6 +341,7 @@ class HybridRunner:
         self.fuse_norm = os.environ.get("OWL_FUSE_NORM", "0") == "1"
         self._norm_count = None
         self._attn_ws = None         # scratch of the GEMM-form prefill attention
+        self._ahead = None           # dequantisation one projection ahead (long chunks)
         # decode activations: 15-bit fixed point (exact for bf16 inputs up to rounding at 2^-14 of the group maximum), or 8
         # bits per group (the W4A8 decode arm: half the integer products per weight byte)
         self.act_bits = int(os.environ.get("OWL_ACT_BITS", "15"))
@@ -981,13 +982,27 @@ class HybridRunner:
         self._pf = ws
         return ws
 
-    def _gemm(self, w, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    def _gemm(self, w, x: torch.Tensor, out: torch.Tensor, ahead=None) -> torch.Tensor:
         """out[T, N] = x[T, K] @ dequant(w)^T for a prefill chunk."""
         from ..ops import linear
 
         if w.layout == "nvfp4":
             return linear.nvfp4_gemm(w, x, out, arm=self.prefill_gemm)
-        return linear.w4_gemm(w, x, out, arm=self.prefill_gemm)
+        return linear.w4_gemm(w, x, out, arm=self.prefill_gemm, ahead=ahead)
+
+    def _dequant_ahead(self, t: int):
+        """The ``DequantAhead`` of a ``t``-row chunk, started on this model's weights, or None: chunks above the sizes that read
+        the int4 records directly, on the arm that dequantises per chunk."""
+        from ..ops import gemm_tc, linear
+
+        if self.prefill_gemm not in ("tc", "tc4") or t <= gemm_tc.ROWS_UPTO or self.w.layout not in ("slice", "block") or not self.w.layers \
+                or torch.cuda.is_current_stream_capturing():
+            return None
+        if self._ahead is None:
+            self._ahead = linear.DequantAhead(self.device)
+        order = [w for lw in self.w.layers
+                 for w in ((lw.qkvz, lw.out_proj) if lw.kind == "gdn" else (lw.qkv, lw.o_proj)) + (lw.gate_up, lw.down)]
+        return self._ahead if self._ahead.start(order) else None
 
     def _gdn_prefill(self, lw, gi: int, wide, nq: int, ab, conv, mix, t: int, gdn_slot: int, use_state: bool, snap) -> None:
         """Convolution + delta-rule scan of one GDN layer over the chunk's rows. With ``snap = (rows, state_row)`` the
@@ -1044,22 +1059,23 @@ class HybridRunner:
             h.copy_(embeds)
         fi = gi = 0
         use_state = pos0 > 0
+        ahead = self._dequant_ahead(t)
         y = None                    # the last MLP's output, not yet added to h: the next norm adds it on its way
         for i, lw in enumerate(self.w.layers):
             K.rmsnorm_pack(h, lw.ln1, delta=y, out_h=h if y is not None else None, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps)
             if lw.kind == "gdn":
                 nq = sp.conv_dim + sp.value_dim
                 wide = ws["wide"].view(-1)[:t * nq].view(t, nq)
-                self._gemm(lw.qkvz, x, wide)
+                self._gemm(lw.qkvz, x, wide, ahead)
                 ab = ws["ab"][:t]
                 linear.dense_gemm(x, lw.ab_dense, ab, arm="baseline" if self.prefill_gemm == "baseline" else "tc")
                 mix = ws["mix"].view(-1)[:t * sp.value_dim].view(t, sp.value_dim)
                 self._gdn_prefill(lw, gi, wide, nq, ab, ws["conv"][:t], mix, t, gdn_slot, use_state, snap)
-                self._gemm(lw.out_proj, mix, ws["y"][:t])
+                self._gemm(lw.out_proj, mix, ws["y"][:t], ahead)
                 gi += 1
             else:
                 wide = ws["wide"].view(-1)[:t * self.qkv_n].view(t, self.qkv_n)
-                self._gemm(lw.qkv, x, wide)
+                self._gemm(lw.qkv, x, wide, ahead)
                 qn = 2 * sp.hq * sp.hd
                 K.qknorm_rope_insert(wide, self.qkv_n, wide[:, qn:], self.qkv_n, wide[:, qn + sp.hkv * sp.hd:],
                                      self.qkv_n, lw.q_norm, lw.k_norm, pos3_v, self.inv_freq, self.section, kv_slot,
@@ -1067,16 +1083,16 @@ class HybridRunner:
                                      sp.eps, self.rope_scale, scales=pool.scales(fi))
                 mix = ws["mix"].view(-1)[:t * sp.hq * sp.hd].view(t, sp.hq * sp.hd)
                 self._prefill_attention(ws, pool, fi, wide, mix, t, pos0, seq_row, ng, tail)
-                self._gemm(lw.o_proj, mix, ws["y"][:t])
+                self._gemm(lw.o_proj, mix, ws["y"][:t], ahead)
                 fi += 1
             if self.comm is not None and sp.tp_world > 1:
                 self.comm.allreduce_prefill(ws["y"][:t])
             K.rmsnorm_pack(h, lw.ln2, delta=ws["y"][:t], out_h=h, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps)
-            if not linear.w4_gemm_silu(lw.gate_up, x, ws["act"][:t], arm=self.prefill_gemm):
+            if not linear.w4_gemm_silu(lw.gate_up, x, ws["act"][:t], arm=self.prefill_gemm, ahead=ahead):
                 gu = ws["wide"].view(-1)[:t * 2 * sp.inter].view(t, 2 * sp.inter)
-                self._gemm(lw.gate_up, x, gu)
+                self._gemm(lw.gate_up, x, gu, ahead)
                 K.silu_mul(gu, t, sp.inter, out=ws["act"][:t], group=self.G)
-            self._gemm(lw.down, ws["act"][:t], ws["y"][:t])
+            self._gemm(lw.down, ws["act"][:t], ws["y"][:t], ahead)
             if self.comm is not None and sp.tp_world > 1:
                 self.comm.allreduce_prefill(ws["y"][:t])
             y = ws["y"][:t]
