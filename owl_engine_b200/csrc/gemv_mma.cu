@@ -106,7 +106,10 @@ template <int FMT, int MT> __host__ __device__ constexpr int mm_stage() {
 }
 // The partial tiles arrive in a buffer behind the ring, or in the ring's own bytes where both would cost a stage too many.
 template <int MT> __host__ __device__ constexpr int mm_in_bytes() { return MM_TILES * 16 * mm_red_ld(MT) * 4; }
-template <int FMT, int MT> __host__ __device__ constexpr bool mm_alias() { return FMT == MF_G32 && MT == 4; }
+template <int FMT, int MT> __host__ __device__ constexpr bool mm_alias() { return FMT != MF_NV4 && MT > 2; }
+// Token blocks per pass over a record's nibbles: above 16 rows the int4 forms unpack a record twice (the integer pipe has the
+// room beside the MMAs), which keeps the sums of one pass in registers that leave four CTAs per SM.
+template <int FMT, int MT> __host__ __device__ constexpr int mm_pass() { return FMT != MF_NV4 && MT > 2 ? 2 : MT; }
 // Ring stages: what CT resident CTAs per SM leave room for.
 template <int FMT, int MT, int CT> __host__ __device__ constexpr int mm_stages() {
   return (227 * 1024 / CT - 1024 - (mm_alias<FMT, MT>() ? 0 : mm_in_bytes<MT>())) / mm_stage<FMT, MT>();
@@ -367,7 +370,10 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
       }
     } else {
       constexpr bool G32 = FMT == MF_G32;
-      float dot[MM_R][MT][4];
+      constexpr int MP = mm_pass<FMT, MT>();
+#pragma unroll
+      for (int mb = 0; mb < MT; mb += MP) {
+      float dot[MM_R][MP][4];
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         uint32_t fa[MM_R][8];
@@ -385,8 +391,8 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
           }
         const bool first = G32 || w == 0, last = G32 || w == 3;
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-          const uint4 xv = xf[m * 128 + w * 32];
+        for (int m = 0; m < MP && mb + m < MT; ++m) {
+          const uint4 xv = xf[(mb + m) * 128 + w * 32];
 #pragma unroll
           for (int r = 0; r < MM_R; ++r) {
             if (first) mm_bf16_z(dot[r][m], fa[r][0], fa[r][1], fa[r][2], fa[r][3], xv.x, xv.y);
@@ -404,19 +410,21 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
             s1[r] = __half22float2(*reinterpret_cast<const __half2*>(rec + r * REC + 1024 + q * 64 + 32 + g * 4));
           }
 #pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            const float4 xv = xg[m * GPR * 4 + q * 4];       // (scale, sum) of tokens 2t and 2t + 1
+          for (int m = 0; m < MP && mb + m < MT; ++m) {
+            const float4 xv = xg[(mb + m) * GPR * 4 + q * 4];       // (scale, sum) of tokens 2t and 2t + 1
 #pragma unroll
             for (int r = 0; r < MM_R; ++r) {
               float* d = dot[r][m];
               if (A8) { d[0] *= xv.x; d[1] *= xv.z; d[2] *= xv.x; d[3] *= xv.z; }
-              acc[r][m][0] = fmaf(s0[r].x, fmaf(-s0[r].y, xv.y, d[0]), acc[r][m][0]);
-              acc[r][m][1] = fmaf(s0[r].x, fmaf(-s0[r].y, xv.w, d[1]), acc[r][m][1]);
-              acc[r][m][2] = fmaf(s1[r].x, fmaf(-s1[r].y, xv.y, d[2]), acc[r][m][2]);
-              acc[r][m][3] = fmaf(s1[r].x, fmaf(-s1[r].y, xv.w, d[3]), acc[r][m][3]);
+              float* o = acc[r][mb + m];
+              o[0] = fmaf(s0[r].x, fmaf(-s0[r].y, xv.y, d[0]), o[0]);
+              o[1] = fmaf(s0[r].x, fmaf(-s0[r].y, xv.w, d[1]), o[1]);
+              o[2] = fmaf(s1[r].x, fmaf(-s1[r].y, xv.y, d[2]), o[2]);
+              o[3] = fmaf(s1[r].x, fmaf(-s1[r].y, xv.w, d[3]), o[3]);
             }
           }
         }
+      }
       }
     }
   }
@@ -505,8 +513,8 @@ static int dispatch_mma(MmaParams& p, int epi, int pdl, cudaStream_t st) {
   switch ((p.M + 7) / 8) {
     case 1: return three ? launch_mma<FMT, 1, A8, 3>(p, epi, KS, blocks, pdl, st) : launch_mma<FMT, 1, A8, 4>(p, epi, KS, blocks, pdl, st);
     case 2: return three ? launch_mma<FMT, 2, A8, 3>(p, epi, KS, blocks, pdl, st) : launch_mma<FMT, 2, A8, 4>(p, epi, KS, blocks, pdl, st);
-    case 3: return launch_mma<FMT, 3, A8, 3>(p, epi, KS, blocks, pdl, st);
-    default: return launch_mma<FMT, 4, A8, 3>(p, epi, KS, blocks, pdl, st);
+    case 3: return three || FMT == MF_NV4 ? launch_mma<FMT, 3, A8, 3>(p, epi, KS, blocks, pdl, st) : launch_mma<FMT, 3, A8, FMT == MF_NV4 ? 3 : 4>(p, epi, KS, blocks, pdl, st);
+    default: return three || FMT == MF_NV4 ? launch_mma<FMT, 4, A8, 3>(p, epi, KS, blocks, pdl, st) : launch_mma<FMT, 4, A8, FMT == MF_NV4 ? 3 : 4>(p, epi, KS, blocks, pdl, st);
   }
 }
 
