@@ -106,17 +106,21 @@ template <int FMT, int MT> __host__ __device__ constexpr int mm_stage() {
 }
 // The partial tiles arrive in a buffer behind the ring, or in the ring's own bytes where both would cost a stage too many.
 template <int MT> __host__ __device__ constexpr int mm_in_bytes() { return MM_TILES * 16 * mm_red_ld(MT) * 4; }
-template <int FMT, int MT> __host__ __device__ constexpr bool mm_alias() { return FMT != MF_NV4 && MT > 2; }
-// Token blocks per pass over a record's nibbles: above 16 rows the int4 forms unpack a record twice (the integer pipe has the
-// room beside the MMAs), which keeps the sums of one pass in registers that leave four CTAs per SM.
-template <int FMT, int MT> __host__ __device__ constexpr int mm_pass() { return FMT != MF_NV4 && MT > 2 ? 2 : MT; }
+template <int FMT, int MT, int CT> __host__ __device__ constexpr bool mm_alias() { return FMT != MF_NV4 && MT > 2 && (CT == 4 || (FMT == MF_G32 && MT == 4)); }
+// Token blocks per pass over a record's nibbles: above 16 rows the int4 forms of four CTAs per SM unpack a record twice, which
+// keeps the sums of one pass in the registers that leaves (34816 x 5120, 20 / 32 rows: 34 / 44 us against 37 / 45 in two waves of
+// three; 16384 x 5120: 20 / 25 against 24 / 29). With three CTAs per SM one pass is faster (5120 x 17408, 32 rows: 28.5 against
+// 31.4), but for 32 rows of group 32, whose sums spill (37 against 40).
+template <int FMT, int MT, int CT> __host__ __device__ constexpr int mm_pass() {
+  return FMT != MF_NV4 && MT > 2 && (CT == 4 || (FMT == MF_G32 && MT == 4)) ? 2 : MT;
+}
 // Ring stages: what CT resident CTAs per SM leave room for.
 template <int FMT, int MT, int CT> __host__ __device__ constexpr int mm_stages() {
-  return (227 * 1024 / CT - 1024 - (mm_alias<FMT, MT>() ? 0 : mm_in_bytes<MT>())) / mm_stage<FMT, MT>();
+  return (227 * 1024 / CT - 1024 - (mm_alias<FMT, MT, CT>() ? 0 : mm_in_bytes<MT>())) / mm_stage<FMT, MT>();
 }
 template <int FMT, int MT, int CT> __host__ __device__ constexpr int mm_ring() { return mm_stages<FMT, MT, CT>() * mm_stage<FMT, MT>(); }
 template <int FMT, int MT, int CT> constexpr int mm_smem() {
-  return mm_ring<FMT, MT, CT>() + (mm_alias<FMT, MT>() ? 0 : mm_in_bytes<MT>());
+  return mm_ring<FMT, MT, CT>() + (mm_alias<FMT, MT, CT>() ? 0 : mm_in_bytes<MT>());
 }
 
 // Every CTA of the cluster owns 8 / KS of the row block's tiles. The CTAs push their partial tiles into the owners' buffers
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
       }
     } else {
       constexpr bool G32 = FMT == MF_G32;
-      constexpr int MP = mm_pass<FMT, MT>();
+      constexpr int MP = mm_pass<FMT, MT, CT>();
 #pragma unroll
       for (int mb = 0; mb < MT; mb += MP) {
       float dot[MM_R][MP][4];
@@ -430,8 +434,8 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
   }
   mm_wait<0>();
   cl_wait();
-  float* in = reinterpret_cast<float*>(smem + (mm_alias<FMT, MT>() ? 0 : mm_ring<FMT, MT, CT>()));
-  if (mm_alias<FMT, MT>()) { cl_arrive(); cl_wait(); }      // every ring of the cluster is drained
+  float* in = reinterpret_cast<float*>(smem + (mm_alias<FMT, MT, CT>() ? 0 : mm_ring<FMT, MT, CT>()));
+  if (mm_alias<FMT, MT, CT>()) { cl_arrive(); cl_wait(); }      // every ring of the cluster is drained
   const int per = MM_TILES / KS;
   const uint32_t in_s = smem_u32(in) + ((rank * per * 16 + g) * LD + 2 * t) * 4;
 #pragma unroll
@@ -507,8 +511,8 @@ static int dispatch_mma(MmaParams& p, int epi, int pdl, cudaStream_t st) {
   int KS = 8;
   while (KS > 1 && (row_blocks * KS > 4 * sms || KS > (p.K >> 7))) KS >>= 1;
   // Grids of up to three CTAs per SM run with three resident and a deeper ring: with four slots per SM the scheduler fills
-  // some SMs with four CTAs and others with two (5120 x 17408, one row: 12.9 against 15.3 us). Above 16 rows three is all the
-  // registers allow.
+  // some SMs with four CTAs and others with two (5120 x 17408, one row: 12.9 against 15.3 us). NVFP4 above 16 rows has registers
+  // for three only.
   const bool three = KS * blocks <= 3 * sms;
   switch ((p.M + 7) / 8) {
     case 1: return three ? launch_mma<FMT, 1, A8, 3>(p, epi, KS, blocks, pdl, st) : launch_mma<FMT, 1, A8, 4>(p, epi, KS, blocks, pdl, st);
