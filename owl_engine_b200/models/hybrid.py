@@ -284,6 +284,9 @@ class StatePool:
 
     def copy_slot(self, src: int, dst: int) -> None:
         """Snapshot / restore of a GDN row (speculative rollback, prefix-boundary snapshots)."""
+        if self.rec_state.is_cuda and self.rec_state.shape[0] and src >= 0 and dst >= 0:
+            K.gdn_copy_slot(self.conv_state, self.rec_state, src, dst)
+            return
         self.conv_state[:, dst].copy_(self.conv_state[:, src])
         self.rec_state[:, dst].copy_(self.rec_state[:, src])
 

@@ -341,6 +341,16 @@ def gdn_decode(qkvz, ld: int, ab, ldab: int, conv_w, a_log, dt_bias, gamma, conv
          ptr(tlen), int(pdl), stream())
 
 
+register("owl_gdn_copy_slot", [_P, _P, _I, _I, c_longlong, c_longlong, _I, _I, _P])
+
+
+def gdn_copy_slot(conv_state, rec_state, src: int, dst: int) -> None:
+    """Copy slot ``src`` of both GDN state pools ([layers, slots, ...], contiguous) to slot ``dst``."""
+    ng, ns = rec_state.shape[:2]
+    call("owl_gdn_copy_slot", ptr(conv_state), ptr(rec_state), ng, ns, conv_state[0, 0].numel() * conv_state.element_size(),
+         rec_state[0, 0].numel() * rec_state.element_size(), src, dst, stream())
+
+
 def gdn_conv_fwd(x, ld: int, conv_w, conv_state, slot: int, out, t: int, nk: int, nv: int, use_state: bool) -> None:
     call("owl_gdn_conv_fwd", ptr(x), ld, ptr(conv_w), ptr(conv_state), slot, ptr(out), t, nk, nv, int(use_state),
          stream())

@@ -42,6 +42,7 @@ _T = [
     KernelSpec("owl_w4_gemm_rows", "gemm_w4.cu", "gemm_act", gen="tcgen05+tma"),
     KernelSpec("owl_gemm_w4_status", "gemm_w4.cu", "status", capture=False),
     KernelSpec("owl_gemm_silu", "gemm_dense.cu", "gemm_act", gen="tcgen05+tma"),
+    KernelSpec("owl_gdn_copy_slot", "gdn.cu", "gdn"),
     KernelSpec("owl_w4_mma", "gemv_mma.cu", "gemv", gen="mma.sync+cp.async+dsmem"),
     KernelSpec("owl_nvfp4_mma", "gemv_mma.cu", "gemv", gen="mma.sync+cp.async+dsmem"),
     KernelSpec("owl_w4_fma", "gemv_fma.cu", "gemv", gen="hfma2+bulk-copy"),

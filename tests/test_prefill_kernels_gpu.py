@@ -136,3 +136,13 @@ def test_rows_gemm_dequantises_once(t, n, k, group):
     assert (act[:, n // 2:] == 0).all()
     torch.testing.assert_close(act[:, :n // 2].float(), _silu_ref(out[:, :n].contiguous()).float(), rtol=2.0 ** -9, atol=2.0 ** -20)
     assert K.all_status()["gemm_w4"] == 0
+
+
+@pytest.mark.parametrize("vec", [4, 4096, 5000])
+def test_copy_slot_moves_one_row_of_every_layer(vec):
+    gen = torch.Generator(device=DEV).manual_seed(vec)
+    conv, rec = torch.randn(3, 4, 12, device=DEV, generator=gen), torch.randn(3, 4, vec * 4, device=DEV, generator=gen)
+    c2, r2 = conv.clone(), rec.clone()
+    K.gdn_copy_slot(conv, rec, 1, 3)
+    c2[:, 3], r2[:, 3] = c2[:, 1], r2[:, 1]
+    assert torch.equal(conv, c2) and torch.equal(rec, r2)
