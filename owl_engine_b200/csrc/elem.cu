@@ -90,6 +90,54 @@ __global__ void __launch_bounds__(1024) rmsnorm_pack_kernel(const __nv_bfloat16*
   }
 }
 
+// The same where a row has a chunk of 8 per thread (K <= 8 * blockDim): the row stays in registers between the sum and the
+// scaling instead of being read again, and the weights are there before the dependency wait. Same sums in the same order.
+__global__ void __launch_bounds__(1024) rmsnorm_pack_row_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ delta,
+                                                                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* out_h,
+                                                                __nv_bfloat16* normed, uint4* xpack, float2* xs, int K, int G, float eps,
+                                                                int one_plus_w, int normed_f16) {
+  __shared__ float red[32];
+  const int c = threadIdx.x, nchunks = K >> 3, row = blockIdx.x;
+  const bool live = c < nchunks;
+  const uint4 wv = live ? __ldg(reinterpret_cast<const uint4*>(w) + c) : make_uint4(0, 0, 0, 0);
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tiles = G & ACT_TILES;
+  G &= ~ACT_TILES;
+  float v[8], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = 0.f;
+  if (live) {
+    unpack_bf16x8(reinterpret_cast<const uint4*>(h + (size_t)row * K)[c], v);
+    if (delta) {
+      float u[8];
+      unpack_bf16x8(reinterpret_cast<const uint4*>(delta + (size_t)row * K)[c], u);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = __bfloat162float(__float2bfloat16(v[i] + u[i]));
+      if (out_h) reinterpret_cast<uint4*>(out_h + (size_t)row * K)[c] = pack_bf16x8(v);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
+  }
+  ss = block_sum(ss, red);
+  const float rinv = rsqrtf(ss / (float)K + eps);
+  if (!normed && !xpack) return;
+  float wf[8];
+  unpack_bf16x8(wv, wf);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float g = one_plus_w ? 1.f + wf[i] : wf[i];
+    const float y = v[i] * rinv * g;
+    v[i] = live ? (normed_f16 ? __half2float(__float2half_rn(clamp_h(y))) : __bfloat162float(__float2bfloat16(y))) : 0.f;
+  }
+  if (live && normed) reinterpret_cast<uint4*>(normed + (size_t)row * K)[c] = normed_f16 ? pack_f16x8(v) : pack_bf16x8(v);
+  if (xpack) {
+    float sx, xsum;
+    const uint4 pk = actpack_emit(v, G >> 3, sx, xsum);
+    if (live) actpack_store(xpack, xs, tiles, G, row, c, nchunks, pk, sx, xsum);
+  }
+}
+
 // bf16 [M][K] -> ActPack.
 __global__ void __launch_bounds__(256) act_pack_kernel(const __nv_bfloat16* __restrict__ x, int ldx, uint4* xpack,
                                                        float2* xs, int K, int G) {
@@ -299,6 +347,10 @@ OWL_API int owl_rmsnorm_pack(const void* h, const void* delta, const void* w, vo
   if (M < 1 || (K & 127) || !actpack_group_ok(G, M)) return OWL_ERR_BAD_ARG;
   int threads = ((K / 8 + 31) / 32) * 32;
   if (threads > 1024) threads = 1024;
+  if (K / 8 <= threads)
+    return launch_pdl(rmsnorm_pack_row_kernel, dim3(M), dim3(threads), pdl, st, (const __nv_bfloat16*)h,
+                      (const __nv_bfloat16*)delta, (const __nv_bfloat16*)w, (__nv_bfloat16*)out_h,
+                      (__nv_bfloat16*)normed, (uint4*)xpack, (float2*)xs, K, G, eps, one_plus_w, normed_f16);
   return launch_pdl(rmsnorm_pack_kernel, dim3(M), dim3(threads), pdl, st, (const __nv_bfloat16*)h,
                     (const __nv_bfloat16*)delta, (const __nv_bfloat16*)w, (__nv_bfloat16*)out_h,
                     (__nv_bfloat16*)normed, (uint4*)xpack, (float2*)xs, K, G, eps, one_plus_w, normed_f16);

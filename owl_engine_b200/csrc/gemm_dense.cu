@@ -557,9 +557,11 @@ OWL_API int owl_gemm_dense_set_scratch(void* ptr, long long bytes) {
   return OWL_OK;
 }
 
+OWL_API int owl_gemm_w4_status();
 OWL_API int owl_gemm_dense_status() {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_gemm_dense_status, sizeof(int)) != cudaSuccess) return -1;
   if (v != 0) cudaMemcpyToSymbol(g_gemm_dense_status, &zero, sizeof(int));
-  return v;
+  const int w = owl_gemm_w4_status();       // the row GEMM of gemm_w4.cu reports here
+  return v ? v : w;
 }

@@ -135,7 +135,7 @@ def test_rows_gemm_dequantises_once(t, n, k, group):
     gemm_tc.w4_gemm_rows(w, x, act, silu=True)
     assert (act[:, n // 2:] == 0).all()
     torch.testing.assert_close(act[:, :n // 2].float(), _silu_ref(out[:, :n].contiguous()).float(), rtol=2.0 ** -9, atol=2.0 ** -20)
-    assert K.all_status()["gemm_w4"] == 0
+    assert K.all_status()["gemm_dense"] == 0
 
 
 @pytest.mark.parametrize("vec", [4, 4096, 5000])
