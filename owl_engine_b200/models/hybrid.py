@@ -437,11 +437,11 @@ class HybridRunner:
                     gslot=i[lay.gslot:lay.gslot + lay.b], bt_row=i[lay.bt_row:lay.bt_row + lay.b])
 
     # -- building blocks ---------------------------------------------------------------------
-    def _grp(self, m: int) -> int:
+    def _grp(self, m: int, ab: bool = False) -> int:
         """``group`` argument for the ActPack producers of an ``m``-row step: the tile layout when the tcgen05 streaming kernel
-        consumes it, fragments for the 16-bit tensor streaming kernel."""
+        consumes it, fragments for the 16-bit tensor streaming kernel (``ab``: for the GDN input projection)."""
         g = (self.G | K.ACT_TILES) if self.tiles else self.G
-        if self._mma(m):
+        if self._mma(m, ab):
             g |= K.ACT_FRAG | (K.ACT_NV if self.w.layout == "nvfp4" else 0)
         return g | K.ACT_A8 if self.act_bits == 8 else g
 
@@ -452,15 +452,18 @@ class HybridRunner:
         return m >= self.BATCH_GEMM_FROM and self.prefill_gemm in ("tcr", "tc8r") and self.w.layout == "slice" \
             and not self.uniform_rows and not any(k % 128 for k in (sp.hidden, sp.inter, sp.value_dim, sp.hq * sp.hd))
 
-    def _mma(self, m: int) -> bool:
-        """The projections of an ``m``-row step run on the 16-bit tensor streaming kernel (``csrc/gemv_mma.cu``): one GPU,
+    def _mma(self, m: int, ab: bool = False) -> bool:
+        """The projections of an ``m``-row step (``ab``: the GDN input projection, which takes the a / b rows along) run on the 16-bit tensor streaming kernel (``csrc/gemv_mma.cu``): one GPU,
         slice-major int4 or NVFP4 weights. The tensor-parallel arms (push, symmetric all-reduce) and the fused-norm variant
         stay on the integer kernels, whose epilogues they are."""
         sp = self.spec
         if self._dense16(m):
             return False
         if m == 1 and self.act_bits == 8 and not self.uniform_rows and self.w.layout == "slice":
-            return False          # one row of 8-bit activations: dp4a needs half the products and streams faster (10 against 13 us)
+            # one row of 8-bit activations: dp4a needs half the products and streams faster (10 against 13 us a projection on
+            # average), but for the GDN input projection, whose a / b rows cost the integer arm a forked branch (10 us a layer)
+            return ab and not self.fuse_norm and self.decode_gemv != "dp4a" and (self.comm is None or sp.tp_world == 1) \
+                and sp.hidden % 128 == 0
         if self.decode_gemv == "dp4a" or self.fuse_norm or self.w.layout not in ("slice", "nvfp4") or not self.w.layers:
             return False
         return (self.comm is None or sp.tp_world == 1) and not any(k % 128 for k in (sp.hidden, sp.inter, sp.value_dim, sp.hq * sp.hd))
@@ -491,7 +494,7 @@ class HybridRunner:
         """out[m] = W x on the weight-streaming kernel that matches the weight's record layout. ``ab``: the dense rows that
         the 16-bit tensor kernel computes beside the matrix."""
         self._pf_hook(w, False)
-        if self._mma(m):
+        if self._mma(m, bool(ab)):
             K.w4_mma(w, xp, xs, out, m, residual=residual, epi=epi, ldo=ldo, a8=self.act_bits == 8, pdl=pdl, **ab)
         else:
             self._gemv_inner(w, xp, xs, out, m, residual=residual, epi=epi, ldo=ldo, pdl=pdl)
@@ -573,9 +576,10 @@ class HybridRunner:
             raise ValueError(f"NVFP4 arm: epilogue {epi} is not built")
 
     def _norm(self, m: int, w, *, want_xn: bool, want_pack: bool = True) -> None:
+        # (a norm whose plain rows are wanted feeds a GDN layer's input projection)
         sp = self.spec
         K.rmsnorm_pack(self.h, w, normed=self.xn if want_xn else None, xpack=self.xp_h if want_pack else None,
-                       xs=self.xs_h if want_pack else None, m=m, k=sp.hidden, group=self._grp(m), eps=sp.eps, pdl=self.pdl)
+                       xs=self.xs_h if want_pack else None, m=m, k=sp.hidden, group=self._grp(m, want_xn), eps=sp.eps, pdl=self.pdl)
 
     def _row_parallel(self, which: int, w, xp, xs, m: int, next_norm, *, want_xn: bool, want_pack: bool = True) -> None:
         """h += W x for a row-parallel projection, then x_next = rmsnorm(h) * (1 + next_norm).
@@ -626,8 +630,8 @@ class HybridRunner:
         sp, m = self.spec, lay.m
         # a speculative verify step keeps every layer's GDN inputs so that fold() can replay a prefix
         qo, ao = (self.qkvz_out, self.ab_out) if self.gdn_save is None else (self.gdn_save[0][li], self.gdn_save[1][li])
-        pdl = self._mma(m) and self.pdl
-        if self._mma(m):
+        pdl = self._mma(m, True) and self.pdl
+        if self._mma(m, True):
             # the small dense a/b projection runs on CTAs of the qkvz launch (a forked branch of the graph cost 10 us a layer)
             self._gemv(lw.qkvz, self.xp_h, self.xs_h, qo, m, pdl=pdl, ab_w=lw.ab_dense, ab_x=self.xn, ab_out=ao)
         else:
