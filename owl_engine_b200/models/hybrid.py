@@ -1005,10 +1005,12 @@ class HybridRunner:
         if self.prefill_gemm not in ("tc", "tc4") or t <= gemm_tc.ROWS_UPTO or self.w.layout not in ("slice", "block") or not self.w.layers \
                 or torch.cuda.is_current_stream_capturing():
             return None
-        if self._ahead is None:
-            self._ahead = linear.DequantAhead(self.device)
         order = [w for lw in self.w.layers
                  for w in ((lw.qkvz, lw.out_proj) if lw.kind == "gdn" else (lw.qkv, lw.o_proj)) + (lw.gate_up, lw.down)]
+        if any(w.layout not in ("slice", "block") for w in order):
+            return None
+        if self._ahead is None:
+            self._ahead = linear.DequantAhead(self.device)
         return self._ahead if self._ahead.start(order) else None
 
     def _gdn_prefill(self, lw, gi: int, wide, nq: int, ab, conv, mix, t: int, gdn_slot: int, use_state: bool, snap) -> None:

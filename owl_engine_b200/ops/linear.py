@@ -24,6 +24,8 @@ two arms:
 """
 from __future__ import annotations
 
+import weakref
+
 import torch
 
 from . import kernels as K
@@ -63,6 +65,11 @@ def _fp8_scratch(tag: str, r: int, k: int, device):
     return buf[0][:r * k].view(r, k), buf[1][:r]
 
 
+def _release_all(ledger, names: list) -> None:
+    for nm in names:
+        ledger.release(nm)
+
+
 class DequantAhead:
     """Dequantises a chunk's weights one projection ahead, on a stream of its own: the dequantisation is bound by memory (44 us a
     projection of the 27B model, 11 of 112 ms at 2048 tokens), the GEMM beside it by the tensor cores. Two buffers alternate; a
@@ -72,6 +79,8 @@ class DequantAhead:
     def __init__(self, device):
         self.device, self.side = torch.device(device), torch.cuda.Stream(device=device)
         self.buf, self.elems = [], 0
+        self.names = [f"dequant ahead {id(self)} {i}" for i in range(2)]
+        weakref.finalize(self, _release_all, _ledger(self.device), self.names)
 
     def start(self, weights: list) -> bool:
         """Begin a chunk that multiplies ``weights`` in this order; False where the buffers do not fit the device's budget."""
@@ -81,13 +90,12 @@ class DequantAhead:
 
             led = _ledger(self.device)
             torch.cuda.current_stream(self.device).wait_stream(self.side)
-            for i in range(len(self.buf)):
-                led.release(f"dequant ahead {id(self)} {i}")
+            _release_all(led, self.names)
             self.buf, self.elems = [], 0
             try:
-                self.buf = [led.alloc(f"dequant ahead {id(self)} {i}", "workspace", (need,), torch.float16) for i in range(2)]
+                self.buf = [led.alloc(nm, "workspace", (need,), torch.float16) for nm in self.names]
             except BudgetError:
-                led.release(f"dequant ahead {id(self)} 0")
+                _release_all(led, self.names)
                 return False
             self.elems = need
         self.weights, self.i = weights, -1
@@ -154,6 +162,10 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: Dequa
             rows = (t + 7) // 8 * 8
             xp = torch.empty(rows, 2 * k, dtype=torch.uint8, device=x.device)
             xs = torch.empty(rows, k // w.group, 2, dtype=torch.float32, device=x.device)
+            if out.stride(0) % 2 or out.data_ptr() % 4:          # the integer arm stores single values
+                K.act_pack(xb, xp, xs, t, k, w.group)
+                K.w4a16_skinny(w, xp, xs, out, t, ldo=out.stride(0))
+                return out
             K.act_pack(xb, xp, xs, t, k, w.group | K.ACT_FRAG)
             K.w4_mma(w, xp, xs, out, t, ldo=out.stride(0))
             return out

@@ -146,3 +146,18 @@ def test_copy_slot_moves_one_row_of_every_layer(vec):
     K.gdn_copy_slot(conv, rec, 1, 3)
     c2[:, 3], r2[:, 3] = c2[:, 1], r2[:, 1]
     assert torch.equal(conv, c2) and torch.equal(rec, r2)
+
+
+def test_dequantising_ahead_gives_each_weight_in_turn():
+    """More weights than buffers, of different sizes, over two chunks: every copy is the weight's own, and products made while the
+    next one is dequantised equal those made one after the other."""
+    gen = torch.Generator().manual_seed(4)
+    ws = [Q.pack_skinny(Q.quantize_w4(torch.randn(n, k, generator=gen) * 0.05, 128)).to(DEV) for n, k in ((512, 256), (256, 1024), (1024, 128), (768, 512))]
+    ahead = linear.DequantAhead(DEV)
+    for _ in range(2):
+        assert ahead.start(ws)
+        for w in ws:
+            x = torch.randn(300, w.k, generator=gen).half().to(DEV)
+            out = linear.w4_gemm(w, x, torch.empty(300, w.n, dtype=torch.bfloat16, device=DEV), ahead=ahead)
+            want = linear.w4_gemm(w, x, torch.empty(300, w.n, dtype=torch.bfloat16, device=DEV))
+            assert torch.equal(out, want)
