@@ -45,8 +45,9 @@ __device__ __forceinline__ float clamp_h(float x) { return fminf(fmaxf(x, -65504
 constexpr int ACT_A8 = 0x2000;
 // With ACT_FRAG the chunk is for the 16-bit tensor path (gemv_mma.cu): eight bf16 = x * 2^64, an exponent shift; elements 2, 3,
 // 6 and 7, which meet the nibbles that carry a factor 16, are x * 2^60 (with ACT_A8, x is the 8-bit integer and sx its scale).
-// xsum is stored in the unit of the products, n * 2^-133 * x * 2^64. With ACT_NV as well (NVFP4 weights) the elements come in
-// the order 0 4 1 5 2 6 3 7, all times 2^64 (and with ACT_A8 the rounded activations themselves: there is no scale to apply).
+// xsum is stored in the unit of the products, n * 2^-133 * x * 2^64. With ACT_NV as well (NVFP4 weights) the elements are fp16 in
+// their order, x * 2^e with the largest of 128 in [2^13, 2^14) (exact for bf16 values down to 2^-27 of it) and sx = 2^-e; with
+// ACT_A8 x is the rounded activation.
 constexpr int ACT_FRAG = 0x4000, ACT_NV = 0x8000;
 constexpr float ACT_FRAG_UNIT = 590295810358705651712.f;      // 2^69 = 2^133 / 2^64
 __device__ __forceinline__ uint4 actpack_frag(const float* v, int cpg, float& sx, float& xsum) {
@@ -71,15 +72,24 @@ __device__ __forceinline__ uint4 actpack_frag(const float* v, int cpg, float& sx
   for (int i = 0; i < 8; ++i) sum += x[i];
   for (int o = cpg >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   xsum = sum * sx * (1.f / ACT_FRAG_UNIT);
-  if (nv && a8) {
+  if (nv) {
+    float amax = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] *= sx;
+    for (int i = 0; i < 8; ++i) {
+      if (a8) x[i] = __bfloat162float(__float2bfloat16(x[i] * sx));
+      amax = fmaxf(amax, fabsf(x[i]));
+    }
+    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));     // 16 lanes: 128 elements
+    const int ex = amax > 0.f ? min(max(127 + 13 - ((int)(__float_as_uint(amax) >> 23) - 127), 1), 253) : 127;
+    const float up = __uint_as_float((uint32_t)ex << 23);
+    sx = __uint_as_float((uint32_t)(254 - ex) << 23);
+    return make_uint4(pack_f16(x[0] * up, x[1] * up), pack_f16(x[2] * up, x[3] * up), pack_f16(x[4] * up, x[5] * up),
+                      pack_f16(x[6] * up, x[7] * up));
   }
-  const float e = 18446744073709551616.f, e16 = nv ? e : e / 16.f;
+  const float e = 18446744073709551616.f, e16 = e / 16.f;
   float y[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) y[i] = x[i] * ((i & 2) ? e16 : e);
-  if (nv) return make_uint4(pack_bf16(y[0], y[4]), pack_bf16(y[1], y[5]), pack_bf16(y[2], y[6]), pack_bf16(y[3], y[7]));
   return make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
 }
 __device__ __forceinline__ uint4 actpack_emit(const float* v, int cpg, float& sx, float& xsum) {
@@ -165,7 +175,8 @@ __device__ __forceinline__ void actpack_store(uint4* xpack, float2* xs, int tile
     const int kt = c8 >> 4, hi = (c8 >> 2) & 3, lo = c8 & 3, w = nv ? lo : hi, t = nv ? hi : lo;
     const size_t blk = (size_t)(token >> 3);
     xpack[(blk * (nchunks >> 4) + kt) * 128 + w * 32 + (token & 7) * 4 + t] = pk;
-    if (!nv && (c8 % cpg) == 0) xs[(blk * (nchunks / cpg) + c8 / cpg) * 8 + (token & 7)] = make_float2(sx, xsum);
+    const int per = nv ? 16 : cpg;           // chunks of one (scale, sum) pair
+    if ((c8 % per) == 0) xs[(blk * (nchunks / per) + c8 / per) * 8 + (token & 7)] = make_float2(sx, xsum);
     return;
   }
   if (!tiles) {

@@ -12,13 +12,14 @@
 //     y += s * (dot - z * sum(x)).
 // The integer arm (gemv.cu) rounds the activations to 15 bits, needs two MMAs per 32 k and converts its int32 sums; this
 // one rounds nothing before the fp32 sums. Activations of magnitude 2^63 and above become infinite here.
-// NVFP4: the code bits are moved to the sign and exponent places of a bf16 (value * 2^-126, exact) and multiplied by the
-// block scale (4 x 2 significant bits: exact in bf16), so its whole k range is one accumulator chain.
+// NVFP4: the codes are converted to fp16 pairs by the conversion unit (6.6 clocks a word of eight; moving their bits to the
+// sign and exponent places of a bf16 took 15 integer instructions, 19 clocks) and multiplied by the block scale (4 x 2
+// significant bits: exact in fp16); the activations are fp16 with a power of two per 128 that the sums are rescaled by.
 //
 // What bounds it: 0.53 bytes per weight over HBM. An SM receives about 23.5 bytes per clock, one 1088-byte record per 185
 // clocks and sub-core; per record this kernel issues 40 mask / shift instructions (two clocks each), 8 MMAs per 8 rows at 8
 // clocks each, and about 30 others. Up to 8 rows the stream and the launch-to-launch dependency (about 4 us) are the bound,
-// at 32 rows the MMAs and the shared-memory reads of their fragments; NVFP4 is bound by its 15 integer instructions a word.
+// at 32 rows the MMAs and the shared-memory reads of their fragments.
 //
 // Shape of the work. A CTA is 4 warps x 2 row tiles = 128 rows over one part of k; the KS parts of a row block form a
 // thread-block cluster and reduce through distributed shared memory in rank order, so a row's sums have one order that
@@ -52,7 +53,7 @@ struct MmaParams {
   const uint8_t* sf;              // NVFP4: e4m3 block scales [N][K/16]
   const float* row_scale;         // NVFP4, optional: fp32 [N]
   const uint4* x;                 // ACT_FRAG chunks
-  const float4* xs;               // int4: ACT_FRAG (scale, sum) pairs of two tokens
+  const float4* xs;               // ACT_FRAG (scale, sum) pairs of two tokens
   __nv_bfloat16* out;
   const __nv_bfloat16* residual;
   const __nv_bfloat16* ab_w;      // optional dense rows [ab_rows][K] ...
@@ -74,10 +75,28 @@ __device__ __forceinline__ void mm_bf16_z(float* c, uint32_t a0, uint32_t a1, ui
       : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
+__device__ __forceinline__ void mm_f16(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mm_f16_z(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ uint32_t mm_mul2(uint32_t a, uint32_t b) {
   uint32_t d;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
+}
+// eight e2m1 codes -> four fp16 pairs
+__device__ __forceinline__ void mm_e2m1x8(uint32_t q, uint32_t* d) {
+  asm("{\n\t.reg .b8 a, b, c, d;\n\tmov.b32 {a, b, c, d}, %4;\n\tcvt.rn.f16x2.e2m1x2 %0, a;\n\tcvt.rn.f16x2.e2m1x2 %1, b;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %2, c;\n\tcvt.rn.f16x2.e2m1x2 %3, d;\n\t}"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(q));
 }
 __device__ __forceinline__ void mm_cp16(uint32_t smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
@@ -100,7 +119,7 @@ __device__ __forceinline__ void cl_store2(uint32_t addr, float a, float b) {
 template <int FMT> __host__ __device__ constexpr int mm_rec() { return FMT == MF_G128 ? 1088 : FMT == MF_G32 ? 1280 : 1152; }
 __host__ __device__ constexpr int mm_red_ld(int mt) { return mt * 8 + 2; }
 // One ring stage: the record of every tile, the activation fragments of the record column, their (scale, sum) pairs.
-template <int FMT> __host__ __device__ constexpr int mm_pairs() { return FMT == MF_NV4 ? 0 : FMT == MF_G32 ? 4 : 1; }
+template <int FMT> __host__ __device__ constexpr int mm_pairs() { return FMT == MF_G32 ? 4 : 1; }
 template <int FMT, int MT> __host__ __device__ constexpr int mm_stage() {
   return MM_TILES * mm_rec<FMT>() + MT * (2048 + mm_pairs<FMT>() * 64);
 }
@@ -336,17 +355,18 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
     }
     if constexpr (FMT == MF_NV4) {
       // this lane's blocks: 16-k blocks 2t and 2t + 1 of rows g and g + 8
-      uint32_t sc[MM_R][2][2];          // [tile][row half][block]: scale * 2^63 in both halves of a bf16 pair
+      uint32_t sc[MM_R][2][2];          // [tile][row half][block]: the scale in both halves of an fp16 pair
 #pragma unroll
       for (int r = 0; r < MM_R; ++r)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const uint16_t b2 = *reinterpret_cast<const uint16_t*>(rec + r * REC + 1024 + (g + 8 * h) * 8 + 2 * t);
-          const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(b2, __NV_E4M3);
-          const float2 f = __half22float2(__half2(hr));
-          sc[r][h][0] = pack_bf16(f.x * 9.223372036854775808e18f, f.x * 9.223372036854775808e18f);
-          sc[r][h][1] = pack_bf16(f.y * 9.223372036854775808e18f, f.y * 9.223372036854775808e18f);
+          const __half2 s2 = __half2(__nv_cvt_fp8x2_to_halfraw2(b2, __NV_E4M3));
+          const __half2 s0 = __low2half2(s2), s1 = __high2half2(s2);
+          sc[r][h][0] = *reinterpret_cast<const uint32_t*>(&s0);
+          sc[r][h][1] = *reinterpret_cast<const uint32_t*>(&s1);
         }
+      float dot[MM_R][MT][4];
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         uint32_t fa[MM_R][8];
@@ -355,21 +375,32 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const uint4& u = h ? hi[r] : lo[r];
-            const uint32_t q = w == 0 ? u.x : w == 1 ? u.y : w == 2 ? u.z : u.w;
-            const uint32_t s = sc[r][h][w >> 1];
-            // nibble pairs (j, j + 4): sign to bit 15, exponent and mantissa to bits 8..6
-            fa[r][0 + h] = mm_mul2(((q << 12) & 0x80008000u) | ((q << 6) & 0x01C001C0u), s);
-            fa[r][2 + h] = mm_mul2(((q << 8) & 0x80008000u) | ((q << 2) & 0x01C001C0u), s);
-            fa[r][4 + h] = mm_mul2(((q << 4) & 0x80008000u) | ((q >> 2) & 0x01C001C0u), s);
-            fa[r][6 + h] = mm_mul2((q & 0x80008000u) | ((q >> 6) & 0x01C001C0u), s);
+            uint32_t d[4];
+            mm_e2m1x8(w == 0 ? u.x : w == 1 ? u.y : w == 2 ? u.z : u.w, d);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) fa[r][2 * i + h] = mm_mul2(d[i], sc[r][h][w >> 1]);
           }
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
           const uint4 xv = xf[m * 128 + w * 32];
 #pragma unroll
-          for (int r = 0; r < MM_R; ++r) mm_bf16(acc[r][m], fa[r][0], fa[r][1], fa[r][2], fa[r][3], xv.x, xv.y);
+          for (int r = 0; r < MM_R; ++r) {
+            if (w == 0) mm_f16_z(dot[r][m], fa[r][0], fa[r][1], fa[r][2], fa[r][3], xv.x, xv.y);
+            else mm_f16(dot[r][m], fa[r][0], fa[r][1], fa[r][2], fa[r][3], xv.x, xv.y);
+          }
 #pragma unroll
-          for (int r = 0; r < MM_R; ++r) mm_bf16(acc[r][m], fa[r][4], fa[r][5], fa[r][6], fa[r][7], xv.z, xv.w);
+          for (int r = 0; r < MM_R; ++r) mm_f16(dot[r][m], fa[r][4], fa[r][5], fa[r][6], fa[r][7], xv.z, xv.w);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const float4 xv = xg[m * 4];     // the powers of two of tokens 2t and 2t + 1
+#pragma unroll
+        for (int r = 0; r < MM_R; ++r) {
+          acc[r][m][0] = fmaf(dot[r][m][0], xv.x, acc[r][m][0]);
+          acc[r][m][1] = fmaf(dot[r][m][1], xv.z, acc[r][m][1]);
+          acc[r][m][2] = fmaf(dot[r][m][2], xv.x, acc[r][m][2]);
+          acc[r][m][3] = fmaf(dot[r][m][3], xv.z, acc[r][m][3]);
         }
       }
     } else {
@@ -556,17 +587,18 @@ OWL_API int owl_w4_mma(const void* records, const void* x, const void* xs, void*
   return a8 ? dispatch_mma<MF_G32, true>(p, epi, pdl, st) : dispatch_mma<MF_G32, false>(p, epi, pdl, st);
 }
 
-// codes [N][K/2], sf [N][K/16], y = alpha * row_scale[n] * sum; x: activations packed with ACT_FRAG | ACT_NV.
-OWL_API int owl_nvfp4_mma(const void* codes, const void* sf, float alpha, const void* row_scale, const void* x, void* out,
+// codes [N][K/2], sf [N][K/16], y = alpha * row_scale[n] * sum; x / xs: activations packed with ACT_FRAG | ACT_NV.
+OWL_API int owl_nvfp4_mma(const void* codes, const void* sf, float alpha, const void* row_scale, const void* x, const void* xs, void* out,
                           const void* residual, const void* ab_w, const void* ab_x, void* ab_out, int ab_rows, int ab_ld, int M,
                           int N, int K, int ldo, int epi, int pdl, cudaStream_t st) {
-  if (!codes || !sf || (reinterpret_cast<uintptr_t>(codes) & 15) || (reinterpret_cast<uintptr_t>(sf) & 7) ||
+  if (!codes || !sf || !xs || ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(xs)) & 15) ||
+      (reinterpret_cast<uintptr_t>(sf) & 7) ||
       !mma_args_ok(x, out, residual, ab_w, ab_x, ab_out, ab_rows, ab_ld, M, N, K, ldo, epi))
     return OWL_ERR_BAD_ARG;
   MmaParams p = {};
   p.w = (const uint8_t*)codes; p.sf = (const uint8_t*)sf; p.row_scale = (const float*)row_scale; p.x = (const uint4*)x;
-  p.xs = (const float4*)x; p.out = (__nv_bfloat16*)out; p.residual = (const __nv_bfloat16*)residual;
+  p.xs = (const float4*)xs; p.out = (__nv_bfloat16*)out; p.residual = (const __nv_bfloat16*)residual;
   p.ab_w = (const __nv_bfloat16*)ab_w; p.ab_x = (const __nv_bfloat16*)ab_x; p.ab_out = (__nv_bfloat16*)ab_out;
-  p.ab_rows = ab_rows; p.ab_ld = ab_ld; p.out_scale = alpha * 0.5f; p.M = M; p.N = N; p.K = K; p.ldo = ldo; p.n_tiles = N / 16;
+  p.ab_rows = ab_rows; p.ab_ld = ab_ld; p.out_scale = alpha; p.M = M; p.N = N; p.K = K; p.ldo = ldo; p.n_tiles = N / 16;
   return dispatch_mma<MF_NV4, false>(p, epi, pdl, st);
 }

@@ -182,7 +182,7 @@ class StreamTcWorkspace:
 ACT_TILES = 0x1000     # OR into a producer's ``group`` argument: write ActPack in the tile layout
 ACT_A8 = 0x2000        # OR into a producer's ``group`` argument: round the activations to 8 bits (low plane zero)
 ACT_FRAG = 0x4000      # OR into a producer's ``group`` argument: bf16 fragments for w4_mma (buffers hold rows rounded up to 8)
-ACT_NV = 0x8000        # with ACT_FRAG: the element order of nvfp4_mma
+ACT_NV = 0x8000        # with ACT_FRAG: the fp16 form that w4_mma wants for NVFP4 weights
 
 
 def act_tile_bytes(k: int, group: int) -> int:
@@ -238,7 +238,7 @@ def w4_fma(w, x, out, *, norm_w=None, residual=None, epi: int = EPI_STORE, ab_w=
 
 
 register("owl_w4_mma", [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P])
-register("owl_nvfp4_mma", [_P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P])
+register("owl_nvfp4_mma", [_P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P])
 
 
 def w4_mma(w, xpack, xs, out, m: int, *, residual=None, epi: int = EPI_STORE, ldo: int | None = None, a8: bool = False,
@@ -249,8 +249,8 @@ def w4_mma(w, xpack, xs, out, m: int, *, residual=None, epi: int = EPI_STORE, ld
     ldo = out.shape[-1] if ldo is None else ldo
     ab = (ptr(ab_w), ptr(ab_x), ptr(ab_out), ab_w.shape[0] if ab_w is not None else 0, ab_out.shape[-1] if ab_w is not None else 0)
     if w.layout == "nvfp4":
-        call("owl_nvfp4_mma", ptr(w.codes), ptr(w.scales), float(w.alpha), ptr(w.row_scale), ptr(xpack), ptr(out), ptr(residual), *ab,
-             m, w.n, w.k, ldo, epi, int(pdl), stream())
+        call("owl_nvfp4_mma", ptr(w.codes), ptr(w.scales), float(w.alpha), ptr(w.row_scale), ptr(xpack), ptr(xs), ptr(out), ptr(residual),
+             *ab, m, w.n, w.k, ldo, epi, int(pdl), stream())
         return
     assert w.layout == "slice", "w4_mma reads slice-major records"
     call("owl_w4_mma", ptr(w.records), ptr(xpack), ptr(xs), ptr(out), ptr(residual), *ab, m, w.n, w.k, ldo, w.group, epi, int(a8),

@@ -68,13 +68,14 @@ def test_mma_streaming_matches_dequantised_product(fmt, shape, m):
         assert torch.equal(one[0], out[m - 1])
 
 
-@pytest.mark.parametrize("group,m", [(128, 1), (32, 5), (128, 20)])
-def test_eight_bit_activations(group, m):
+@pytest.mark.parametrize("fmt,m", [("g128", 1), ("g32", 5), ("g128", 20), ("nvfp4", 3)])
+def test_eight_bit_activations(fmt, m):
     n, k = 512, 1024
     gen = torch.Generator().manual_seed(m)
-    w, deq = _weight(f"g{group}", n, k, gen)
+    w, deq = _weight(fmt, n, k, gen)
+    group = w.group
     x = torch.randn(m, k, generator=gen).to(torch.bfloat16)
-    xp, xs = _pack(w, x, K.ACT_A8)
+    xp, xs = _pack(w, x, K.ACT_A8 | (K.ACT_NV if fmt == "nvfp4" else 0))
     out = torch.zeros(m, n, dtype=torch.bfloat16, device=DEV)
     K.w4_mma(w, xp, xs, out, m, a8=True)
     xg = x.float().view(m, k // group, group)
@@ -99,18 +100,19 @@ def test_dense_rows_beside_the_matrix(rows, m):
         assert (got.double().cpu() - want).norm() / want.norm() < 4e-3
 
 
-def test_extremes_of_the_activations():
+@pytest.mark.parametrize("fmt", ["g128", "nvfp4"])
+def test_extremes_of_the_activations(fmt):
     """Zero rows, rows of very small and very large values, NaN only where its row is."""
     n, k, m = 64, 512, 5
     gen = torch.Generator().manual_seed(3)
-    w, deq = _weight("g128", n, k, gen)
+    w, deq = _weight(fmt, n, k, gen)
     x = torch.randn(m, k, generator=gen)
     x[0] = 0
     x[1] *= 2.0 ** -40
     x[2] *= 2.0 ** 55
     x[3, 7] = float("nan")
     x = x.to(torch.bfloat16)
-    xp, xs = _pack(w, x, 0)
+    xp, xs = _pack(w, x, K.ACT_NV if fmt == "nvfp4" else 0)
     out = torch.zeros(m, n, dtype=torch.bfloat16, device=DEV)
     K.w4_mma(w, xp, xs, out, m)
     want = x.double() @ deq.t()
