@@ -165,9 +165,8 @@ __device__ __forceinline__ void mma_f16_16816_z(float* c, uint32_t a0, uint32_t 
 // CTA that owns row tiles nt0.. therefore reads ONE contiguous byte stream, cut into fixed-size
 // chunks that ignore row-tile boundaries (one bulk copy + one mbarrier per chunk).
 // SIMT = true (single token only): the contraction runs on the CUDA cores with dp4a instead of the
-// warp-level tensor-core path. On sm_100 the legacy mma.sync path issues one m16n8k16/k32 MMA per
-// ~34 cycles per SM sub-core, which caps a W4 stream at ~4 TB/s (8 MMAs per 1088-byte record
-// whatever the token count); for one token 32 dp4a per lane per record are cheaper than that.
+// warp-level tensor-core path: 32 dp4a per lane and record (2 clocks each) against 8 MMAs (8 clocks each on a
+// sub-core, 21 in a dependent chain) whose columns would hold one token in eight.
 template <int MT, int KIND, bool SIMT, bool A8>
 __global__ void __launch_bounds__(SK_WARPS * 32, MT == 1 ? 4 : 2) skinny_stream_kernel(SkinnyParams p, int epi) {
   constexpr int REC = RecInfo<KIND>::BYTES, KREC = RecInfo<KIND>::KREC;

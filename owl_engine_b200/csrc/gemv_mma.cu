@@ -30,9 +30,9 @@
 // latency was exposed four times a record.
 //
 // Measured (one B200, graph of dependent launches over rotating weights, group 128; HBM time of the weights; 1 / 8 / 32 rows):
-//   16384 x 5120  6.7 us: 10.6 / 10.8 / 28      5120 x 6144   2.5 us: 6.8 / 6.9 / 14.6
-//   34816 x 5120 14.2 us: 18.7 / 19.5 / 45      5120 x 17408  7.1 us: 12.9 / 13.2 / 28.7
-// (the integer arm in a step of 8 / 32 rows: 23 / 82 us on average over the four; the NVFP4 GEMV 88 us at 4 rows, here 24.)
+//   16384 x 5120  6.7 us: 10.5 / 10.8 / 25.3    5120 x 6144   2.5 us: 6.9 / 7.0 / 14.6
+//   34816 x 5120 14.2 us: 18.8 / 19.5 / 44.0    5120 x 17408  7.1 us: 12.9 / 13.1 / 28.5
+// (the integer arm in a step of 8 / 32 rows: 23 / 82 us on average over the four; the NVFP4 GEMV 88 us at 4 rows, here 20.)
 //
 // Role in the reference: the Marlin W4A16 decode path and the NVFP4 GEMV (crates/kernels/cu/marlin/*,
 // crates/kernels/cu/nvfp4/nvfp4_gemv.cu).
@@ -100,6 +100,10 @@ __device__ __forceinline__ void mm_e2m1x8(uint32_t q, uint32_t* d) {
 }
 __device__ __forceinline__ void mm_cp16(uint32_t smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
+}
+// The same for rows of which a stage takes 64 bytes: the rest of the line is fetched along (NVFP4: 3 % at 4 rows).
+__device__ __forceinline__ void mm_cp16_ahead(uint32_t smem_dst, const void* gsrc) {
+  asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
 }
 __device__ __forceinline__ void mm_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -282,10 +286,10 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
   auto issue = [&](uint32_t st) {
     if (to_issue > 0) {
       if (FMT == MF_NV4) {
-        mm_cp16(ring_s + st, src_a);
-        mm_cp16(ring_s + st + 512, src_a + row8);
-        mm_cp16(ring_s + st + REC, src_b);
-        mm_cp16(ring_s + st + REC + 512, src_b + row8);
+        mm_cp16_ahead(ring_s + st, src_a);
+        mm_cp16_ahead(ring_s + st + 512, src_a + row8);
+        mm_cp16_ahead(ring_s + st + REC, src_b);
+        mm_cp16_ahead(ring_s + st + REC + 512, src_b + row8);
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(ring_s - lane * 16 + st + (lane >> 4) * REC + 1024 + (lane & 15) * 8),
                      "l"(sfp) : "memory");
         src_a += 64;
