@@ -12,8 +12,9 @@
 // Why this arm exists. One token makes the projection a pure weight stream: 0.53 bytes per weight, every byte
 // read once. At 6.4 TB/s an SM receives about 22 bytes per clock, i.e. 44 weights, so the instruction budget is
 // about three instructions per weight BYTE and lane. The integer arm (dp4a, issued at a quarter of the rate on
-// this part, two 8-bit planes per activation) needs five; the warp-level MMA issues once per ~34 clocks per
-// sub-core. This arm needs nine instructions per 32-bit word of eight weights:
+// this part, two 8-bit planes per activation) needs five. This arm needs nine instructions per 32-bit word of eight
+// weights (the same nibbles in warp-level MMAs with one used column of eight: 8 MMAs of 8 clocks a record, fewer
+// instructions, but their dependent chains made the 27B step 4.24 ms against 3.95):
 //
 //   * A nibble masked in place (q & 0x000f000f, q & 0x00f000f0, and the same on q >> 8) IS a pair of fp16
 //     subnormals with the values n * 2^-24 and 16 n * 2^-24: no bias to subtract, no conversion. The record
