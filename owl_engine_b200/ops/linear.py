@@ -279,8 +279,9 @@ def w4_dense(w, dtype, device, resident: bool = False) -> torch.Tensor:
     return K.w4_dequant(w, _dense_scratch(w.n, w.k, device, dtype))
 
 
-def dense_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.Tensor:
-    """out[T, N] (bf16) = x @ w^T for a small dense bf16 weight (GDN a/b projections, draft heads)."""
+def dense_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, arm: str = "tc", split: bool = False) -> torch.Tensor:
+    """out[T, N] (bf16) = x @ w^T for a small dense bf16 weight (GDN a/b projections, draft heads). ``split``: cut k so that
+    every SM has a part (the 96 rows of a / b are one or two tiles at a short prompt)."""
     if arm == "baseline":
         torch.matmul(x.to(w.dtype), w.t(), out=out)
         return out
@@ -294,4 +295,4 @@ def dense_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, arm: str = "
             cache = w.to(x.dtype)
             w._owl_cast = cache
         w = cache
-    return gemm_tc.f16_gemm(x, w, out)
+    return gemm_tc.f16_gemm(x, w, out, force_persist=split)

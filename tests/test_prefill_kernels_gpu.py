@@ -161,3 +161,13 @@ def test_dequantising_ahead_gives_each_weight_in_turn():
             out = linear.w4_gemm(w, x, torch.empty(300, w.n, dtype=torch.bfloat16, device=DEV), ahead=ahead)
             want = linear.w4_gemm(w, x, torch.empty(300, w.n, dtype=torch.bfloat16, device=DEV))
             assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("t", [33, 128, 137, 256])
+def test_dense_rows_cut_along_k(t):
+    gen = torch.Generator(device=DEV).manual_seed(t)
+    x, w = torch.randn(t, 1280, device=DEV, generator=gen).half(), (torch.randn(96, 1280, device=DEV, generator=gen) * 0.05).half()
+    out = linear.dense_gemm(x, w, torch.zeros(t, 96, dtype=torch.bfloat16, device=DEV), split=True)
+    want = x.double() @ w.double().t()
+    # bf16 result + fp32 sums
+    assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * 2.0 ** -19).all()
