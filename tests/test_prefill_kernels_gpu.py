@@ -171,3 +171,32 @@ def test_dense_rows_cut_along_k(t):
     want = x.double() @ w.double().t()
     # bf16 result + fp32 sums
     assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * 2.0 ** -19).all()
+
+
+def _big_zeros(n, k, layout):
+    """Group-32 records with zero points outside 0..15, each in whole 16 x 128 records: whole numbers that fp16 sums of 1024 + z would
+    round or overflow (a dead Q4_K sub-block has scale 1.2e-7 and its zero point clipped to 65504), negative ones, and fractional."""
+    gen = torch.Generator().manual_seed(n + k)
+    c = Q.quantize_w4(torch.randn(n, k, generator=gen) * 0.05, 32)
+    z = c.zeros.half()
+    for i, (zero, scale) in enumerate(((1024, 1e-3), (1025, 1e-3), (3001, 2e-4), (65504, 1.2e-7), (-3, 0.01), (-2040, 2e-4), (15.3, 0.01))):
+        r, q = 16 * (i % (n // 16)), 4 * (i // (n // 16))
+        z[r:r + 16, q:q + 4], c.scales[r:r + 16, q:q + 4] = zero, scale
+    c.zeros = z
+    return Q.pack_skinny(c, layout).to(DEV)
+
+
+def _check_against_dequant(w, x, out):
+    dense = K.w4_dequant(w, torch.empty(w.n, w.k, dtype=torch.float16, device=DEV)).double()
+    assert dense.isfinite().all()
+    want, size = x.double() @ dense.t(), x.double().abs() @ dense.abs().t()
+    # bf16 result + fp32 sums of products of the same fp16 weights
+    assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -18).all()
+
+
+@pytest.mark.parametrize("t", [33, 137])
+@pytest.mark.parametrize("n,k", [(112, 256), (32, 1024)])
+def test_rows_gemm_with_large_zero_points(t, n, k):
+    w = _big_zeros(n, k, "slice")
+    x = torch.randn(t, k, generator=torch.Generator().manual_seed(t)).half().to(DEV)
+    _check_against_dequant(w, x, gemm_tc.w4_gemm_rows(w, x, torch.zeros(t, n, dtype=torch.bfloat16, device=DEV)))
