@@ -9,8 +9,9 @@
 //   warp 1      allocates TMEM, then one thread issues tcgen05.mma (M128 N128 K16 x 4 per stage) and
 //               tcgen05.commit -> the stage's "empty" barrier; a last commit signals the epilogue
 //   warps 2-5   W4 path: stream the int4 records of 8 row tiles, dequantise ((q - z) * s in exact
-//               fp16: lop3 bias trick, one hsub2 + one hmul2 per pair) and write the swizzled
-//               B tile; afterwards they are the epilogue: tcgen05.ld 32x32b -> bf16 -> global
+//               fp16: lop3 bias trick, one hsub2 + one hmul2 per pair; records with fractional zero
+//               points or such above 1024 in fp32) and write the swizzled B tile; afterwards they are
+//               the epilogue: tcgen05.ld 32x32b -> bf16 -> global
 // Two CTAs fit per SM (3 stages x 32 KB, 128 TMEM columns each) so one CTA's epilogue overlaps the
 // other's main loop.
 //
@@ -20,6 +21,7 @@
 // Role in the reference: the Marlin / cuBLAS prefill GEMMs (crates/kernels/cu/marlin/*,
 // crates/kernels/src/family/cublas.rs); the reference has no tcgen05 path.
 #include <cuda.h>
+#include <type_traits>
 #include "common.cuh"
 #include "records.cuh"
 
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(GT_THREADS, 2) gemm_tc_kernel(const __grid_con
       const int NT = p.N / 16, KT = p.K / 128;
       const __half2 k1024 = __floats2half2_rn(1024.f, 1024.f), k64 = __floats2half2_rn(64.f, 64.f);
       const __half2 k16th = __floats2half2_rn(0.0625f, 0.0625f);
+      const __half z_max = __float2half_rn(1024.f);
       uint4 cur[4], nxt[4];                  // [jt*2 + half]
       uint32_t csz[4][4], nsz[4][4];         // (scale, zero) half2 per [jt*2+half][group of record]
       auto load_rec = [&](int kt, uint4* q, uint32_t (*sz)[4]) {
@@ -166,53 +169,84 @@ __global__ void __launch_bounds__(GT_THREADS, 2) gemm_tc_kernel(const __grid_con
             q[jt * 2 + 0] = ldg_stream(reinterpret_cast<const uint4*>(rec) + lane);
             q[jt * 2 + 1] = ldg_stream(reinterpret_cast<const uint4*>(rec) + 32 + lane);
             const uint32_t* szr = reinterpret_cast<const uint32_t*>(rec + 1024);
-            for (int qg = 0; qg < GPT; ++qg) {
+#pragma unroll
+            for (int qg = 0; qg < 4; ++qg) {
+              if (qg >= GPT) break;
               sz[jt * 2 + 0][qg] = __ldg(szr + qg * 16 + g);
               sz[jt * 2 + 1][qg] = __ldg(szr + qg * 16 + 8 + g);
             }
           } else {
             q[jt * 2 + 0] = q[jt * 2 + 1] = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);
+#pragma unroll
             for (int qg = 0; qg < 4; ++qg) sz[jt * 2 + 0][qg] = sz[jt * 2 + 1][qg] = 0x48000000u;  // s = 0, z = 8
           }
         }
       };
       load_rec(0, cur, csz);
+      bool exact = true;
       for (int it = 0; it < KI; ++it) {
         const int s = it % GT_STAGES;
         const uint32_t ph = (uint32_t)(it / GT_STAGES) & 1u;
         const int sp = it & 1;
-        if (sp == 0) load_rec(it / 2 + 1, nxt, nsz);   // prefetch the next 128-k record
+        if (sp == 0) {
+          load_rec(it / 2 + 1, nxt, nsz);              // prefetch the next 128-k record
+          // whole zero points of at most 1024 in size: every step of the fp16 arithmetic below is exact. One vote per record and
+          // two unrolled bodies: with a branch per word the eight words could not overlap (34816 x 5120, group 128, 127 tokens:
+          // 180 us, so 112; 148 before the test, with the pairs of the loop in local memory)
+          exact = true;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int qg = 0; qg < 4; ++qg) {
+              if (qg > 0 && GPT == 1) continue;
+              const __half z = __high2half(*reinterpret_cast<const __half2*>(&csz[i][qg]));
+              exact = exact && __heq(hrint(z), z) && __hle(__habs(z), z_max);
+            }
+          exact = __all_sync(0xffffffffu, exact);
+        }
         if (!gt_wait(&sm->empty[s], ph ^ 1u, sm, OWL_ERR_WAIT_MMA)) { ok = false; break; }
         uint8_t* tileB = sB + s * GT_TILE_BYTES;
+        auto dequant_stage = [&](auto whole) {
 #pragma unroll
-        for (int jh = 0; jh < 4; ++jh) {
-          const int r8 = (wq * 2 + (jh >> 1)) * 2 + (jh & 1);     // 8-row group index inside the 128-row tile
-          const uint32_t qw[4] = {cur[jh].x, cur[jh].y, cur[jh].z, cur[jh].w};
+          for (int jh = 0; jh < 4; ++jh) {
+            const int r8 = (wq * 2 + (jh >> 1)) * 2 + (jh & 1);     // 8-row group index inside the 128-row tile
+            const uint32_t qw[4] = {cur[jh].x, cur[jh].y, cur[jh].z, cur[jh].w};
 #pragma unroll
-          for (int wl = 0; wl < 2; ++wl) {
-            const int w = sp * 2 + wl;
-            const uint32_t szv = (p.group == 32) ? (sp ? (wl ? csz[jh][3] : csz[jh][2]) : (wl ? csz[jh][1] : csz[jh][0]))
-                                                 : csz[jh][0];
-            const __half2 szh = *reinterpret_cast<const __half2*>(&szv);
-            const __half sc = __low2half(szh), z = __high2half(szh);
-            const __half2 s2 = __half2half2(sc);
-            const __half2 z_lo = __hadd2(k1024, __half2half2(z));       // 1024 + z
-            const __half2 z_hi = __hneg2(__hadd2(k64, __half2half2(z))); // -(64 + z)
-            const uint32_t q = qw[w], q8 = q >> 8;
-            uint32_t t0 = (q & 0x000F000Fu) | 0x64006400u, t1 = (q & 0x00F000F0u) | 0x64006400u;
-            uint32_t t2 = (q8 & 0x000F000Fu) | 0x64006400u, t3 = (q8 & 0x00F000F0u) | 0x64006400u;
-            // low nibbles: (1024 + q) - (1024 + z); high nibbles: (1024 + 16 q) / 16 - (64 + z); both exact
-            __half2 h0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&t0), z_lo), s2);
-            __half2 h1 = __hmul2(__hfma2(*reinterpret_cast<__half2*>(&t1), k16th, z_hi), s2);
-            __half2 h2 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&t2), z_lo), s2);
-            __half2 h3 = __hmul2(__hfma2(*reinterpret_cast<__half2*>(&t3), k16th, z_hi), s2);
-            const int c = wl * 4 + t;        // 16-byte chunk inside the 128-byte row
-            uint4 o;
-            o.x = *reinterpret_cast<uint32_t*>(&h0); o.y = *reinterpret_cast<uint32_t*>(&h1);
-            o.z = *reinterpret_cast<uint32_t*>(&h2); o.w = *reinterpret_cast<uint32_t*>(&h3);
-            *reinterpret_cast<uint4*>(tileB + r8 * 1024 + g * 128 + ((c ^ g) << 4)) = o;
+            for (int wl = 0; wl < 2; ++wl) {
+              const int w = sp * 2 + wl;
+              const uint32_t szv = (p.group == 32) ? (sp ? (wl ? csz[jh][3] : csz[jh][2]) : (wl ? csz[jh][1] : csz[jh][0]))
+                                                   : csz[jh][0];
+              const __half2 szh = *reinterpret_cast<const __half2*>(&szv);
+              const __half sc = __low2half(szh), z = __high2half(szh);
+              const __half2 s2 = __half2half2(sc);
+              const uint32_t q = qw[w], q8 = q >> 8;
+              uint4 o;
+              if constexpr (decltype(whole)::value) {
+                const __half2 z_lo = __hadd2(k1024, __half2half2(z));       // 1024 + z
+                const __half2 z_hi = __hneg2(__hadd2(k64, __half2half2(z))); // -(64 + z)
+                uint32_t t0 = (q & 0x000F000Fu) | 0x64006400u, t1 = (q & 0x00F000F0u) | 0x64006400u;
+                uint32_t t2 = (q8 & 0x000F000Fu) | 0x64006400u, t3 = (q8 & 0x00F000F0u) | 0x64006400u;
+                // low nibbles: (1024 + q) - (1024 + z); high nibbles: (1024 + 16 q) / 16 - (64 + z); both exact
+                __half2 h0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&t0), z_lo), s2);
+                __half2 h1 = __hmul2(__hfma2(*reinterpret_cast<__half2*>(&t1), k16th, z_hi), s2);
+                __half2 h2 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&t2), z_lo), s2);
+                __half2 h3 = __hmul2(__hfma2(*reinterpret_cast<__half2*>(&t3), k16th, z_hi), s2);
+                o.x = *reinterpret_cast<uint32_t*>(&h0); o.y = *reinterpret_cast<uint32_t*>(&h1);
+                o.z = *reinterpret_cast<uint32_t*>(&h2); o.w = *reinterpret_cast<uint32_t*>(&h3);
+              } else {                         // fractional or large zero points (converted Q4_K blocks): 1024 + z would be rounded
+                const float sf = __half2float(sc), zf = __half2float(z);
+                float f[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) f[i] = ((float)((q >> (4 * ((i >> 1) + (i & 1) * 4))) & 0xF) - zf) * sf;
+                o = make_uint4(pack_f16(f[0], f[1]), pack_f16(f[2], f[3]), pack_f16(f[4], f[5]), pack_f16(f[6], f[7]));
+              }
+              const int c = wl * 4 + t;        // 16-byte chunk inside the 128-byte row
+              *reinterpret_cast<uint4*>(tileB + r8 * 1024 + g * 128 + ((c ^ g) << 4)) = o;
+            }
           }
-        }
+        };
+        if (exact) dequant_stage(std::true_type{});
+        else dequant_stage(std::false_type{});
         fence_async_smem();                  // generic-proxy writes -> visible to the MMA (async proxy)
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm->full_b[s]);

@@ -200,3 +200,12 @@ def test_rows_gemm_with_large_zero_points(t, n, k):
     w = _big_zeros(n, k, "slice")
     x = torch.randn(t, k, generator=torch.Generator().manual_seed(t)).half().to(DEV)
     _check_against_dequant(w, x, gemm_tc.w4_gemm_rows(w, x, torch.zeros(t, n, dtype=torch.bfloat16, device=DEV)))
+
+
+@pytest.mark.parametrize("layout", ["slice", "block"])
+@pytest.mark.parametrize("t", [33, 127])
+def test_tiled_gemm_with_large_zero_points(t, layout):
+    n, k = 112, 256
+    w = _big_zeros(n, k, layout)
+    x = torch.randn(t, k, generator=torch.Generator().manual_seed(t)).half().to(DEV)
+    _check_against_dequant(w, x, gemm_tc.w4a16_gemm(w, x, torch.zeros(t, n, dtype=torch.bfloat16, device=DEV)))
