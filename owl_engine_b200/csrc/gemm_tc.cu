@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(GT_THREADS, 2) gemm_tc_kernel(const __grid_con
           load_rec(it / 2 + 1, nxt, nsz);              // prefetch the next 128-k record
           // whole zero points of at most 1024 in size: every step of the fp16 arithmetic below is exact. One vote per record and
           // two unrolled bodies: with a branch per word the eight words could not overlap (34816 x 5120, group 128, 127 tokens:
-          // 180 us, so 112; 148 before the test, with the pairs of the loop in local memory)
+          // 180 us, so 116; 148 before the test, with the pairs of the loop in local memory)
           exact = true;
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -204,7 +204,9 @@ __global__ void __launch_bounds__(GT_THREADS, 2) gemm_tc_kernel(const __grid_con
             }
           exact = __all_sync(0xffffffffu, exact);
         }
-        if (!gt_wait(&sm->empty[s], ph ^ 1u, sm, OWL_ERR_WAIT_MMA)) { ok = false; break; }
+        // (the lanes leave together after a timeout: the others would wait for them in the next sync)
+        ok = __all_sync(0xffffffffu, gt_wait(&sm->empty[s], ph ^ 1u, sm, OWL_ERR_WAIT_MMA));
+        if (!ok) break;
         uint8_t* tileB = sB + s * GT_TILE_BYTES;
         auto dequant_stage = [&](auto whole) {
 #pragma unroll
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(GT_THREADS, 2) gemm_tc_kernel(const __grid_con
       }
     }
     // epilogue: warp reads its TMEM lane quarter (warp id % 4), one token row per thread
-    if (ok) ok = gt_wait(&sm->acc_full, 0, sm, OWL_ERR_WAIT_MMA);
+    if (ok) ok = __all_sync(0xffffffffu, gt_wait(&sm->acc_full, 0, sm, OWL_ERR_WAIT_MMA));
     if (ok) {
       tc_fence_after();
       const int q4 = warp & 3;
