@@ -999,7 +999,7 @@ class HybridRunner:
 
     def _dequant_ahead(self, t: int):
         """The ``DequantAhead`` of a ``t``-row chunk, started on this model's weights, or None: chunks above the sizes that read
-        the int4 records directly, on the arm that dequantises per chunk."""
+        the int4 records directly, on the arm that dequantises per chunk, with products long enough to hide it behind."""
         from ..ops import gemm_tc, linear
 
         if self.prefill_gemm not in ("tc", "tc4") or t <= gemm_tc.ROWS_UPTO or self.w.layout not in ("slice", "block") or not self.w.layers \
@@ -1007,7 +1007,7 @@ class HybridRunner:
             return None
         order = [w for lw in self.w.layers
                  for w in ((lw.qkvz, lw.out_proj) if lw.kind == "gdn" else (lw.qkv, lw.o_proj)) + (lw.gate_up, lw.down)]
-        if any(w.layout not in ("slice", "block") for w in order):
+        if any(w.layout not in ("slice", "block") for w in order) or not linear.ahead_pays(order, t):
             return None
         if self._ahead is None:
             self._ahead = linear.DequantAhead(self.device)

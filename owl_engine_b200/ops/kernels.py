@@ -654,11 +654,12 @@ def gguf_gemv(blocks, type_id: int, n: int, k: int, x, out, m: int) -> None:
     call("owl_gguf_gemv", ptr(blocks), type_id, ptr(x), x.stride(0), ptr(out), out.stride(0), m, n, k, stream())
 
 
-def w4_dequant(w, out=None):
-    """Dense bf16 (or fp16, by ``out.dtype``) [N, K] copy of a ``W4Skinny`` weight."""
+def w4_dequant(w, out=None, on: int | None = None):
+    """Dense bf16 (or fp16, by ``out.dtype``) [N, K] copy of a ``W4Skinny`` weight, launched on the current stream or on the
+    stream handle ``on``."""
     if out is None:
         out = torch.empty(w.n, w.k, dtype=torch.bfloat16, device=w.records.device)
-    call("owl_w4_dequant", ptr(w.records), ptr(out), w.n, w.k, w.group, w.layout_id, _is_f16(out), stream())
+    call("owl_w4_dequant", ptr(w.records), ptr(out), w.n, w.k, w.group, w.layout_id, _is_f16(out), stream() if on is None else on)
     return out
 
 

@@ -70,6 +70,17 @@ def _release_all(ledger, names: list) -> None:
         ledger.release(nm)
 
 
+# Weights x tokens of a chunk's projections, on average, from which they are dequantised one ahead: the hand-over between the two
+# streams costs the host about 7 us a projection, which a pass that waits for the host pays in full. Prompts with / without, ms:
+# 5 M weights a projection (0.8B) 400 tokens 6.2 / 6.0, 1000 6.5 / 6.7, 2048 8.2 / 8.6; 15 M 257 tokens 7.7 / 7.2, 700 8.6 / 9.0;
+# 28 M 400 tokens 10.6 / 10.7; 54 M 257 tokens 12.4 / 13.3; 95 M (27B) 257 tokens 37.9 / 39.2, 2048 115.9 / 118.9.
+AHEAD_FROM = 8e9
+
+
+def ahead_pays(weights: list, t: int) -> bool:
+    return sum(w.n * w.k for w in weights) * t >= AHEAD_FROM * len(weights)
+
+
 class DequantAhead:
     """Dequantises a chunk's weights one projection ahead, on a stream of its own: the dequantisation is bound by memory (44 us a
     projection of the 27B model, 11 of 112 ms at 2048 tokens), the GEMM beside it by the tensor cores. Two buffers alternate; a
@@ -78,6 +89,7 @@ class DequantAhead:
 
     def __init__(self, device):
         self.device, self.side = torch.device(device), torch.cuda.Stream(device=device)
+        self.free, self.ready = torch.cuda.Event(), torch.cuda.Event()      # a wait takes the state an event has when it is called
         self.buf, self.elems = [], 0
         self.names = [f"dequant ahead {id(self)} {i}" for i in range(2)]
         weakref.finalize(self, _release_all, _ledger(self.device), self.names)
@@ -99,7 +111,8 @@ class DequantAhead:
                 return False
             self.elems = need
         self.weights, self.i = weights, -1
-        self.free = torch.cuda.current_stream(self.device).record_event()
+        self.main = torch.cuda.current_stream(self.device)
+        self.free.record(self.main)
         self.kick()
         return True
 
@@ -111,17 +124,15 @@ class DequantAhead:
             return
         w = self.weights[j]
         self.side.wait_event(self.free)
-        with torch.cuda.stream(self.side):
-            K.w4_dequant(w, self.buf[j % 2][:w.n * w.k].view(w.n, w.k))
-            self.ready = self.side.record_event()
+        K.w4_dequant(w, self.buf[j % 2][:w.n * w.k].view(w.n, w.k), on=self.side.cuda_stream)
+        self.ready.record(self.side)
 
     def take(self, w) -> torch.Tensor:
-        """The dense copy of the chunk's next weight, valid for the GEMM launched next on the current stream."""
+        """The dense copy of the chunk's next weight, valid for the GEMM launched next on the chunk's stream."""
         self.i += 1
         assert self.weights[self.i] is w, "weights are taken in the order given to start()"
-        main = torch.cuda.current_stream(self.device)
-        main.wait_event(self.ready)
-        self.free = main.record_event()          # the other buffer's GEMM has been launched before this point
+        self.main.wait_event(self.ready)
+        self.free.record(self.main)              # the other buffer's GEMM has been launched before this point
         return self.buf[self.i % 2][:w.n * w.k].view(w.n, w.k)
 
 
