@@ -28,6 +28,7 @@ import weakref
 
 import torch
 
+from . import gemm_tc
 from . import kernels as K
 
 _scratch: dict = {}
@@ -138,16 +139,12 @@ class DequantAhead:
 
 def _rows_ok(w, x: torch.Tensor, out: torch.Tensor) -> bool:
     """Up to 256 rows of fp16: one launch reads the int4 records and dequantises each weight once."""
-    from . import gemm_tc
-
     return w.layout == "slice" and x.dtype == torch.float16 and x.shape[0] <= gemm_tc.ROWS_UPTO and x.stride(0) % 8 == 0 \
         and out.stride(0) % 8 == 0 and (x.data_ptr() | out.data_ptr()) % 16 == 0
 
 
 def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: DequantAhead | None = None) -> torch.Tensor:
     if ahead is not None:
-        from . import gemm_tc
-
         gemm_tc.f16_gemm(x, ahead.take(w), out)
         ahead.kick()
         return out
@@ -158,21 +155,17 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: Dequa
         return out
     resident = arm in ("tcr", "tc8r")
     if arm in ("tc8", "tc8r") and x.shape[0] >= DEQUANT_FROM and w.k % 128 == 0:
-        from . import gemm_tc
-
         wq, sw = _e4m3_weight(w, x.device, resident)
         xq, sx = gemm_tc.quant_e4m3_rows(x, *_fp8_scratch("x", x.shape[0], w.k, x.device))
         return gemm_tc.e4m3_gemm(xq, sx, wq, sw, out)
     if arm in ("tc", "tc8", "tcr", "tc8r"):
-        from . import gemm_tc
-
         if x.shape[0] <= SKINNY_UPTO and w.layout == "slice":
             # a handful of rows (the tail chunk after the last block boundary): the weight-streaming kernel
             t, k = x.shape
             xb = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
             rows = (t + 7) // 8 * 8
-            xp = torch.empty(rows, 2 * k, dtype=torch.uint8, device=x.device)
-            xs = torch.empty(rows, k // w.group, 2, dtype=torch.float32, device=x.device)
+            xp = torch.empty(rows * (2 * k + k // w.group * 8), dtype=torch.uint8, device=x.device)
+            xs = xp[rows * 2 * k:]                               # (scale, sum) pairs behind the packed rows
             if out.stride(0) % 2 or out.data_ptr() % 4:          # the integer arm stores single values
                 K.act_pack(xb, xp, xs, t, k, w.group)
                 K.w4a16_skinny(w, xp, xs, out, t, ldo=out.stride(0))
@@ -190,8 +183,6 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: Dequa
 
 def _e4m3_weight(w, device, resident: bool):
     """The weight as e4m3 rows with their scales: its resident copy (made on first use), or the shared scratch."""
-    from . import gemm_tc
-
     cached = getattr(w, "_owl_e4m3", None) if resident else None
     if cached is None:
         dense = K.w4_dequant(w, _dense_scratch(w.n, w.k, device, torch.float16))
@@ -208,8 +199,6 @@ SILU_FROM = 256         # tokens from which the persistent GEMM, which has the s
 def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: DequantAhead | None = None) -> bool:
     """out[T, N/2] (fp16) = silu(gate) * up of the merged gate / up projection in one launch. False (and nothing done) where the
     arm or the shape has no such epilogue: the caller multiplies and activates in two steps."""
-    from . import gemm_tc
-
     t = x.shape[0]
     if ahead is not None:
         if t < SILU_FROM or w.n < 512 or out.stride(0) % 8:
@@ -239,8 +228,6 @@ def nvfp4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.
     (W4A4) quantises the chunk's activations to NVFP4 with one scale per token and multiplies codes by codes on the
     block-scaled tensor-core path (``ops/nvfp4_tc.py``), with no dense copy of the weight at all; a handful of rows take the
     streaming GEMV."""
-    from . import gemm_tc
-
     t = x.shape[0]
     if arm == "tc4":
         from . import nvfp4_tc
@@ -264,8 +251,6 @@ def nvfp4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc") -> torch.
 
 def w4_e4m3(w, device):
     """Resident per-row e4m3 copy of a W4 weight: (bytes [N, K], fp32 row scales [N]), created on first use."""
-    from . import gemm_tc
-
     cached = getattr(w, "_owl_e4m3", None)
     if cached is None:
         dense = K.w4_dequant(w, _dense_scratch(w.n, w.k, device, torch.float16))
@@ -296,8 +281,6 @@ def dense_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, arm: str = "
     if arm == "baseline":
         torch.matmul(x.to(w.dtype), w.t(), out=out)
         return out
-    from . import gemm_tc
-
     if x.dtype != w.dtype:
         # the converted copy lives on the weight tensor itself (a cache keyed by address would hand a stale copy to the
         # next tensor allocated at that address)
