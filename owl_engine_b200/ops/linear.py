@@ -28,6 +28,7 @@ import weakref
 
 import torch
 
+from ..utils.ledger import BudgetError, ledger_for
 from . import gemm_tc
 from . import kernels as K
 
@@ -50,8 +51,6 @@ def _dense_scratch(n: int, k: int, device, dtype=torch.bfloat16) -> torch.Tensor
 
 
 def _ledger(device):
-    from ..utils.ledger import ledger_for
-
     return ledger_for(device)
 
 
@@ -91,26 +90,30 @@ class DequantAhead:
     def __init__(self, device):
         self.device, self.side = torch.device(device), torch.cuda.Stream(device=device)
         self.free, self.ready = torch.cuda.Event(), torch.cuda.Event()      # a wait takes the state an event has when it is called
-        self.buf, self.elems = [], 0
+        self.buf, self.elems, self.refused = [], 0, None
         self.names = [f"dequant ahead {id(self)} {i}" for i in range(2)]
         weakref.finalize(self, _release_all, _ledger(self.device), self.names)
 
     def start(self, weights: list) -> bool:
-        """Begin a chunk that multiplies ``weights`` in this order; False where the buffers do not fit the device's budget."""
+        """Begin a chunk that multiplies ``weights`` in this order; False where the buffers do not fit the device's budget or
+        its memory (asked again only once the ledger has more room than it had then)."""
         need = max(w.n * w.k for w in weights)
         if need > self.elems:
-            from ..utils.ledger import BudgetError
-
             led = _ledger(self.device)
+            if self.refused is not None and need >= self.refused[0] and led.room() <= self.refused[1]:
+                return False
             torch.cuda.current_stream(self.device).wait_stream(self.side)
             _release_all(led, self.names)
             self.buf, self.elems = [], 0
             try:
-                self.buf = [led.alloc(nm, "workspace", (need,), torch.float16) for nm in self.names]
-            except BudgetError:
+                for nm in self.names:
+                    self.buf.append(led.alloc(nm, "workspace", (need,), torch.float16))
+            except (BudgetError, torch.cuda.OutOfMemoryError):
+                self.buf = []
                 _release_all(led, self.names)
+                self.refused = (need, led.room())
                 return False
-            self.elems = need
+            self.elems, self.refused = need, None
         self.weights, self.i = weights, -1
         self.main = torch.cuda.current_stream(self.device)
         self.free.record(self.main)

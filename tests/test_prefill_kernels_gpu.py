@@ -6,6 +6,7 @@ from owl_engine_b200.ops import gemm_tc, linear
 from owl_engine_b200.ops import kernels as K
 from owl_engine_b200.ops import quant as Q
 from owl_engine_b200.ops import reference as R
+from owl_engine_b200.utils.ledger import DeviceLedger
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -209,3 +210,28 @@ def test_tiled_gemm_with_large_zero_points(t, layout):
     w = _big_zeros(n, k, layout)
     x = torch.randn(t, k, generator=torch.Generator().manual_seed(t)).half().to(DEV)
     _check_against_dequant(w, x, gemm_tc.w4a16_gemm(w, x, torch.zeros(t, n, dtype=torch.bfloat16, device=DEV)))
+
+
+class _FullDevice(DeviceLedger):
+    """A ledger without a budget on a device that has no memory left."""
+    tries = 0
+
+    def alloc(self, *a, **kw):
+        self.tries += 1
+        raise torch.cuda.OutOfMemoryError("out of memory")
+
+
+@pytest.mark.parametrize("full", [False, True])
+def test_dequantising_ahead_is_refused_without_room(full, monkeypatch):
+    """No room for the buffers, in the declared budget or on the device: start() says so, and asks again only once there is more."""
+    gen = torch.Generator().manual_seed(9)
+    w = Q.pack_skinny(Q.quantize_w4(torch.randn(512, 256, generator=gen) * 0.05, 128)).to(DEV)
+    led = _FullDevice("cuda:0") if full else DeviceLedger("cuda:0", total_bytes=512 * 256 * 2 + 100, enforce=True)
+    monkeypatch.setattr(linear, "ledger_for", lambda dev: led)
+    ahead = linear.DequantAhead(DEV)
+    assert not ahead.start([w]) and not led.entries
+    tries, refused = getattr(led, "tries", 0), led.refused
+    assert not ahead.start([w]) and (getattr(led, "tries", 0), led.refused) == (tries, refused)
+    if not full:
+        led.total *= 4
+        assert ahead.start([w])
