@@ -24,6 +24,7 @@ two arms:
 """
 from __future__ import annotations
 
+import threading
 import weakref
 
 import torch
@@ -39,6 +40,9 @@ SKINNY_UPTO = 32        # rows up to which the decode-shape weight-streaming ker
 
 def _dense_scratch(n: int, k: int, device, dtype=torch.bfloat16) -> torch.Tensor:
     key = (str(device), dtype)
+    shared = _ahead.get(str(torch.device(device))) if dtype == torch.float16 else None
+    if shared is not None and not shared.leave_scratch():
+        return torch.empty(n, k, dtype=dtype, device=device)
     buf = _scratch.get(key)
     if buf is None or buf.numel() < n * k:
         led = _ledger(device)
@@ -65,11 +69,6 @@ def _fp8_scratch(tag: str, r: int, k: int, device):
     return buf[0][:r * k].view(r, k), buf[1][:r]
 
 
-def _release_all(ledger, names: list) -> None:
-    for nm in names:
-        ledger.release(nm)
-
-
 # Weights x tokens of a chunk's projections, on average, from which they are dequantised one ahead: the hand-over between the two
 # streams costs the host about 7 us a projection, which a pass that waits for the host pays in full. Prompts with / without, ms:
 # 5 M weights a projection (0.8B) 400 tokens 6.2 / 6.0, 1000 6.5 / 6.7, 2048 8.2 / 8.6; 15 M 257 tokens 7.7 / 7.2, 700 8.6 / 9.0;
@@ -81,63 +80,144 @@ def ahead_pays(weights: list, t: int) -> bool:
     return sum(w.n * w.k for w in weights) * t >= AHEAD_FROM * len(weights)
 
 
+class _AheadShared:
+    """What the ``DequantAhead`` objects of a device share: the stream, and beside the dequantisation scratch one more buffer of
+    its size (356 MB for the 27B model), a ledger entry that goes when the last of them does. One chunk at a time holds both
+    buffers; a second one that starts meanwhile is refused and dequantises in line."""
+
+    NAME = "dequant ahead buffer"
+
+    def __init__(self, device):
+        self.device, self.side = device, torch.cuda.Stream(device=device)
+        self.free, self.ready = torch.cuda.Event(), torch.cuda.Event()      # a wait takes the state an event has when it is called
+        self.lock = threading.RLock()
+        self.users = weakref.WeakSet()
+        self.holder = self.last = None       # the object whose chunk has the buffers (weakly), and that chunk's stream
+        self.extra = self.ledger = self.refused = None
+        self.pending = False                 # a dequantisation has been launched that no stream but ``side`` waits for
+
+    def reserve(self, need: int):
+        """The second buffer, or None where it does not fit the device's budget or its memory (asked again only once the ledger
+        has more room than it had then)."""
+        led = _ledger(self.device)
+        if self.extra is None or self.extra.numel() < need or self.ledger is not led:
+            if self.refused is not None and self.refused[0] is led and need >= self.refused[1] and led.room() <= self.refused[2]:
+                return None
+            self.release()
+            try:
+                self.extra = led.alloc(self.NAME, "workspace", (need,), torch.float16)
+            except (BudgetError, torch.cuda.OutOfMemoryError):
+                self.refused = (led, need, led.room())
+                return None
+            self.ledger, self.refused = led, None
+        return self.extra
+
+    def release(self) -> None:
+        if self.extra is not None:
+            self.ledger.release(self.NAME)
+            self.extra = self.ledger = None
+
+    def leave_scratch(self) -> bool:
+        """The scratch is wanted for something else: a chunk of this thread that was not finished gives up its buffers, and the
+        current stream waits for what may still be written. False while a chunk of another thread holds them."""
+        with self.lock:
+            h = self.holder() if self.holder is not None else None
+            if h is not None and h.running:
+                if h.thread != threading.get_ident():
+                    return False
+                h.running = False
+            if self.pending:
+                torch.cuda.current_stream(self.device).wait_event(self.ready)
+                self.pending = False
+        return True
+
+    def user_gone(self) -> None:
+        # (from a finaliser: a thread that holds the lock is a user itself, and waiting for it here could be waiting for oneself)
+        if not list(self.users) and self.lock.acquire(blocking=False):
+            try:
+                self.release()
+            finally:
+                self.lock.release()
+
+
+_ahead: dict = {}         # device -> _AheadShared
+_ahead_lock = threading.Lock()
+
+
 class DequantAhead:
     """Dequantises a chunk's weights one projection ahead, on a stream of its own: the dequantisation is bound by memory (44 us a
     projection of the 27B model, 11 of 112 ms at 2048 tokens), the GEMM beside it by the tensor cores. Two buffers alternate; a
-    buffer is written again only after the GEMM that read it. One object per runner, used from the stream of its chunks: every
-    use of a buffer on either stream is ordered by events, and the buffers live as long as the object."""
+    buffer is written again only after the GEMM that read it. One object per runner; every use of a buffer on either stream is
+    ordered by events, and the allocator knows both streams. Once a chunk has lost its buffers ``take`` returns None."""
 
     def __init__(self, device):
-        self.device, self.side = torch.device(device), torch.cuda.Stream(device=device)
-        self.free, self.ready = torch.cuda.Event(), torch.cuda.Event()      # a wait takes the state an event has when it is called
-        self.buf, self.elems, self.refused = [], 0, None
-        self.names = [f"dequant ahead {id(self)} {i}" for i in range(2)]
-        weakref.finalize(self, _release_all, _ledger(self.device), self.names)
+        dev = torch.device(device)
+        if dev.index is None:
+            dev = torch.device(dev.type, torch.cuda.current_device())
+        with _ahead_lock:
+            if str(dev) not in _ahead:
+                _ahead[str(dev)] = _AheadShared(dev)
+        self.shared = sh = _ahead[str(dev)]
+        self.running, self.thread, self.buf = False, 0, ()
+        sh.users.add(self)
+        weakref.finalize(self, sh.user_gone).atexit = False
 
     def start(self, weights: list) -> bool:
-        """Begin a chunk that multiplies ``weights`` in this order; False where the buffers do not fit the device's budget or
-        its memory (asked again only once the ledger has more room than it had then)."""
-        need = max(w.n * w.k for w in weights)
-        if need > self.elems:
-            led = _ledger(self.device)
-            if self.refused is not None and need >= self.refused[0] and led.room() <= self.refused[1]:
+        """Begin a chunk that multiplies ``weights`` in this order on the current stream; False where there is no second buffer
+        or another chunk holds it."""
+        sh, need = self.shared, max(w.n * w.k for w in weights)
+        with sh.lock:
+            h = sh.holder() if sh.holder is not None else None
+            if h is not None and h is not self and h.running and h.thread != threading.get_ident():
                 return False
-            torch.cuda.current_stream(self.device).wait_stream(self.side)
-            _release_all(led, self.names)
-            self.buf, self.elems = [], 0
-            try:
-                for nm in self.names:
-                    self.buf.append(led.alloc(nm, "workspace", (need,), torch.float16))
-            except (BudgetError, torch.cuda.OutOfMemoryError):
-                self.buf = []
-                _release_all(led, self.names)
-                self.refused = (need, led.room())
+            if h is not None:
+                h.running = False
+            scratch = _dense_scratch(1, need, sh.device, torch.float16).view(-1)
+            extra = sh.reserve(need)
+            if extra is None:
                 return False
-            self.elems, self.refused = need, None
-        self.weights, self.i = weights, -1
-        self.main = torch.cuda.current_stream(self.device)
-        self.free.record(self.main)
+            self.main = torch.cuda.current_stream(sh.device)
+            if sh.last is not None and sh.last != self.main:
+                self.main.wait_stream(sh.last)       # the last chunk's products, on another stream
+            sh.last, sh.holder = self.main, weakref.ref(self)
+            self.buf = (scratch, extra)
+            for b in self.buf:
+                b.record_stream(sh.side)
+                b.record_stream(self.main)
+            self.weights, self.i, self.running, self.thread = weights, -1, True, threading.get_ident()
+            sh.free.record(self.main)
         self.kick()
         return True
 
     def kick(self) -> None:
         """Launch the next weight's dequantisation. Called after the GEMM beside which it is to run has been launched: the GEMM's
         CTAs take their place on the SMs first."""
-        j = self.i + 1
-        if j >= len(self.weights):
-            return
-        w = self.weights[j]
-        self.side.wait_event(self.free)
-        K.w4_dequant(w, self.buf[j % 2][:w.n * w.k].view(w.n, w.k), on=self.side.cuda_stream)
-        self.ready.record(self.side)
+        sh, j = self.shared, self.i + 1
+        with sh.lock:
+            if not self.running:
+                return
+            if j >= len(self.weights):
+                self.running, self.buf = False, ()
+                return
+            w = self.weights[j]
+            sh.side.wait_event(sh.free)
+            K.w4_dequant(w, self.buf[j % 2][:w.n * w.k].view(w.n, w.k), on=sh.side.cuda_stream)
+            sh.ready.record(sh.side)
+            sh.pending = True
 
-    def take(self, w) -> torch.Tensor:
+    def take(self, w) -> torch.Tensor | None:
         """The dense copy of the chunk's next weight, valid for the GEMM launched next on the chunk's stream."""
-        self.i += 1
-        assert self.weights[self.i] is w, "weights are taken in the order given to start()"
-        self.main.wait_event(self.ready)
-        self.free.record(self.main)              # the other buffer's GEMM has been launched before this point
-        return self.buf[self.i % 2][:w.n * w.k].view(w.n, w.k)
+        sh = self.shared
+        with sh.lock:
+            self.i += 1
+            assert self.weights[self.i] is w, "weights are taken in the order given to start()"
+            if not self.running:
+                self.buf = ()
+                return None
+            self.main.wait_event(sh.ready)
+            sh.pending = False
+            sh.free.record(self.main)            # the other buffer's GEMM has been launched before this point
+            return self.buf[self.i % 2][:w.n * w.k].view(w.n, w.k)
 
 
 def _rows_ok(w, x: torch.Tensor, out: torch.Tensor) -> bool:
@@ -147,8 +227,9 @@ def _rows_ok(w, x: torch.Tensor, out: torch.Tensor) -> bool:
 
 
 def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: DequantAhead | None = None) -> torch.Tensor:
-    if ahead is not None:
-        gemm_tc.f16_gemm(x, ahead.take(w), out)
+    dense = ahead.take(w) if ahead is not None else None
+    if dense is not None:
+        gemm_tc.f16_gemm(x, dense, out)
         ahead.kick()
         return out
     arm = "tc" if arm == "tc4" else arm                    # the 4-bit float product exists for NVFP4 weights only
@@ -204,9 +285,12 @@ def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: 
     arm or the shape has no such epilogue: the caller multiplies and activates in two steps."""
     t = x.shape[0]
     if ahead is not None:
-        if t < SILU_FROM or w.n < 512 or out.stride(0) % 8:
+        if w.n < 512 or out.stride(0) % 8:
             return False
-        gemm_tc.gemm_silu(x, ahead.take(w), out)
+        dense = ahead.take(w)
+        if dense is None:
+            dense = w4_dense(w, x.dtype, x.device)
+        gemm_tc.gemm_silu(x, dense, out)
         ahead.kick()
         return True
     if w.layout == "nvfp4" or x.dtype != torch.float16 or out.dtype != torch.float16 or out.stride(0) % 8:

@@ -1,4 +1,7 @@
 """Prompt-sized forms of the prefill kernels against the forms that short inputs take."""
+import gc
+from concurrent.futures import ThreadPoolExecutor
+
 import pytest
 import torch
 
@@ -221,17 +224,67 @@ class _FullDevice(DeviceLedger):
         raise torch.cuda.OutOfMemoryError("out of memory")
 
 
+def _int4(shapes, seed):
+    gen = torch.Generator().manual_seed(seed)
+    return [Q.pack_skinny(Q.quantize_w4(torch.randn(n, k, generator=gen) * 0.05, 128)).to(DEV) for n, k in shapes]
+
+
 @pytest.mark.parametrize("full", [False, True])
 def test_dequantising_ahead_is_refused_without_room(full, monkeypatch):
-    """No room for the buffers, in the declared budget or on the device: start() says so, and asks again only once there is more."""
-    gen = torch.Generator().manual_seed(9)
-    w = Q.pack_skinny(Q.quantize_w4(torch.randn(512, 256, generator=gen) * 0.05, 128)).to(DEV)
-    led = _FullDevice("cuda:0") if full else DeviceLedger("cuda:0", total_bytes=512 * 256 * 2 + 100, enforce=True)
+    """No room for the second buffer, in the declared budget or on the device: start() says so, and asks again only once there is
+    more."""
+    (w,) = _int4([(512, 256)], 9)
+    linear._dense_scratch(512, 256, w.records.device, torch.float16)       # the first one is the scratch
+    led = _FullDevice("cuda:0") if full else DeviceLedger("cuda:0", total_bytes=1000, enforce=True)
     monkeypatch.setattr(linear, "ledger_for", lambda dev: led)
     ahead = linear.DequantAhead(DEV)
     assert not ahead.start([w]) and not led.entries
     tries, refused = getattr(led, "tries", 0), led.refused
     assert not ahead.start([w]) and (getattr(led, "tries", 0), led.refused) == (tries, refused)
     if not full:
-        led.total *= 4
+        led.total *= 1000
         assert ahead.start([w])
+
+
+def test_runners_of_a_device_share_the_buffer(monkeypatch):
+    """One second buffer per device, held by one chunk at a time, given back with the last runner."""
+    ws = _int4([(512, 256), (256, 512)], 10)
+    led = DeviceLedger("cuda:0")
+    monkeypatch.setattr(linear, "ledger_for", lambda dev: led)
+    linear._dense_scratch(512, 256, ws[0].records.device, torch.float16)
+    mine = lambda: [e for n, e in led.entries.items() if n.startswith("dequant ahead")]
+    a, b = linear.DequantAhead(DEV), linear.DequantAhead(DEV)
+    with ThreadPoolExecutor(1) as other:
+        assert a.start(ws) and len(mine()) == 1
+        assert not other.submit(b.start, ws).result()                     # a's chunk has the buffers
+        x = torch.randn(300, 256, device=DEV).half()
+        # the scratch is one of them: another thread's product in line must not write it
+        got = other.submit(linear.w4_gemm, ws[0], x, torch.empty(300, 512, dtype=torch.bfloat16, device=DEV)).result()
+        for w in ws:
+            xw = torch.randn(300, w.k, device=DEV).half()
+            out = linear.w4_gemm(w, xw, torch.empty(300, w.n, dtype=torch.bfloat16, device=DEV), ahead=a)
+            assert torch.equal(out, gemm_tc.f16_gemm(xw, K.w4_dequant(w, torch.empty(w.n, w.k, dtype=torch.float16, device=DEV)), torch.empty_like(out)))
+        assert torch.equal(got, linear.w4_gemm(ws[0], x, torch.empty_like(got)))
+        assert other.submit(b.start, ws).result() and len(mine()) == 1    # a's chunk has ended
+    del a, b
+    gc.collect()
+    assert not mine()
+
+
+def test_unfinished_chunk_gives_its_buffers_up():
+    """A chunk that ended in an exception leaves a dequantisation under way: the next user of the scratch waits for it, and the
+    chunk's object dequantises in line until it starts again."""
+    ws = _int4([(512, 256), (256, 512), (1024, 256)], 11)
+    ahead = linear.DequantAhead(DEV)
+    x = [torch.randn(300, w.k, device=DEV).half() for w in ws]
+    empty = lambda w: torch.empty(300, w.n, dtype=torch.bfloat16, device=DEV)
+    want = [linear.w4_gemm(w, xw, empty(w)) for w, xw in zip(ws, x)]
+    assert ahead.start(ws)
+    first = linear.w4_gemm(ws[0], x[0], empty(ws[0]), ahead=ahead)
+    inline = linear.w4_gemm(ws[2], x[2], empty(ws[2]))
+    rest = [linear.w4_gemm(w, xw, empty(w), ahead=ahead) for w, xw in zip(ws[1:], x[1:])]
+    for got, w in zip([first, inline] + rest, [want[0], want[2], want[1], want[2]]):
+        assert torch.equal(got, w)
+    assert ahead.start(ws)
+    for w, xw, y in zip(ws, x, want):
+        assert torch.equal(linear.w4_gemm(w, xw, empty(w), ahead=ahead), y)
