@@ -82,8 +82,8 @@ def ahead_pays(weights: list, t: int) -> bool:
 
 class _AheadShared:
     """What the ``DequantAhead`` objects of a device share: the stream, and beside the dequantisation scratch one more buffer of
-    its size (356 MB for the 27B model), a ledger entry that goes when the last of them does. One chunk at a time holds both
-    buffers; a second one that starts meanwhile is refused and dequantises in line."""
+    its size (356 MB for the 27B model), a ledger entry that goes when the last of them does or when another entry needs the
+    room. One chunk at a time holds both buffers; a second one that starts meanwhile is refused and dequantises in line."""
 
     NAME = "dequant ahead buffer"
 
@@ -105,12 +105,25 @@ class _AheadShared:
                 return None
             self.release()
             try:
+                # allocations that no ledger makes cannot ask for it back: as much again has to stay free
+                free = torch.cuda.mem_get_info(self.device)[0]
+                if free + torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device) < 4 * need:
+                    raise BudgetError(self.NAME)
                 self.extra = led.alloc(self.NAME, "workspace", (need,), torch.float16)
             except (BudgetError, torch.cuda.OutOfMemoryError):
                 self.refused = (led, need, led.room())
                 return None
             self.ledger, self.refused = led, None
+            led.on_pressure(self.give_back)
         return self.extra
+
+    def give_back(self) -> None:
+        """Another entry needs the room: a chunk under way dequantises its other weights in line."""
+        with self.lock:
+            h = self.holder() if self.holder is not None else None
+            if h is not None:
+                h.running = False
+            self.release()
 
     def release(self) -> None:
         if self.extra is not None:

@@ -48,6 +48,7 @@ class DeviceLedger:
         self._storages: dict[int, str] = {}
         self._lock = threading.Lock()
         self.refused = 0
+        self._give_back: list = []
 
     # -- budget ---------------------------------------------------------------------------------------------------------
     def _total(self) -> int:
@@ -69,8 +70,20 @@ class DeviceLedger:
     def room(self) -> int:
         return self.avail - self.used()
 
+    def on_pressure(self, give_back) -> None:
+        """``give_back()`` is called, from any thread, when a request does not fit: it releases entries that are only a
+        convenience to their owner."""
+        if give_back not in self._give_back:
+            self._give_back.append(give_back)
+
+    def _make_room(self) -> None:
+        for f in list(self._give_back):
+            f()
+
     def check(self, name: str, nbytes: int) -> None:
         """Refuse (when enforcing) a request that does not fit what is left of the declared budget."""
+        if self.enforce and nbytes > self.room():
+            self._make_room()
         if self.enforce and nbytes > self.room():
             self.refused += 1
             raise BudgetError(f"{name}: {nbytes / 2**20:.1f} MiB requested, {max(0, self.room()) / 2**20:.1f} MiB left of the "
@@ -89,7 +102,14 @@ class DeviceLedger:
             n *= int(s)
         nbytes = n * torch.empty(0, dtype=dtype).element_size()
         self.check(name, nbytes)
-        t = (torch.zeros if zero else torch.empty)(shape, dtype=dtype, device=self.device)
+        make = torch.zeros if zero else torch.empty
+        try:
+            t = make(shape, dtype=dtype, device=self.device)
+        except torch.cuda.OutOfMemoryError:
+            if not self._give_back:
+                raise
+            self._make_room()
+            t = make(shape, dtype=dtype, device=self.device)
         self.track(name, klass, t)
         return t
 

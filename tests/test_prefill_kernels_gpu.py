@@ -243,6 +243,9 @@ def test_dequantising_ahead_is_refused_without_room(full, monkeypatch):
     assert not ahead.start([w]) and (getattr(led, "tries", 0), led.refused) == (tries, refused)
     if not full:
         led.total *= 1000
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev: (-(1 << 50), 0))      # nothing would stay free
+        assert not ahead.start([w])
+        monkeypatch.undo()
         assert ahead.start([w])
 
 
@@ -288,3 +291,20 @@ def test_unfinished_chunk_gives_its_buffers_up():
     assert ahead.start(ws)
     for w, xw, y in zip(ws, x, want):
         assert torch.equal(linear.w4_gemm(w, xw, empty(w), ahead=ahead), y)
+
+
+def test_second_buffer_makes_room_for_other_entries(monkeypatch):
+    """An entry that does not fit the budget beside the second buffer gets its room, in the middle of a chunk."""
+    ws = _int4([(512, 256), (256, 512), (1024, 128)], 12)
+    led = DeviceLedger("cuda:0", total_bytes=512 * 256 * 2 + 1000, enforce=True)
+    linear._dense_scratch(512, 256, ws[0].records.device, torch.float16)
+    monkeypatch.setattr(linear, "ledger_for", lambda dev: led)
+    ahead = linear.DequantAhead(DEV)
+    assert ahead.start(ws)
+    for i, w in enumerate(ws):
+        x = torch.randn(300, w.k, device=DEV).half()
+        out = linear.w4_gemm(w, x, torch.empty(300, w.n, dtype=torch.bfloat16, device=DEV), ahead=ahead)
+        if i == 0:
+            led.alloc("other", "workspace", (5000,), torch.uint8)
+        assert torch.equal(out, gemm_tc.f16_gemm(x, K.w4_dequant(w, torch.empty(w.n, w.k, dtype=torch.float16, device=DEV)), torch.empty_like(out)))
+    assert list(led.entries) == ["other"] and not ahead.start(ws)
