@@ -308,3 +308,31 @@ def test_second_buffer_makes_room_for_other_entries(monkeypatch):
             led.alloc("other", "workspace", (5000,), torch.uint8)
         assert torch.equal(out, gemm_tc.f16_gemm(x, K.w4_dequant(w, torch.empty(w.n, w.k, dtype=torch.float16, device=DEV)), torch.empty_like(out)))
     assert list(led.entries) == ["other"] and not ahead.start(ws)
+
+
+# products that take longer than a dequantisation, and the other way round
+@pytest.mark.parametrize("t,shapes", [(4096, ((2048, 1024), (1024, 2048), (2048, 512), (512, 1024), (1024, 1024))),
+                                      (16, ((34816, 1280), (5120, 8704), (16384, 2560)))])
+def test_dequantising_ahead_without_host_waits(t, shapes):
+    """Two chunks with nothing between the projections that the host or the stream would wait for: results are looked at after the
+    last launch only."""
+    ws = _int4(shapes, t)
+    gen = torch.Generator(device=DEV).manual_seed(t)
+    x = [torch.randn(t, w.k, device=DEV, generator=gen).half() for w in ws]
+    empty = lambda w: torch.empty(t, w.n, dtype=torch.bfloat16, device=DEV)
+    dense = [K.w4_dequant(w, torch.empty(w.n, w.k, dtype=torch.float16, device=DEV)) for w in ws]
+    want = [gemm_tc.f16_gemm(xw, d, empty(w)) for w, xw, d in zip(ws, x, dense)]
+    out = [[empty(w).zero_() for w in ws] for _ in range(2)]
+    ahead = linear.DequantAhead(DEV)
+    assert ahead.start(ws)                                                # (allocates)
+    for w, xw, y in zip(ws, x, out[0]):
+        linear.w4_gemm(w, xw, y, ahead=ahead)
+    torch.cuda.synchronize()
+    out[0][0].zero_()
+    for o in out:
+        ahead.start(ws)
+        for w, xw, y in zip(ws, x, o):
+            linear.w4_gemm(w, xw, y, ahead=ahead)
+    for o in out:
+        for got, y in zip(o, want):
+            assert torch.equal(got, y)
