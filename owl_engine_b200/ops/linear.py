@@ -35,6 +35,8 @@ from . import kernels as K
 
 _scratch: dict = {}
 DEQUANT_FROM = 128      # tokens per chunk from which dequantise-once + dense GEMM wins
+SILU_FROM = 256         # tokens from which the persistent GEMM, which has the silu(gate) * up epilogue, multiplies fp16 weights
+SMS = 148               # of the part all sizes here were measured on
 SKINNY_UPTO = 32        # rows up to which the decode-shape weight-streaming kernel is used instead of a GEMM
 
 
@@ -233,9 +235,25 @@ class DequantAhead:
             return self.buf[self.i % 2][:w.n * w.k].view(w.n, w.k)
 
 
-def _rows_ok(w, x: torch.Tensor, out: torch.Tensor) -> bool:
-    """Up to 256 rows of fp16: one launch reads the int4 records and dequantises each weight once."""
-    return w.layout == "slice" and x.dtype == torch.float16 and x.shape[0] <= gemm_tc.ROWS_UPTO and x.stride(0) % 8 == 0 \
+def rows_pay(n: int, k: int, t: int, resident: bool) -> bool:
+    """Whether ``t`` tokens times an [n, k] int4 weight read the records (``gemm_w4.cu``) rather than a dense copy.
+
+    Up to 256 tokens, all that one launch takes (from 257 a second pass over the records would cost 109 us at 16384 x 5120, the
+    dequantisation and the dense GEMM 111 and, one projection ahead, less). A resident copy needs no dequantisation: it is the
+    better operand at 256 tokens (the persistent kernel: 16384 x 5120 44 against 63 us, 34816 x 5120 87 / 115, 5120 x 17408 60 / 73;
+    the 27B prompt 23.2 / 27.0 ms) and, from 128, where its 128 x 128 tiles fit two per SM and k is short (16384 x 5120 46 / 49 us at
+    137 tokens, 50 / 63 at 255); not where a tile walks a long k alone or the tiles take two waves (5120 x 17408 118 / 52 us,
+    34816 x 5120 121 / 89)."""
+    if t > gemm_tc.ROWS_UPTO:
+        return False
+    if not resident or t < DEQUANT_FROM:
+        return True
+    return t < SILU_FROM and (n < 2 * k or -(-n // 128) * -(-t // 128) > 2 * SMS)
+
+
+def _rows_ok(w, x: torch.Tensor, out: torch.Tensor, resident: bool) -> bool:
+    """One launch reads the int4 records and dequantises each weight once."""
+    return w.layout == "slice" and x.dtype == torch.float16 and rows_pay(w.n, w.k, x.shape[0], resident) and x.stride(0) % 8 == 0 \
         and out.stride(0) % 8 == 0 and (x.data_ptr() | out.data_ptr()) % 16 == 0
 
 
@@ -270,7 +288,7 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: Dequa
             K.act_pack(xb, xp, xs, t, k, w.group | K.ACT_FRAG)
             K.w4_mma(w, xp, xs, out, t, ldo=out.stride(0))
             return out
-        if _rows_ok(w, x, out):
+        if _rows_ok(w, x, out, resident):
             return gemm_tc.w4_gemm_rows(w, x, out)
         if x.shape[0] >= DEQUANT_FROM:
             return gemm_tc.f16_gemm(x, w4_dense(w, x.dtype, x.device, resident=resident), out)
@@ -288,9 +306,6 @@ def _e4m3_weight(w, device, resident: bool):
             _ledger(device).track("resident e4m3 weight copy", "resident copies", cached[0])
             w._owl_e4m3 = cached
     return cached
-
-
-SILU_FROM = 256         # tokens from which the persistent GEMM, which has the silu(gate) * up epilogue, multiplies fp16 weights
 
 
 def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: DequantAhead | None = None) -> bool:
@@ -313,7 +328,7 @@ def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: 
         xq, sx = gemm_tc.quant_e4m3_rows(x, *_fp8_scratch("x", t, w.k, x.device))
         gemm_tc.gemm_silu(xq, wq, out, sx, sw)
         return True
-    if arm in ("tc", "tc4", "tcr", "tc8", "tc8r") and t > SKINNY_UPTO and _rows_ok(w, x, out):
+    if arm in ("tc", "tc4", "tcr", "tc8", "tc8r") and t > SKINNY_UPTO and _rows_ok(w, x, out, arm in ("tcr", "tc8r")):
         gemm_tc.w4_gemm_rows(w, x, out, silu=True)
         return True
     if arm in ("tc", "tc4", "tcr", "tc8", "tc8r") and t >= SILU_FROM and w.n >= 512:

@@ -21,3 +21,11 @@ def _projections(name):
                                           ("qwen3.5-0.8b", 1000, False), ("qwen3.5-0.8b", 2048, True)])
 def test_small_models_do_not_pay_for_dequantising_ahead(model, t, pays):
     assert linear.ahead_pays(_projections(model), t) == pays
+
+
+@pytest.mark.parametrize("n,k,t,resident,rows", [(16384, 5120, 256, False, True), (16384, 5120, 257, False, False), (1024, 3584, 256, False, True),
+                                                 (16384, 5120, 256, True, False), (5120, 17408, 256, True, False), (5120, 17408, 255, True, True),
+                                                 (16384, 5120, 255, True, False), (34816, 5120, 128, True, False), (34816, 5120, 129, True, True),
+                                                 (16384, 5120, 127, True, True), (5120, 17408, 33, True, True)])
+def test_operand_of_a_short_prompt(n, k, t, resident, rows):
+    assert linear.rows_pay(n, k, t, resident) == rows

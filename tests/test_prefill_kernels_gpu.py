@@ -336,3 +336,19 @@ def test_dequantising_ahead_without_host_waits(t, shapes):
     for o in out:
         for got, y in zip(o, want):
             assert torch.equal(got, y)
+
+
+@pytest.mark.parametrize("t", [127, 128, 255, 256, 257])
+def test_resident_copy_and_records_give_one_product(t):
+    """Both sides of every limit of the resident arm, with the activation and without, against the 16-bit product of the same
+    weights (bf16 results of fp32 sums)."""
+    (w,) = _int4([(1024, 512)], t)
+    x = torch.randn(t, 512, generator=torch.Generator().manual_seed(t)).half().to(DEV)
+    dense = K.w4_dequant(w, torch.empty(1024, 512, dtype=torch.float16, device=DEV)).double()
+    want, size = x.double() @ dense.t(), x.double().abs() @ dense.abs().t()
+    out = linear.w4_gemm(w, x, torch.empty(t, 1024, dtype=torch.bfloat16, device=DEV), arm="tcr")
+    assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -18).all()
+    act = torch.empty(t, 512, dtype=torch.float16, device=DEV)
+    if not linear.w4_gemm_silu(w, x, act, arm="tcr"):
+        K.silu_mul(out, t, 512, out=act)
+    torch.testing.assert_close(act.float(), _silu_ref(out).float(), rtol=2.0 ** -9, atol=2.0 ** -20)
