@@ -542,9 +542,11 @@ static int dispatch_mma(MmaParams& p, int epi, int pdl, cudaStream_t st) {
   p.ab_blocks = (p.ab_rows + 15) / 16;
   const int row_blocks = (p.n_tiles + MM_TILES - 1) / MM_TILES;
   const int blocks = row_blocks + p.ab_blocks, sms = mm_sms();
-  // k parts: as many as one wave of four CTAs per SM holds, at most one record column each; independent of M
+  // k parts: as many as one wave of four CTAs per SM holds, each of at least two record columns; independent of M. With one
+  // column a part is all start-up and exchange (8192 x 1024, group 128, 1 / 8 / 32 rows: 8 parts 4.6 / 5.0 / 11.6 us, 4 parts 3.8 /
+  // 4.0 / 8.1; a column more loses where it takes CTAs away: 1024 x 2048 2.8 -> 3.1).
   int KS = 8;
-  while (KS > 1 && (row_blocks * KS > 4 * sms || KS > (p.K >> 7))) KS >>= 1;
+  while (KS > 1 && (row_blocks * KS > 4 * sms || 2 * KS > (p.K >> 7))) KS >>= 1;
   // Grids of up to three CTAs per SM run with three resident and a deeper ring: with four slots per SM the scheduler fills
   // some SMs with four CTAs and others with two (5120 x 17408, one row: 12.9 against 15.3 us). NVFP4 above 16 rows has registers
   // for three only.

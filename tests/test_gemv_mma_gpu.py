@@ -119,3 +119,11 @@ def test_extremes_of_the_activations(fmt):
     assert (out[0] == 0).all() and out[3].isnan().all()
     for r in (1, 2, 4):
         assert (out[r].double().cpu() - want[r]).norm() / want[r].norm() < 4e-3
+
+
+# k parts of two record columns at least: 3 and 4 columns in one and two parts, 7 in two, 8 in four
+@pytest.mark.parametrize("fmt", ["g128", "g32", "nvfp4"])
+@pytest.mark.parametrize("shape", [(144, 512), (144, 896), (16, 1024), (20480, 1024)])
+@pytest.mark.parametrize("m", [1, 32])
+def test_k_parts_of_narrow_matrices(fmt, shape, m):
+    test_mma_streaming_matches_dequantised_product(fmt, shape, m)
