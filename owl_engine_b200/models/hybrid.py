@@ -654,9 +654,14 @@ class HybridRunner:
         if self.uniform_rows:
             b = 8        # a speculating engine: the split of the keys (and with it the order of the partial sums) must not
                          # depend on how many sequences share the step, or batched verify rows round differently from plain ones
-        # two CTAs per SM, four for many sequences: with unequal lengths the longest part is what the launch takes (32 sequences of
-        # 1k to 8k tokens: 125 against 149 us a layer; 8 sequences: 24 against 20, the parts get too short)
-        want = max(1, ((4 if b >= 16 else 2) * 148) // max(1, b * self.spec.hkv))
+        # two CTAs per SM; four for many sequences, whose lengths differ, where a part keeps 16 pages: the longest part is what the
+        # launch takes. A layer (projection to reduction) at twice the parts: 32 sequences of 1k to 8k tokens 238 -> 150 us, 16 90 ->
+        # 66, 24 of 500 to 4000 76 -> 64, 32 of 100 to 2000 86 -> 66. Equal lengths lose: 24 of 2000 57.9 -> 63.2, 32 96 -> 99, of
+        # 8000 267 -> 270; with less than 16 pages a part everything does: 16 of 2000 44.6 -> 47.6, of 300 to 600 32.2 -> 35.2. So do
+        # few sequences: 8 of 2000 31.7 -> 35.6, of 400 to 4000 36.7 -> 37.1
+        want = max(1, 2 * 148 // max(1, b * self.spec.hkv))
+        if b >= 16 and pages >= 16 * (4 * 148 // (b * self.spec.hkv)):
+            want = max(1, 4 * 148 // (b * self.spec.hkv))
         return max(1, min(self.max_splits, want, (pages + 3) // 4))
 
     def _full(self, lw: LayerWeights, li: int, lay: StepLayout, v: dict, splits: int, ctx_hint: int = 0) -> None:

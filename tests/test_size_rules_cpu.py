@@ -1,8 +1,9 @@
-"""Size rules of the prompt path (no GPU: the rules look at sizes only)."""
+"""Size rules of the prompt and step paths (no GPU: the rules look at sizes only)."""
 from types import SimpleNamespace
 
 import pytest
 
+from owl_engine_b200.models.hybrid import HybridRunner
 from owl_engine_b200.models.spec import PRESETS
 from owl_engine_b200.ops import linear
 
@@ -29,3 +30,12 @@ def test_small_models_do_not_pay_for_dequantising_ahead(model, t, pays):
                                                  (16384, 5120, 127, True, True), (5120, 17408, 33, True, True)])
 def test_operand_of_a_short_prompt(n, k, t, resident, rows):
     assert linear.rows_pay(n, k, t, resident) == rows
+
+
+# (sequences, longest context, uniform rows) -> parts of a sequence's keys, 27B head geometry (4 kv heads)
+@pytest.mark.parametrize("b,ctx,uniform,parts", [(1, 2048, False, 32), (8, 8192, False, 9), (15, 8192, False, 4), (16, 8192, False, 9),
+                                                 (16, 2048, False, 4), (16, 2304, False, 9), (24, 2048, False, 6), (32, 1024, False, 4),
+                                                 (32, 1008, False, 2), (32, 8192, True, 9), (32, 16, False, 1)])
+def test_parts_of_the_keys(b, ctx, uniform, parts):
+    r = SimpleNamespace(attn_splits=0, uniform_rows=uniform, max_splits=64, spec=PRESETS["qwen3.8-27b"]())
+    assert HybridRunner._pick_splits(r, b, ctx) == parts
