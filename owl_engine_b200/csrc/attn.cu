@@ -555,10 +555,11 @@ static int insert_launch(const void* qraw, int ldq, const void* kraw, int ldk, c
   p.k_pool = (uint8_t*)k_pool; p.v_pool = (uint8_t*)v_pool; p.k_scale = (float*)k_scale; p.v_scale = (float*)v_scale;
   p.rows = rows; p.hq = hq; p.hkv = hkv; p.hd = hd; p.kv16 = kv16;
   p.rot = rot; p.eps = eps; p.rope_scale = rope_scale;
-  // A CTA per row fills the chip from about 148 rows on; decode steps of a few rows want a CTA per head (3.6 us at 1 to 32 rows).
+  // A CTA per row takes 5.7 us up to 148 rows of 24 + 8 heads and 3.8 of 8 + 4; a CTA per (row, head) grows with their product: 24 +
+  // 8 heads 137 rows 5.65 us, 160 6.47 (by rows 6.16), 256 9.6 (6.3), 2048 68.8 (20.8); 8 + 4 heads 192 rows 3.5 (4.0), 256 4.8 (4.0).
   const uintptr_t al = (uintptr_t)qraw | (uintptr_t)kraw | (uintptr_t)vraw | (uintptr_t)qnorm_w | (uintptr_t)knorm_w |
                        (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool;
-  if (rows >= 128 && !pdl && hd == 256 && !(rot & 15) && !((ldq | ldk | ldv) & 7) && !(al & 15)) {
+  if (rows >= 160 && (long long)rows * (hq + 2 * hkv) >= 3072 && !pdl && hd == 256 && !(rot & 15) && !((ldq | ldk | ldv) & 7) && !(al & 15)) {
     qknorm_rope_insert_rows_kernel<<<rows, QI_WARPS * 32, 0, st>>>(p);
     OWL_LAUNCH_CHECK();
     return OWL_OK;
