@@ -281,8 +281,10 @@ __global__ void __launch_bounds__(256) gdn_decode_kernel(GdnDecodeParams p) {
 // Prefill conv: one warp per (TR consecutive t, 128-channel segment). Segments 0..2nk-1 are q/k heads (get
 // l2norm), the rest are v heads. Reads the 3-sample history from conv_state for t < 3. Output bf16 [T][conv_dim].
 // Memory bound (every input read once, every output written once: 13 us at 2048 tokens of 10240 channels). With one t per
-// warp (TR = 1) the four taps were four loads and the weights four more per output row: 56 us; TR = 8 loads 11 rows for 8
-// outputs, all of them before the first is used. Short prompts keep TR = 1 for its eight times as many warps.
+// warp the four taps were four loads and the weights four more per output row: 56 us; TR = 8 loads 11 rows for 8 outputs, all
+// of them before the first is used: 34. Shorter prompts want more warps than that: TR = 2 below 512 rows (10240 / 6144 channels:
+// 511 rows 12.7 / 9.5 us, one t per warp 16.8 / 11.8; 128 rows 6.0 / 4.9 against 7.0 / 5.4; 16 rows 4.1 / 4.0 against 3.9 / 3.8;
+// TR = 8 there 7.1 / 6.7 at 128).
 // ---------------------------------------------------------------------------------------
 template <int TR>
 __global__ void __launch_bounds__(256) gdn_conv_fwd_kernel(const __nv_bfloat16* __restrict__ x, int ld,
@@ -617,13 +619,13 @@ OWL_API int owl_gdn_conv_fwd(const void* x, int ld, const void* conv_w, void* co
                              int nk, int nv, int use_state, cudaStream_t st) {
   if (T < 1 || nk < 1 || nv < 1 || (ld & 3)) return OWL_ERR_BAD_ARG;
   const int conv_dim = (2 * nk + nv) * GD;
-  const int tr = T >= 512 ? 8 : 1;
+  const int tr = T >= 512 ? 8 : 2;
   const dim3 grid(2 * nk + nv, (T + 8 * tr - 1) / (8 * tr));
   if (tr == 8)
     gdn_conv_fwd_kernel<8><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (const float*)conv_w, (float*)conv_state, slot,
                                                  (__nv_bfloat16*)out, T, nk, nv, use_state);
   else
-    gdn_conv_fwd_kernel<1><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (const float*)conv_w, (float*)conv_state, slot,
+    gdn_conv_fwd_kernel<2><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (const float*)conv_w, (float*)conv_state, slot,
                                                  (__nv_bfloat16*)out, T, nk, nv, use_state);
   OWL_LAUNCH_CHECK();
   gdn_conv_state_kernel<<<(conv_dim + 255) / 256, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (float*)conv_state, slot, T,
