@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes
+import threading
 from ctypes import c_int, c_void_p
 
 import torch
@@ -18,6 +19,24 @@ K.register("owl_quant_e4m3_rows", [c_void_p, c_int, c_int, c_void_p, c_int, c_vo
 K.register("owl_gemm_dense_set_scratch", [c_void_p, ctypes.c_longlong])
 _scratch: dict = {}
 KS_SCRATCH_BYTES = 160 * 128 * 256 * 4
+
+
+_order = threading.Lock()
+_last: dict = {}         # device -> the stream whose product used the scratch last
+
+
+def _call(device, name: str, *args) -> None:
+    """Launch a GEMM that may cut k into parts on the current stream, after the products that other streams (of this or another
+    thread) launched before it: the parts of all of them lie in the device's one scratch. (Inside a capture the graph's launches
+    are ordered by whoever replays it.)"""
+    with _order:
+        st = torch.cuda.current_stream(device)
+        last = _last.get(device)
+        if last is not st and last != st and not torch.cuda.is_current_stream_capturing():
+            if last is not None:
+                st.wait_stream(last)
+            _last[device] = st
+        K.call(name, *args, st.cuda_stream)
 
 
 def ensure_scratch(device) -> None:
@@ -52,8 +71,8 @@ def e4m3_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Te
     assert xq.dtype == torch.uint8 and wq.dtype == torch.uint8 and out.dtype == torch.bfloat16
     ensure_scratch(xq.device)
     t, k = xq.shape
-    K.call("owl_e4m3_gemm", K.ptr(xq), xq.stride(0), K.ptr(sx), K.ptr(wq), wq.stride(0), K.ptr(sw), K.ptr(out), t, wq.shape[0], k,
-           out.stride(0), K.stream())
+    _call(xq.device, "owl_e4m3_gemm", K.ptr(xq), xq.stride(0), K.ptr(sx), K.ptr(wq), wq.stride(0), K.ptr(sw), K.ptr(out), t, wq.shape[0], k,
+           out.stride(0))
     return out
 
 
@@ -72,9 +91,11 @@ def f16_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, force_small: b
     ensure_scratch(x.device)
     t, k = x.shape
     # long chunks x wide weights: the persistent 128 x 256 kernel; otherwise the 128 x 128 kernel (two CTAs per SM)
-    entry = "owl_f16_gemm_persist" if (force_persist or (t >= 256 and w.shape[0] >= 512 and not force_small)) else "owl_f16_gemm_tc"
-    K.call(entry, K.ptr(x), x.stride(0), K.ptr(w), w.stride(0), K.ptr(out), t, w.shape[0], k, out.stride(0),
-           1 if x.dtype == torch.bfloat16 else 0, K.stream())
+    args = (K.ptr(x), x.stride(0), K.ptr(w), w.stride(0), K.ptr(out), t, w.shape[0], k, out.stride(0), 1 if x.dtype == torch.bfloat16 else 0)
+    if force_persist or (t >= 256 and w.shape[0] >= 512 and not force_small):
+        _call(x.device, "owl_f16_gemm_persist", *args)
+    else:
+        K.call("owl_f16_gemm_tc", *args, K.stream())
     return out
 
 
@@ -88,8 +109,8 @@ def w4_gemm_rows(w, x: torch.Tensor, out: torch.Tensor, silu: bool = False) -> t
     assert w.layout == "slice" and x.dtype == torch.float16 and x.stride(-1) == 1 and out.stride(-1) == 1
     assert out.dtype == (torch.float16 if silu else torch.bfloat16)
     ensure_scratch(x.device)
-    K.call("owl_w4_gemm_rows", K.ptr(x), x.stride(0), K.ptr(w.records), K.ptr(out), x.shape[0], w.n, w.k, out.stride(0), w.group,
-           int(silu), K.stream())
+    _call(x.device, "owl_w4_gemm_rows", K.ptr(x), x.stride(0), K.ptr(w.records), K.ptr(out), x.shape[0], w.n, w.k, out.stride(0), w.group,
+           int(silu))
     return out
 
 
@@ -102,8 +123,8 @@ def gemm_silu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, sx: torch.Ten
     assert x.dtype == w.dtype and out.dtype == torch.float16 and out.stride(-1) == 1
     ensure_scratch(x.device)
     fmt = 2 if sx is not None else 1 if x.dtype == torch.bfloat16 else 0
-    K.call("owl_gemm_silu", K.ptr(x), x.stride(0), K.ptr(sx), K.ptr(w), w.stride(0), K.ptr(sw), K.ptr(out), x.shape[0], w.shape[0],
-           x.shape[1], out.stride(0), fmt, K.stream())
+    _call(x.device, "owl_gemm_silu", K.ptr(x), x.stride(0), K.ptr(sx), K.ptr(w), w.stride(0), K.ptr(sw), K.ptr(out), x.shape[0], w.shape[0],
+           x.shape[1], out.stride(0), fmt)
     return out
 
 

@@ -352,3 +352,26 @@ def test_resident_copy_and_records_give_one_product(t):
     if not linear.w4_gemm_silu(w, x, act, arm="tcr"):
         K.silu_mul(out, t, 512, out=act)
     torch.testing.assert_close(act.float(), _silu_ref(out).float(), rtol=2.0 ** -9, atol=2.0 ** -20)
+
+
+def test_streams_share_the_scratch_of_cut_products():
+    """Two threads, each on a stream of its own, with products that are cut along k (5120 x 1024, the a / b rows): the fp32 parts lie
+    in one scratch."""
+    (w, v), gen = _int4([(5120, 1024), (5120, 1024)], 21), torch.Generator(device=DEV).manual_seed(21)
+    ab = (torch.randn(96, 1024, device=DEV, generator=gen) * 0.05).half()
+    jobs = []
+    for m, t in ((w, 64), (v, 137)):
+        x = torch.randn(t, 1024, device=DEV, generator=gen).half()
+        jobs.append((m, x, gemm_tc.w4_gemm_rows(m, x, torch.empty(t, 5120, dtype=torch.bfloat16, device=DEV)),
+                     linear.dense_gemm(x, ab, torch.empty(t, 96, dtype=torch.bfloat16, device=DEV), split=True)))
+    torch.cuda.synchronize()
+
+    def work(m, x, want, want_ab):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            y = [(torch.empty_like(want), torch.empty_like(want_ab)) for _ in range(40)]
+            for a, b in y:
+                gemm_tc.w4_gemm_rows(m, x, a)
+                linear.dense_gemm(x, ab, b, split=True)
+            return all(torch.equal(a, want) and torch.equal(b, want_ab) for a, b in y)
+    with ThreadPoolExecutor(2) as ex:
+        assert all(ex.map(lambda j: work(*j), jobs))
