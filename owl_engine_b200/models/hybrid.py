@@ -284,7 +284,8 @@ class StatePool:
 
     def copy_slot(self, src: int, dst: int) -> None:
         """Snapshot / restore of a GDN row (speculative rollback, prefix-boundary snapshots)."""
-        if self.rec_state.is_cuda and self.rec_state.shape[0] and src >= 0 and dst >= 0:
+        slots = range(self.rec_state.shape[1])
+        if self.rec_state.is_cuda and self.rec_state.shape[0] and src in slots and dst in slots:      # else what indexing does
             K.gdn_copy_slot(self.conv_state, self.rec_state, src, dst)
             return
         self.conv_state[:, dst].copy_(self.conv_state[:, src])

@@ -5,6 +5,8 @@ from concurrent.futures import ThreadPoolExecutor
 import pytest
 import torch
 
+from owl_engine_b200.models.hybrid import StatePool
+from owl_engine_b200.models.spec import PRESETS
 from owl_engine_b200.ops import gemm_tc, linear
 from owl_engine_b200.ops import kernels as K
 from owl_engine_b200.ops import quant as Q
@@ -375,3 +377,17 @@ def test_streams_share_the_scratch_of_cut_products():
             return all(torch.equal(a, want) and torch.equal(b, want_ab) for a, b in y)
     with ThreadPoolExecutor(2) as ex:
         assert all(ex.map(lambda j: work(*j), jobs))
+
+
+def test_copy_slot_indexes_like_a_tensor():
+    pool = StatePool(PRESETS["test-hybrid"](), torch.device(DEV), 4, 5)
+    pool.conv_state.normal_()
+    pool.rec_state.normal_()
+    a = [t.clone() for t in (pool.conv_state, pool.rec_state)]
+    pool.copy_slot(-1, 0)
+    for t, u in zip((pool.conv_state, pool.rec_state), a):
+        u[:, 0] = u[:, -1]
+        assert torch.equal(t, u)
+    for src, dst in ((0, 5), (5, 0), (-6, 0)):
+        with pytest.raises(IndexError):
+            pool.copy_slot(src, dst)
