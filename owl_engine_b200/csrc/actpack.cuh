@@ -1,6 +1,7 @@
-// ActPack: the activation format consumed by the W4A16 weight-streaming kernels (gemv.cu).
+// ActPack: the activation formats consumed by the weight-streaming kernels: this one by the integer arms (gemv.cu, in tiles
+// gemv_tc.cu), the fragment form (ACT_FRAG, below) by the 16-bit tensor path (gemv_mma.cu).
 //
-// The streaming kernels feed the int4 weights to the integer tensor-core path as bytes: one AND
+// The integer kernels feed the int4 weights to the integer tensor-core path as bytes: one AND
 // gives the four low nibbles of a 32-bit weight word, one shift + AND the four high nibbles, and
 // that is the entire "dequantisation" (zero point and scale are applied once per group on the
 // int32 accumulators). The activations therefore have to be integers too: the producer stores

@@ -11,7 +11,8 @@
 // carry 2^60), so a product is an exact 12-bit integer times a power of two, accumulated in fp32 per group:
 //     y += s * (dot - z * sum(x)).
 // The integer arm (gemv.cu) rounds the activations to 15 bits, needs two MMAs per 32 k and converts its int32 sums; this
-// one rounds nothing before the fp32 sums. Activations of magnitude 2^63 and above become infinite here.
+// one rounds nothing before the fp32 sums. Activations of magnitude 2^63 and above become infinite here, and below about 2^-57 fp32
+// ends under the products; prompts and the one-token arm carry activations as fp16, whose range is inside that.
 // NVFP4: the codes are converted to fp16 pairs by the conversion unit (6.6 clocks a word of eight; moving their bits to the
 // sign and exponent places of a bf16 took 15 integer instructions, 19 clocks) and multiplied by the block scale (4 x 2
 // significant bits: exact in fp16); the activations are fp16 with a power of two per 128 that the sums are rescaled by.

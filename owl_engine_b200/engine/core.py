@@ -43,10 +43,11 @@ class EngineConfig:
     prefill_chunk: int = 2048
     pdl: bool = True
     prefill_gemm: str = "tc"
-    act_bits: int = 15             # decode activations: 15-bit fixed point, or 8 (the W4A8 decode arm, `[model] quant = "w4a8"`)
-    decode_gemv: str = "fma"       # W4 decode arm: "fma" (one-token steps on the half-precision FMA projection with fused norm /
-                                   # residual / activation; other row counts on the integer arm), "dp4a" (integer arm only) or
-                                   # "tc" (tcgen05 streaming kernel, block-major records)
+    act_bits: int = 15             # decode activations: as they are (15-bit fixed point on the integer arms), or rounded to 8 bits
+                                   # per group (the W4A8 decode arm, `[model] quant = "w4a8"`)
+    decode_gemv: str = "fma"       # W4 decode arm: "fma" (one-token steps of group 128 on the half-precision FMA projection with fused
+                                   # norm / residual / activation; other steps on the 16-bit tensor path), "dp4a" (the integer arms,
+                                   # whatever the row count) or "tc" (tcgen05 streaming kernel, block-major records)
     seed: int = 0
     n_layers: int | None = None    # override (tests / smoke)
     snap_cut: bool = False         # cut a separate chunk at the prompt's last block boundary instead of snapshotting inside a chunk

@@ -61,7 +61,7 @@ def main() -> None:
     n_seq = a.prompt + a.out + 64
     cfg = EngineConfig(model="qwen3.8-27b", group=a.group, n_pages=a.batch * (n_seq // 16 + 2) + 64, n_slots=a.batch, n_snap_rows=1,
                        spec_rows=min(per, a.batch), max_seqs=a.batch, max_seq=n_seq, lm_head_int8=True, n_layers=a.layers,
-                       decode_gemv="dp4a" if a.group != 128 else "fma", prefill_gemm=a.prefill_gemm)
+                       prefill_gemm=a.prefill_gemm)
     eng = Engine(cfg, comm=comm)
     eng.runner.uniform_rows = True
     g = torch.Generator().manual_seed(21)

@@ -346,8 +346,8 @@ class HybridRunner:
         self._norm_count = None
         self._attn_ws = None         # scratch of the GEMM-form prefill attention
         self._ahead = None           # dequantisation one projection ahead (long chunks)
-        # decode activations: 15-bit fixed point (exact for bf16 inputs up to rounding at 2^-14 of the group maximum), or 8
-        # bits per group (the W4A8 decode arm: half the integer products per weight byte)
+        # decode activations: bf16 as they are on the 16-bit tensor path, 15-bit fixed point (rounded at 2^-14 of the group
+        # maximum) on the integer arms, fp16 on the one-token FMA arm; with 8 bits (the W4A8 decode arm) rounded per group
         self.act_bits = int(os.environ.get("OWL_ACT_BITS", "15"))
         # L2 prefetch of the next projection's weights on a side branch of the step graph (MB per projection, 0 = off) and
         # where the branch forks: "before" the current projection (concurrent with it) or "after" it (in the gap that follows)
@@ -414,7 +414,7 @@ class HybridRunner:
         self.tap_sink = None            # callable(pos0, t, {layer: [t, H]}) called after every prefill chunk when taps are on
         self.pre_hook = None            # callable(m): rewrites self.h after the embedding (draft heads mix in the target's hidden)
         self.uniform_rows = False       # per-row arithmetic independent of the number of rows in the step (speculative
-                                        # verify must reproduce plain decoding bit for bit): one GEMV arm for 1..8 rows,
+                                        # verify must reproduce plain decoding bit for bit): one streaming arm for 1..32 rows,
                                         # KV splits aligned to positions instead of to the row's length
         self.pf_pipe = None             # explicit prefill pipe (parallel/symm.PrefillPipe); default: the communicator's
         self.sp_prefill = True          # tensor-parallel prefill through the GEMM-fused reduce-scatter / all-gather path
@@ -454,8 +454,8 @@ class HybridRunner:
             and not self.uniform_rows and not any(k % 128 for k in (sp.hidden, sp.inter, sp.value_dim, sp.hq * sp.hd))
 
     def _mma(self, m: int, ab: bool = False) -> bool:
-        """The projections of an ``m``-row step (``ab``: the GDN input projection, which takes the a / b rows along) run on the 16-bit tensor streaming kernel (``csrc/gemv_mma.cu``): one GPU,
-        slice-major int4 or NVFP4 weights. The tensor-parallel arms (push, symmetric all-reduce) and the fused-norm variant
+        """The projections of an ``m``-row step (``ab``: the GDN input projection, which takes the a / b rows along) run on the
+        16-bit tensor streaming kernel (``csrc/gemv_mma.cu``): one GPU, slice-major int4 or NVFP4 weights. The tensor-parallel arms (push, symmetric all-reduce) and the fused-norm variant
         stay on the integer kernels, whose epilogues they are."""
         sp = self.spec
         if self._dense16(m):
@@ -523,9 +523,8 @@ class HybridRunner:
     BATCH_GEMM_FROM = 24   # rows from which a batched step multiplies the resident dense weight copy on the tcgen05 GEMM
 
     def _gemv_dense16(self, w, xp, xs, out, m: int, residual, epi: int, ldo) -> None:
-        """Wide batched steps (16+ rows) with a resident dense copy of the weights (``prefill_gemm = "tcr"``: fp16, 4x the
-        int4 bytes; ``"tc8r"``: e4m3 rows, 2x, activations quantised per token): the integer weight-streaming arms run on
-        warp-level MMA and grow linearly with the row count from 8 rows on, while the persistent tcgen05 GEMM streams the
+        """Wide batched steps (24+ rows) with a resident dense copy of the weights (``prefill_gemm = "tcr"``: fp16, 4x the
+        int4 bytes; ``"tc8r"``: e4m3 rows, 2x, activations quantised per token): the persistent tcgen05 GEMM streams the
         dense matrix once for all rows."""
         from ..ops import gemm_tc, linear
 
@@ -705,7 +704,7 @@ class HybridRunner:
     def _fma_ok(self, lay: StepLayout) -> bool:
         """The fused one-token path applies: one row, slice-major group-128 int4 weights, 15-bit-equivalent activations, and no
         mode that needs row-count-independent arithmetic (speculative verify reproduces plain decoding bit for bit on the
-        integer arm). Under tensor parallelism it needs the symmetric workspace (the collective lives inside the
+        kernels that take several rows). Under tensor parallelism it needs the symmetric workspace (the collective lives inside the
         projections) and no hidden-state taps (the residual stream is only materialised inside the next projection)."""
         w0 = self.w.layers[0].gate_up if self.w.layers else None
         if not (self.decode_gemv == "fma" and lay.m == 1 and not self.uniform_rows and self.act_bits == 15

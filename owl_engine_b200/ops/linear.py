@@ -1,23 +1,24 @@
 """Prefill-shape linear layers over quantised weights.
 
-``w4_gemm`` computes ``out[T, N] = x[T, K] @ dequant(w)^T`` for a ``W4Skinny`` weight with one of
-two arms:
+``w4_gemm`` computes ``out[T, N] = x[T, K] @ dequant(w)^T`` for a ``W4Skinny`` weight with one of these arms:
 
-* ``"tc"``        the product path, both steps our own sm_100a kernels: for short chunks (fewer than
-                  ``DEQUANT_FROM`` tokens) the tcgen05 / TMEM W4A16 GEMM that dequantises inside the kernel
-                  (``csrc/gemm_tc.cu``); for long chunks the weight is dequantised ONCE into a dense
-                  scratch matrix (``csrc/dequant.cu``, runs at copy bandwidth) and the dense tcgen05 GEMM
-                  multiplies it -- the in-kernel dequantisation repeats per 128-token tile and caps
-                  the fused kernel near 300 TFLOP/s, the dense kernel runs at 750-1000;
-* ``"tc8"``       the W4A8 arm on tensor cores: like ``"tc"``, but for long chunks the dequantised weight is
+* ``"tc"``        the product path, all steps our own sm_100a kernels. Slice-major weights: up to ``SKINNY_UPTO`` tokens the
+                  decode-shape streaming kernel (``csrc/gemv_mma.cu``), up to 256 (``rows_pay``) the tcgen05 GEMM that reads the
+                  int4 records and dequantises each once (``csrc/gemm_w4.cu``), above that the weight is dequantised into a dense
+                  fp16 matrix (``csrc/dequant.cu``, beside the GEMM before it where ``DequantAhead`` applies) and the dense
+                  tcgen05 GEMM multiplies it. Block-layout weights and operands that are not 16-byte aligned: below
+                  ``DEQUANT_FROM`` tokens the tiled GEMM that dequantises in the kernel once per 128 tokens
+                  (``csrc/gemm_tc.cu``), from there the dense form;
+* ``"tc8"``       the W4A8 arm on tensor cores: like ``"tc"``, but from ``DEQUANT_FROM`` tokens the dequantised weight is
                   re-quantised per output row to e4m3 and the activations per token, and the product runs as
                   ``tcgen05.mma kind::f8f6f4`` at twice the 16-bit rate (the reference's W4A8 arm quantises
                   activations per token to int8 for IMMA, ``crates/kernels/cu/elems/quant_i8_act.cu:80-98``; int4
                   values times a group scale do not survive an integer MMA without a per-group epilogue, an
                   8-bit float product with per-row scales does);
 * ``"tcr"`` / ``"tc8r"``  the same two arms with the dequantised (fp16) resp. re-quantised (e4m3) weight kept RESIDENT
-                  on the weight object after its first use: 4 resp. 2 extra bytes per weight in HBM (54 / 27 GB for the
-                  27B model on one GPU, which 180 GB leave room for) buy back the per-call dequantisation pass;
+                  on the weight object after its first use: 2 resp. 1 extra bytes per weight in HBM (48.7 / 24.3 GB for the
+                  27B model on one GPU, which 180 GB leave room for) buy back the per-call dequantisation pass. The fp16
+                  copies serve chunks above 256 tokens, and from 128 those where ``rows_pay`` says so;
 * ``"baseline"``  dequantise to a dense bf16 scratch matrix, then the library GEMM
                   (``torch.matmul`` = cuBLAS). This is the comparison arm, like the reference's
                   range-dequant -> cuBLAS arm (``crates/kernels/cu/gguf/gguf_smem.cu:415-552``).
@@ -34,7 +35,9 @@ from . import gemm_tc
 from . import kernels as K
 
 _scratch: dict = {}
-DEQUANT_FROM = 128      # tokens per chunk from which dequantise-once + dense GEMM wins
+DEQUANT_FROM = 128      # tokens per chunk from which the 8-bit arms re-quantise, and from which weights that gemm_w4.cu does not
+                        # take are dequantised once (34816 x 5120: tiled form 116 us per 128 tokens, dense form 150 at 128,
+                        # 204 at 137)
 SILU_FROM = 256         # tokens from which the persistent GEMM, which has the silu(gate) * up epilogue, multiplies fp16 weights
 SMS = 148               # of the part all sizes here were measured on
 SKINNY_UPTO = 32        # rows up to which the decode-shape weight-streaming kernel is used instead of a GEMM
