@@ -45,6 +45,7 @@ struct GdnDecodeParams {
   uint4* xpack;                 // ActPack of out (optional)
   float2* xs;
   int ld, ldab, nk, nv, T, G;
+  int z8;                       // the z columns can be read 8 bytes at a time (row stride and base allow it)
   float eps;
 };
 
@@ -237,8 +238,15 @@ __global__ void __launch_bounds__(256) gdn_decode_kernel(GdnDecodeParams p) {
       ss = warp_sum(ss);
       const float rinv = rsqrtf(ss / (float)GD + p.eps);
       float y[4];
-      const uint2 zu = live ? *reinterpret_cast<const uint2*>(xr + 2 * K + V + h * GD + lane * 4) : make_uint2(0, 0);
-      const float z[4] = {bf16_lo(zu.x), bf16_hi(zu.x), bf16_lo(zu.y), bf16_hi(zu.y)};
+      const __nv_bfloat16* zp = xr + 2 * K + V + h * GD + lane * 4;
+      float z[4] = {0.f, 0.f, 0.f, 0.f};
+      if (live && p.z8) {
+        const uint2 zu = *reinterpret_cast<const uint2*>(zp);
+        z[0] = bf16_lo(zu.x); z[1] = bf16_hi(zu.x); z[2] = bf16_lo(zu.y); z[3] = bf16_hi(zu.y);
+      } else if (live) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) z[j] = __bfloat162float(zp[j]);
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         y[j] = __bfloat162float(__float2bfloat16(o[j] * rinv * gam[j] * silu_f(z[j])));
@@ -593,6 +601,7 @@ OWL_API int owl_gdn_decode(const void* qkvz, int ld, const void* ab, int ldab, c
   p.conv_state = (float*)conv_state; p.state = (float*)state; p.slots = (const int*)slots; p.tlen = (const int*)tlen;
   p.out = (__nv_bfloat16*)out; p.xpack = (uint4*)xpack; p.xs = (float2*)xs;
   p.ld = ld; p.ldab = ldab; p.nk = nk; p.nv = nv; p.T = T; p.G = G; p.eps = eps;
+  p.z8 = !(ld & 3) && !(reinterpret_cast<uintptr_t>(qkvz) & 7);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nv, batch); cfg.blockDim = dim3(256); cfg.stream = st;
   cudaLaunchAttribute attr[2];

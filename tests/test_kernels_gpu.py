@@ -297,6 +297,37 @@ def test_gdn_decode(nk, nv, t):
     torch.testing.assert_close(xs.cpu(), ws, rtol=1e-5, atol=1e-3)
 
 
+@pytest.mark.parametrize("nk,nv", [(2, 6), (2, 2)])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_gdn_decode_of_part_of_the_rows(nk, nv, pad):
+    """Eight rows a sequence, of which ``tlen`` count (none, some, all, more than there are); ``pad``: an odd row stride. The state
+    alone (a fold) and with outputs."""
+    t, tlens, order = 8, [0, 3, 8, 11], [2, 0, -1, 1]
+    s = _gdn_setup(nk, nv, t, 4, 23)
+    d = {k: (v.to(DEV) if torch.is_tensor(v) else v) for k, v in s.items()}
+    wide = torch.full((4 * t, d["qkvz"].shape[1] + pad), float("nan"), dtype=torch.bfloat16, device=DEV)
+    wide[:, :d["qkvz"].shape[1]] = d["qkvz"]
+    slots, tlen = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in (order, tlens))
+    for fold in (False, True):
+        conv, state = d["conv_state"].clone(), d["state"].clone()
+        out = torch.full((4 * t, s["vdim"]), 7.0, dtype=torch.bfloat16, device=DEV)
+        K.gdn_decode(wide, wide.shape[1], d["ab"], 2 * nv, d["conv_w"], d["a_log"], d["dt_bias"], d["gamma"], conv, state, slots,
+                     out=None if fold else out, batch=4, t=t, nk=nk, nv=nv, tlen=tlen)
+        for b, (slot, n) in enumerate(zip(order, tlens)):
+            n = min(n, t)
+            if slot < 0:
+                continue
+            assert (out[b * t + (0 if fold else n):(b + 1) * t] == 7.0).all()            # rows that do not count are not written
+            if n == 0:
+                assert torch.equal(state[slot], d["state"][slot]) and torch.equal(conv[slot], d["conv_state"][slot])
+                continue
+            want, st, hist = _gdn_ref(s, slice(b * t, b * t + n), slot, n)
+            if not fold:
+                torch.testing.assert_close(out[b * t:b * t + n].float().cpu(), want, rtol=2e-2, atol=2e-2)
+            torch.testing.assert_close(state[slot].cpu(), st, rtol=1e-3, atol=1e-3)
+            torch.testing.assert_close(conv[slot].cpu(), hist, rtol=0, atol=0)
+
+
 @pytest.mark.parametrize("t,use_state,split", [(70, True, None), (33, False, None), (5, False, None), (2, True, None),
                                                (64, False, "chunked"), (70, True, "chunked"), (200, True, None),
                                                (333, False, None)])
