@@ -127,3 +127,51 @@ def test_extremes_of_the_activations(fmt):
 @pytest.mark.parametrize("m", [1, 32])
 def test_k_parts_of_narrow_matrices(fmt, shape, m):
     test_mma_streaming_matches_dequantised_product(fmt, shape, m)
+
+
+def _same_pack(got, want, m, k, group):
+    (xp, xs), (wp, ws) = got, want
+    assert torch.equal(xp, wp)
+    torch.testing.assert_close(xs, ws, rtol=2.0 ** -18, atol=0, equal_nan=True)          # the sums' order may differ
+
+
+# what the kernels before a projection write for it, against the pack kernel on their plain outputs
+@pytest.mark.parametrize("flags", [0, K.ACT_A8, K.ACT_NV, K.ACT_NV | K.ACT_A8])
+@pytest.mark.parametrize("group", [128, 32])
+@pytest.mark.parametrize("m", [1, 9])
+def test_producers_write_the_fragments_of_their_outputs(flags, group, m):
+    g = group | K.ACT_FRAG | flags
+    gen = torch.Generator(device=DEV).manual_seed(m + group)
+    rn = lambda *s: torch.randn(*s, device=DEV, generator=gen).bfloat16()
+    rows = (m + 7) // 8 * 8
+
+    def buffers(k):
+        return (torch.full((rows, 2 * k), 0x5a, dtype=torch.uint8, device=DEV),
+                torch.full((rows, k // (128 if flags & K.ACT_NV else group), 2), 3.0, device=DEV))
+
+    def packed(x):
+        b = buffers(x.shape[1])
+        K.act_pack(x, *b, m, x.shape[1], g)
+        return b
+    for k in (384, 5120, 8192, 8320):              # the row kernel up to 8192, half a warp of chunks at 384 and 8320
+        h, w, y, b = rn(m, k), rn(k), torch.empty(m, k, dtype=torch.bfloat16, device=DEV), buffers(k)
+        K.rmsnorm_pack(h, w, normed=y, xpack=b[0], xs=b[1], m=m, k=k, group=g)
+        _same_pack(b, packed(y), m, k, group)
+    # attention: two parts a head, three heads of 256
+    hq, hd, splits = 3, 256, 2
+    part_o, part_ml = torch.randn(m * hq * splits * hd, device=DEV, generator=gen), torch.rand(m * hq * splits * 2, device=DEV, generator=gen) + 0.5
+    y, b = torch.empty(m, hq * hd, dtype=torch.bfloat16, device=DEV), buffers(hq * hd)
+    K.attn_reduce(part_o, part_ml, splits, None, 0, m, hq, out=y)
+    K.attn_reduce(part_o, part_ml, splits, None, 0, m, hq, xpack=b[0], xs=b[1], group=g)
+    _same_pack(b, packed(y), m, hq * hd, group)
+    # the recurrence: m rows of one sequence (at most 8) or m sequences
+    nk, nv = 1, 3
+    ld = (2 * nk + 2 * nv) * 128
+    batch, t = (m, 1) if m > 8 else (1, m)
+    args = (rn(m, ld), ld, rn(m, 2 * nv), 2 * nv, torch.randn((2 * nk + nv) * 128, 4, device=DEV, generator=gen), torch.zeros(nv, device=DEV),
+            torch.ones(nv, device=DEV), torch.ones(128, device=DEV))
+    conv, state = torch.zeros(batch, (2 * nk + nv) * 128, 3, device=DEV), torch.zeros(batch, nv, 128, 128, device=DEV)
+    slots = torch.arange(batch, dtype=torch.int32, device=DEV)
+    y, b = torch.empty(m, nv * 128, dtype=torch.bfloat16, device=DEV), buffers(nv * 128)
+    K.gdn_decode(*args, conv, state, slots, out=y, xpack=b[0], xs=b[1], batch=batch, t=t, nk=nk, nv=nv, group=g)
+    _same_pack(b, packed(y), m, nv * 128, group)
