@@ -45,24 +45,25 @@ struct GdnDecodeParams {
   uint4* xpack;                 // ActPack of out (optional)
   float2* xs;
   int ld, ldab, nk, nv, T, G;
-  int z8;                       // the z columns can be read 8 bytes at a time (row stride and base allow it)
   float eps;
 };
 
 // The rows' inputs (convolution, norms, gates) do not depend on the state, so all T rows are prepared first: one exchange
 // between the CTAs of a k-head and three barriers for the whole launch, then one barrier per row (the partial sums of k^T S and
 // q^T S; their buffers alternate). With an exchange and four barriers per row a step of 8 sequences x 4 rows took 41 us a layer
-// (state traffic: 8). OUT = false (a fold: the state only) leaves out the q side.
-template <bool OUT>
+// (state traffic: 8). OUT = false (a fold: the state only) leaves out the q side. MT: rows the buffers hold; one row has its own
+// form, whose 14 KB (33 for 8 rows) of shared memory let it start beside the projection before it (one-row step, 0.8B / 27B: 19.0
+// / 57.2 us a layer, with the buffers of 8 rows 19.9 / 57.8). Z8: the z columns are read 8 bytes at a time.
+template <bool OUT, int MT, bool Z8>
 __global__ void __launch_bounds__(256) gdn_decode_kernel(GdnDecodeParams p) {
   cg::cluster_group cluster = cg::this_cluster();
-  __shared__ float qk_s[GDN_MAX_T][256];   // per row: q[0..127], k[128..255]
-  __shared__ float v_s[GDN_MAX_T][128];
-  __shared__ float part[2][2][8][128];     // [row parity][kS|qS][warp][v]
+  __shared__ float qk_s[MT][256];   // per row: q[0..127], k[128..255]
+  __shared__ float v_s[MT][128];
+  __shared__ float part[MT > 1 ? 2 : 1][2][8][128];     // [row parity][kS|qS][warp][v]
   __shared__ float o_s[8][128];            // per epilogue warp
-  __shared__ float red[GDN_MAX_T][8];
-  __shared__ float scal[GDN_MAX_T][2];     // e^g, beta
-  __shared__ float qk_dot[GDN_MAX_T];      // q.k
+  __shared__ float red[MT][8];
+  __shared__ float scal[MT][2];     // e^g, beta
+  __shared__ float qk_dot[MT];      // q.k
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int h = blockIdx.x, b = blockIdx.y;
@@ -119,11 +120,11 @@ __global__ void __launch_bounds__(256) gdn_decode_kernel(GdnDecodeParams p) {
   {
     const __nv_bfloat16* x0 = p.qkvz + (size_t)b * p.T * p.ld;
     if (rank == 0) {
-      float y[GDN_MAX_T];
+      float y[MT];
 #pragma unroll
-      for (int r = 0; r < GDN_MAX_T; ++r) y[r] = (live && r < Tn) ? __bfloat162float(x0[(size_t)r * p.ld + ch_qk]) : 0.f;
+      for (int r = 0; r < MT; ++r) y[r] = (live && r < Tn) ? __bfloat162float(x0[(size_t)r * p.ld + ch_qk]) : 0.f;
 #pragma unroll
-      for (int r = 0; r < GDN_MAX_T; ++r) {
+      for (int r = 0; r < MT; ++r) {
         if (r >= Tn) break;
         const float x = y[r];
         float v = cwq[0] * wq[0] + cwq[1] * wq[1] + cwq[2] * wq[2] + cwq[3] * x;
@@ -137,18 +138,18 @@ __global__ void __launch_bounds__(256) gdn_decode_kernel(GdnDecodeParams p) {
       __syncthreads();
       const int base = (tid < 128) ? 0 : 4;
 #pragma unroll
-      for (int r = 0; r < GDN_MAX_T; ++r) {
+      for (int r = 0; r < MT; ++r) {
         if (r >= Tn) break;
         const float tot = red[r][base] + red[r][base + 1] + red[r][base + 2] + red[r][base + 3];
         qk_s[r][tid] = y[r] * rsqrtf(tot + 1e-6f);
       }
     }
     if (tid < 128) {
-      float y[GDN_MAX_T];
+      float y[MT];
 #pragma unroll
-      for (int r = 0; r < GDN_MAX_T; ++r) y[r] = (live && r < Tn) ? __bfloat162float(x0[(size_t)r * p.ld + ch_v]) : 0.f;
+      for (int r = 0; r < MT; ++r) y[r] = (live && r < Tn) ? __bfloat162float(x0[(size_t)r * p.ld + ch_v]) : 0.f;
 #pragma unroll
-      for (int r = 0; r < GDN_MAX_T; ++r) {
+      for (int r = 0; r < MT; ++r) {
         if (r >= Tn) break;
         const float x = y[r];
         const float v = cwv[0] * wv[0] + cwv[1] * wv[1] + cwv[2] * wv[2] + cwv[3] * x;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(256) gdn_decode_kernel(GdnDecodeParams p) {
       if (rank != 0) {
         const float* remote = cluster.map_shared_rank(&qk_s[0][0], 0);
 #pragma unroll
-        for (int r = 0; r < GDN_MAX_T; ++r) {
+        for (int r = 0; r < MT; ++r) {
           if (r >= Tn) break;
           qk_s[r][tid] = remote[r * 256 + tid];
         }
@@ -239,14 +240,14 @@ __global__ void __launch_bounds__(256) gdn_decode_kernel(GdnDecodeParams p) {
       const float rinv = rsqrtf(ss / (float)GD + p.eps);
       float y[4];
       const __nv_bfloat16* zp = xr + 2 * K + V + h * GD + lane * 4;
-      float z[4] = {0.f, 0.f, 0.f, 0.f};
-      if (live && p.z8) {
-        const uint2 zu = *reinterpret_cast<const uint2*>(zp);
-        z[0] = bf16_lo(zu.x); z[1] = bf16_hi(zu.x); z[2] = bf16_lo(zu.y); z[3] = bf16_hi(zu.y);
+      uint2 zu = make_uint2(0, 0);
+      if (live && Z8) {
+        zu = *reinterpret_cast<const uint2*>(zp);
       } else if (live) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) z[j] = __bfloat162float(zp[j]);
+        const unsigned short* z1 = reinterpret_cast<const unsigned short*>(zp);
+        zu = make_uint2(z1[0] | (uint32_t)z1[1] << 16, z1[2] | (uint32_t)z1[3] << 16);
       }
+      const float z[4] = {bf16_lo(zu.x), bf16_hi(zu.x), bf16_lo(zu.y), bf16_hi(zu.y)};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         y[j] = __bfloat162float(__float2bfloat16(o[j] * rinv * gam[j] * silu_f(z[j])));
@@ -601,7 +602,6 @@ OWL_API int owl_gdn_decode(const void* qkvz, int ld, const void* ab, int ldab, c
   p.conv_state = (float*)conv_state; p.state = (float*)state; p.slots = (const int*)slots; p.tlen = (const int*)tlen;
   p.out = (__nv_bfloat16*)out; p.xpack = (uint4*)xpack; p.xs = (float2*)xs;
   p.ld = ld; p.ldab = ldab; p.nk = nk; p.nv = nv; p.T = T; p.G = G; p.eps = eps;
-  p.z8 = !(ld & 3) && !(reinterpret_cast<uintptr_t>(qkvz) & 7);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nv, batch); cfg.blockDim = dim3(256); cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -618,7 +618,11 @@ OWL_API int owl_gdn_decode(const void* qkvz, int ld, const void* ab, int ldab, c
     ++na;
   }
   cfg.attrs = attr; cfg.numAttrs = na;
-  cudaError_t e = (out || xpack) ? cudaLaunchKernelEx(&cfg, gdn_decode_kernel<true>, p) : cudaLaunchKernelEx(&cfg, gdn_decode_kernel<false>, p);
+  const bool z8 = !(ld & 3) && !(reinterpret_cast<uintptr_t>(qkvz) & 7);
+  auto kernel = !(out || xpack) ? (T == 1 ? gdn_decode_kernel<false, 1, true> : gdn_decode_kernel<false, GDN_MAX_T, true>)
+              : !z8 ? gdn_decode_kernel<true, GDN_MAX_T, false>
+              : T == 1 ? gdn_decode_kernel<true, 1, true> : gdn_decode_kernel<true, GDN_MAX_T, true>;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) return (int)OWL_ERR_LAUNCH * 1000 - (int)e;
   return OWL_OK;
 }
