@@ -110,9 +110,10 @@ class _AheadShared:
                 return None
             self.release()
             try:
-                # allocations that no ledger makes cannot ask for it back: as much again has to stay free
-                free = torch.cuda.mem_get_info(self.device)[0]
-                if free + torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device) < 4 * need:
+                # allocations that no ledger makes cannot ask for it back: as much again has to stay free (by this process' own
+                # count: asking the driver took up to 9 ms after a large release, in the first pass of a new engine)
+                left = torch.cuda.get_device_properties(self.device).total_memory - torch.cuda.memory_allocated(self.device)
+                if left < 4 * need + (2 << 30):
                     raise BudgetError(self.NAME)
                 self.extra = led.alloc(self.NAME, "workspace", (need,), torch.float16)
             except (BudgetError, torch.cuda.OutOfMemoryError):

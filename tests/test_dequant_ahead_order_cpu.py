@@ -54,8 +54,8 @@ class _Model:
                 self.at = stream.last
         self.main = Stream()
         self.cuda = SimpleNamespace(Stream=Stream, Event=Event, current_stream=lambda device=None: self.main, current_device=lambda: 0,
-                                    OutOfMemoryError=MemoryError, mem_get_info=lambda dev: (1 << 40, 1 << 40),
-                                    memory_reserved=lambda dev: 0, memory_allocated=lambda dev: 0)
+                                    OutOfMemoryError=MemoryError, memory_allocated=lambda dev: 0,
+                                    get_device_properties=lambda dev: SimpleNamespace(total_memory=1 << 40))
 
     def op(self, after):
         self.before.append(set().union(*({a} | self.before[a] for a in after if a is not None), set()))

@@ -245,7 +245,7 @@ def test_dequantising_ahead_is_refused_without_room(full, monkeypatch):
     assert not ahead.start([w]) and (getattr(led, "tries", 0), led.refused) == (tries, refused)
     if not full:
         led.total *= 1000
-        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev: (-(1 << 50), 0))      # nothing would stay free
+        monkeypatch.setattr(torch.cuda, "memory_allocated", lambda dev: 1 << 50)          # nothing would stay free
         assert not ahead.start([w])
         monkeypatch.undo()
         assert ahead.start([w])
