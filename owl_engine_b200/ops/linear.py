@@ -242,12 +242,11 @@ class DequantAhead:
 def rows_pay(n: int, k: int, t: int, resident: bool) -> bool:
     """Whether ``t`` tokens times an [n, k] int4 weight read the records (``gemm_w4.cu``) rather than a dense copy.
 
-    Up to 256 tokens, all that one launch takes (from 257 a second pass over the records would cost 109 us at 16384 x 5120, the
-    dequantisation and the dense GEMM 111 and, one projection ahead, less). A resident copy needs no dequantisation: it is the
-    better operand at 256 tokens (the persistent kernel: 16384 x 5120 44 against 63 us, 34816 x 5120 87 / 115, 5120 x 17408 60 / 73;
-    the 27B prompt 23.2 / 27.0 ms) and, from 128, where its 128 x 128 tiles fit two per SM and k is short (16384 x 5120 46 / 49 us at
-    137 tokens, 50 / 63 at 255); not where a tile walks a long k alone or the tiles take two waves (5120 x 17408 118 / 52 us,
-    34816 x 5120 121 / 89)."""
+    Up to 256 tokens, all that one launch takes. A resident copy needs no dequantisation; where it exists it is used at 256 tokens (the
+    persistent kernel: 16384 x 5120 44 us, 34816 x 5120 87, 5120 x 17408 60; the records 34, 76 and 49) and, from 128, where its
+    128 x 128 tiles fit two per SM and k is short (16384 x 5120 46 us at 137 tokens, the records 23): limits measured against the
+    records through shared memory (63, 115, 73 us and 49), which the present kernel no longer needs them for; not where a tile walks a
+    long k alone or the tiles take two waves (5120 x 17408 118 / 32 us, 34816 x 5120 121 / 45)."""
     if t > gemm_tc.ROWS_UPTO:
         return False
     if not resident or t < DEQUANT_FROM:
