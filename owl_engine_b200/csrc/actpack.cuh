@@ -49,7 +49,8 @@ constexpr int ACT_A8 = 0x2000;
 // xsum is stored in the unit of the products, n * 2^-133 * x * 2^64. With ACT_NV as well (NVFP4 weights) the elements are fp16 in
 // their order, x * 2^e with the largest of 128 in [2^13, 2^14) (exact for bf16 values down to 2^-27 of it) and sx = 2^-e; with
 // ACT_A8 x is the rounded activation.
-constexpr int ACT_FRAG = 0x4000, ACT_NV = 0x8000;
+// With ACT_TM as well the chunks and sums are laid out for the form that unpacks into tensor memory (gemv_tm.cu).
+constexpr int ACT_FRAG = 0x4000, ACT_NV = 0x8000, ACT_TM = 0x10000, ACT_BLOCKS = 17;
 constexpr float ACT_FRAG_UNIT = 590295810358705651712.f;      // 2^69 = 2^133 / 2^64
 __device__ __forceinline__ uint4 actpack_frag(const float* v, int cpg, float& sx, float& xsum) {
   const bool a8 = (cpg & (ACT_A8 >> 3)) != 0, nv = (cpg & (ACT_NV >> 3)) != 0;
@@ -156,10 +157,12 @@ __device__ __forceinline__ uint4 actpack_emit(const float* v, int cpg, float& sx
 constexpr int ACT_TILES = 0x1000;
 __host__ __device__ constexpr int actpack_tile_bytes(int G) { return 2048 + 64 * (128 / G); }
 
-// Group argument check of the producers' launchers: 32 / 128, optionally | ACT_TILES.
-inline bool actpack_group_ok(int G, int tokens) {
-  const int g = G & ~(ACT_TILES | ACT_A8 | ACT_FRAG | ACT_NV);
-  (void)tokens;
+// Group argument check of the producers' launchers: 32 / 128, optionally | ACT_TILES or ACT_FRAG and their variants. With ACT_TM the
+// kernel's argument also carries the number of token blocks (from bit ACT_BLOCKS), from which a chunk's place follows.
+inline bool actpack_group_ok(int& G, int tokens) {
+  const int g = G & ~(ACT_TILES | ACT_A8 | ACT_FRAG | ACT_NV | ACT_TM);
+  if ((G & ACT_TM) && (!(G & ACT_FRAG) || tokens < 1 || tokens > 32)) return false;
+  if (G & ACT_TM) G |= (tokens + 7) / 8 << ACT_BLOCKS;
   if ((G & ACT_FRAG) && (G & ACT_TILES)) return false;
   if ((G & ACT_NV) && !(G & ACT_FRAG)) return false;
   return g == 32 || g == 128;
@@ -167,9 +170,23 @@ inline bool actpack_group_ok(int G, int tokens) {
 
 __device__ __forceinline__ void actpack_store(uint4* xpack, float2* xs, int tiles, int G, int token, int c8, int nchunks,
                                               const uint4& pk, float sx, float xsum) {
-  const int frag = G & ACT_FRAG, nv = G & ACT_NV;
-  G &= ~(ACT_A8 | ACT_FRAG | ACT_NV);
+  const int frag = G & ACT_FRAG, nv = G & ACT_NV, blocks = G >> ACT_BLOCKS;
+  G &= ACT_A8 - 1;
   const int cpg = G >> 3;
+  if (blocks) {
+    // tensor-memory layout: a 128-k record of all tokens is contiguous, in blocks of 8 tokens; per block [4 words][8 tokens][4 quarters]
+    // chunks and, in `xs`, per group [8 scales][8 sums]. A word's 8 rows of 64 bytes carry the MMA's 64-byte swizzle: quarter t lies at
+    // place t ^ (token / 2) % 4. NVFP4 codes run the other way round.
+    const int kt = c8 >> 4, hi = (c8 >> 2) & 3, lo = c8 & 3, w = nv ? lo : hi, t = nv ? hi : lo, blk = token >> 3;
+    xpack[((size_t)kt * blocks + blk) * 128 + w * 32 + (token & 7) * 4 + (t ^ ((token >> 1) & 3))] = pk;
+    const int sh = nv || G == 128 ? 4 : 2;   // log2 of the chunks of one (scale, sum) pair
+    if ((c8 & ((1 << sh) - 1)) == 0) {
+      float* f = reinterpret_cast<float*>(xs) + ((((size_t)kt * blocks + blk) << (4 - sh)) + ((c8 & 15) >> sh)) * 16 + (token & 7);
+      f[0] = sx;
+      f[8] = xsum;
+    }
+    return;
+  }
   if (frag) {
     // fragment layout: blocks of 8 tokens; per block and 128-k record [4 words][8 tokens][4 quarters] chunks and per group
     // [8 tokens] pairs. A lane of the consumer reads word w of quarter t; NVFP4 codes run the other way round.

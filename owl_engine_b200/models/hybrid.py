@@ -443,7 +443,7 @@ class HybridRunner:
         consumes it, fragments for the 16-bit tensor streaming kernel (``ab``: for the GDN input projection)."""
         g = (self.G | K.ACT_TILES) if self.tiles else self.G
         if self._mma(m, ab):
-            g |= K.ACT_FRAG | (K.ACT_NV if self.w.layout == "nvfp4" else 0)
+            g |= K.ACT_FRAG | (K.ACT_NV if self.w.layout == "nvfp4" else 0) | (K.ACT_TM if self._tm(m) else 0)
         return g | K.ACT_A8 if self.act_bits == 8 else g
 
     def _dense16(self, m: int) -> bool:
@@ -468,6 +468,18 @@ class HybridRunner:
         if self.decode_gemv == "dp4a" or self.fuse_norm or self.w.layout not in ("slice", "nvfp4") or not self.w.layers:
             return False
         return (self.comm is None or sp.tp_world == 1) and not any(k % 128 for k in (sp.hidden, sp.inter, sp.value_dim, sp.hq * sp.hd))
+
+    def _tm(self, m: int) -> bool:
+        """The projections of an ``m``-row step unpack their weights into tensor memory (``csrc/gemv_tm.cu``) instead of registers.
+
+        Four blocks of 8 rows cost the warp-level form four times the MMAs, the other one nothing: us at 24 / 25 / 32 rows, warp-level
+        and tensor memory: int4 16384 x 5120 20.4 / 26.3 / 26.1 and 20.4 / 20.6 / 20.9, 34816 x 5120 35.8 / 44.7 / 45.3 and 36.3 / 36.4
+        / 37.5, 5120 x 6144 11.5 / 13.7 / 13.9 and 11.9 / 12.3 / 12.3 (group 32, 32 rows: 33.3 and 30.1, 59.1 and 56.8, 18.0 and 16.2);
+        NVFP4 at 16 / 17 rows 20.8 / 29.9 and 20.2 / 20.9. The 0.8B model's matrices are all start-up: its four together 26.8 and 26.2 us
+        at 32 rows, NVFP4 at 17 rows 22.8 and 25.3. Not under ``uniform_rows``: the sums' order differs from the warp-level form's."""
+        if self.uniform_rows:
+            return False
+        return m > 24 or (m > 16 and self.w.layout == "nvfp4" and self.spec.hidden >= 2048)
 
     def _pf_hook(self, w, after: bool) -> None:
         """Weight-stream bookkeeping around a projection: the warm-up pass of a capture records the weight tensors in launch
@@ -496,7 +508,7 @@ class HybridRunner:
         the 16-bit tensor kernel computes beside the matrix."""
         self._pf_hook(w, False)
         if self._mma(m, bool(ab)):
-            K.w4_mma(w, xp, xs, out, m, residual=residual, epi=epi, ldo=ldo, a8=self.act_bits == 8, pdl=pdl, **ab)
+            (K.w4_tm if self._tm(m) else K.w4_mma)(w, xp, xs, out, m, residual=residual, epi=epi, ldo=ldo, a8=self.act_bits == 8, pdl=pdl, **ab)
         else:
             self._gemv_inner(w, xp, xs, out, m, residual=residual, epi=epi, ldo=ldo, pdl=pdl)
         self._pf_hook(w, True)

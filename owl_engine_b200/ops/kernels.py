@@ -182,6 +182,7 @@ class StreamTcWorkspace:
 ACT_TILES = 0x1000     # OR into a producer's ``group`` argument: write ActPack in the tile layout
 ACT_A8 = 0x2000        # OR into a producer's ``group`` argument: round the activations to 8 bits (low plane zero)
 ACT_FRAG = 0x4000      # OR into a producer's ``group`` argument: bf16 fragments for w4_mma (buffers hold rows rounded up to 8)
+ACT_TM = 0x10000       # with ACT_FRAG: laid out for w4_tm
 ACT_NV = 0x8000        # with ACT_FRAG: the fp16 form that w4_mma wants for NVFP4 weights
 
 
@@ -238,6 +239,8 @@ def w4_fma(w, x, out, *, norm_w=None, residual=None, epi: int = EPI_STORE, ab_w=
 
 
 register("owl_w4_mma", [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P])
+register("owl_w4_tm", [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P])
+register("owl_nvfp4_tm", [_P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P])
 register("owl_nvfp4_mma", [_P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P])
 
 
@@ -257,6 +260,21 @@ def w4_mma(w, xpack, xs, out, m: int, *, residual=None, epi: int = EPI_STORE, ld
          int(pdl), stream())
 
 
+def w4_tm(w, xpack, xs, out, m: int, *, residual=None, epi: int = EPI_STORE, ldo: int | None = None, a8: bool = False,
+          ab_w=None, ab_x=None, ab_out=None, pdl: bool = False) -> None:
+    """``w4_mma`` with the weights unpacked into tensor memory (``csrc/gemv_tm.cu``): the same arithmetic, sums in another order;
+    the activations are packed with ``ACT_TM`` beside ``ACT_FRAG``, for the same number of rows."""
+    ldo = out.shape[-1] if ldo is None else ldo
+    ab = (ptr(ab_w), ptr(ab_x), ptr(ab_out), ab_w.shape[0] if ab_w is not None else 0, ab_out.shape[-1] if ab_w is not None else 0)
+    if w.layout == "nvfp4":
+        call("owl_nvfp4_tm", ptr(w.codes), ptr(w.scales), float(w.alpha), ptr(w.row_scale), ptr(xpack), ptr(xs), ptr(out), ptr(residual),
+             *ab, m, w.n, w.k, ldo, epi, int(pdl), stream())
+        return
+    assert w.layout == "slice", "w4_tm reads slice-major records"
+    call("owl_w4_tm", ptr(w.records), ptr(xpack), ptr(xs), ptr(out), ptr(residual), *ab, m, w.n, w.k, ldo, w.group, epi, int(a8),
+         int(pdl), stream())
+
+
 def fma_status() -> int:
     """First bounded-wait failure recorded by the FMA-arm projection kernels (0 = none); clears it."""
     f = fn("owl_fma_status")
@@ -264,7 +282,7 @@ def fma_status() -> int:
     return f()
 
 
-_STATUS_WORDS = {"skinny": "owl_skinny_status", "fma": "owl_fma_status", "stream_tc": "owl_stream_tc_status",
+_STATUS_WORDS = {"skinny": "owl_skinny_status", "fma": "owl_fma_status", "stream_tc": "owl_stream_tc_status", "stream_tm": "owl_gemv_tm_status",
                  "gemm": "owl_gemm_status", "gemm_dense": "owl_gemm_dense_status", "gemm_nvfp4": "owl_gemm_nvfp4_status", "attn_tc": "owl_attn_tc_status", "comm": "owl_comm_status"}
 
 

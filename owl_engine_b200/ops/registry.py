@@ -45,6 +45,9 @@ _T = [
     KernelSpec("owl_gdn_copy_slot", "gdn.cu", "gdn"),
     KernelSpec("owl_w4_mma", "gemv_mma.cu", "gemv", gen="mma.sync+cp.async+dsmem"),
     KernelSpec("owl_nvfp4_mma", "gemv_mma.cu", "gemv", gen="mma.sync+cp.async+dsmem"),
+    KernelSpec("owl_w4_tm", "gemv_tm.cu", "gemv", gen="tcgen05+tmem+cp.async+bulk-copy+dsmem"),
+    KernelSpec("owl_nvfp4_tm", "gemv_tm.cu", "gemv", gen="tcgen05+tmem+cp.async+bulk-copy+dsmem"),
+    KernelSpec("owl_gemv_tm_status", "gemv_tm.cu", "status", capture=False),
     KernelSpec("owl_w4_fma", "gemv_fma.cu", "gemv", gen="hfma2+bulk-copy"),
     KernelSpec("owl_w4_fma_tp", "gemv_fma.cu", "gemv", gen="hfma2+bulk-copy+p2p"),
     KernelSpec("owl_fma_status", "gemv_fma.cu", "status", capture=False),

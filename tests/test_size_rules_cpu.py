@@ -39,3 +39,12 @@ def test_operand_of_a_short_prompt(n, k, t, resident, rows):
 def test_parts_of_the_keys(b, ctx, uniform, parts):
     r = SimpleNamespace(attn_splits=0, uniform_rows=uniform, max_splits=64, spec=PRESETS["qwen3.8-27b"]())
     assert HybridRunner._pick_splits(r, b, ctx) == parts
+
+
+# projections through tensor memory: four blocks of 8 rows (three for a large NVFP4 model), never in a speculating engine
+@pytest.mark.parametrize("layout,model,m,uniform,tm", [("slice", "qwen3.8-27b", 24, False, False), ("slice", "qwen3.8-27b", 25, False, True),
+                                                       ("slice", "qwen3.8-27b", 32, True, False), ("slice", "qwen3.5-0.8b", 32, False, True),
+                                                       ("nvfp4", "qwen3.8-27b", 16, False, False), ("nvfp4", "qwen3.8-27b", 17, False, True),
+                                                       ("nvfp4", "qwen3.5-0.8b", 17, False, False), ("nvfp4", "qwen3.5-0.8b", 25, False, True)])
+def test_projections_through_tensor_memory(layout, model, m, uniform, tm):
+    assert HybridRunner._tm(SimpleNamespace(uniform_rows=uniform, w=SimpleNamespace(layout=layout), spec=PRESETS[model]()), m) == tm
