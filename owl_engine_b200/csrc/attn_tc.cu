@@ -11,15 +11,20 @@
 //
 // One CTA = one (row tile, kv head), 320 threads, key tiles of 64:
 //   warp 0      producer: Q once (64 KB), then K_j (32 KB) and V_j (32 KB) through two-stage rings of their own
-//   warp 1      one thread issues S_j = Q K_j^T (16 x M128 N64 K16, bf16) into one of two 64-column S buffers, then
-//               O += P_{j-1} V_{j-1} (4 x M128 N256 K16, fp16) into the 256 O columns: S_{j} runs while the softmax of tile j-1
-//               is still busy
+//   warp 1      the whole warp walks the tiles, an elected lane issues S_j = Q K_j^T (16 x M128 N64 K16, bf16) into one of two 64-column
+//               S buffers, then O += P_{j-1} V_{j-1} (4 x M128 N256 K16, fp16) into the 256 O columns: S_{j} runs while the softmax of
+//               tile j-1 is still busy. Q is the A operand from tensor memory (the softmax warps put it there once): from shared memory
+//               an MMA of 64 columns reads 6 KB in its 32 clocks and takes 49, and issued by one lane 51
 //   warps 2-9   softmax, two threads per query row (each half of the tile's key columns; the halves' row maxima meet through
 //               shared memory at an mbarrier): tcgen05.ld S_j, causal mask on the diagonal tiles, running maximum,
 //               P_j = 2^(s - m) as fp16 into swizzled shared memory (the A operand of the second MMA), row sums. The maximum
 //               in use only moves when the new one exceeds it by more than 8 (a factor 256, far inside fp16 / fp32 range);
 //               then, after the PV product in flight has completed, the warp rescales its O rows in tensor memory
-//               (tcgen05.ld / st). At the end O / l goes out as bf16.
+//               (tcgen05.ld / st). At the end O / l goes out as bf16. S_j may be there before P_{j-2} V_{j-2} is done (products into
+//               different accumulators are not ordered): the wait for a product tells its round from the one two back
+// Measured (24 q heads, 4 kv heads): 2048 rows at 8192 keys 440 -> 323 us (1116 TFLOP/s of causal work), 2000 at 34816 1916 -> 1463
+// (1136), 2048 at 2048 92 -> 72. Bound: a tile takes about 1850 clocks, its MMAs 1040, its exponentials 512 of the special-function
+// unit; the rest is the softmax's chain (load, maximum, meeting point, exponentials, stores, proxy fence).
 // Every wait is bounded; on a timeout the CTA records an error code, the roles leave their loops, copies in flight are waited
 // for (bounded) and TMEM is freed.
 //
@@ -41,7 +46,7 @@ constexpr int AT_OFF_K = AT_Q_BYTES, AT_OFF_V = AT_OFF_K + 2 * AT_K_BYTES, AT_OF
 constexpr int AT_OFF_CTL = AT_OFF_P + 2 * AT_P_BYTES;    // 224 KB
 constexpr int AT_SMEM = AT_OFF_CTL + 2304;          // 231,680 bytes: the dynamic region is declared 1024-aligned
 constexpr int AT_THREADS = 320;        // producer warp, MMA warp, 8 softmax warps
-constexpr uint32_t AT_COL_S = 0, AT_COL_O = 128;         // TMEM columns: S0, S1 (64 each), O (256)
+constexpr uint32_t AT_COL_S = 0, AT_COL_O = 128, AT_COL_Q = 384;      // TMEM columns: S0, S1 (64 each), O (256), Q (128)
 constexpr float AT_LAZY = 8.f;
 
 struct AtParams {
@@ -50,7 +55,7 @@ struct AtParams {
   float scale_log2;
 };
 struct AtCtl {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full[2], p_empty[2], o_done;
+  uint64_t q_full, q_tmem, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full[2], p_empty[2], o_done[2];
   uint64_t pair[4];            // meeting point of the two softmax warps of a lane quarter (64 arrivals per phase)
   uint32_t tmem_base;
   volatile int abort_flag;
@@ -60,6 +65,7 @@ struct AtCtl {
 static_assert(sizeof(AtCtl) <= 2304, "control block exceeds its reservation");
 
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, AtCtl* c, int code) {
+  if (mbar_try_wait(bar, parity)) return true;       // the clock is read only when there is something to wait for
   const uint64_t t0 = global_ns();
   for (uint32_t i = 0; i < (1u << 22); ++i) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -71,25 +77,19 @@ __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, AtCtl* c
   return false;
 }
 // The same wait for the hand-offs on the critical path of a tile (scores ready, probabilities ready, the warps' meeting
-// point): test_wait polls instead of suspending the thread, whose wake-up costs more than the work it waits for.
+// point), by a whole warp, whose lanes leave together: a look at a time instead of a suspended thread, whose wake-up costs more than the
+// work it waits for. The clock is not read before a thousand looks: reading it takes longer than most of these waits.
 __device__ __forceinline__ bool at_spin(uint64_t* bar, uint32_t parity, AtCtl* c, int code) {
-  const uint64_t t0 = global_ns();
+  uint64_t t0 = 0;
   for (uint32_t i = 0;; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    if (ok) return true;
-    if ((i & 63u) == 63u) {
-      if (c->abort_flag) return false;
-      if (wait_expired(t0)) break;
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    if ((i & 1023u) == 1023u) {
+      bool stop = c->abort_flag != 0;
+      if (t0 == 0) t0 = global_ns();
+      else if (wait_expired(t0)) { stop = true; c->abort_flag = 1; atomicCAS(&g_attn_tc_status, 0, code); }
+      if (__any_sync(0xffffffffu, stop)) return false;
     }
   }
-  c->abort_flag = 1;
-  atomicCAS(&g_attn_tc_status, 0, code);
-  return false;
 }
 // 32 lanes x 32 consecutive 32-bit columns <- 32 registers per thread (lane = TMEM lane)
 __device__ __forceinline__ void at_tmem_st_x32(uint32_t taddr, const uint32_t* r) {
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     if (threadIdx.x == 0) atomicCAS(&g_attn_tc_status, 0, OWL_ERR_BAD_ARG);
     return;
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // the row tiles with the most key tiles start first
   const int tile = p.row_tiles - 1 - (int)blockIdx.x, kh = blockIdx.y;
   const int row0 = tile * AT_BM;
@@ -128,13 +128,14 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
 
   if (threadIdx.x == 0) {
     mbar_init(&ctl->q_full, 1);
+    mbar_init(&ctl->q_tmem, 8);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&ctl->k_full[s], 1); mbar_init(&ctl->k_empty[s], 1);
       mbar_init(&ctl->v_full[s], 1); mbar_init(&ctl->v_empty[s], 1);
       mbar_init(&ctl->s_full[s], 1); mbar_init(&ctl->s_empty[s], 8);
       mbar_init(&ctl->p_full[s], 8); mbar_init(&ctl->p_empty[s], 1);
     }
-    mbar_init(&ctl->o_done, 1);
+    mbar_init(&ctl->o_done[0], 1); mbar_init(&ctl->o_done[1], 1);
     for (int q = 0; q < 4; ++q) mbar_init(&ctl->pair[q], 64);
     ctl->abort_flag = 0;
     mbar_fence_init();
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -178,46 +179,45 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_s = umma_idesc_f16(AT_BM, AT_BN, 1), idesc_o = umma_idesc_f16(AT_BM, AT_HD, 0);
-      const uint32_t sq = smem_u32(base);
-      bool ok = at_wait(&ctl->q_full, 0, ctl, OWL_ERR_WAIT_TMA);
-      auto pv = [&](int j) -> bool {        // O (+)= P_j V_j
-        const int s = j & 1;
-        const uint32_t ph = ((uint32_t)(j >> 1)) & 1u;
-        if (!at_spin(&ctl->p_full[s], ph, ctl, OWL_ERR_WAIT_EPI)) return false;
-        if (!at_spin(&ctl->v_full[s], ph, ctl, OWL_ERR_WAIT_TMA)) return false;
-        tc_fence_after();
-        const uint64_t dp = umma_desc_k128(smem_u32(base + AT_OFF_P + s * AT_P_BYTES));
-        const uint64_t dv = umma_desc_k128(smem_u32(base + AT_OFF_V + s * AT_V_BYTES));
+    // the whole warp runs the loop, an elected lane issues (see common.cuh)
+    const uint32_t idesc_s = umma_idesc_f16(AT_BM, AT_BN, 1), idesc_o = umma_idesc_f16(AT_BM, AT_HD, 0);
+    const uint32_t sb = smem_u32(base);
+    bool ok = at_spin(&ctl->q_tmem, 0, ctl, OWL_ERR_WAIT_EPI);
+    auto pv = [&](int j) -> bool {        // O (+)= P_j V_j
+      const int s = j & 1;
+      const uint32_t ph = ((uint32_t)(j >> 1)) & 1u;
+      if (!at_spin(&ctl->p_full[s], ph, ctl, OWL_ERR_WAIT_EPI)) return false;
+      if (!at_spin(&ctl->v_full[s], ph, ctl, OWL_ERR_WAIT_TMA)) return false;
+      tc_fence_after();
+      const uint64_t dp = umma_desc_k128(sb + AT_OFF_P + s * AT_P_BYTES), dv = umma_desc_k128(sb + AT_OFF_V + s * AT_V_BYTES);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)          // 16 keys = 32 bytes of the 128-byte rows per instruction
-          tc_mma_f16(tmem + AT_COL_O, dp + (uint64_t)(i * 2), dv + (uint64_t)(i * 2), idesc_o, (j > 0 || i > 0) ? 1u : 0u);
-        tc_commit(&ctl->v_empty[s]);
-        tc_commit(&ctl->p_empty[s]);
-        tc_commit(&ctl->o_done);
-        return true;
-      };
-      for (int j = 0; ok && j < n_kv; ++j) {
-        const int s = j & 1;
-        const uint32_t ph = ((uint32_t)(j >> 1)) & 1u;
-        if (!at_spin(&ctl->k_full[s], ph, ctl, OWL_ERR_WAIT_TMA)) { ok = false; break; }
-        if (!at_spin(&ctl->s_empty[s], ph ^ 1u, ctl, OWL_ERR_WAIT_EPI)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t sk = smem_u32(base + AT_OFF_K + s * AT_K_BYTES);
+      for (int i = 0; i < 4; ++i)          // 16 keys = 32 bytes of the 128-byte rows per instruction
+        tc_mma_f16_warp(tmem + AT_COL_O, dp + (uint64_t)(i * 2), dv + (uint64_t)(i * 2), idesc_o, (j > 0 || i > 0) ? 1u : 0u);
+      tc_commit_warp(&ctl->v_empty[s]);
+      tc_commit_warp(&ctl->p_empty[s]);
+      tc_commit_warp(&ctl->o_done[s]);
+      return true;
+    };
+    for (int j = 0; ok && j < n_kv; ++j) {
+      const int s = j & 1;
+      const uint32_t ph = ((uint32_t)(j >> 1)) & 1u;
+      if (!at_spin(&ctl->k_full[s], ph, ctl, OWL_ERR_WAIT_TMA)) { ok = false; break; }
+      if (!at_spin(&ctl->s_empty[s], ph ^ 1u, ctl, OWL_ERR_WAIT_EPI)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t sk = sb + AT_OFF_K + s * AT_K_BYTES;
 #pragma unroll
-        for (int kb = 0; kb < 4; ++kb) {
-          const uint64_t dq = umma_desc_k128(sq + kb * (AT_BM * 128)), dk = umma_desc_k128(sk + kb * (AT_BN * 128));
+      for (int kb = 0; kb < 4; ++kb) {
+        const uint64_t dk = umma_desc_k128(sk + kb * (AT_BN * 128));
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            tc_mma_f16(tmem + AT_COL_S + s * AT_BN, dq + (uint64_t)(i * 2), dk + (uint64_t)(i * 2), idesc_s, (kb > 0 || i > 0) ? 1u : 0u);
-        }
-        tc_commit(&ctl->k_empty[s]);
-        tc_commit(&ctl->s_full[s]);
-        if (j > 0 && !pv(j - 1)) { ok = false; break; }
+        for (int i = 0; i < 4; ++i)
+          tc_mma_f16_ts_warp(tmem + AT_COL_S + s * AT_BN, tmem + AT_COL_Q + kb * 32 + i * 8, dk + (uint64_t)(i * 2), idesc_s,
+                             (kb > 0 || i > 0) ? 1u : 0u);
       }
-      if (ok && n_kv > 0) pv(n_kv - 1);
+      tc_commit_warp(&ctl->k_empty[s]);
+      tc_commit_warp(&ctl->s_full[s]);
+      if (j > 0 && !pv(j - 1)) { ok = false; break; }
     }
+    if (ok && n_kv > 0) pv(n_kv - 1);
   } else {
     // Two warps per TMEM lane quarter: both own the same 32 query rows, each half of a tile's 64 key columns (and half of
     // the O columns when rows are rescaled). They meet once per tile, at an mbarrier of 64 arrivals (a bounded wait like every other), to exchange the
@@ -227,12 +227,31 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     const int limit = grow < p.rows ? p.pos0 + grow / p.gq + 1 : 1;      // keys visible to this row (padding rows: one key)
     const uint32_t lane_addr = tmem + ((uint32_t)(q4 * 32) << 16);
     uint8_t* prow_base = base + AT_OFF_P + (r_loc >> 3) * 1024 + (r_loc & 7) * 128;
+    // Q to tensor memory as the A operand of the first product: this thread's row, half of its 256 elements
+    bool q_ok = __all_sync(0xffffffffu, at_wait(&ctl->q_full, 0, ctl, OWL_ERR_WAIT_TMA));
+    if (q_ok) {
+#pragma unroll 1
+      for (int kb = 2 * hf; kb < 2 * hf + 2; ++kb) {
+        uint32_t q[32];
+        const uint8_t* src = base + kb * (AT_BM * 128) + r_loc * 128;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint4 v = *reinterpret_cast<const uint4*>(src + ((c ^ (r_loc & 7)) << 4));
+          q[c * 4] = v.x; q[c * 4 + 1] = v.y; q[c * 4 + 2] = v.z; q[c * 4 + 3] = v.w;
+        }
+        at_tmem_st_x32(lane_addr + AT_COL_Q + kb * 32, q);
+      }
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->q_tmem);
+    }
     float m_used = -INFINITY, l = 0.f;                       // l: this thread's half of the row sum
-    bool ok = true;
-    for (int j = 0; j < n_kv; ++j) {
+    bool ok = q_ok;
+    for (int j = 0; ok && j < n_kv; ++j) {
       const int s = j & 1;
       const uint32_t ph = ((uint32_t)(j >> 1)) & 1u;
-      if (!__all_sync(0xffffffffu, at_spin(&ctl->s_full[s], ph, ctl, OWL_ERR_WAIT_MMA))) { ok = false; break; }
+      if (!at_spin(&ctl->s_full[s], ph, ctl, OWL_ERR_WAIT_MMA)) { ok = false; break; }
       tc_fence_after();
       uint32_t sv[32];
       tmem_ld_32x32b_x32(lane_addr + AT_COL_S + s * AT_BN + hf * 32, sv);
@@ -256,7 +275,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
       ctl->mx[s][hf][r_loc] = mx;
       mbar_arrive(&ctl->pair[q4]);                           // (arrive has release, the wait acquire semantics)
-      if (!__all_sync(0xffffffffu, at_spin(&ctl->pair[q4], (uint32_t)j & 1u, ctl, OWL_ERR_WAIT_EPI))) { ok = false; break; }
+      if (!at_spin(&ctl->pair[q4], (uint32_t)j & 1u, ctl, OWL_ERR_WAIT_EPI)) { ok = false; break; }
       mx = fmaxf(mx, ctl->mx[s][hf ^ 1][r_loc]);             // both warps of the row now hold the same maximum
       // Rows whose every key of this tile is masked keep their maximum (a tile past the row's limit inside the row tile).
       const bool grow_m = mx > m_used + AT_LAZY;
@@ -266,7 +285,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         const float f = (m_used == -INFINITY) ? 0.f : at_ex2(m_used - m_new);
         if (j > 0) {
           // the product that still adds to O must have completed before its rows are rescaled
-          if (!__all_sync(0xffffffffu, at_wait(&ctl->o_done, ((uint32_t)(j - 1)) & 1u, ctl, OWL_ERR_WAIT_MMA))) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, at_wait(&ctl->o_done[s ^ 1], ((uint32_t)((j - 1) >> 1)) & 1u, ctl, OWL_ERR_WAIT_MMA))) { ok = false; break; }
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < AT_HD / 64; ++c) {             // this warp's half of the O columns
@@ -284,7 +303,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         m_used = m_new;
       }
       // P_j (fp16) into the swizzled A-operand tile; the buffer is free once the product two tiles back has read it
-      if (!__all_sync(0xffffffffu, at_spin(&ctl->p_empty[s], ph ^ 1u, ctl, OWL_ERR_WAIT_MMA))) { ok = false; break; }
+      if (!at_spin(&ctl->p_empty[s], ph ^ 1u, ctl, OWL_ERR_WAIT_MMA)) { ok = false; break; }
       uint8_t* prow = prow_base + s * AT_P_BYTES;
       float s4[4] = {0.f, 0.f, 0.f, 0.f};
       const float nm = -m_used;
@@ -311,7 +330,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       ok = __all_sync(0xffffffffu, at_wait(&ctl->pair[q4], (uint32_t)n_kv & 1u, ctl, OWL_ERR_WAIT_EPI));
     }
     l += ctl->mx[n_kv & 1][hf ^ 1][r_loc];
-    if (ok && n_kv > 0 && __all_sync(0xffffffffu, at_wait(&ctl->o_done, ((uint32_t)(n_kv - 1)) & 1u, ctl, OWL_ERR_WAIT_MMA))) {
+    if (ok && n_kv > 0 && __all_sync(0xffffffffu, at_wait(&ctl->o_done[(n_kv - 1) & 1], ((uint32_t)((n_kv - 1) >> 1)) & 1u, ctl, OWL_ERR_WAIT_MMA))) {
       tc_fence_after();
       const float inv = 1.f / l;
       __nv_bfloat16* orow = p.out + ((size_t)kh * p.rows + grow) * AT_HD + hf * (AT_HD / 2);
