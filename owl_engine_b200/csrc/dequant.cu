@@ -1,6 +1,6 @@
-// Expand a W4 skinny-tile weight to dense fp16 or bf16 [N][K]: prompts above 256 tokens (one projection ahead of the dense GEMM),
-// resident dense copies, the baseline arm (dequant -> library GEMM) and tests. Shorter prompts dequantise inside the GEMM
-// (gemm_w4.cu; block-layout weights gemm_tc.cu).
+// Expand a W4 skinny-tile weight to dense fp16 or bf16 [N][K]: resident dense copies, the 8-bit arms, long prompts of block-layout
+// weights (one projection ahead of the dense GEMM), the baseline arm (dequant -> library GEMM) and tests. Prompts on slice-major
+// weights dequantise inside the GEMM (gemm_w4.cu; short ones of block-layout weights gemm_tc.cu).
 // Reference counterpart: owl_gguf_dequant_range_* + cuBLAS arm (crates/kernels/cu/gguf/gguf_smem.cu).
 #include "common.cuh"
 

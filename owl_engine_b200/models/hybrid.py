@@ -1015,11 +1015,11 @@ class HybridRunner:
         return linear.w4_gemm(w, x, out, arm=self.prefill_gemm, ahead=ahead)
 
     def _dequant_ahead(self, t: int):
-        """The ``DequantAhead`` of a ``t``-row chunk, started on this model's weights, or None: chunks above the sizes that read
-        the int4 records directly, on the arm that dequantises per chunk, with products long enough to hide it behind."""
+        """The ``DequantAhead`` of a ``t``-row chunk, started on this model's weights, or None: long chunks of block-layout weights (the
+        others' records are dequantised inside the GEMM), with products long enough to hide it behind."""
         from ..ops import gemm_tc, linear
 
-        if self.prefill_gemm not in ("tc", "tc4") or t <= gemm_tc.ROWS_UPTO or self.w.layout not in ("slice", "block") or not self.w.layers \
+        if self.prefill_gemm not in ("tc", "tc4") or t <= gemm_tc.ROWS_UPTO or self.w.layout != "block" or not self.w.layers \
                 or torch.cuda.is_current_stream_capturing():
             return None
         order = [w for lw in self.w.layers

@@ -3,12 +3,12 @@
 ``w4_gemm`` computes ``out[T, N] = x[T, K] @ dequant(w)^T`` for a ``W4Skinny`` weight with one of these arms:
 
 * ``"tc"``        the product path, all steps our own sm_100a kernels. Slice-major weights: up to ``SKINNY_UPTO`` tokens the
-                  decode-shape streaming kernel (``csrc/gemv_mma.cu``), up to 256 (``rows_pay``) the tcgen05 GEMM that reads the
-                  int4 records and dequantises each once (``csrc/gemm_w4.cu``), above that the weight is dequantised into a dense
-                  fp16 matrix (``csrc/dequant.cu``, beside the GEMM before it where ``DequantAhead`` applies) and the dense
-                  tcgen05 GEMM multiplies it. Block-layout weights and operands that are not 16-byte aligned: below
-                  ``DEQUANT_FROM`` tokens the tiled GEMM that dequantises in the kernel once per 128 tokens
-                  (``csrc/gemm_tc.cu``), from there the dense form;
+                  decode-shape streaming kernel (``csrc/gemv_mma.cu``), above that the tcgen05 GEMM that reads the int4 records and
+                  dequantises them into tensor memory, once per 256 tokens (``csrc/gemm_w4.cu``). Matrices under a million weights
+                  above 256 tokens: dequantised into a dense fp16 matrix (``csrc/dequant.cu``) that the dense tcgen05 GEMM multiplies.
+                  Block-layout weights and operands that are not 16-byte aligned: below ``DEQUANT_FROM`` tokens the tiled GEMM that
+                  dequantises in the kernel once per 128 tokens (``csrc/gemm_tc.cu``), from there the dense form (beside the GEMM
+                  before it where ``DequantAhead`` applies);
 * ``"tc8"``       the W4A8 arm on tensor cores: like ``"tc"``, but from ``DEQUANT_FROM`` tokens the dequantised weight is
                   re-quantised per output row to e4m3 and the activations per token, and the product runs as
                   ``tcgen05.mma kind::f8f6f4`` at twice the 16-bit rate (the reference's W4A8 arm quantises
@@ -255,8 +255,12 @@ def rows_pay(n: int, k: int, t: int, resident: bool) -> bool:
 
 
 def _rows_ok(w, x: torch.Tensor, out: torch.Tensor, resident: bool) -> bool:
-    """One launch reads the int4 records and dequantises each weight once."""
-    return w.layout == "slice" and x.dtype == torch.float16 and rows_pay(w.n, w.k, x.shape[0], resident) and x.stride(0) % 8 == 0 \
+    """One launch reads the int4 records and dequantises each weight once per chunk of at most 256 tokens. Above 256 tokens that takes
+    the place of the dense copy made per call (small matrices, which are all start-up in either form, keep it: from 2 M weights the
+    records are faster at every count, 1024 x 2048 at 257 / 2048 tokens 9.9 / 12.9 us against 15.3 / 20.4)."""
+    t = x.shape[0]
+    long = t > gemm_tc.ROWS_UPTO and not resident and w.n * w.k >= 1 << 20
+    return w.layout == "slice" and x.dtype == torch.float16 and (long or rows_pay(w.n, w.k, t, resident)) and x.stride(0) % 8 == 0 \
         and out.stride(0) % 8 == 0 and (x.data_ptr() | out.data_ptr()) % 16 == 0
 
 

@@ -145,15 +145,20 @@ def test_rows_gemm_dequantises_once(t, n, k, group):
 
 
 # the last and first token counts of every stage and accumulator layout; two units of an odd number of steps a CTA (one set starts the
-# second unit), a lone step, and parts cut along k (whose sums go through the scratch)
-@pytest.mark.parametrize("t", [128, 129, 160, 161])
-@pytest.mark.parametrize("n,k", [(20480, 640), (19088, 384), (1040, 4736)])
+# second unit), a lone step, parts cut along k (whose sums go through the scratch), one row tile; one to six chunks of tokens
+@pytest.mark.parametrize("t", [128, 129, 160, 161, 257, 515, 1300])
+@pytest.mark.parametrize("n,k", [(20480, 640), (19088, 384), (1040, 4736), (48, 128)])
 def test_rows_gemm_walks_units_and_stages(t, n, k):
     gen = torch.Generator(device=DEV).manual_seed(n + k + t)
     w = Q.random_skinny(n, k, 32, DEV, 0.05, n + k)
     x = torch.randn(t, k, generator=gen, device=DEV).half()
-    _check_against_dequant(w, x, gemm_tc.w4_gemm_rows(w, x, torch.zeros(t, n, dtype=torch.bfloat16, device=DEV)))
-    assert K.all_status()["gemm_dense"] == 0
+    out = torch.zeros(t, n + 8, dtype=torch.bfloat16, device=DEV)
+    gemm_tc.w4_gemm_rows(w, x, out)
+    _check_against_dequant(w, x, out[:, :n])
+    act = torch.zeros(t, n // 2 + 8, dtype=torch.float16, device=DEV)
+    gemm_tc.w4_gemm_rows(w, x, act, silu=True)
+    torch.testing.assert_close(act[:, :n // 2].float(), _silu_ref(out[:, :n].contiguous()).float(), rtol=2.0 ** -9, atol=2.0 ** -20)
+    assert (out[:, n:] == 0).all() and (act[:, n // 2:] == 0).all() and K.all_status()["gemm_dense"] == 0
 
 
 @pytest.mark.parametrize("vec", [4, 4096, 5000])
