@@ -560,8 +560,10 @@ OWL_API int owl_stream_tc_trace(void* host_dst) {
 }
 #endif
 
+OWL_API int owl_gemv_tm_status();
 OWL_API int owl_stream_tc_status() {
+  const int w = owl_gemv_tm_status();       // the streaming projections of gemv_tm.cu report here
   int v = 0;
   cudaMemcpyFromSymbol(&v, g_stream_tc_status, sizeof(int));
-  return v;
+  return v != 0 ? v : w;
 }

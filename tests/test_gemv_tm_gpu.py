@@ -15,7 +15,7 @@ def _through_tensor_memory(monkeypatch):
     monkeypatch.setattr(K, "ACT_FRAG", K.ACT_FRAG | K.ACT_TM)
     yield
     torch.cuda.synchronize()
-    assert K.all_status()["stream_tm"] == 0
+    assert K.all_status()["stream_tc"] == 0
 
 
 @pytest.mark.parametrize("fmt", ["g128", "g32", "nvfp4"])
