@@ -22,7 +22,7 @@ KS_SCRATCH_BYTES = 160 * 128 * 256 * 4
 
 
 _order = threading.Lock()
-_last: dict = {}         # device -> the stream whose product used the scratch last
+_last: dict = {}         # device index -> (handle, stream) whose product used the scratch last
 
 
 def _call(device, name: str, *args) -> None:
@@ -30,13 +30,15 @@ def _call(device, name: str, *args) -> None:
     thread) launched before it: the parts of all of them lie in the device's one scratch. (Inside a capture the graph's launches
     are ordered by whoever replays it.)"""
     with _order:
-        st = torch.cuda.current_stream(device)
-        last = _last.get(device)
-        if last is not st and last != st and not torch.cuda.is_current_stream_capturing():
+        dev = torch._C._cuda_getDevice() if device.index is None else device.index
+        raw = torch._C._cuda_getCurrentRawStream(dev)
+        last = _last.get(dev)
+        if (last is None or last[0] != raw) and not torch.cuda.is_current_stream_capturing():
+            st = torch.cuda.current_stream(dev)
             if last is not None:
-                st.wait_stream(last)
-            _last[device] = st
-        K.call(name, *args, st.cuda_stream)
+                st.wait_stream(last[1])
+            _last[dev] = (raw, st)
+        K.call(name, *args, raw)
 
 
 def ensure_scratch(device) -> None:

@@ -73,7 +73,8 @@ def ptr(t) -> int | None:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle (without the stream object: making one took 7 of the 13 us of a launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 # Ring of the most recent native launches (entry name + raw arguments), formatted on demand by ``recent_launches``:
