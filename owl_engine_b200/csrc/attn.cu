@@ -128,6 +128,8 @@ __global__ void __launch_bounds__(QI_WARPS * 32) qknorm_rope_insert_rows_kernel(
   __shared__ float sn_s[128], cs_s[128];
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, hd = 256;
   const int half = p.rot >> 1;
+  pdl_launch_dependents();
+  pdl_wait();
   for (int j = tid; j < half; j += QI_WARPS * 32) {
     const int pos = p.pos3[(size_t)p.section[j] * p.rows + row];
     float sn, cs;
@@ -562,9 +564,7 @@ static int insert_launch(const void* qraw, int ldq, const void* kraw, int ldk, c
   const uintptr_t al = (uintptr_t)qraw | (uintptr_t)kraw | (uintptr_t)vraw | (uintptr_t)qnorm_w | (uintptr_t)knorm_w |
                        (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool;
   if (rows >= 160 && (long long)rows * (hq + 2 * hkv) >= 3072 && !pdl && hd == 256 && !(rot & 15) && !((ldq | ldk | ldv) & 7) && !(al & 15)) {
-    qknorm_rope_insert_rows_kernel<<<rows, QI_WARPS * 32, 0, st>>>(p);
-    OWL_LAUNCH_CHECK();
-    return OWL_OK;
+    return launch_dep(rows, qknorm_rope_insert_rows_kernel, dim3(rows), dim3(QI_WARPS * 32), 0, st, p);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(rows, hq + 2 * hkv); cfg.blockDim = dim3(128); cfg.stream = st;

@@ -139,6 +139,8 @@ __global__ void __launch_bounds__(512) causal_softmax_smem_kernel(__half* __rest
 __global__ void __launch_bounds__(256) attn_gate_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ qraw,
                                                         int ldq, int D, void* __restrict__ out, int HD, int out_f16, int gq,
                                                         const float* __restrict__ inv_sum) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= (HD >> 3)) return;
   const int e = c * 8, head = e / D, off = e % D;
@@ -165,6 +167,8 @@ using namespace owl;
 
 // q bf16 [rows][hq][D] -> qg [hkv][rows][gq][D]: the q heads of one kv head become consecutive rows of one GEMM operand.
 __global__ void __launch_bounds__(256) q_group_kernel(const uint4* __restrict__ q, uint4* __restrict__ qg, int hq, int gq, int cpd) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.y, rows = gridDim.y, c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= hq * cpd) return;
   const int head = c / cpd, off = c % cpd;
@@ -174,19 +178,15 @@ __global__ void __launch_bounds__(256) q_group_kernel(const uint4* __restrict__ 
 OWL_API int owl_q_group(const void* q, void* qg, int rows, int hq, int hkv, int D, cudaStream_t st) {
   if (rows < 1 || hkv < 1 || hq % hkv || (D & 7) || !q || !qg) return OWL_ERR_BAD_ARG;
   const int cpd = D / 8;
-  q_group_kernel<<<dim3((hq * cpd + 255) / 256, rows), 256, 0, st>>>((const uint4*)q, (uint4*)qg, hq, hq / hkv, cpd);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  return launch_dep(rows, q_group_kernel, dim3((hq * cpd + 255) / 256, rows), dim3(256), 0, st, (const uint4*)q, (uint4*)qg, hq, hq / hkv, cpd);
 }
 
 // gq > 0: `o` is the grouped layout [hkv][rows][gq][D]; gq = 0: [rows][HD].
 OWL_API int owl_attn_gate(const void* o, const void* qraw, int ldq, int D, void* out, int rows, int HD, int out_f16, int gq,
                           const void* inv_sum, cudaStream_t st) {
   if (rows < 1 || (HD & 7) || (D & 7) || (ldq & 7) || !o || !qraw || !out || gq < 0) return OWL_ERR_BAD_ARG;
-  attn_gate_kernel<<<dim3((HD / 8 + 255) / 256, rows), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)qraw, ldq, D, out,
-                                                                   HD, out_f16, gq, (const float*)inv_sum);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  return launch_dep(rows, attn_gate_kernel, dim3((HD / 8 + 255) / 256, rows), dim3(256), 0, st, (const __nv_bfloat16*)o, (const __nv_bfloat16*)qraw,
+                    ldq, D, out, HD, out_f16, gq, (const float*)inv_sum);
 }
 
 // bt: the sequence's block-table row (int32 page numbers). fmt: 0 e4m3, 1 int8 with k_scale / v_scale [pages][16][hkv], 2 fp16.

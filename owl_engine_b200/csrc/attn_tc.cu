@@ -151,6 +151,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -416,9 +418,7 @@ OWL_API int owl_attn_tc(const void* qg, const void* k, const void* vt, void* og,
   p.out = (__nv_bfloat16*)og; p.rows = rows; p.gq = gq; p.pos0 = pos0; p.hkv = hkv;
   p.row_tiles = (rows + AT_BM - 1) / AT_BM;
   p.scale_log2 = scale * 1.4426950408889634f;
-  attn_tc_kernel<<<dim3(p.row_tiles, hkv), AT_THREADS, AT_SMEM, st>>>(mq, mk, mv, p);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  return launch_dep(rows / gq, attn_tc_kernel, dim3(p.row_tiles, hkv), dim3(AT_THREADS), AT_SMEM, st, mq, mk, mv, p);
 }
 
 OWL_API int owl_attn_tc_status() {

@@ -51,6 +51,8 @@ namespace owl {
 __global__ void __launch_bounds__(256) quant_e4m3_rows_kernel(const uint16_t* __restrict__ x, int ldx, int f16,
                                                               uint8_t* __restrict__ out, int ldo, float* __restrict__ scales,
                                                               int K) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[32];
   const int row = blockIdx.x;
   const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * ldx);
@@ -96,7 +98,6 @@ __global__ void __launch_bounds__(256) quant_e4m3_rows_kernel(const uint16_t* __
 OWL_API int owl_quant_e4m3_rows(const void* x, int ldx, int f16, void* out, int ldo, void* scales, int R, int K,
                                 cudaStream_t st) {
   if (R < 1 || K < 8 || (K & 7) || (ldx & 7) || (ldo & 7) || !scales) return OWL_ERR_BAD_ARG;
-  owl::quant_e4m3_rows_kernel<<<R, 256, 0, st>>>((const uint16_t*)x, ldx, f16, (uint8_t*)out, ldo, (float*)scales, K);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  return owl::launch_dep(R, owl::quant_e4m3_rows_kernel, dim3(R), dim3(256), 0, st, (const uint16_t*)x, ldx, f16, (uint8_t*)out, ldo,
+                         (float*)scales, K);
 }

@@ -300,6 +300,8 @@ __global__ void __launch_bounds__(256) gdn_conv_fwd_kernel(const __nv_bfloat16* 
                                                            const float* __restrict__ conv_w, float* conv_state,
                                                            int slot, __nv_bfloat16* out, int T, int nk, int nv,
                                                            int use_state) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int seg = blockIdx.x;
   const int t0 = (blockIdx.y * 8 + warp) * TR;
@@ -343,6 +345,8 @@ __global__ void __launch_bounds__(256) gdn_conv_fwd_kernel(const __nv_bfloat16* 
 // when the chunk is shorter than 3). One thread per channel. Runs after gdn_conv_fwd_kernel.
 __global__ void gdn_conv_state_kernel(const __nv_bfloat16* __restrict__ x, int ld, float* conv_state, int slot, int T,
                                       int conv_dim, int use_state) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= conv_dim) return;
   float* cs = conv_state + ((size_t)slot * conv_dim + ch) * 3;
@@ -570,6 +574,8 @@ __global__ void __launch_bounds__(256) gdn_scan2_kernel(GdnScanParams p, float* 
 __global__ void __launch_bounds__(256) gdn_norm_gate_kernel(const float* __restrict__ raw, const __nv_bfloat16* __restrict__ z,
                                                             int ldz, const float* __restrict__ gamma, __nv_bfloat16* out,
                                                             int T, int nv, float eps, int out_f16) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long wid = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (wid >= (long long)T * nv) return;
@@ -634,17 +640,11 @@ OWL_API int owl_gdn_conv_fwd(const void* x, int ld, const void* conv_w, void* co
   const int conv_dim = (2 * nk + nv) * GD;
   const int tr = T >= 512 ? 8 : 2;
   const dim3 grid(2 * nk + nv, (T + 8 * tr - 1) / (8 * tr));
-  if (tr == 8)
-    gdn_conv_fwd_kernel<8><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (const float*)conv_w, (float*)conv_state, slot,
-                                                 (__nv_bfloat16*)out, T, nk, nv, use_state);
-  else
-    gdn_conv_fwd_kernel<2><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (const float*)conv_w, (float*)conv_state, slot,
-                                                 (__nv_bfloat16*)out, T, nk, nv, use_state);
-  OWL_LAUNCH_CHECK();
-  gdn_conv_state_kernel<<<(conv_dim + 255) / 256, 256, 0, st>>>((const __nv_bfloat16*)x, ld, (float*)conv_state, slot, T,
-                                                                conv_dim, use_state);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  const int rc = launch_dep(T, tr == 8 ? gdn_conv_fwd_kernel<8> : gdn_conv_fwd_kernel<2>, grid, dim3(256), 0, st, (const __nv_bfloat16*)x, ld,
+                            (const float*)conv_w, (float*)conv_state, slot, (__nv_bfloat16*)out, T, nk, nv, use_state);
+  if (rc != OWL_OK) return rc;
+  return launch_dep(T, gdn_conv_state_kernel, dim3((conv_dim + 255) / 256), dim3(256), 0, st, (const __nv_bfloat16*)x, ld, (float*)conv_state,
+                    slot, T, conv_dim, use_state);
 }
 
 OWL_API int owl_gdn_scan(const void* qkv, const void* z, int ldz, const void* ab, int ldab, const void* a_log,
@@ -668,10 +668,8 @@ OWL_API int owl_gdn_norm_gate(const void* raw, const void* z, int ldz, const voi
                               int out_f16, cudaStream_t st) {
   if (T < 1 || nv < 1 || (ldz & 3) || !raw || !out) return OWL_ERR_BAD_ARG;
   const long long warps = (long long)T * nv;
-  gdn_norm_gate_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>((const float*)raw, (const __nv_bfloat16*)z, ldz,
-                                                                   (const float*)gamma, (__nv_bfloat16*)out, T, nv, eps, out_f16);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  return launch_dep(T, gdn_norm_gate_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, (const float*)raw, (const __nv_bfloat16*)z, ldz,
+                    (const float*)gamma, (__nv_bfloat16*)out, T, nv, eps, out_f16);
 }
 
 OWL_API int owl_gdn_scan_split(const void* qkv, const void* z, int ldz, const void* ab, int ldab, const void* a_log,

@@ -100,6 +100,8 @@ __device__ __forceinline__ uint4 scale2_bf16x8(const uint4& u, float s, float e)
                     pack_bf16(bf16_lo(u.z) * s * e, bf16_hi(u.z) * s * e), pack_bf16(bf16_lo(u.w) * s * e, bf16_hi(u.w) * s * e));
 }
 __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t ck_smem[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(ck_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
@@ -287,6 +289,8 @@ struct ScanSmem {
   __nv_bfloat16 vn[CK_C][CK_LT];    // v': [token][value column]
 };
 __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t ck_smem[];
   ScanSmem& sm = *reinterpret_cast<ScanSmem*>(ck_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
@@ -453,9 +457,7 @@ OWL_API int owl_gdn_chunk_scan(const void* qkv, const void* ab, int ldab, const 
   p.kd = base + 4 * rows;
   p.attn = p.kd + (size_t)nv * p.chunks * CK_D * CK_C;
   p.eglast = reinterpret_cast<float*>(p.attn + (size_t)nv * p.chunks * CK_C * CK_C);
-  gdn_chunk_prep_kernel<<<dim3(p.chunks, nv), 256, sizeof(PrepSmem), st>>>(p);
-  OWL_LAUNCH_CHECK();
-  gdn_chunk_scan_kernel<<<dim3(nv, CK_D / CK_NC), 256, sizeof(ScanSmem), st>>>(p);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  const int rc = launch_dep(T, gdn_chunk_prep_kernel, dim3(p.chunks, nv), dim3(256), sizeof(PrepSmem), st, p);
+  if (rc != OWL_OK) return rc;
+  return launch_dep(T, gdn_chunk_scan_kernel, dim3(nv, CK_D / CK_NC), dim3(256), sizeof(ScanSmem), st, p);
 }

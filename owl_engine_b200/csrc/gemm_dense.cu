@@ -151,6 +151,8 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_dense_kernel(const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl->tmem_base;
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -324,6 +326,8 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_dense_kernel(const __grid_
 // out[row][col] = bf16(sum over parts): grid (ceil(N / 1024), T), 256 threads x 4 columns
 __global__ void __launch_bounds__(256) gemm_ksplit_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out,
                                                                  int T, int N, int ldp, int ldo, int ks) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.y, col = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (col >= N) return;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -343,6 +347,8 @@ __global__ void __launch_bounds__(256) gemm_ksplit_reduce_kernel(const float* __
 // The same with the silu(gate) * up epilogue: grid (ceil(N / 4096), T), 256 threads x 16 columns
 __global__ void __launch_bounds__(256) gemm_ksplit_silu_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out,
                                                                int T, int N, int ldp, int ldo, int ks) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.y, col = (blockIdx.x * 256 + threadIdx.x) * 16;
   if (col >= N) return;
   float v[16];
@@ -402,12 +408,8 @@ float* gd_split_scratch(size_t* bytes) {
   return g_ks_scratch[dev];
 }
 int gd_split_reduce(const float* partial, void* out, int T, int N, int ldp, int ldo, int ks, int silu, cudaStream_t st) {
-  if (silu)
-    gemm_ksplit_silu_kernel<<<dim3((N + 4095) / 4096, T), 256, 0, st>>>(partial, (__nv_bfloat16*)out, T, N, ldp, ldo, ks);
-  else
-    gemm_ksplit_reduce_kernel<<<dim3((N + 1023) / 1024, T), 256, 0, st>>>(partial, (__nv_bfloat16*)out, T, N, ldp, ldo, ks);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  return launch_dep(T, silu ? gemm_ksplit_silu_kernel : gemm_ksplit_reduce_kernel, silu ? dim3((N + 4095) / 4096, T) : dim3((N + 1023) / 1024, T),
+                    dim3(256), 0, st, partial, (__nv_bfloat16*)out, T, N, ldp, ldo, ks);
 }
 }  // namespace owl
 
@@ -455,19 +457,16 @@ static int gd_launch(const void* x, int ldx, const void* w, int ldw, GdParams& p
     }
   }
   const int grid = tiles < sms ? tiles : sms;
-  if (mode == 0) gemm_dense_kernel<false, false, false><<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
-  else if (mode == 1) gemm_dense_kernel<true, false, false><<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
-  else if (mode == 2) gemm_dense_kernel<false, true, false><<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
-  else gemm_dense_kernel<false, false, true><<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
-  OWL_LAUNCH_CHECK();
-  if (p.ksplit > 1 && p.silu) {
-    gemm_ksplit_silu_kernel<<<dim3((p.N + 4095) / 4096, p.T), 256, 0, st>>>(p.partial, p.out, p.T, p.N, p.ldp, p.ldo, p.ksplit);
+  if (mode == 1 || mode == 2) {         // the forms that exchange with other ranks start after the kernel before
+    if (mode == 1) gemm_dense_kernel<true, false, false><<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
+    else gemm_dense_kernel<false, true, false><<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
     OWL_LAUNCH_CHECK();
-  } else if (p.ksplit > 1) {
-    gemm_ksplit_reduce_kernel<<<dim3((p.N + 1023) / 1024, p.T), 256, 0, st>>>(p.partial, p.out, p.T, p.N, p.ldp, p.ldo, p.ksplit);
-    OWL_LAUNCH_CHECK();
+  } else {
+    const int rc = launch_dep(p.T, mode == 0 ? gemm_dense_kernel<false, false, false> : gemm_dense_kernel<false, false, true>, dim3(grid),
+                              dim3(GD_THREADS), GD_SMEM, st, a, b, p);
+    if (rc != OWL_OK) return rc;
   }
-  return OWL_OK;
+  return p.ksplit > 1 ? gd_split_reduce(p.partial, p.out, p.T, p.N, p.ldp, p.ldo, p.ksplit, p.silu, st) : OWL_OK;
 }
 
 // x: [T][ldx], w: [N][ldw], both fp16 (fmt 0) or both bf16 (fmt 1); out bf16 [T][ldo]. K multiple of 64.

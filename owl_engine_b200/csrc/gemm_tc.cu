@@ -96,6 +96,8 @@ __global__ void __launch_bounds__(GT_THREADS, 2) gemm_tc_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_d = sm->tmem_base;
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------- TMA producer ---------------------------------------------
@@ -337,9 +339,7 @@ static int launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const GemmTcP
     attr_done = true;
   }
   dim3 grid((p.N + GT_BN - 1) / GT_BN, (p.T + GT_BM - 1) / GT_BM);
-  kernel<<<grid, GT_THREADS, GT_SMEM, st>>>(a, b, p);
-  OWL_LAUNCH_CHECK();
-  return OWL_OK;
+  return launch_dep(p.T, kernel, grid, dim3(GT_THREADS), GT_SMEM, st, a, b, p);
 }
 
 }  // namespace owl

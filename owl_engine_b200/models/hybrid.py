@@ -1084,11 +1084,12 @@ class HybridRunner:
         else:
             h.copy_(embeds)
         fi = gi = 0
+        pdl = self.pdl and t <= self.PDL_UPTO
         use_state = pos0 > 0
         ahead = self._dequant_ahead(t)
         y = None                    # the last MLP's output, not yet added to h: the next norm adds it on its way
         for i, lw in enumerate(self.w.layers):
-            K.rmsnorm_pack(h, lw.ln1, delta=y, out_h=h if y is not None else None, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps)
+            K.rmsnorm_pack(h, lw.ln1, delta=y, out_h=h if y is not None else None, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps, pdl=pdl)
             if lw.kind == "gdn":
                 nq = sp.conv_dim + sp.value_dim
                 wide = ws["wide"].view(-1)[:t * nq].view(t, nq)
@@ -1116,7 +1117,7 @@ class HybridRunner:
                 fi += 1
             if self.comm is not None and sp.tp_world > 1:
                 self.comm.allreduce_prefill(ws["y"][:t])
-            K.rmsnorm_pack(h, lw.ln2, delta=ws["y"][:t], out_h=h, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps)
+            K.rmsnorm_pack(h, lw.ln2, delta=ws["y"][:t], out_h=h, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps, pdl=pdl)
             if not linear.w4_gemm_silu(lw.gate_up, x, ws["act"][:t], arm=self.prefill_gemm, ahead=ahead):
                 gu = ws["wide"].view(-1)[:t * 2 * sp.inter].view(t, 2 * sp.inter)
                 self._gemm(lw.gate_up, x, gu, ahead)
@@ -1140,6 +1141,7 @@ class HybridRunner:
         self._head(1, sample=True)
         return self.out_tok[:1]
 
+    PDL_UPTO = 288      # tokens per chunk up to which its kernels start while the one before drains (DEP_ROWS of csrc/common.cuh)
     SP_FROM = 256       # tokens per chunk from which the sequence-parallel fused path is used under tensor parallelism
 
     # keys from which a prefill chunk's attention runs as tcgen05 GEMMs (0: never)
@@ -1159,16 +1161,17 @@ class HybridRunner:
             K.attn_gemm_prefill(ws["q"], pool.k_pool[fi], pool.v_pool[fi], pool.scales(fi), self.block_table[seq_row], pos0, t,
                                 sp.hq, sp.hkv, sp.hd, self.scale, aw, wide, self.qkv_n, mix)
             return
+        pdl = self.pdl and t <= self.PDL_UPTO
         if ng:
             K.paged_attn(ws["q"], pool.k_pool[fi], pool.v_pool[fi], self.block_table, ws["bt_row"], ws["ctx"],
                          ws["part_o"], ws["part_ml"], ng, 8, sp.hq, sp.hkv, sp.hd, self.max_blocks, 1, self.scale,
-                         scales=pool.scales(fi))
+                         pdl=pdl, scales=pool.scales(fi))
         if tail:
             off = ng * 8
             K.paged_attn(ws["q"][off:], pool.k_pool[fi], pool.v_pool[fi], self.block_table, ws["bt_row"][ng:],
                          ws["ctx"][ng:], ws["part_o"][off * sp.hq * sp.hd:], ws["part_ml"][off * sp.hq * 2:], 1,
-                         tail, sp.hq, sp.hkv, sp.hd, self.max_blocks, 1, self.scale, scales=pool.scales(fi))
-        K.attn_reduce(ws["part_o"], ws["part_ml"], 1, wide, self.qkv_n, t, sp.hq, out=mix, group=self.G)
+                         tail, sp.hq, sp.hkv, sp.hd, self.max_blocks, 1, self.scale, pdl=pdl, scales=pool.scales(fi))
+        K.attn_reduce(ws["part_o"], ws["part_ml"], 1, wide, self.qkv_n, t, sp.hq, out=mix, group=self.G, pdl=pdl)
 
     def _pipe(self):
         """The prefill pipe of the tensor-parallel communicator (or one set explicitly, e.g. a world of one)."""

@@ -37,6 +37,36 @@ def test_conv_of_long_chunks_equals_short_chunks(t, use_state):
     assert torch.equal(a, b) and torch.equal(h1, h2)
 
 
+@pytest.mark.parametrize("t", [40, 128, 288, 289])
+def test_prompt_kernels_that_start_early_wait_for_the_rows_before(t):
+    """Up to 288 rows a kernel starts while the one before drains. Three layers back to back, which read and overwrite the same
+    buffers, against the same launches with a synchronisation after each: the same bits."""
+    nk, nv, slot = 2, 6, 1
+    gen = torch.Generator(device=DEV).manual_seed(t)
+    cd, vd = (2 * nk + nv) * 128, nv * 128
+    wide = torch.randn(t, cd + vd, device=DEV, generator=gen).bfloat16()
+    cw = torch.randn(cd, 4, device=DEV, generator=gen)
+    ab = torch.randn(t, 2 * nv, device=DEV, generator=gen).bfloat16()
+    a_log, dt, gamma = (torch.randn(n, device=DEV, generator=gen) for n in (nv, nv, 128))
+    w = (torch.randn(cd + vd, vd, device=DEV, generator=gen) * vd ** -0.5).half()
+    runs = []
+    for sync in (True, False):
+        hist, st = torch.zeros(2, cd, 3, device=DEV), torch.zeros(2, nv, 128, 128, device=DEV)
+        conv, mix = torch.zeros(t, cd, dtype=torch.bfloat16, device=DEV), torch.zeros(t, vd, dtype=torch.float16, device=DEV)
+        cur = wide.clone()
+        torch.cuda.synchronize()
+        for _ in range(3):
+            for step in (lambda: K.gdn_conv_fwd(cur, cd + vd, cw, hist, slot, conv, t, nk, nv, True),
+                         lambda: K.gdn_scan(conv, cur[:, cd:], cd + vd, ab, 2 * nv, a_log, dt, gamma, st, slot, mix, t, nk, nv, True),
+                         lambda: gemm_tc.f16_gemm(mix, w, cur)):
+                step()
+                if sync:
+                    torch.cuda.synchronize()
+        runs.append((cur, hist, st, mix))
+    assert torch.isfinite(runs[0][0].float()).all()
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
 @pytest.mark.parametrize("pool", ["fp8", "int8", "f16"])
 @pytest.mark.parametrize("rows,hq,hkv,rot", [(128, 24, 4, 64), (131, 6, 2, 256), (200, 2, 1, 16)])
 def test_qknorm_rope_of_many_rows_equals_few_rows(pool, rows, hq, hkv, rot):
