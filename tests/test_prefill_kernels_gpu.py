@@ -67,6 +67,34 @@ def test_prompt_kernels_that_start_early_wait_for_the_rows_before(t):
     assert all(torch.equal(a, b) for a, b in zip(*runs))
 
 
+@pytest.mark.parametrize("fmt", [0, 1, 2])
+@pytest.mark.parametrize("ctx,pad,hkv", [(1, 64, 1), (63, 64, 2), (64, 128, 4), (65, 128, 1), (200, 320, 3)])
+def test_gathered_keys_and_values(fmt, ctx, pad, hkv):
+    """Tiles of 64 keys: whole, ragged and empty ones; every e4m3 and int8 value is exact in both outputs but for the scale's rounding."""
+    gen = torch.Generator(device=DEV).manual_seed(ctx + fmt)
+    pages = (ctx + 15) // 16
+    bt = torch.randperm(pages + 3, device=DEV, generator=gen)[:pages].int()
+    shape = (pages + 3, 16, hkv, 256)
+    raw = [torch.randint(0, 256, shape, device=DEV, generator=gen, dtype=torch.uint8) for _ in range(2)]
+    sc = [torch.rand(shape[:3], device=DEV, generator=gen) + 0.01 for _ in range(2)]
+    if fmt == 0:
+        pools = [r.masked_fill((r & 0x7f) == 0x7f, 0x7e) for r in raw]
+        vals = [p.view(torch.float8_e4m3fn).float() for p in pools]
+    elif fmt == 1:
+        pools = raw
+        vals = [p.view(torch.int8).float() * s[..., None] for p, s in zip(pools, sc)]
+    else:
+        pools = [torch.randn(shape, device=DEV, generator=gen).half() for _ in range(2)]
+        vals = [p.float() for p in pools]
+    k = torch.full((hkv, pad, 256), float("nan"), dtype=torch.bfloat16, device=DEV)
+    vt = torch.full((hkv, 256, pad), float("nan"), dtype=torch.float16, device=DEV)
+    K.call("owl_kv_gather", K.ptr(pools[0]), K.ptr(pools[1]), K.ptr(sc[0]), K.ptr(sc[1]), fmt, K.ptr(bt), ctx, pad, hkv, 256,
+           K.ptr(k), K.ptr(vt), K.stream())
+    flat = [v[bt.long()].reshape(-1, hkv, 256)[:ctx] for v in vals]
+    assert torch.equal(k[:, :ctx], flat[0].bfloat16().permute(1, 0, 2)) and torch.equal(vt[..., :ctx], flat[1].half().permute(1, 2, 0))
+    assert not k[:, ctx:].any() and not vt[..., ctx:].any()
+
+
 @pytest.mark.parametrize("pool", ["fp8", "int8", "f16"])
 @pytest.mark.parametrize("rows,hq,hkv,rot", [(128, 24, 4, 64), (131, 6, 2, 256), (200, 2, 1, 16)])
 def test_qknorm_rope_of_many_rows_equals_few_rows(pool, rows, hq, hkv, rot):
