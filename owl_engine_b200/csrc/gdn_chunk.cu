@@ -10,7 +10,7 @@
 //   gdn_chunk_prep_kernel  one CTA per (chunk, v-head), all chunks in parallel: the 64x64 products and the two 64x128
 //                          products on mma.sync (bf16 in, fp32 accumulate), the triangular inverse by forward substitution
 //                          with four threads per column; writes w, u, scaled q, scaled k and attn
-//   gdn_chunk_scan_kernel  one CTA per (v-head, half of the value columns), the chunks in order: three small tensor-core
+//   gdn_chunk_scan_kernel  one CTA per (v-head, part of the value columns), the chunks in order: three small tensor-core
 //                          products per chunk against the fp32 state kept in MMA accumulator registers (a bf16 copy in
 //                          shared memory is the B operand), operands prefetched one chunk ahead with cp.async
 // Every tile stays in the row order it has in global memory; the products that need it the other way round read it with
@@ -31,7 +31,7 @@ constexpr int CK_C = 64;            // chunk length
 constexpr int CK_D = 128;           // head dim (k and v)
 constexpr int CK_LD = CK_D + 8;     // row stride of [64][128] bf16 tiles (68 words: conflict-free fragment loads)
 constexpr int CK_LT = CK_C + 8;     // row stride of [*][64] bf16 tiles
-constexpr int CK_NC = 64;           // value columns per CTA of the recurrence kernel
+constexpr int CK_NC = 64;           // most value columns per CTA of the recurrence kernel
 
 __device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -275,7 +275,13 @@ __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkParams p
   }
 }
 
-// ---- the recurrence over chunks: one CTA per (v-head, 64 value columns), 256 threads ----------------------------------
+// ---- the recurrence over chunks: one CTA per (v-head, part of the value columns), 256 threads ----------------------------
+// Bound by the chain of chunks, of which each takes 1.7 us with next to no products in it. The only split is by columns: into as many
+// parts (2, 3, 4 or 8, of whole 8-column tiles) as leave every CTA an SM of its own; a part reads the other operands again, from L2.
+// us a layer at 2048 tokens, two parts / the rule's: 48 heads 92 / 82 (three), 32 heads 90 / 64 (four), 16 heads 90 / 53 (eight); the 0.8B
+// model's prompt of 2048 tokens 6.9 / 6.2 ms. The
+// number of tiles is a template argument: as a variable it cost two parts 25 us. What lost: warps 8 to 15 for the outputs, so
+// that 0 to 7 walk the chain alone (99 against 92 us): the state's fragments are then read twice.
 struct ScanBuf {
   __nv_bfloat16 w[CK_C][CK_LD];
   __nv_bfloat16 qg[CK_C][CK_LD];
@@ -288,18 +294,19 @@ struct ScanSmem {
   __nv_bfloat16 s[CK_D][CK_LT];     // the state as bf16: [k][value column]
   __nv_bfloat16 vn[CK_C][CK_LT];    // v': [token][value column]
 };
-__global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
-  pdl_launch_dependents();
-  pdl_wait();
+// Column tiles tile0 .. tile0 + NT - 1 (8 columns each) of one head.
+template <int NT>
+__device__ __forceinline__ void gdn_scan_part(const GdnChunkParams& p, int tile0) {
+  constexpr int H1 = (NT + 1) / 2;                  // tiles of warps 0 to 3; warps 4 to 7 have one less of an odd number
   extern __shared__ __align__(16) uint8_t ck_smem[];
   ScanSmem& sm = *reinterpret_cast<ScanSmem*>(ck_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
-  const int h = blockIdx.x, cb = blockIdx.y * CK_NC, V = p.nv * CK_D;
-  // state rows 16 warp .. +15, all 64 columns: 8 n-tiles of accumulator registers
-  float S[8][4];
+  const int h = blockIdx.x, V = p.nv * CK_D, cb = tile0 * 8;
+  // state rows 16 warp .. +15, all columns of the part
+  float S[NT][4];
   float* sp = p.state + ((size_t)p.slot * p.nv + h) * CK_D * CK_D;
 #pragma unroll
-  for (int n = 0; n < 8; ++n)
+  for (int n = 0; n < NT; ++n)
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int k = warp * 16 + g + half * 8, col = cb + n * 8 + 2 * t4;
@@ -317,7 +324,7 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
         ck_cp16(&b.w[t][piece], p.w + o);
         ck_cp16(&b.qg[t][piece], p.qg + o);
         ck_cp16(&b.kd[t][piece], p.kd + (((size_t)h * p.chunks + c) * CK_C + t) * CK_D + piece);
-        ck_cp16(&b.u[t][piece / 2], p.u + ((size_t)(r0 + t) * p.nv + h) * CK_D + cb + piece / 2);
+        if (NT == 8 || piece < NT * 16) ck_cp16(&b.u[t][piece / 2], p.u + ((size_t)(r0 + t) * p.nv + h) * CK_D + cb + piece / 2);
       }
       for (int i = tid; i < CK_C * 8; i += 256) {
         const int t = i >> 3, piece = (i & 7) * 8;
@@ -333,18 +340,19 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
     const float eg = p.eglast[(size_t)h * p.chunks + c];
     // the state as the B operand of this chunk (the last reads of s are two barriers back)
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int half = 0; half < 2; ++half)
         *reinterpret_cast<uint32_t*>(&sm.s[warp * 16 + g + half * 8][n * 8 + 2 * t4]) = pack_bf16(S[n][half * 2], S[n][half * 2 + 1]);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                 // chunk c and the state copy are visible; everyone is done with chunk c - 1
     issue(c + 1);
-    // v' = u - w S and o = qg S: warp -> rows 16 (warp & 3), columns 32 (warp >> 2); K = 128
-    const int m0 = (warp & 3) * 16, nh = (warp >> 2) * 32;
-    float pv[4][4], ov[4][4];
+    // v' = u - w S and o = qg S: warp -> rows 16 (warp & 3), the first or second half of the column tiles (mine, from nh); K = 128
+    const int m0 = (warp & 3) * 16, nh = (warp >> 2) * H1 * 8;
+    const bool last = NT % 2 == 0 || warp < 4;       // this warp has a tile H1 - 1
+    float pv[H1][4], ov[H1][4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < H1; ++n)
 #pragma unroll
       for (int i = 0; i < 4; ++i) pv[n][i] = ov[n][i] = 0.f;
 #pragma unroll
@@ -353,27 +361,30 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
       frag_a(aw, &b.w[0][0], CK_LD, m0, ks * 16, lane);
       frag_a(aq, &b.qg[0][0], CK_LD, m0, ks * 16, lane);
 #pragma unroll
-      for (int n = 0; n < 4; n += 2) {
+      for (int n = 0; n < H1; n += 2) {
+        if (n == H1 - 1 && !last) continue;
         uint32_t bs[4];
         frag_bt(bs, &sm.s[0][0], CK_LT, nh + n * 8, ks * 16, lane);
         mma_bf16(pv[n], aw[0], aw[1], aw[2], aw[3], bs[0], bs[1]);
         mma_bf16(ov[n], aq[0], aq[1], aq[2], aq[3], bs[0], bs[1]);
+        if (n + 1 == H1 || (n + 1 == H1 - 1 && !last)) continue;
         mma_bf16(pv[n + 1], aw[0], aw[1], aw[2], aw[3], bs[2], bs[3]);
         mma_bf16(ov[n + 1], aq[0], aq[1], aq[2], aq[3], bs[2], bs[3]);
       }
     }
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < H1; ++n)
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
+        if (n == H1 - 1 && !last) continue;
         const int i = m0 + g + half * 8, col = nh + n * 8 + 2 * t4;
         const float2 uw = *reinterpret_cast<const float2*>(&b.u[i][col]);
         *reinterpret_cast<uint32_t*>(&sm.vn[i][col]) = pack_bf16(uw.x - pv[n][half * 2], uw.y - pv[n][half * 2 + 1]);
       }
     __syncthreads();
-    // S <- e^{gc_last} S + (e^{gc_last - gc} k)^T v': warp -> state rows 16 warp .. +15, all 64 columns
+    // S <- e^{gc_last} S + (e^{gc_last - gc} k)^T v': warp -> state rows 16 warp .. +15, all columns
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int i = 0; i < 4; ++i) S[n][i] *= eg;
     // and o += attn v'  (K = 64 tokens)
@@ -383,38 +394,49 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
       frag_at(ak, &b.kd[0][0], CK_LD, warp * 16, ks * 16, lane);
       frag_a(a, &b.attn[0][0], CK_LT, m0, ks * 16, lane);
 #pragma unroll
-      for (int n = 0; n < 8; n += 2) {
+      for (int n = 0; n < NT; n += 2) {
         uint32_t bv[4];
         frag_bt(bv, &sm.vn[0][0], CK_LT, n * 8, ks * 16, lane);
         mma_bf16(S[n], ak[0], ak[1], ak[2], ak[3], bv[0], bv[1]);
+        if (n + 1 == NT) continue;
         mma_bf16(S[n + 1], ak[0], ak[1], ak[2], ak[3], bv[2], bv[3]);
       }
 #pragma unroll
-      for (int n = 0; n < 4; n += 2) {
+      for (int n = 0; n < H1; n += 2) {
+        if (n == H1 - 1 && !last) continue;
         uint32_t bv[4];
         frag_bt(bv, &sm.vn[0][0], CK_LT, nh + n * 8, ks * 16, lane);
         mma_bf16(ov[n], a[0], a[1], a[2], a[3], bv[0], bv[1]);
+        if (n + 1 == H1 || (n + 1 == H1 - 1 && !last)) continue;
         mma_bf16(ov[n + 1], a[0], a[1], a[2], a[3], bv[2], bv[3]);
       }
     }
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < H1; ++n)
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int r = r0 + m0 + g + half * 8;
-        if (r < p.T)
+        if (r < p.T && (n < H1 - 1 || last))
           *reinterpret_cast<float2*>(p.raw + (size_t)r * V + h * CK_D + cb + nh + n * 8 + 2 * t4) =
               make_float2(ov[n][half * 2], ov[n][half * 2 + 1]);
       }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
-  for (int n = 0; n < 8; ++n)
+  for (int n = 0; n < NT; ++n)
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int k = warp * 16 + g + half * 8, col = cb + n * 8 + 2 * t4;
       *reinterpret_cast<float2*>(sp + (size_t)k * CK_D + col) = make_float2(S[n][half * 2], S[n][half * 2 + 1]);
     }
+}
+template <int PARTS>
+__global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(GdnChunkParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tile0 = (int)blockIdx.y * 16 / PARTS;
+  if (PARTS == 3 && blockIdx.y == 2) gdn_scan_part<6>(p, tile0);
+  else gdn_scan_part<16 / PARTS>(p, tile0);
 }
 
 }  // namespace owl
@@ -439,10 +461,16 @@ OWL_API int owl_gdn_chunk_scan(const void* qkv, const void* ab, int ldab, const 
   if (T < 1 || nk < 1 || nv % nk || !raw || !work || work_bytes < ck_work_bytes(T, nv) ||
       (reinterpret_cast<uintptr_t>(work) & 255))
     return OWL_ERR_BAD_ARG;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+  const int fit = sms / nv, parts = fit >= 8 ? 8 : fit >= 4 ? 4 : fit == 3 ? 3 : 2;
+  auto scan = parts == 8 ? gdn_chunk_scan_kernel<8> : parts == 4 ? gdn_chunk_scan_kernel<4> : parts == 3 ? gdn_chunk_scan_kernel<3> : gdn_chunk_scan_kernel<2>;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(gdn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PrepSmem)) != cudaSuccess ||
-        cudaFuncSetAttribute(gdn_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ScanSmem)) != cudaSuccess)
+    for (auto k : {gdn_chunk_scan_kernel<8>, gdn_chunk_scan_kernel<4>, gdn_chunk_scan_kernel<3>, gdn_chunk_scan_kernel<2>})
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ScanSmem)) != cudaSuccess)
+        return OWL_ERR_LAUNCH * 1000;
+    if (cudaFuncSetAttribute(gdn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PrepSmem)) != cudaSuccess)
       return OWL_ERR_LAUNCH * 1000;
     attr = true;
   }
@@ -459,5 +487,5 @@ OWL_API int owl_gdn_chunk_scan(const void* qkv, const void* ab, int ldab, const 
   p.eglast = reinterpret_cast<float*>(p.attn + (size_t)nv * p.chunks * CK_C * CK_C);
   const int rc = launch_dep(T, gdn_chunk_prep_kernel, dim3(p.chunks, nv), dim3(256), sizeof(PrepSmem), st, p);
   if (rc != OWL_OK) return rc;
-  return launch_dep(T, gdn_chunk_scan_kernel, dim3(nv, CK_D / CK_NC), dim3(256), sizeof(ScanSmem), st, p);
+  return launch_dep(T, scan, dim3(nv, parts), dim3(256), sizeof(ScanSmem), st, p);
 }

@@ -67,6 +67,35 @@ def test_prompt_kernels_that_start_early_wait_for_the_rows_before(t):
     assert all(torch.equal(a, b) for a, b in zip(*runs))
 
 
+@pytest.mark.parametrize("nv", [18, 36, 48, 75])
+def test_chunked_scan_splits_its_columns(nv):
+    """8, 4, 3 (of 5, 5 and 6 column tiles) and 2 parts: the sums of a column do not depend on the part it lies in, so three heads alone
+    (8 parts) give the same bits. A ragged last chunk."""
+    t, slot = 130, 1
+    gen = torch.Generator(device=DEV).manual_seed(nv)
+    nk = nv // 3
+    q, k, v = (torch.randn(t, n, 128, device=DEV, generator=gen) for n in (nk, nk, nv))
+    q, k = (x / x.norm(dim=2, keepdim=True) for x in (q, k))
+    z, a, b = (torch.randn(t, n, device=DEV, generator=gen).bfloat16() for n in (nv * 128, nv, nv))
+    a_log, dt, gamma = (torch.randn(n, device=DEV, generator=gen) for n in (nv, nv, 128))
+    s0 = torch.randn(2, nv, 128, 128, device=DEV, generator=gen)
+
+    def run(h0, n):
+        kh = slice(h0 // 3, (h0 + n) // 3)
+        qkv = torch.cat([x.reshape(t, -1) for x in (q[:, kh], k[:, kh], v[:, h0:h0 + n])], 1).bfloat16()
+        st, out = s0[:, h0:h0 + n].clone(memory_format=torch.contiguous_format), torch.zeros(t, n * 128, dtype=torch.float16, device=DEV)
+        ab = torch.cat([a[:, h0:h0 + n], b[:, h0:h0 + n]], 1).contiguous()
+        K.gdn_scan(qkv, z[:, h0 * 128:(h0 + n) * 128].contiguous(), n * 128, ab, 2 * n, a_log[h0:h0 + n].contiguous(),
+                   dt[h0:h0 + n].contiguous(), gamma, st, slot, out, t, n // 3, n, True, split="chunked")
+        return out, st
+
+    out, st = run(0, nv)
+    for h0 in (0, nv - 3):
+        o3, s3 = run(h0, 3)
+        assert torch.isfinite(o3.float()).all()
+        assert torch.equal(out[:, h0 * 128:(h0 + 3) * 128], o3) and torch.equal(st[:, h0:h0 + 3], s3)
+
+
 @pytest.mark.parametrize("fmt", [0, 1, 2])
 @pytest.mark.parametrize("ctx,pad,hkv", [(1, 64, 1), (63, 64, 2), (64, 128, 4), (65, 128, 1), (200, 320, 3)])
 def test_gathered_keys_and_values(fmt, ctx, pad, hkv):
