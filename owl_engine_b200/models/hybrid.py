@@ -1052,7 +1052,7 @@ class HybridRunner:
         pos0..pos0+T-1 must already be in ``block_table[seq_row]``. Returns the argmax token of
         the last row when ``want_logits``. ``snap = (rows, state_row)``: also leave the GDN state after the first
         ``rows`` rows of the chunk in ``state_row`` (0 < rows < T)."""
-        from ..ops import gemm_tc, linear
+        from ..ops import linear
 
         sp, pool = self.spec, self.pool
         t = ids.shape[0]
@@ -1095,10 +1095,11 @@ class HybridRunner:
                 wide = ws["wide"].view(-1)[:t * nq].view(t, nq)
                 self._gemm(lw.qkvz, x, wide, ahead)
                 ab = ws["ab"][:t]
-                # short prompts cut k (137 rows: 35 us on two CTAs); long ones and the 8-bit arms keep one sum, whose rounding the
-                # activations' 8-bit steps would spread
+                # one CTA per 128 rows walks all of k: cut where that takes longer than a second launch that adds the parts (96 rows of
+                # k 5120, 512 / 2048 tokens: 27.4 / 28.0 us whole, 14.1 / 16.4 cut; 32 of k 1024: 7.8 / 8.0 and 11.3 / 14.9). The 8-bit
+                # arms keep one sum, whose rounding the activations' 8-bit steps would spread
                 linear.dense_gemm(x, lw.ab_dense, ab, arm="baseline" if self.prefill_gemm == "baseline" else "tc",
-                                  split=t <= gemm_tc.ROWS_UPTO and self.prefill_gemm in ("tc", "tc4", "tcr"))
+                                  split=sp.hidden >= 3072 and self.prefill_gemm in ("tc", "tc4", "tcr"))
                 mix = ws["mix"].view(-1)[:t * sp.value_dim].view(t, sp.value_dim)
                 self._gdn_prefill(lw, gi, wide, nq, ab, ws["conv"][:t], mix, t, gdn_slot, use_state, snap)
                 self._gemm(lw.out_proj, mix, ws["y"][:t], ahead)

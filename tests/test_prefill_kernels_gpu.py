@@ -67,6 +67,20 @@ def test_prompt_kernels_that_start_early_wait_for_the_rows_before(t):
     assert all(torch.equal(a, b) for a, b in zip(*runs))
 
 
+@pytest.mark.parametrize("t", [1, 128, 257, 2048, 9473])
+def test_narrow_product_cut_along_k(t):
+    """96 rows of k 5120 (the a / b projection of long prompts): from one row tile to more than half as many as there are SMs (not cut)."""
+    n, k = 96, 5120
+    gen = torch.Generator(device=DEV).manual_seed(t)
+    x = torch.randn(t, k, device=DEV, generator=gen).half()
+    w = (torch.randn(n, k, device=DEV, generator=gen) * 0.05).half()
+    out = torch.zeros(t, n, dtype=torch.bfloat16, device=DEV)
+    gemm_tc.f16_gemm(x, w, out, force_persist=True)
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    # one rounding to bf16 and fp32 sums (of at most 16 parts) of k / 16 MMA steps
+    assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + size * (k / 16 + 16) * 2.0 ** -24).all()
+
+
 @pytest.mark.parametrize("nv", [18, 36, 48, 75])
 def test_chunked_scan_splits_its_columns(nv):
     """8, 4, 3 (of 5, 5 and 6 column tiles) and 2 parts: the sums of a column do not depend on the part it lies in, so three heads alone
