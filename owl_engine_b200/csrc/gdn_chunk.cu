@@ -278,10 +278,9 @@ __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkParams p
 // ---- the recurrence over chunks: one CTA per (v-head, part of the value columns), 256 threads ----------------------------
 // Bound by the chain of chunks, of which each takes 1.7 us with next to no products in it. The only split is by columns: into as many
 // parts (2, 3, 4 or 8, of whole 8-column tiles) as leave every CTA an SM of its own; a part reads the other operands again, from L2.
-// us a layer at 2048 tokens, two parts / the rule's: 48 heads 92 / 82 (three), 32 heads 90 / 64 (four), 16 heads 90 / 53 (eight); the 0.8B
-// model's prompt of 2048 tokens 6.9 / 6.2 ms. The
-// number of tiles is a template argument: as a variable it cost two parts 25 us. What lost: warps 8 to 15 for the outputs, so
-// that 0 to 7 walk the chain alone (99 against 92 us): the state's fragments are then read twice.
+// us a layer at 2048 tokens, two parts / the rule's: 48 heads 92 / 82 (three), 32 heads 90 / 64 (four), 16 heads 90 / 53 (eight; the 0.8B
+// model's prompt of 2048 tokens 6.9 / 6.2 ms). The number of tiles is a template argument: as a variable it cost two parts 25 us. What
+// lost: warps 8 to 15 for the outputs, so that 0 to 7 walk the chain alone (99 against 92 us): the state's fragments are read twice.
 struct ScanBuf {
   __nv_bfloat16 w[CK_C][CK_LD];
   __nv_bfloat16 qg[CK_C][CK_LD];
