@@ -40,7 +40,7 @@ constexpr int GD_BM = 128, GD_BN = 256, GD_BK = 64, GD_STAGES = 4;
 constexpr int GD_A_BYTES = GD_BM * GD_BK * 2, GD_B_BYTES = GD_BN * GD_BK * 2;
 constexpr int GD_STAGE_BYTES = GD_A_BYTES + GD_B_BYTES;          // 48 KB
 constexpr int GD_THREADS = 192;
-constexpr int GD_SMEM = GD_STAGES * GD_STAGE_BYTES + 1024 + 256;
+constexpr int GD_CTL_BYTES = 256, GD_SMEM = GD_STAGES * GD_STAGE_BYTES + 1024 + GD_CTL_BYTES;
 
 struct GdParams {
   __nv_bfloat16* out;
@@ -66,6 +66,7 @@ struct GdCtl {
   uint32_t tmem_base;
   volatile int abort_flag;
 };
+static_assert(sizeof(GdCtl) <= GD_CTL_BYTES, "control block exceeds its reservation");
 
 __device__ __forceinline__ bool gd_wait(uint64_t* bar, uint32_t parity, GdCtl* c, int code) {
   const uint64_t t0 = global_ns();

@@ -35,7 +35,7 @@ constexpr int NF_BM = 128, NF_BN = 128, NF_BKB = 128, NF_STAGES = 5;      // NF_
 constexpr int NF_A_BYTES = NF_BM * NF_BKB, NF_B_BYTES = NF_BN * NF_BKB, NF_SF_BYTES = 2048;
 constexpr int NF_STAGE_BYTES = NF_A_BYTES + NF_B_BYTES + 2 * NF_SF_BYTES;    // 36 KB
 constexpr int NF_THREADS = 192;
-constexpr int NF_SMEM = NF_STAGES * NF_STAGE_BYTES + 1024 + 256;
+constexpr int NF_CTL_BYTES = 256, NF_SMEM = NF_STAGES * NF_STAGE_BYTES + 1024 + NF_CTL_BYTES;
 constexpr uint32_t NF_SFA_COL = 256, NF_SFB_COL = 272;                        // TMEM columns of the scale atoms
 
 struct NfParams {
@@ -52,6 +52,7 @@ struct NfCtl {
   uint32_t tmem_base;
   volatile int abort_flag;
 };
+static_assert(sizeof(NfCtl) <= NF_CTL_BYTES, "control block exceeds its reservation");
 
 __device__ __forceinline__ bool nf_wait(uint64_t* bar, uint32_t parity, NfCtl* c, int code) {
   const uint64_t t0 = global_ns();

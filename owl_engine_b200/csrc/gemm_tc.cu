@@ -32,7 +32,8 @@ __device__ int g_gemm_status = 0;
 constexpr int GT_BM = 128, GT_BN = 128, GT_BK = 64, GT_STAGES = 3;
 constexpr int GT_TILE_BYTES = GT_BM * GT_BK * 2;   // 16 KB per operand per stage
 constexpr int GT_THREADS = 192;
-constexpr int GT_SMEM = GT_STAGES * 2 * GT_TILE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+constexpr int GT_CTL_BYTES = 256;
+constexpr int GT_SMEM = GT_STAGES * 2 * GT_TILE_BYTES + 1024 /*align slack*/ + GT_CTL_BYTES;
 
 struct GemmTcParams {
   const uint8_t* wrec;   // W4 records or nullptr for the dense path
@@ -48,6 +49,7 @@ struct GemmSmem {
   uint32_t tmem_base;
   volatile int abort_flag;
 };
+static_assert(sizeof(GemmSmem) <= GT_CTL_BYTES, "control block exceeds its reservation");
 
 // Bounded wait that also leaves when another role aborted.
 __device__ __forceinline__ bool gt_wait(uint64_t* bar, uint32_t parity, GemmSmem* sm, int code) {

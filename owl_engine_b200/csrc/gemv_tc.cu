@@ -63,6 +63,7 @@ constexpr int VT_ACC0 = 256;
 
 enum { VEPI_STORE = 0, VEPI_RESIDUAL = 1, VEPI_SILU_MUL = 2, VEPI_F32 = 3 };
 
+constexpr int VT_CTL_BYTES = 512;
 template <int G> struct VtCfg {
   static constexpr int GPT = 128 / G;                       // scale groups per record
   static constexpr int REC = 1024 + 64 * GPT;
@@ -73,7 +74,7 @@ template <int G> struct VtCfg {
   static constexpr int STAGES = 16;                         // multiple of VT_NG: a stage always serves the same group
   static constexpr int OFF_RED = STAGES * STAGE;
   static constexpr int OFF_CTL = OFF_RED + (VT_NG - 1) * 128 * 8 * 4;
-  static constexpr int SMEM = OFF_CTL + 512 + 128 /*alignment slack*/;
+  static constexpr int SMEM = OFF_CTL + VT_CTL_BYTES + 128 /*alignment slack*/;
 };
 
 struct VtCtl {
@@ -82,6 +83,7 @@ struct VtCtl {
   uint32_t tmem_base;
   volatile int abort_flag;
 };
+static_assert(sizeof(VtCtl) <= VT_CTL_BYTES, "control block exceeds its reservation");
 
 struct VtParams {
   const uint8_t* w;       // block-major record stream

@@ -63,9 +63,21 @@ template <int F> __host__ __device__ constexpr int tm_slots() { return F == TF_G
 // Steps whose weight scales are kept: a set that writes those of step `it` has seen the MMAs of step it - TM_AS done, which had waited for
 // the readers of step it - TM_AS - slots.
 template <int F> __host__ __device__ constexpr int tm_info() { return 8; }
-template <int F> constexpr int tm_smem() {
-  return TM_XPOOL + TM_XPOOL / 2048 * tm_gpr<F>() * 64 + tm_info<F>() * tm_gpr<F>() * 512 + TM_DEQ * tm_raw<F>() * 2 * tm_rec<F>() + TM_IN + 1024 + 256;
+struct TmCtl {
+  // full_a / full_x: a step's weights (an arrival per warp of the set) and activations are here; done: its sums are there (the MMAs'
+  // commit, and an arrival that passes on what full_a and full_x showed); acc_free / empty_x: the readers have the sums, and are
+  // through with the step's activations
+  uint64_t full_a[TM_AS], done[TM_AS], full_x[TM_XMAX], empty_x[TM_XMAX], acc_free[4];
+  uint32_t tmem_base;
+  volatile int abort_flag;
+};
+// Activations, their sums, weight scales, weights, partial sums; the control block lies behind them.
+template <int F> __host__ __device__ constexpr int tm_ctl_off() {
+  return TM_XPOOL + TM_XPOOL / 2048 * tm_gpr<F>() * 64 + tm_info<F>() * tm_gpr<F>() * 512 + TM_DEQ * tm_raw<F>() * 2 * tm_rec<F>() + TM_IN;
 }
+static_assert(tm_ctl_off<TF_G128>() % 8 == 0 && tm_ctl_off<TF_G32>() % 8 == 0 && tm_ctl_off<TF_NV4>() % 8 == 0, "mbarriers");
+// 1024 bytes let the base be rounded up to the swizzle's boundary, from wherever dynamic shared memory begins.
+template <int F> constexpr int tm_smem() { return tm_ctl_off<F>() + (int)sizeof(TmCtl) + 1024; }
 
 struct TmParams {
   const uint8_t* w;               // int4: record stream; NVFP4: codes [N][K/2]
@@ -81,15 +93,6 @@ struct TmParams {
   float out_scale;
   int M, N, K, ldo, n_tiles, row_blocks, ab_rows, ab_ld, ab_blocks, epi;
 };
-struct TmCtl {
-  // full_a / full_x: a step's weights (an arrival per warp of the set) and activations are here; done: its sums are there (the MMAs'
-  // commit, and an arrival that passes on what full_a and full_x showed); acc_free / empty_x: the readers have the sums, and are
-  // through with the step's activations
-  uint64_t full_a[TM_AS], done[TM_AS], full_x[TM_XMAX], empty_x[TM_XMAX], acc_free[4];
-  uint32_t tmem_base;
-  volatile int abort_flag;
-};
-
 __device__ __forceinline__ bool tm_wait(uint64_t* bar, uint32_t parity, TmCtl* c, int code) {
   if (mbar_try_wait(bar, parity)) return true;      // the clock is read only when there is something to wait for
   const uint64_t t0 = global_ns();
@@ -223,7 +226,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) w4_tm_kernel(TmParams p, int KS
   uint8_t* side_all = raw_all + TM_DEQ * RAW * 2 * REC;                // (scale, zero) [step % INFO][group][128 rows]
   uint8_t* sums_all = side_all + INFO * GPR * 512;                  // [stage][block of 8 tokens][group][8 scales, 8 sums]
   float* in = reinterpret_cast<float*>(sums_all + TM_XPOOL / 2048 * GPR * 64);
-  TmCtl* ctl = reinterpret_cast<TmCtl*>(reinterpret_cast<uint8_t*>(in) + TM_IN);
+  TmCtl* ctl = reinterpret_cast<TmCtl*>(base + tm_ctl_off<F>());
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int KT = p.K >> 7;
   const int rank = blockIdx.x % KS, cl = blockIdx.x / KS, n_cl = gridDim.x / KS - p.ab_blocks;

@@ -88,6 +88,24 @@ def test_testkit():
     assert not rep.ok and rep.worst_index == (1,) and "MISMATCH" in str(rep)
 
 
+def test_control_blocks_in_shared_memory_fit_their_reservation():
+    """A kernel's barriers and flags (the struct with its abort flag) lie behind its tiles in dynamic shared memory: the launch asks for
+    the struct's own size, or the build checks it against the bytes reserved."""
+    import re
+
+    from owl_engine_b200.ops import registry as R
+
+    seen = []
+    for f in sorted(R.CSRC.glob("*.cu")):
+        text = f.read_text()
+        for name in re.findall(r"struct (\w+) \{[^}]*\babort_flag;[^}]*\};", text):
+            seen.append(name)
+            asked = re.search(r"_smem\(\) \{ return [^;]*sizeof\(%s\)" % name, text)
+            checked = re.search(r"static_assert\(sizeof\(%s\) <= " % name, text)
+            assert asked or checked, f"{f.name}: nothing bounds {name}"
+    assert len(seen) >= 7
+
+
 def test_kernel_registry_matches_sources_and_bindings():
     from owl_engine_b200.ops import registry as R
 
