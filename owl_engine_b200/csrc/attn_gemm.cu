@@ -255,12 +255,9 @@ OWL_API int owl_causal_softmax(void* s, int rows, int ld, int ncols, int pos0, f
   if (rows < 1 || ncols < 1 || ld < ncols || pos0 < 0 || rows_per_tok < 1 || !inv_sum) return OWL_ERR_BAD_ARG;
   const size_t smem = (size_t)ncols * 2;
   if (!(ld & 7) && !(ncols & 7) && !(reinterpret_cast<uintptr_t>(s) & 15) && smem <= 200 * 1024) {
-    static bool attr_done = false;
-    if (!attr_done) {
-      if (cudaFuncSetAttribute(causal_softmax_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
-        return OWL_ERR_LAUNCH * 1000;
-      attr_done = true;
-    }
+    static SmemLimit limit;
+    const int lrc = limit.raise(causal_softmax_smem_kernel, 200 * 1024);
+    if (lrc != OWL_OK) return lrc;
     causal_softmax_smem_kernel<<<rows, 512, smem, st>>>((__half*)s, ld, ncols, pos0, scale * 1.4426950408889634f, rows_per_tok,
                                                         (float*)inv_sum);
   } else {

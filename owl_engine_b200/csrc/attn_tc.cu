@@ -408,12 +408,9 @@ OWL_API int owl_attn_tc(const void* qg, const void* k, const void* vt, void* og,
   if (r) return r;
   r = at_map(&mv, vt, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, ctx_pad, AT_HD, hkv, AT_HD);
   if (r) return r;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) != cudaSuccess)
-      return OWL_ERR_LAUNCH * 1000;
-    attr = true;
-  }
+  static SmemLimit limit;
+  const int lrc = limit.raise(attn_tc_kernel, AT_SMEM);
+  if (lrc != OWL_OK) return lrc;
   AtParams p = {};
   p.out = (__nv_bfloat16*)og; p.rows = rows; p.gq = gq; p.pos0 = pos0; p.hkv = hkv;
   p.row_tiles = (rows + AT_BM - 1) / AT_BM;

@@ -460,19 +460,12 @@ OWL_API int owl_gdn_chunk_scan(const void* qkv, const void* ab, int ldab, const 
   if (T < 1 || nk < 1 || nv % nk || !raw || !work || work_bytes < ck_work_bytes(T, nv) ||
       (reinterpret_cast<uintptr_t>(work) & 255))
     return OWL_ERR_BAD_ARG;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-  const int fit = sms / nv, parts = fit >= 8 ? 8 : fit >= 4 ? 4 : fit == 3 ? 3 : 2;
+  const int fit = sm_count() / nv, parts = fit >= 8 ? 8 : fit >= 4 ? 4 : fit == 3 ? 3 : 2;
   auto scan = parts == 8 ? gdn_chunk_scan_kernel<8> : parts == 4 ? gdn_chunk_scan_kernel<4> : parts == 3 ? gdn_chunk_scan_kernel<3> : gdn_chunk_scan_kernel<2>;
-  static bool attr = false;
-  if (!attr) {
-    for (auto k : {gdn_chunk_scan_kernel<8>, gdn_chunk_scan_kernel<4>, gdn_chunk_scan_kernel<3>, gdn_chunk_scan_kernel<2>})
-      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ScanSmem)) != cudaSuccess)
-        return OWL_ERR_LAUNCH * 1000;
-    if (cudaFuncSetAttribute(gdn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PrepSmem)) != cudaSuccess)
-      return OWL_ERR_LAUNCH * 1000;
-    attr = true;
-  }
+  static SmemLimit prep_limit, scan_limit[9];
+  int lrc = prep_limit.raise(gdn_chunk_prep_kernel, (int)sizeof(PrepSmem));
+  if (lrc == OWL_OK) lrc = scan_limit[parts].raise(scan, (int)sizeof(ScanSmem));
+  if (lrc != OWL_OK) return lrc;
   GdnChunkParams p = {};
   p.qkv = (const __nv_bfloat16*)qkv; p.ab = (const __nv_bfloat16*)ab; p.a_log = (const float*)a_log; p.dt_bias = (const float*)dt_bias;
   p.state = (float*)state; p.raw = (float*)raw; p.ldab = ldab; p.nk = nk; p.nv = nv; p.T = T; p.slot = slot; p.use_state = use_state;

@@ -425,19 +425,12 @@ static int gd_launch(const void* x, int ldx, const void* w, int ldw, GdParams& p
   r = gd_map(&b, w, p.N, p.K, ldw, p.fmt, GD_BN);
   if (r) return r;
   p.m_tiles = (p.T + GD_BM - 1) / GD_BM; p.n_tiles = (p.N + GD_BN - 1) / GD_BN;
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaFuncSetAttribute(gemm_dense_kernel<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GD_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_dense_kernel<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GD_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_dense_kernel<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GD_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_dense_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GD_SMEM) != cudaSuccess) {
-      sms = 0;
-      return OWL_ERR_LAUNCH * 1000;
-    }
-  }
+  const int sms = sm_count();
+  auto kernel = mode == 0 ? gemm_dense_kernel<false, false, false> : mode == 1 ? gemm_dense_kernel<true, false, false>
+              : mode == 2 ? gemm_dense_kernel<false, true, false> : gemm_dense_kernel<false, false, true>;
+  static SmemLimit limit[4];
+  const int lrc = limit[mode].raise(kernel, GD_SMEM);
+  if (lrc != OWL_OK) return lrc;
   int tiles = p.m_tiles * p.n_tiles;
   // few output tiles (small T and a narrow weight): cut k so that every SM streams a share of the weight; the fp32
   // partial tiles (at most 148 tiles of 128 x 256 floats = 19.4 MB) live in a scratch buffer the CALLER registers per
@@ -459,12 +452,10 @@ static int gd_launch(const void* x, int ldx, const void* w, int ldw, GdParams& p
   }
   const int grid = tiles < sms ? tiles : sms;
   if (mode == 1 || mode == 2) {         // the forms that exchange with other ranks start after the kernel before
-    if (mode == 1) gemm_dense_kernel<true, false, false><<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
-    else gemm_dense_kernel<false, true, false><<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
+    kernel<<<grid, GD_THREADS, GD_SMEM, st>>>(a, b, p);
     OWL_LAUNCH_CHECK();
   } else {
-    const int rc = launch_dep(p.T, mode == 0 ? gemm_dense_kernel<false, false, false> : gemm_dense_kernel<false, false, true>, dim3(grid),
-                              dim3(GD_THREADS), GD_SMEM, st, a, b, p);
+    const int rc = launch_dep(p.T, kernel, dim3(grid), dim3(GD_THREADS), GD_SMEM, st, a, b, p);
     if (rc != OWL_OK) return rc;
   }
   return p.ksplit > 1 ? gd_split_reduce(p.partial, p.out, p.T, p.N, p.ldp, p.ldo, p.ksplit, p.silu, st) : OWL_OK;

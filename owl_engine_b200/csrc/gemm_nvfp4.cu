@@ -371,16 +371,10 @@ OWL_API int owl_nvfp4_gemm(const void* xcodes, const void* xsf, const void* sx, 
   p.out = (__nv_bfloat16*)out; p.sfa = (const uint8_t*)xsf; p.sfb = (const uint8_t*)wsf; p.sx = (const float*)sx;
   p.row_scale = (const float*)row_scale; p.alpha = alpha; p.T = T; p.N = N; p.ldo = ldo; p.KI = (K + 255) / 256;
   p.m_tiles = (T + NF_BM - 1) / NF_BM; p.n_tiles = (N + NF_BN - 1) / NF_BN;
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaFuncSetAttribute(gemm_nvfp4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NF_SMEM) != cudaSuccess) {
-      sms = 0;
-      return OWL_ERR_LAUNCH * 1000;
-    }
-  }
+  const int sms = sm_count();
+  static SmemLimit limit;
+  const int lrc = limit.raise(gemm_nvfp4_kernel, NF_SMEM);
+  if (lrc != OWL_OK) return lrc;
   const int tiles = p.m_tiles * p.n_tiles;
   gemm_nvfp4_kernel<<<tiles < sms ? tiles : sms, NF_THREADS, NF_SMEM, st>>>(a, b, p);
   OWL_LAUNCH_CHECK();

@@ -334,12 +334,9 @@ static int make_map(CUtensorMap* m, const void* ptr, int rows, int K, int ld, in
 template <bool DEQ>
 static int launch_gemm(const CUtensorMap& a, const CUtensorMap& b, const GemmTcParams& p, cudaStream_t st) {
   auto kernel = gemm_tc_kernel<DEQ>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM) != cudaSuccess)
-      return OWL_ERR_LAUNCH * 1000;
-    attr_done = true;
-  }
+  static SmemLimit limit;
+  const int lrc = limit.raise(kernel, GT_SMEM);
+  if (lrc != OWL_OK) return lrc;
   dim3 grid((p.N + GT_BN - 1) / GT_BN, (p.T + GT_BM - 1) / GT_BM);
   return launch_dep(p.T, kernel, grid, dim3(GT_THREADS), GT_SMEM, st, a, b, p);
 }

@@ -601,12 +601,9 @@ template <int MT, int KIND, bool SIMT = false, bool A8 = false>
 static int launch_skinny(const SkinnyParams& p, int epi, int pdl, cudaStream_t st) {
   auto kernel = skinny_stream_kernel<MT, KIND, SIMT, A8>;
   constexpr int smem = skinny_smem_bytes<MT, KIND>();
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)OWL_ERR_LAUNCH * 1000 - (int)e;
-    attr_done = true;
-  }
+  static SmemLimit limit;
+  const int lrc = limit.raise(kernel, smem);
+  if (lrc != OWL_OK) return lrc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((p.n_tiles + p.tiles_per_cta - 1) / p.tiles_per_cta);
   cfg.blockDim = dim3(SK_WARPS * 32);

@@ -425,14 +425,10 @@ __global__ void __launch_bounds__(VC * FM_WARPS * 32, 4 / VC) w4_fma_kernel(FmaP
 template <int VC, int MODE, int EPI>
 static int launch_fma(const FmaParams& p, int grid, int pdl, cudaStream_t st) {
   auto kernel = w4_fma_kernel<VC, MODE, EPI>;
-  static int attr_smem = 0;
   const int smem = fma_smem_bytes(VC, p.K);
-  if (smem > attr_smem) {
-    const int want = smem > 96 * 1024 ? smem : 96 * 1024;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
-    if (e != cudaSuccess) return (int)OWL_ERR_LAUNCH * 1000 - (int)e;
-    attr_smem = want;
-  }
+  static SmemLimit limit;
+  const int lrc = limit.raise(kernel, smem > 96 * 1024 ? smem : 96 * 1024);
+  if (lrc != OWL_OK) return lrc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(VC * FM_WARPS * 32);
@@ -459,18 +455,6 @@ static int dispatch_fma(const FmaParams& p, int mode, int epi, int grid, int pdl
   return OWL_ERR_BAD_ARG;
 }
 
-static int fma_sm_count() {
-  static int sms[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!sms[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
-    sms[dev] = n;
-  }
-  return sms[dev];
-}
-
 }  // namespace owl
 using namespace owl;
 
@@ -495,7 +479,7 @@ OWL_API int owl_w4_fma(const void* records, const void* x, const void* norm_w, v
   p.N = N; p.K = K; p.n_tiles = N / 16; p.eps = eps; p.one_plus = one_plus_w;
   const int vc = groups_per_cta ? groups_per_cta : (K > 8192 ? 4 : 2);
   if (vc != 2 && vc != 4) return OWL_ERR_BAD_ARG;
-  const int grid = fma_sm_count() * (4 / vc);
+  const int grid = sm_count() * (4 / vc);
   if (p.ab_rows > grid * vc * FM_WARPS) return OWL_ERR_BAD_ARG;
   return vc == 4 ? dispatch_fma<4>(p, mode, epi, grid, pdl, st) : dispatch_fma<2>(p, mode, epi, grid, pdl, st);
 }
@@ -521,7 +505,7 @@ OWL_API int owl_w4_fma_tp(const void* records, const void* x, const void* norm_w
   p.ab_w = (const __nv_bfloat16*)ab_w; p.ab_out = (__nv_bfloat16*)ab_out; p.ab_rows = ab_rows;
   const int vc = groups_per_cta ? groups_per_cta : (K > 8192 ? 4 : 2);
   if (vc != 2 && vc != 4) return OWL_ERR_BAD_ARG;
-  const int grid = fma_sm_count() * (4 / vc);
+  const int grid = sm_count() * (4 / vc);
   if (ab_rows < 0 || (ab_rows > 0 && (!ab_w || !ab_out)) || ab_rows > grid * vc * FM_WARPS) return OWL_ERR_BAD_ARG;
   if (kparts < 1 || world * kparts > FM_MAX_RANKS) return OWL_ERR_BAD_ARG;
   p.kparts = kparts;

@@ -494,28 +494,13 @@ __global__ void __launch_bounds__(MM_WARPS * 32, CT) w4_mma_kernel(MmaParams p, 
   }
 }
 
-static int mm_sms() {
-  static int sms[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!sms[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
-    sms[dev] = n;
-  }
-  return sms[dev];
-}
-
 template <int FMT, int MT, bool A8, int CT>
 static int launch_mma(const MmaParams& p, int epi, int KS, int blocks, int pdl, cudaStream_t st) {
   auto kernel = w4_mma_kernel<FMT, MT, A8, CT>;
   constexpr int smem = mm_smem<FMT, MT, CT>();
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)OWL_ERR_LAUNCH * 1000 - (int)e;
-    attr_done = true;
-  }
+  static SmemLimit limit;
+  const int lrc = limit.raise(kernel, smem);
+  if (lrc != OWL_OK) return lrc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(KS * blocks);
   cfg.blockDim = dim3(MM_WARPS * 32);
@@ -542,7 +527,7 @@ template <int FMT, bool A8>
 static int dispatch_mma(MmaParams& p, int epi, int pdl, cudaStream_t st) {
   p.ab_blocks = (p.ab_rows + 15) / 16;
   const int row_blocks = (p.n_tiles + MM_TILES - 1) / MM_TILES;
-  const int blocks = row_blocks + p.ab_blocks, sms = mm_sms();
+  const int blocks = row_blocks + p.ab_blocks, sms = sm_count();
   // k parts: as many as one wave of four CTAs per SM holds, each of at least two record columns; independent of M. With one
   // column a part is all start-up and exchange (8192 x 1024, group 128, 1 / 8 / 32 rows: 8 parts 4.6 / 5.0 / 11.6 us, 4 parts 3.8 /
   // 4.0 / 8.1; a column more loses where it takes CTAs away: 1024 x 2048 2.8 -> 3.1).

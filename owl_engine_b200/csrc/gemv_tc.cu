@@ -482,18 +482,19 @@ static int launch_stream_tc(VtParams p, int epi, int ctas, long long scratch_byt
                             cudaStream_t st) {
   auto kernel = stream_tc_kernel<G, MT>;
   constexpr int smem = VtCfg<G>::SMEM;
-  static int resident = 0;     // CTAs that fit on the device at once (SMs x occupancy)
-  if (!resident) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)OWL_ERR_LAUNCH * 1000 - (int)e;
-    int dev = 0, sms = 0, occ = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, VT_THREADS, smem);
-    if (e != cudaSuccess || occ < 1 || sms < 1) return (int)OWL_ERR_LAUNCH * 1000 - (int)e;
+  static SmemLimit limit;
+  const int lrc = limit.raise(kernel, smem);
+  if (lrc != OWL_OK) return lrc;
+  static std::atomic<int> per_sm[OWL_DEVICES];          // CTAs that fit on an SM at once
+  const int dev = current_device();
+  int occ = dev >= 0 && dev < OWL_DEVICES ? per_sm[dev].load(std::memory_order_relaxed) : 0;
+  if (!occ) {
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, VT_THREADS, smem);
+    if (e != cudaSuccess || occ < 1) return (int)OWL_ERR_LAUNCH * 1000 - (int)e;
     if (occ > 512 / VT_TMEM_COLS) occ = 512 / VT_TMEM_COLS;     // tensor memory: 512 columns per SM
-    resident = sms * occ;
+    if (dev >= 0 && dev < OWL_DEVICES) per_sm[dev].store(occ, std::memory_order_relaxed);
   }
+  const int resident = sm_count() * occ;
   int grid;
   vt_plan(p.KT, p.TB, ctas > 0 ? ctas : resident, &grid, &p.per, &p.slots);
   if ((long long)p.NRB * p.slots * 128 * MT * 4 > scratch_bytes || (long long)p.NRB * 16 > counter_bytes)

@@ -559,34 +559,19 @@ __global__ void __launch_bounds__(TM_THREADS, 1) w4_tm_kernel(TmParams p, int KS
   }
 }
 
-static int tm_sms() {
-  static int sms[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!sms[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
-    sms[dev] = n;
-  }
-  return sms[dev];
-}
-
 template <int F, bool A8>
 static int launch_tm(TmParams& p, int pdl, cudaStream_t st) {
   auto kernel = w4_tm_kernel<F, A8>;
   constexpr int smem = tm_smem<F>();
   static_assert(smem <= 227 * 1024, "shared memory");
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)OWL_ERR_LAUNCH * 1000 - (int)e;
-    attr_done = true;
-  }
+  static SmemLimit limit;
+  const int lrc = limit.raise(kernel, smem);
+  if (lrc != OWL_OK) return lrc;
   p.n_tiles = p.N / 16;
   p.row_blocks = (p.n_tiles + 7) / 8;
   p.ab_blocks = (p.ab_rows + 15) / 16;
   // k parts: as many as the SMs hold beside each other, of at least two record columns each; independent of M
-  const int sms = tm_sms();
+  const int sms = sm_count();
   int KS = 1;
   for (int ks : {2, 3, 4, 8})
     if ((p.row_blocks + p.ab_blocks) * ks <= sms && 2 * ks <= (p.K >> 7)) KS = ks;

@@ -106,6 +106,21 @@ def test_control_blocks_in_shared_memory_fit_their_reservation():
     assert len(seen) >= 7
 
 
+def test_launchers_ask_each_device():
+    """A kernel's limit of shared memory and the number of SMs belong to a device. Launchers get both from common.cuh, which remembers
+    them by device: a launcher that asked once per process failed on a second device."""
+    import re
+
+    from owl_engine_b200.ops import registry as R
+
+    for f in sorted(R.CSRC.glob("*.cu")):
+        text = f.read_text()
+        assert "cudaFuncSetAttribute" not in text and "cudaDevAttrMultiProcessorCount" not in text, f.name
+        assert not re.search(r"static (bool|int) \w+ = (false|0);", text), f.name
+    helper = (R.CSRC / "common.cuh").read_text()
+    assert re.search(r"have\[dev\]\.load\([^)]*\) >= bytes", helper) and re.search(r"have\[dev\]\.store\(bytes", helper)
+
+
 def test_kernel_registry_matches_sources_and_bindings():
     from owl_engine_b200.ops import registry as R
 
