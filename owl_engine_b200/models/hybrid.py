@@ -1012,7 +1012,7 @@ class HybridRunner:
 
         if w.layout == "nvfp4":
             return linear.nvfp4_gemm(w, x, out, arm=self.prefill_gemm)
-        return linear.w4_gemm(w, x, out, arm=self.prefill_gemm, ahead=ahead)
+        return linear.w4_gemm(w, x, out, arm=self.prefill_gemm, ahead=ahead, pdl=self.pdl)
 
     def _dequant_ahead(self, t: int):
         """The ``DequantAhead`` of a ``t``-row chunk, started on this model's weights, or None: long chunks of block-layout weights (the
@@ -1119,7 +1119,7 @@ class HybridRunner:
             if self.comm is not None and sp.tp_world > 1:
                 self.comm.allreduce_prefill(ws["y"][:t])
             K.rmsnorm_pack(h, lw.ln2, delta=ws["y"][:t], out_h=h, normed=x, m=t, k=sp.hidden, group=self.G, eps=sp.eps, pdl=pdl)
-            if not linear.w4_gemm_silu(lw.gate_up, x, ws["act"][:t], arm=self.prefill_gemm, ahead=ahead):
+            if not linear.w4_gemm_silu(lw.gate_up, x, ws["act"][:t], arm=self.prefill_gemm, ahead=ahead, pdl=self.pdl):
                 gu = ws["wide"].view(-1)[:t * 2 * sp.inter].view(t, 2 * sp.inter)
                 self._gemm(lw.gate_up, x, gu, ahead)
                 K.silu_mul(gu, t, sp.inter, out=ws["act"][:t], group=self.G)

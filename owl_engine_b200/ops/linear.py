@@ -264,7 +264,9 @@ def _rows_ok(w, x: torch.Tensor, out: torch.Tensor, resident: bool) -> bool:
         and out.stride(0) % 8 == 0 and (x.data_ptr() | out.data_ptr()) % 16 == 0
 
 
-def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: DequantAhead | None = None) -> torch.Tensor:
+def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: DequantAhead | None = None, pdl: bool = False) -> torch.Tensor:
+    """out[T, N] = x[T, K] @ dequant(w)^T on one of the arms above. ``pdl``: kernels that read the weight's records may do so while the
+    kernel before them on the stream still runs (for weights that nothing on it writes any more)."""
     dense = ahead.take(w) if ahead is not None else None
     if dense is not None:
         gemm_tc.f16_gemm(x, dense, out)
@@ -296,7 +298,7 @@ def w4_gemm(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: Dequa
             K.w4_mma(w, xp, xs, out, t, ldo=out.stride(0))
             return out
         if _rows_ok(w, x, out, resident):
-            return gemm_tc.w4_gemm_rows(w, x, out)
+            return gemm_tc.w4_gemm_rows(w, x, out, pdl=pdl)
         if x.shape[0] >= DEQUANT_FROM:
             return gemm_tc.f16_gemm(x, w4_dense(w, x.dtype, x.device, resident=resident), out)
         return gemm_tc.w4a16_gemm(w, x, out)
@@ -315,9 +317,9 @@ def _e4m3_weight(w, device, resident: bool):
     return cached
 
 
-def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: DequantAhead | None = None) -> bool:
+def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: DequantAhead | None = None, pdl: bool = False) -> bool:
     """out[T, N/2] (fp16) = silu(gate) * up of the merged gate / up projection in one launch. False (and nothing done) where the
-    arm or the shape has no such epilogue: the caller multiplies and activates in two steps."""
+    arm or the shape has no such epilogue: the caller multiplies and activates in two steps. ``pdl``: as for ``w4_gemm``."""
     t = x.shape[0]
     if ahead is not None:
         if w.n < 512 or out.stride(0) % 8:
@@ -336,7 +338,7 @@ def w4_gemm_silu(w, x: torch.Tensor, out: torch.Tensor, arm: str = "tc", ahead: 
         gemm_tc.gemm_silu(xq, wq, out, sx, sw)
         return True
     if arm in ("tc", "tc4", "tcr", "tc8", "tc8r") and t > SKINNY_UPTO and _rows_ok(w, x, out, arm in ("tcr", "tc8r")):
-        gemm_tc.w4_gemm_rows(w, x, out, silu=True)
+        gemm_tc.w4_gemm_rows(w, x, out, silu=True, pdl=pdl)
         return True
     if arm in ("tc", "tc4", "tcr", "tc8", "tc8r") and t >= SILU_FROM and w.n >= 512:
         gemm_tc.gemm_silu(x, w4_dense(w, x.dtype, x.device, resident=arm in ("tcr", "tc8r")), out)
