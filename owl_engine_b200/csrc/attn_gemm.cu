@@ -42,10 +42,19 @@ __device__ __forceinline__ void ag_floats(const uint4* raw, float scale, float* 
 // Bound by memory: a key and head is read once (512 bytes of e4m3) and written once (1 KB). grid (ctx_pad / 64, hkv), 256 threads: 64
 // keys of one head; a thread takes 16 dims (16-byte loads) of two neighbouring keys at a time, stores K as it is and puts V as pairs
 // of keys into shared memory, [dim][32 pairs], from which a dim's 64 keys leave as one line. A pair lies at place
-// pair ^ 2 * (dim / 16): the 16 lanes that write one pair hold dims 16 apart, which would be one bank.
+// pair ^ 2 * (dim / 16): the 16 lanes that write one pair hold dims 16 apart, which would be one bank. ANY: pools or keys that do not
+// begin at a multiple of 16 bytes (views; an allocation of their own always does), read byte by byte and stored value by value.
 // 34,768 e4m3 keys, 4 heads: 38 us, 32 at copy bandwidth; byte loads and 2-byte stores of 16 keys a CTA took 214.
 constexpr int AG_KEYS = 64;
-template <int FMT>
+template <bool ANY>
+__device__ __forceinline__ uint4 ag_load(const uint8_t* p) {
+  if (!ANY) return __ldg(reinterpret_cast<const uint4*>(p));
+  uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < 16; ++i) w[i >> 2] |= (uint32_t)__ldg(p + i) << (8 * (i & 3));
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+template <int FMT, bool ANY>
 __global__ void __launch_bounds__(256) kv_gather_kernel(const uint8_t* __restrict__ k_pool, const uint8_t* __restrict__ v_pool,
                                                         const float* __restrict__ k_scale, const float* __restrict__ v_scale,
                                                         const int* __restrict__ bt, int ctx, int ctx_pad, int hkv,
@@ -64,8 +73,8 @@ __global__ void __launch_bounds__(256) kv_gather_kernel(const uint8_t* __restric
     vsc[i] = FMT == 1 && live ? v_scale[row] : 1.f;
 #pragma unroll
     for (int r = 0; r < RAW; ++r) {
-      kr[i][r] = live ? __ldg(reinterpret_cast<const uint4*>(k_pool + row * HD * ESZ) + l16 * RAW + r) : make_uint4(0, 0, 0, 0);
-      vr[i][r] = live ? __ldg(reinterpret_cast<const uint4*>(v_pool + row * HD * ESZ) + l16 * RAW + r) : make_uint4(0, 0, 0, 0);
+      kr[i][r] = live ? ag_load<ANY>(k_pool + row * HD * ESZ + (l16 * RAW + r) * 16) : make_uint4(0, 0, 0, 0);
+      vr[i][r] = live ? ag_load<ANY>(v_pool + row * HD * ESZ + (l16 * RAW + r) * 16) : make_uint4(0, 0, 0, 0);
     }
   }
 #pragma unroll
@@ -73,7 +82,13 @@ __global__ void __launch_bounds__(256) kv_gather_kernel(const uint8_t* __restric
     const int key = key0 + (i >> 1) * 32 + (threadIdx.x >> 4) * 2 + (i & 1);
     float f[16];
     ag_floats<FMT>(kr[i], ks[i], f);
-    uint4* ko = reinterpret_cast<uint4*>(kout + ((size_t)h * ctx_pad + key) * HD) + l16 * 2;
+    __nv_bfloat16* kd = kout + ((size_t)h * ctx_pad + key) * HD + l16 * 16;
+    if (ANY) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) kd[k] = __float2bfloat16(f[k]);
+      continue;
+    }
+    uint4* ko = reinterpret_cast<uint4*>(kd);
     ko[0] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
     ko[1] = make_uint4(pack_bf16(f[8], f[9]), pack_bf16(f[10], f[11]), pack_bf16(f[12], f[13]), pack_bf16(f[14], f[15]));
   }
@@ -229,20 +244,14 @@ OWL_API int owl_kv_gather(const void* k_pool, const void* v_pool, const void* k_
                           int ctx, int ctx_pad, int hkv, int hd, void* k_out, void* vt_out, cudaStream_t st) {
   if (hd != 256 || ctx < 1 || ctx_pad < ctx || (ctx_pad & 63) || hkv < 1 || fmt < 0 || fmt > 2 || (fmt == 1 && (!k_scale || !v_scale)))
     return OWL_ERR_BAD_ARG;
-  if ((reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool) | reinterpret_cast<uintptr_t>(k_out) |
-       reinterpret_cast<uintptr_t>(vt_out)) & 15)
-    return OWL_ERR_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(vt_out) & 15) || (reinterpret_cast<uintptr_t>(k_out) & 1)) return OWL_ERR_BAD_ARG;
+  const bool any = (reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool) | reinterpret_cast<uintptr_t>(k_out)) & 15;
   const dim3 grid(ctx_pad / AG_KEYS, hkv);
-  if (fmt == 0)
-    kv_gather_kernel<0><<<grid, 256, 0, st>>>((const uint8_t*)k_pool, (const uint8_t*)v_pool, nullptr, nullptr, (const int*)bt, ctx,
-                                              ctx_pad, hkv, (__nv_bfloat16*)k_out, (__half*)vt_out);
-  else if (fmt == 1)
-    kv_gather_kernel<1><<<grid, 256, 0, st>>>((const uint8_t*)k_pool, (const uint8_t*)v_pool, (const float*)k_scale,
-                                              (const float*)v_scale, (const int*)bt, ctx, ctx_pad, hkv, (__nv_bfloat16*)k_out,
-                                              (__half*)vt_out);
-  else
-    kv_gather_kernel<2><<<grid, 256, 0, st>>>((const uint8_t*)k_pool, (const uint8_t*)v_pool, nullptr, nullptr, (const int*)bt, ctx,
-                                              ctx_pad, hkv, (__nv_bfloat16*)k_out, (__half*)vt_out);
+  auto kernel = fmt == 0 ? (any ? kv_gather_kernel<0, true> : kv_gather_kernel<0, false>)
+              : fmt == 1 ? (any ? kv_gather_kernel<1, true> : kv_gather_kernel<1, false>)
+                         : (any ? kv_gather_kernel<2, true> : kv_gather_kernel<2, false>);
+  kernel<<<grid, 256, 0, st>>>((const uint8_t*)k_pool, (const uint8_t*)v_pool, (const float*)k_scale, (const float*)v_scale, (const int*)bt, ctx,
+                               ctx_pad, hkv, (__nv_bfloat16*)k_out, (__half*)vt_out);
   OWL_LAUNCH_CHECK();
   return OWL_OK;
 }

@@ -509,3 +509,28 @@ def test_copy_slot_indexes_like_a_tensor():
     for src, dst in ((0, 5), (5, 0), (-6, 0)):
         with pytest.raises(IndexError):
             pool.copy_slot(src, dst)
+
+
+@pytest.mark.parametrize("fmt", [0, 1, 2])
+@pytest.mark.parametrize("pool_off,key_off", [(1, 0), (0, 1), (7, 3)])
+def test_gather_of_pools_that_begin_anywhere(fmt, pool_off, key_off):
+    """Pools and keys that are not 16-byte aligned (views into a larger allocation), in elements: what aligned ones give, and nothing
+    beside the keys is written."""
+    ctx, pad, hkv, pages = 83, 128, 2, 8
+    gen = torch.Generator(device=DEV).manual_seed(fmt)
+    bt = torch.randperm(pages, device=DEV, generator=gen)[:6].int()
+    n = pages * 16 * hkv * 256
+    flat = [torch.randn(n, device=DEV, generator=gen).half() if fmt == 2 else torch.randint(0, 0x7e, (n,), device=DEV, generator=gen, dtype=torch.uint8)
+            for _ in range(2)]
+    sc = [torch.rand(pages * 16 * hkv, device=DEV, generator=gen) + 0.01 for _ in range(2)]
+
+    def gather(off_p, off_k):
+        pools = [torch.cat([f[:off_p], f])[off_p:] for f in flat]
+        k = torch.full((hkv * pad * 256 + 16,), 7.0, dtype=torch.bfloat16, device=DEV)
+        vt = torch.zeros(hkv, 256, pad, dtype=torch.float16, device=DEV)
+        K.call("owl_kv_gather", K.ptr(pools[0]), K.ptr(pools[1]), K.ptr(sc[0]), K.ptr(sc[1]), fmt, K.ptr(bt), ctx, pad, hkv, 256,
+               K.ptr(k[off_k:]), K.ptr(vt), K.stream())
+        assert (k[:off_k] == 7).all() and (k[off_k + hkv * pad * 256:] == 7).all()
+        return k[off_k:][:hkv * pad * 256], vt
+    for a, b in zip(gather(pool_off, key_off), gather(0, 0)):
+        assert torch.equal(a, b)
