@@ -102,6 +102,7 @@ def f16_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, force_small: b
 
 
 K.register("owl_w4_gemm_rows", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+K.register("owl_w4_gemm_rows_plan", [c_int, c_int, c_int, c_int, ctypes.c_longlong, c_void_p])
 ROWS_UPTO = 256         # rows of one w4_gemm_rows launch
 
 

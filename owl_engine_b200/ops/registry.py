@@ -40,6 +40,7 @@ _T = [
     KernelSpec("owl_w8a16_skinny", "gemv.cu", "gemv", gen="mma.sync+bulk-copy"),
     KernelSpec("owl_skinny_status", "gemv.cu", "status", capture=False),
     KernelSpec("owl_w4_gemm_rows", "gemm_w4.cu", "gemm_act", gen="tcgen05+tma"),
+    KernelSpec("owl_w4_gemm_rows_plan", "gemm_w4.cu", "status", capture=False),
     KernelSpec("owl_gemm_w4_status", "gemm_w4.cu", "status", capture=False),
     KernelSpec("owl_gemm_silu", "gemm_dense.cu", "gemm_act", gen="tcgen05+tma"),
     KernelSpec("owl_gdn_copy_slot", "gdn.cu", "gdn"),

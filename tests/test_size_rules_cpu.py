@@ -1,11 +1,13 @@
 """Size rules of the prompt and step paths (no GPU: the rules look at sizes only)."""
+import ctypes
 from types import SimpleNamespace
 
 import pytest
 
 from owl_engine_b200.models.hybrid import HybridRunner
 from owl_engine_b200.models.spec import PRESETS
-from owl_engine_b200.ops import linear
+from owl_engine_b200.ops import gemm_tc, linear
+from owl_engine_b200.ops import kernels as K
 
 
 def _projections(name):
@@ -30,6 +32,17 @@ def test_small_models_do_not_pay_for_dequantising_ahead(model, t, pays):
                                                  (16384, 5120, 127, True, True), (5120, 17408, 33, True, True)])
 def test_operand_of_a_short_prompt(n, k, t, resident, rows):
     assert linear.rows_pay(n, k, t, resident) == rows
+
+
+# one chunk of up to 256 tokens; two of a matrix that leaves SMs idle, is not cut along k and whose steps get shorter; longer prompts
+@pytest.mark.parametrize("t,n,k,plan", [(128, 1024, 3584, (1, 1, 128)), (129, 1024, 3584, (1, 2, 80)), (256, 1024, 3584, (1, 2, 128)),
+                                        (256, 9472, 1024, (1, 2, 128)), (256, 9488, 1024, (1, 1, 256)), (256, 16384, 5120, (1, 1, 256)),
+                                        (137, 5120, 6144, (3, 1, 144)), (256, 5120, 17408, (3, 1, 256)), (2048, 5120, 17408, (1, 11, 192))])
+def test_chunks_and_parts_of_an_int4_product(t, n, k, plan):
+    out = (ctypes.c_int * 3)()
+    f = K.fn("owl_w4_gemm_rows_plan")
+    assert f(t, n, k, linear.SMS, gemm_tc.KS_SCRATCH_BYTES, out) == 0
+    assert tuple(out) == plan
 
 
 # (sequences, longest context, uniform rows) -> parts of a sequence's keys, 27B head geometry (4 kv heads)
