@@ -534,3 +534,89 @@ def test_gather_of_pools_that_begin_anywhere(fmt, pool_off, key_off):
         return k[off_k:][:hkv * pad * 256], vt
     for a, b in zip(gather(pool_off, key_off), gather(0, 0)):
         assert torch.equal(a, b)
+
+
+def _one_hot_gates(k, group, cut):
+    """A weight whose tiles give gate row r = scale_r * x[0] and up row = x[1], and rows of x for it: nearly every fp16 value of x[0] (some
+    of them where the product is cut along k), with an up of 1.5 or one that takes silu(gate) * up out of fp16's range."""
+    codes = torch.zeros(256, k, dtype=torch.uint8)
+    codes[:, 0] = 1
+    codes[7::16, 0] = 15                              # 15 * 65504: an infinite fp16 weight, so gates of -inf, +inf and (times 0) NaN
+    up = torch.arange(256) % 16 >= 8
+    codes[up, 0], codes[up, 1] = 0, 1
+    scales = torch.ones(256, k // group)
+    scales[~up] = torch.tensor([1.0, 2.0 ** -8, 2.0 ** -14, 96.0, 3000.0, 65504.0, 0.375, 65504.0]).repeat(16)[:, None]
+    w = Q.pack_skinny(Q.W4Canonical(codes, scales.half(), torch.zeros(256, k // group).half(), group)).to(DEV)
+    v = torch.arange(65535, dtype=torch.int32, device=DEV).to(torch.int16).view(torch.float16)
+    if cut:
+        edge = [0.0, -80.0, -79.5, -80.5, -88.0, -89.0, -104.0, -5000.0, 80.0, 90.0, float("inf"), -float("inf"), float("nan")]
+        v = torch.cat([torch.tensor(edge, device=DEV).half(), v[7::391]])
+    x = torch.zeros(v.numel(), k, dtype=torch.float16, device=DEV)
+    x[:, 0] = v
+    x[:, 1] = torch.where(torch.arange(v.numel(), device=DEV) % 3 == 0, 60000.0, 1.5).half()
+    return w, x
+
+
+# gates of -80 and below, subnormal results, infinities, NaN; one launch of 256 chunks of tokens, and k in parts
+@pytest.mark.parametrize("k,cut", [(128, False), (8192, True)])
+@pytest.mark.parametrize("group", [128, 32])
+def test_activation_of_every_gate(k, cut, group):
+    """The epilogue's silu, which divides without branches, against the two-step form's division on the same rounded products: equal but
+    for the sign of a zero. And both against silu in 64 bits."""
+    w, x = _one_hot_gates(k, group, cut)
+    t = x.shape[0]
+    gu, act = torch.zeros(t, 256, dtype=torch.bfloat16, device=DEV), torch.zeros(t, 128, dtype=torch.float16, device=DEV)
+    gemm_tc.w4_gemm_rows(w, x, gu)
+    gemm_tc.w4_gemm_rows(w, x, act, silu=True)
+    two = torch.zeros_like(act)
+    K.silu_mul(gu, t, 128, out=two)
+    gu = gu.double().view(t, 16, 2, 8)
+    g, u = gu[:, :, 0].reshape(t, 128), gu[:, :, 1].reshape(t, 128)
+    assert torch.isinf(g).any() and torch.isnan(g).any() and ((g < -80) & (g > -90)).any() and (g < -1e8).any()
+    assert (act == two).all()
+    # fp32 exponential, quotient and product, then fp16
+    want = (g / (1 + torch.exp(-g)) * u).clamp(-65504, 65504)
+    assert ((act.double() - want).abs() <= want.abs() * 2.0 ** -10 + 2.0 ** -24)[torch.isfinite(g)].all()
+    assert K.all_status()["gemm_dense"] == 0
+
+
+@pytest.mark.parametrize("t", [40, 137, 256, 288, 289])
+def test_mlp_chain_that_starts_early_equals_the_chain_with_host_waits(t):
+    """Norm (residual added in place), gate / up with its activation, down twice in a row: the int4 GEMM reads weights before it waits,
+    and its k parts (8 of the 512 x 8192 products) meet in the scratch that the next product writes. Four layers back to back against
+    the same launches with a synchronisation after each: the same bits."""
+    n, inter = 512, 8192
+    gen = torch.Generator(device=DEV).manual_seed(t)
+    gu, down, down2 = (Q.random_skinny(a, b, 32, DEV, b ** -0.5, i) for i, (a, b) in enumerate(((2 * inter, n), (n, inter), (n, inter))))
+    gamma = 1 + 0.1 * torch.randn(n, device=DEV, generator=gen)
+    h0 = torch.randn(t, n, device=DEV, generator=gen).bfloat16()
+    runs = []
+    for sync in (True, False):
+        h, x = h0.clone(), torch.zeros(t, n, dtype=torch.float16, device=DEV)
+        y, y2 = torch.zeros_like(h), torch.zeros_like(h)
+        act = torch.zeros(t, inter, dtype=torch.float16, device=DEV)
+        torch.cuda.synchronize()
+        for i in range(4):
+            for step in (lambda: K.rmsnorm_pack(h, gamma, delta=(y, y2)[i % 2], out_h=h, normed=x, m=t, k=n, group=32, eps=1e-6, pdl=True),
+                         lambda: gemm_tc.w4_gemm_rows(gu, x, act, silu=True, pdl=True),
+                         lambda: gemm_tc.w4_gemm_rows(down, act, y, pdl=True),
+                         lambda: gemm_tc.w4_gemm_rows(down2, act, y2, pdl=True)):
+                step()
+                if sync:
+                    torch.cuda.synchronize()
+        runs.append((h, x, act, y, y2))
+    assert torch.isfinite(runs[0][0].float()).all() and runs[0][3].float().std() > 0.01
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
+# several chunks of tokens in groups of 128 (records of another length): two units of an odd number of steps a CTA; k in parts
+@pytest.mark.parametrize("t", [257, 515])
+@pytest.mark.parametrize("n,k", [(19088, 384), (1040, 4736)])
+def test_rows_gemm_walks_units_in_groups_of_128(t, n, k):
+    gen = torch.Generator(device=DEV).manual_seed(n + k + t)
+    w = Q.random_skinny(n, k, 128, DEV, 0.05, n + k)
+    x = torch.randn(t, k, generator=gen, device=DEV).half()
+    out = torch.zeros(t, n + 8, dtype=torch.bfloat16, device=DEV)
+    gemm_tc.w4_gemm_rows(w, x, out)
+    _check_against_dequant(w, x, out[:, :n])
+    assert (out[:, n:] == 0).all() and K.all_status()["gemm_dense"] == 0

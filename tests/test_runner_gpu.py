@@ -370,3 +370,75 @@ def test_wide_batched_step_on_the_resident_dense_weights_matches_the_streaming_a
         runs.append(r)
     assert runs[0]._x16h is not None and runs[1]._x16h is None
     assert rel_err(outs[0], outs[1]) < tol
+
+
+@pytest.mark.parametrize("quant,group", [("w4a16", 128), ("w4a16", 32), ("nvfp4", 128)])
+def test_captured_step_of_32_rows_matches_reference(quant, group):
+    """32 sequences from their first token on, three steps of given tokens through one captured graph: the packing producers of every
+    projection and the form that unpacks into tensor memory, against the fp32 model of the same weights."""
+    b, steps = 32, 3
+    spec = make_spec(n_layers=4)
+    hw, equiv = H.weights_from_dense(spec, init_weights(spec, seed=3, std=0.05), DEV, group=group, quant=quant)
+    run = H.HybridRunner(spec, hw, H.StatePool(spec, DEV, n_pages=b, n_slots=b), max_seqs=b, max_blocks=4, prefill_gemm="tc")
+    ref = RefModel(spec, equiv, kv_fp8=True)
+    ids = torch.randint(0, spec.vocab, (b, steps), generator=torch.Generator().manual_seed(4))
+    rows = torch.arange(b, dtype=torch.int32, device=DEV)
+    run.block_table[:, 0] = rows
+    graph = run.capture(b, 1, ctx_hint=64)
+    entries = run.graph_manifest()[0]["entries"]
+    tm, mma = ("owl_nvfp4_tm", "owl_nvfp4_mma") if quant == "nvfp4" else ("owl_w4_tm", "owl_w4_mma")
+    assert entries.get(tm, 0) == 4 * spec.n_layers and mma not in entries
+    for s in range(b):
+        run.pool.reset_slot(s)
+    lay = H.StepLayout(b, 1)
+    v = run.views(lay)
+    v["gslot"].copy_(rows)
+    v["bt_row"].copy_(rows)
+    states = [ref.new_state() for _ in range(b)]
+    for pos in range(steps):
+        v["ids"].copy_(ids[:, pos].to(torch.int32))
+        v["pos3"][:] = pos
+        v["kv_slot"].copy_(rows * 16 + pos)
+        v["ctx"][:] = pos + 1
+        graph.replay()
+        want = torch.cat([ref.logits(ref.forward(ids[i, pos:pos + 1], states[i])) for i in range(b)])
+        got = run.logits[:b].float().cpu()
+        assert max(rel_err(got[i], want[i]) for i in range(b)) < DECODE_TOL, pos
+    assert K.all_status()["stream_tc"] == 0
+
+
+# rows per chunk x pool x arm; kernels of 289 rows start after the one before. The last three: rows behind a prefix, and the attention
+# over gathered keys
+@pytest.mark.parametrize("t,kv_dtype,arm,attn_from,pos0", [(40, "fp8", "tc", 0, 0), (137, "int8", "tc", 0, 0), (256, "bf16", "tc", 0, 0), (288, "fp8", "tc", 0, 0),
+                                                           (289, "fp8", "tc", 0, 0), (137, "fp8", "tc8r", 0, 0), (288, "bf16", "tc8r", 0, 0),
+                                                           (137, "fp8", "tcr", 0, 48), (200, "fp8", "tc", 32, 0), (137, "int8", "tc", 32, 163)])
+def test_prompt_kernels_that_start_early_leave_what_kernels_with_host_waits_leave(t, kv_dtype, arm, attn_from, pos0, monkeypatch):
+    """A whole chunk, twice over without a pause, against the same launches with a synchronisation after each: logits, keys, values and
+    GDN states bit for bit."""
+    spec = make_spec(n_layers=4, mult=2)
+    hw, _ = H.weights_from_dense(spec, init_weights(spec, seed=3, std=0.05), DEV)
+    gen = torch.Generator().manual_seed(t)
+    ids = torch.randint(0, spec.vocab, (pos0 + t,), generator=gen).to(torch.int32).to(DEV)
+    plain_call = K.call
+
+    def waiting_call(*a):
+        plain_call(*a)
+        torch.cuda.synchronize()
+    runs = []
+    for call in (waiting_call, plain_call):
+        pool = H.StatePool(spec, DEV, n_pages=64, n_slots=3, kv_dtype=kv_dtype)
+        run = H.HybridRunner(spec, hw, pool, max_seqs=4, max_blocks=32, prefill_gemm=arm, pdl=True)
+        run.ATTN_GEMM_FROM = attn_from
+        run.block_table[1, :24] = torch.randperm(64, generator=torch.Generator().manual_seed(1))[:24].to(torch.int32).to(DEV)
+        monkeypatch.setattr(K, "call", call)
+        for _ in range(2):
+            pool.reset_slot(2)
+            if pos0:
+                run.prefill_chunk_forward(ids[:pos0], 0, 1, 2, want_logits=False)
+            run.prefill_chunk_forward(ids[pos0:], pos0, 1, 2)
+        torch.cuda.synchronize()
+        monkeypatch.setattr(K, "call", plain_call)
+        runs.append([run.logits[:1].clone(), pool.k_pool, pool.v_pool, pool.conv_state, pool.rec_state] + (list(pool.scales(0)) if pool.scales(0) else []))
+    assert torch.isfinite(runs[0][0].float()).all()
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+    assert not any(K.all_status().values())
