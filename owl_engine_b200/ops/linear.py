@@ -18,7 +18,7 @@
 * ``"tcr"`` / ``"tc8r"``  the same two arms with the dequantised (fp16) resp. re-quantised (e4m3) weight kept RESIDENT
                   on the weight object after its first use: 2 resp. 1 extra bytes per weight in HBM (48.7 / 24.3 GB for the
                   27B model on one GPU, which 180 GB leave room for) buy back the per-call dequantisation pass. The fp16
-                  copies serve chunks above 256 tokens, and from 128 those where ``rows_pay`` says so;
+                  copies serve chunks above 256 tokens (``rows_pay``);
 * ``"baseline"``  dequantise to a dense bf16 scratch matrix, then the library GEMM
                   (``torch.matmul`` = cuBLAS). This is the comparison arm, like the reference's
                   range-dequant -> cuBLAS arm (``crates/kernels/cu/gguf/gguf_smem.cu:415-552``).
@@ -242,25 +242,22 @@ class DequantAhead:
 def rows_pay(n: int, k: int, t: int, resident: bool) -> bool:
     """Whether ``t`` tokens times an [n, k] int4 weight read the records (``gemm_w4.cu``) rather than a dense copy.
 
-    Up to 256 tokens, all that one launch takes. A resident copy needs no dequantisation; where it exists it is used at 256 tokens (the
-    persistent kernel: 16384 x 5120 44 us, 34816 x 5120 87, 5120 x 17408 60; the records 34, 76 and 49) and, from 128, where its
-    128 x 128 tiles fit two per SM and k is short (16384 x 5120 46 us at 137 tokens, the records 23): limits measured against the
-    records through shared memory (63, 115, 73 us and 49), which the present kernel no longer needs them for; not where a tile walks a
-    long k alone or the tiles take two waves (5120 x 17408 118 / 32 us, 34816 x 5120 121 / 45)."""
-    if t > gemm_tc.ROWS_UPTO:
-        return False
-    if not resident or t < DEQUANT_FROM:
-        return True
-    return t < SILU_FROM and (n < 2 * k or -(-n // 128) * -(-t // 128) > 2 * SMS)
+    Up to 256 tokens always: the records are the faster operand even where a resident fp16 copy needs no dequantisation. us at 128 / 137
+    / 255 / 256 tokens, records and copy: 16384 x 5120 20.4 / 22.6 / 34.5 / 34.3 and 46.7 / 47.0 / 49.6 / 44.4, 5120 x 6144 16.0 / 17.1
+    / 23.3 / 23.3 and 48.0 / 46.5 / 47.3 / 30.3, 34816 x 5120 with the activation 39.5 / 43.7 / 71.3 / 70.9 and 72.6 / 128 / 137 / 92.7,
+    5120 x 17408 40.4 / 30.4 / 43.9 / 44.2 and 156 / 123 / 121 / 57.8.
+
+    Above, an arm with resident copies multiplies them: they are what it is asked for, and steps of 24 and more rows, whose graphs are
+    captured, need them made before. It costs time below about 1400 tokens (257 / 512 / 1000 / 1400 / 2048, records and copy: 16384 x
+    5120 40 / 65 / 129 / 186 / 255 and 71 / 77 / 147 / 194 / 278, 34816 x 5120 80 / 136 / 265 / 423 / 566 and 119 / 161 / 311 / 412 /
+    571, 5120 x 17408 49 / 85 / 141 / 184 / 310 and 70 / 116 / 242 / 234 / 392). The other arms read the records from a million weights
+    on; smaller matrices, all start-up in either form, keep the dense copy made per call."""
+    return t <= gemm_tc.ROWS_UPTO or (not resident and n * k >= 1 << 20)
 
 
 def _rows_ok(w, x: torch.Tensor, out: torch.Tensor, resident: bool) -> bool:
-    """One launch reads the int4 records and dequantises each weight once per chunk of at most 256 tokens. Above 256 tokens that takes
-    the place of the dense copy made per call (small matrices, which are all start-up in either form, keep it: from 2 M weights the
-    records are faster at every count, 1024 x 2048 at 257 / 2048 tokens 9.9 / 12.9 us against 15.3 / 20.4)."""
-    t = x.shape[0]
-    long = t > gemm_tc.ROWS_UPTO and not resident and w.n * w.k >= 1 << 20
-    return w.layout == "slice" and x.dtype == torch.float16 and (long or rows_pay(w.n, w.k, t, resident)) and x.stride(0) % 8 == 0 \
+    """One launch reads the int4 records and dequantises each weight once per chunk of at most 256 tokens."""
+    return w.layout == "slice" and x.dtype == torch.float16 and rows_pay(w.n, w.k, x.shape[0], resident) and x.stride(0) % 8 == 0 \
         and out.stride(0) % 8 == 0 and (x.data_ptr() | out.data_ptr()) % 16 == 0
 
 
