@@ -65,41 +65,11 @@ struct AtCtl {
 static_assert(sizeof(AtCtl) <= 2304, "control block exceeds its reservation");
 
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, AtCtl* c, int code) {
-  if (mbar_try_wait(bar, parity)) return true;       // the clock is read only when there is something to wait for
-  const uint64_t t0 = global_ns();
-  for (uint32_t i = 0; i < (1u << 22); ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 15u) == 15u && wait_expired(t0)) break;
-    if ((i & 255u) == 255u && c->abort_flag) return false;
-  }
-  c->abort_flag = 1;
-  atomicCAS(&g_attn_tc_status, 0, code);
-  return false;
+  return mbar_wait_bounded(bar, parity, &c->abort_flag, &g_attn_tc_status, code);
 }
-// The same wait for the hand-offs on the critical path of a tile (scores ready, probabilities ready, the warps' meeting
-// point), by a whole warp, whose lanes leave together: a look at a time instead of a suspended thread, whose wake-up costs more than the
-// work it waits for. The clock is not read before a thousand looks: reading it takes longer than most of these waits.
+// For the hand-offs on the critical path of a tile: scores ready, probabilities ready, the warps' meeting point.
 __device__ __forceinline__ bool at_spin(uint64_t* bar, uint32_t parity, AtCtl* c, int code) {
-  uint64_t t0 = 0;
-  for (uint32_t i = 0;; ++i) {
-    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
-    if ((i & 1023u) == 1023u) {
-      bool stop = c->abort_flag != 0;
-      if (t0 == 0) t0 = global_ns();
-      else if (wait_expired(t0)) { stop = true; c->abort_flag = 1; atomicCAS(&g_attn_tc_status, 0, code); }
-      if (__any_sync(0xffffffffu, stop)) return false;
-    }
-  }
-}
-// 32 lanes x 32 consecutive 32-bit columns <- 32 registers per thread (lane = TMEM lane)
-__device__ __forceinline__ void at_tmem_st_x32(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
-        "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
-        "r"(r[30]), "r"(r[31]) : "memory");
+  return mbar_wait_warp<false>(bar, parity, &c->abort_flag, &g_attn_tc_status, code);
 }
 
 // 2^x on the special-function unit (ex2.approx: 2^-inf = 0, relative error about 2^-22)
@@ -241,7 +211,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
           const uint4 v = *reinterpret_cast<const uint4*>(src + ((c ^ (r_loc & 7)) << 4));
           q[c * 4] = v.x; q[c * 4 + 1] = v.y; q[c * 4 + 2] = v.z; q[c * 4 + 3] = v.w;
         }
-        at_tmem_st_x32(lane_addr + AT_COL_Q + kb * 32, q);
+        tmem_st_32x32b_x32(lane_addr + AT_COL_Q + kb * 32, q);
       }
       tc_wait_st();
       tc_fence_before();
@@ -296,7 +266,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             tc_wait_ld();
 #pragma unroll
             for (int v = 0; v < 32; ++v) o[v] = __float_as_uint(__uint_as_float(o[v]) * f);
-            at_tmem_st_x32(lane_addr + AT_COL_O + hf * (AT_HD / 2) + c * 32, o);
+            tmem_st_32x32b_x32(lane_addr + AT_COL_O + hf * (AT_HD / 2) + c * 32, o);
           }
           tc_wait_st();
           tc_fence_before();

@@ -24,7 +24,7 @@
 //
 // Shape of the work. A CTA is 4 warps x 2 row tiles = 128 rows over one part of k; the KS parts of a row block form a
 // thread-block cluster and reduce through distributed shared memory in rank order, so a row's sums have one order that
-// depends on (N, K) only: a row computes the same bits whatever the number of rows in the step. KS is chosen so that
+// depends on N, K and the device's SMs only: a row computes the same bits whatever the number of rows in the step. KS is chosen so that
 // one wave of CTAs (4 per SM) covers the matrix: the 5120-row projections would leave 108 SMs idle otherwise. Two row tiles
 // per warp halve the activation bytes per weight byte. The activations come in MMA fragment order (actpack.cuh, ACT_FRAG) and
 // ride in the same ring of asynchronous copies as the weights, shared by the CTA's warps: read through L1 instead, their L2

@@ -32,8 +32,8 @@
 //   warps 2-9    two sets of four: set s unpacks steps s, s + 2, ... into one of four stages of tensor memory, each warp 32 rows, from a ring of
 //                its own that cp.async fills; the weights do not depend on the kernel before, so the rings fill before the wait
 //   warps 10-17  read a step's sums back (a warp: 32 rows x 16 tokens) and keep y in registers
-// The k parts of a row block form a cluster and push their partial sums to the part that owns the rows; KS depends on (N, K) only, so
-// a row computes the same bits whatever the number of rows in the step.
+// The k parts of a row block form a cluster and push their partial sums to the part that owns the rows; KS depends on N, K,
+// the number of dense rows beside the matrix and the device's SMs, not on M: a row computes the same bits in every step that takes this form.
 //
 // Every mbarrier wait is bounded; on a timeout the CTA records an error code, the roles leave their loops, copies in flight are
 // waited for and TMEM is freed.
@@ -94,30 +94,10 @@ struct TmParams {
   int M, N, K, ldo, n_tiles, row_blocks, ab_rows, ab_ld, ab_blocks, epi;
 };
 __device__ __forceinline__ bool tm_wait(uint64_t* bar, uint32_t parity, TmCtl* c, int code) {
-  if (mbar_try_wait(bar, parity)) return true;      // the clock is read only when there is something to wait for
-  const uint64_t t0 = global_ns();
-  for (uint32_t i = 0; i < (1u << 22); ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 15u) == 15u && wait_expired(t0)) break;
-    if ((i & 15u) == 15u && c->abort_flag) return false;
-  }
-  c->abort_flag = 1;
-  atomicCAS(&g_gemv_tm_status, 0, code);
-  return false;
+  return mbar_wait_bounded(bar, parity, &c->abort_flag, &g_gemv_tm_status, code);
 }
-// By a whole warp, whose lanes leave together.
-__device__ __forceinline__ bool tm_spin_warp(uint64_t* bar, uint32_t parity, TmCtl* c, int code) {
-  uint64_t t0 = 0;
-  for (uint32_t i = 0;; ++i) {
-    const bool ok = mbar_try_wait(bar, parity);      // (sleeps: polling takes issue slots from the warps that unpack)
-    if (__all_sync(0xffffffffu, ok)) return true;
-    if ((i & 15u) == 15u) {
-      bool stop = c->abort_flag != 0;
-      if (t0 == 0) t0 = global_ns();
-      else if (wait_expired(t0)) { stop = true; c->abort_flag = 1; atomicCAS(&g_gemv_tm_status, 0, code); }
-      if (__any_sync(0xffffffffu, stop)) return false;
-    }
-  }
+__device__ __forceinline__ bool tm_wait_warp(uint64_t* bar, uint32_t parity, TmCtl* c, int code) {
+  return mbar_wait_warp<true>(bar, parity, &c->abort_flag, &g_gemv_tm_status, code);
 }
 __device__ __forceinline__ void tm_cp16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -324,9 +304,9 @@ __global__ void __launch_bounds__(TM_THREADS, 1) w4_tm_kernel(TmParams p, int KS
     for (int it = 0; it < total; ++it) {
       const int slot = it & (SLOTS - 1), as = it & (TM_AS - 1), n = it + 1;
       if (!__all_sync(0xffffffffu, free & x & a)) {
-        if (!__all_sync(0xffffffffu, x) && !tm_spin_warp(&ctl->full_x[s], phx, ctl, OWL_ERR_WAIT_TMA)) break;
-        if (!__all_sync(0xffffffffu, a) && !tm_spin_warp(&ctl->full_a[as], ((uint32_t)(it / TM_AS)) & 1u, ctl, OWL_ERR_WAIT_EPI)) break;
-        if (!__all_sync(0xffffffffu, free) && !tm_spin_warp(&ctl->acc_free[slot], (((uint32_t)(it / SLOTS)) & 1u) ^ 1u, ctl, OWL_ERR_WAIT_EPI)) break;
+        if (!__all_sync(0xffffffffu, x) && !tm_wait_warp(&ctl->full_x[s], phx, ctl, OWL_ERR_WAIT_TMA)) break;
+        if (!__all_sync(0xffffffffu, a) && !tm_wait_warp(&ctl->full_a[as], ((uint32_t)(it / TM_AS)) & 1u, ctl, OWL_ERR_WAIT_EPI)) break;
+        if (!__all_sync(0xffffffffu, free) && !tm_wait_warp(&ctl->acc_free[slot], (((uint32_t)(it / SLOTS)) & 1u) ^ 1u, ctl, OWL_ERR_WAIT_EPI)) break;
       }
       tc_fence_after();
       uint64_t* done = &ctl->done[as];
