@@ -169,8 +169,8 @@ def main() -> None:
     ttft_ms = (time.perf_counter() - t0) * 1e3
     if comm:
         ttft_ms = comm.max_over_ranks(ttft_ms)
-    # the same prompt length on the arm that keeps NO resident dense copy of the weights (dequantise once per call into a
-    # shared scratch, then the dense GEMM): what time to first token costs without the extra memory of "tcr" / "tc8r"
+    # the same prompt length on the arm that keeps NO resident dense copy of the weights (the GEMM dequantises the int4 records
+    # itself): what time to first token costs without the extra memory of "tcr" / "tc8r"
     ttft_tc_ms = None
     if args.prefill_gemm in ("tcr", "tc8r"):
         eng.runner.prefill_gemm = "tc"

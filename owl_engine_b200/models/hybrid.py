@@ -532,7 +532,9 @@ class HybridRunner:
                               residual=None if residual is None else residual[r0:], epi=epi,
                               ldo=ldo if ldo is not None else out.shape[-1], pdl=pdl)
 
-    BATCH_GEMM_FROM = 24   # rows from which a batched step multiplies the resident dense weight copy on the tcgen05 GEMM
+    # rows from which a batched step multiplies the resident dense weight copy on the tcgen05 GEMM. Set against the integer arms; the
+    # streaming projections have passed it since (27B, 32 rows at 1024 tokens: "tcr" 15.3 ms, "tc8r" 13.6, "tc", which streams, 10.9)
+    BATCH_GEMM_FROM = 24
 
     def _gemv_dense16(self, w, xp, xs, out, m: int, residual, epi: int, ldo) -> None:
         """Wide batched steps (24+ rows) with a resident dense copy of the weights (``prefill_gemm = "tcr"``: fp16, 4x the
@@ -1095,9 +1097,10 @@ class HybridRunner:
                 wide = ws["wide"].view(-1)[:t * nq].view(t, nq)
                 self._gemm(lw.qkvz, x, wide, ahead)
                 ab = ws["ab"][:t]
-                # one CTA per 128 rows walks all of k: cut where that takes longer than a second launch that adds the parts (96 rows of
-                # k 5120, 512 / 2048 tokens: 27.4 / 28.0 us whole, 14.1 / 16.4 cut; 32 of k 1024: 7.8 / 8.0 and 11.3 / 14.9). The 8-bit
-                # arms keep one sum, whose rounding the activations' 8-bit steps would spread
+                # one CTA per 128 rows walks all of k: cut where that takes longer than a second launch that adds the parts. us at 40 /
+                # 300 / 2048 tokens, whole and cut: 96 rows of k 5120 25.7 / 27.7 / 28.6 and 8.6 / 13.1 / 16.1, 48 of 3072 16.6 / 18.9 /
+                # 19.0 and 7.7 / 11.9 / 14.4, 32 of 2048 11.5 / 12.5 / 12.6 and 7.3 / 11.4 / 13.0, 32 of 1024 6.7 / 7.7 / 7.8 and 6.6 /
+                # 10.7 / 13.7. The 8-bit arms keep one sum, whose rounding the activations' 8-bit steps would spread
                 linear.dense_gemm(x, lw.ab_dense, ab, arm="baseline" if self.prefill_gemm == "baseline" else "tc",
                                   split=sp.hidden >= 3072 and self.prefill_gemm in ("tc", "tc4", "tcr"))
                 mix = ws["mix"].view(-1)[:t * sp.value_dim].view(t, sp.value_dim)
@@ -1142,7 +1145,7 @@ class HybridRunner:
         self._head(1, sample=True)
         return self.out_tok[:1]
 
-    PDL_UPTO = 288      # tokens per chunk up to which its kernels start while the one before drains (DEP_ROWS of csrc/common.cuh)
+    PDL_UPTO = 288      # tokens per chunk up to which its kernels start while the one before drains: DEP_ROWS of csrc/common.cuh
     SP_FROM = 256       # tokens per chunk from which the sequence-parallel fused path is used under tensor parallelism
 
     # keys from which a prefill chunk's attention runs as tcgen05 GEMMs (0: never)

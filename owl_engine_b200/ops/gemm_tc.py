@@ -103,11 +103,11 @@ def f16_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, force_small: b
 
 K.register("owl_w4_gemm_rows", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
 K.register("owl_w4_gemm_rows_plan", [c_int, c_int, c_int, c_int, ctypes.c_longlong, c_void_p])
-ROWS_UPTO = 256         # rows of one w4_gemm_rows launch
+ROWS_UPTO = 256         # rows of one chunk of a w4_gemm_rows launch
 
 
 def w4_gemm_rows(w, x: torch.Tensor, out: torch.Tensor, silu: bool = False, pdl: bool = False) -> torch.Tensor:
-    """out[T, N] (bf16) = x[T, K] (fp16) @ dequant(w)^T for up to 256 rows, every weight dequantised once (``csrc/gemm_w4.cu``);
+    """out[T, N] (bf16) = x[T, K] (fp16) @ dequant(w)^T, every weight dequantised once per chunk of at most 256 rows (``csrc/gemm_w4.cu``);
     ``silu``: out[T, N/2] (fp16) = silu(gate) * up of interleaved gate / up rows. ``pdl``: the launch starts while the kernel before
     it drains and reads the records meanwhile (weights that no kernel still at work writes, as an engine's are)."""
     assert w.layout == "slice" and x.dtype == torch.float16 and x.stride(-1) == 1 and out.stride(-1) == 1

@@ -39,8 +39,9 @@ DEQUANT_FROM = 128      # tokens per chunk from which the 8-bit arms re-quantise
                         # take are dequantised once (34816 x 5120: tiled form 116 us per 128 tokens, dense form 150 at 128,
                         # 204 at 137)
 SILU_FROM = 256         # tokens from which the persistent GEMM, which has the silu(gate) * up epilogue, multiplies fp16 weights
-SMS = 148               # of the part all sizes here were measured on
-SKINNY_UPTO = 32        # rows up to which the decode-shape weight-streaming kernel is used instead of a GEMM
+SKINNY_UPTO = 32        # rows up to which the decode-shape weight-streaming kernel is used instead of a GEMM. Set against the tiled GEMM; the
+                        # int4 GEMM has passed it since (17 / 32 rows with packing, streaming and GEMM, us: 16384 x 5120 27.7 / 33.0 and
+                        # 16.0 / 16.2, 34816 x 5120 46.4 / 56.5 and 29.4 / 29.5, 5120 x 17408 45.2 / 52.3 and 27.7 / 29.0)
 
 
 def _dense_scratch(n: int, k: int, device, dtype=torch.bfloat16) -> torch.Tensor:

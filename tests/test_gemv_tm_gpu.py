@@ -1,5 +1,5 @@
 """The streaming projections through tensor memory (csrc/gemv_tm.cu): the tests of the warp-level form on this kernel, which takes the
-same operands. Beside its tile edges: one to four sets of unpacking warps with work, one and two units a CTA, clusters of 1 to 8."""
+same operands. Beside its tile edges: one and both sets of unpacking warps with work, one and two units a CTA, clusters of 1 to 8."""
 import pytest
 import torch
 

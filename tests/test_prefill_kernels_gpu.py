@@ -218,7 +218,7 @@ def test_gate_up_with_activation_matches_two_steps():
             assert torch.equal(out, two)
 
 
-# every token width of the MMA (64, 128, 192, 256) at its edges; one row tile, a last row block of 1 to 7 tiles, slices of unequal
+# every token width of a stage (64, 128, 160, 256) at its edges; one row tile, a last row block of 1 to 7 tiles, slices of unequal
 # length, and row counts that are cut along k (K from 1024 on)
 @pytest.mark.parametrize("t", [1, 17, 64, 65, 137, 192, 241, 256])
 @pytest.mark.parametrize("n,k", [(16, 128), (144, 384), (1040, 2176), (5120, 1024), (20480, 128)])

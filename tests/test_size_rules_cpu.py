@@ -44,7 +44,7 @@ def test_operand_of_a_short_prompt(n, k, t, resident, rows):
 def test_chunks_and_parts_of_an_int4_product(t, n, k, plan):
     out = (ctypes.c_int * 3)()
     f = K.fn("owl_w4_gemm_rows_plan")
-    assert f(t, n, k, linear.SMS, gemm_tc.KS_SCRATCH_BYTES, out) == 0
+    assert f(t, n, k, 148, gemm_tc.KS_SCRATCH_BYTES, out) == 0
     assert tuple(out) == plan
 
 
