@@ -252,7 +252,9 @@ def rows_pay(n: int, k: int, t: int, resident: bool) -> bool:
     captured, need them made before. It costs time below about 1400 tokens (257 / 512 / 1000 / 1400 / 2048, records and copy: 16384 x
     5120 40 / 65 / 129 / 186 / 255 and 71 / 77 / 147 / 194 / 278, 34816 x 5120 80 / 136 / 265 / 423 / 566 and 119 / 161 / 311 / 412 /
     571, 5120 x 17408 49 / 85 / 141 / 184 / 310 and 70 / 116 / 242 / 234 / 392). The other arms read the records from a million weights
-    on; smaller matrices, all start-up in either form, keep the dense copy made per call."""
+    on (257 / 2048 tokens, copy made and multiplied, and records: 1024 x 1024 12.7 / 17.1 and 5.6 / 8.4, 1536 x 1024 17.5 / 15.3 and 5.7
+    / 10.0, 1024 x 2048 14.2 / 20.4 and 7.8 / 11.2); smaller matrices, which only test models have, keep the copy made per call (1024 x
+    512 12.1 / 15.9 and 4.6 / 6.9)."""
     return t <= gemm_tc.ROWS_UPTO or (not resident and n * k >= 1 << 20)
 
 
