@@ -24,11 +24,11 @@ def test_quant_rows_matches_host_codec(t, k):
     wc, ws, wg = nvfp4.quantize_rows(x.float())
     assert torch.allclose(sx.cpu(), wg, rtol=1e-6)
     assert torch.equal(sf.cpu().view(-1, 512), nvfp4.pack_sf_atoms(ws).view(-1, 512))
-    # codes may differ where a value sits on a rounding boundary of the division; the dequantised row must agree closely
-    got = _deq(codes.cpu(), ws, k) * sx.cpu()[:, None]
-    want = _deq(wc, ws, k) * wg[:, None]
+    # codes may differ where a value sits on a rounding boundary of the division, by one place among the eight magnitudes (in five rows of
+    # 64 one such code of the largest block moves the whole by up to 3 %, so the places are bounded and not the norm)
+    place = lambda c: torch.stack([c & 0xF, c >> 4], -1).int().apply_(lambda n: -(n & 7) if n & 8 else n & 7)
     assert (codes.cpu() != wc).float().mean() < 0.01
-    assert ((got - want).norm() / want.norm()) < 0.02
+    assert (place(codes.cpu()) - place(wc)).abs().max() <= 1
     # fp16 input takes the same path
     c2, _, s2 = nvfp4_tc.quant_rows(x.to(DEV).half())
     assert torch.allclose(s2.cpu(), wg, rtol=1e-3) and (c2.cpu() != wc).float().mean() < 0.02
