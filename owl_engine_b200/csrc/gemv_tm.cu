@@ -111,6 +111,12 @@ __device__ __forceinline__ void tm_bulk_warp(uint32_t dst, const void* src, uint
                "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
+// A load that stays where it is written, before the arrival that gives its slot back (see the readers).
+__device__ __forceinline__ float4 tm_ld4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.volatile.shared::cta.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void tm_cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tm_cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tm_push4(uint32_t addr, int rank, float a, float b, float c, float d) {
@@ -448,6 +454,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) w4_tm_kernel(TmParams p, int KS
     const int r = q4 * 32 + lane, own = (((r >> 4) + 1) * KS - 1) >> 3;      // this lane's row of the block, and the part that owns it
     float* dst = in + ((size_t)rank * RM + ((r >> 4) - own * 8 / KS) * 16 + (r & 15)) * TM_LD + h * 16;
     int it = 0, sx = 0;
+    const uint32_t sums_s = smem_u32(sums_all);
     bool ok = true;
     for (int u = 0; u < units; ++u) {
       for (int k = 0; k < len && ok; ++k, ++it) {
@@ -455,8 +462,15 @@ __global__ void __launch_bounds__(TM_THREADS, 1) w4_tm_kernel(TmParams p, int KS
         ok = __all_sync(0xffffffffu, tm_wait(&ctl->done[it & (TM_AS - 1)], ((uint32_t)(it / TM_AS)) & 1u, ctl, OWL_ERR_WAIT_MMA));
         if (!ok) break;
         tc_fence_after();
+        // The slot of the step before goes back now, not at that step's end: a copy writes into it once all readers have arrived, and
+        // nothing orders loads whose values have not been used yet before a copy (given back at the end of its step, a warp that was held
+        // up there found the sums of six steps later in its last loads). The values of the step before have been used by now.
+        if (it > 0) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->empty_x[sx == 0 ? SX - 1 : sx - 1]);
+        }
         const uint32_t a = tmem + ((uint32_t)(q4 * 32) << 16) + TM_ACC + slot * (GPR * 32) + h * 16;
-        const uint8_t* sums = sums_all + sx * sbytes + 2 * h * (GPR * 64);
+        const uint32_t sums = sums_s + sx * sbytes + 2 * h * (GPR * 64);
         const uint8_t* side = side_all + e * GPR * 512 + r * 4;
         constexpr int GB = GPR == 4 ? 2 : 1;         // groups whose sums are fetched together
 #pragma unroll
@@ -470,7 +484,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) w4_tm_kernel(TmParams p, int KS
           for (int i = 0; i < GB; ++i) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              xs[i][j] = reinterpret_cast<const float4*>(sums + (j >> 1) * (GPR * 64) + (q0 + i) * 64)[(j & 1) + (F == TF_NV4 ? 0 : 2)];
+              xs[i][j] = tm_ld4(sums + (j >> 1) * (GPR * 64) + (q0 + i) * 64 + ((j & 1) + (F == TF_NV4 ? 0 : 2)) * 16);
             const __half2 z = F == TF_NV4 ? __half2() : *reinterpret_cast<const __half2*>(side + (q0 + i) * 512);
             s[i] = __low2float(z);
             nz[i] = -__high2float(z);
@@ -493,7 +507,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) w4_tm_kernel(TmParams p, int KS
                 tm_fma2(y[j + 2], y[j + 3], d2, d3, x.z, x.w, y[j + 2], y[j + 3]);
               } else {
                 if (A8) {
-                  const float4 x8 = reinterpret_cast<const float4*>(sums + (i >> 1) * (GPR * 64) + (q0 + g) * 64)[i & 1];
+                  const float4 x8 = tm_ld4(sums + (i >> 1) * (GPR * 64) + (q0 + g) * 64 + (i & 1) * 16);
                   d0 *= x8.x; d1 *= x8.y; d2 *= x8.z; d3 *= x8.w;
                 }
                 const float4 x = xs[g][i];
@@ -504,8 +518,6 @@ __global__ void __launch_bounds__(TM_THREADS, 1) w4_tm_kernel(TmParams p, int KS
               }
             }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl->empty_x[sx]);
         sx = sx + 1 == SX ? 0 : sx + 1;
       }
       if (KS > 1) {                        // (one unit)
