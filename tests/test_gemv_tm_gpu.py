@@ -58,7 +58,7 @@ def test_a_step_repeats_itself():
     gen = torch.Generator(device="cuda").manual_seed(1)
     w = Q.random_skinny(n, h, 128, "cuda", 0.02, 5)
     ws = [replace(w, records=w.records.clone()) for _ in range(8)]
-    x, gamma = torch.randn(m, h, device="cuda", generator=gen).bfloat16(), torch.ones(h, dtype=torch.bfloat16, device="cuda")
+    x, gamma = torch.randn(m, h, device="cuda", generator=gen).bfloat16(), torch.zeros(h, dtype=torch.bfloat16, device="cuda")      # 1 + gamma
     xp = torch.empty(32 * 2 * h, dtype=torch.uint8, device="cuda")
     xs = torch.empty(32 * h // 128 * 8, dtype=torch.uint8, device="cuda")
     out = torch.zeros(16, m, n, dtype=torch.bfloat16, device="cuda")
